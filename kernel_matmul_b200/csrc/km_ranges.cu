@@ -13,29 +13,13 @@
 //   make_ranges:            start[i] = max_{i' <= i} lb_i' ;  end[i] = max(start[i], max_{i' <= i} ub_i')
 //   make_ranges_symmetric:  end[i] = max(block, max_{i' <= i} ub_i') ;
 //                           start[k] = block * (first i <= k with ceil(end[i] / block) > k), else n
-// with every predicate evaluated in fp32 exactly as the reference writes it.  A first kernel
-// checks monotonicity per batch row (NaNs count as unsorted); batch rows that fail it are
-// processed by a sequential scan kernel that restates the reference loop, so the int32
-// results are bit-identical to the reference for every input.
+// with every predicate evaluated in fp32 exactly as the reference writes it.  Monotonicity
+// is checked per batch row (NaNs count as unsorted); batch rows that fail it are processed by a
+// sequential scan that restates the reference loop, so the int32 results are bit-identical to the
+// reference for every input.
 #include "km_common.cuh"
 
 namespace km {
-
-// flags[b] = 1 iff x[b, :] is non-decreasing.  flags must be preset to 1.
-// `xs`: elements between batch rows of x (n, or 0 when every batch row shares one x).
-__global__ void check_sorted_kernel(int64_t B, int64_t n, const float *x, int64_t xs, int32_t *flags) {
-    const int64_t total = B * n;
-    for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
-         idx += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t j = idx % n, b = idx / n;
-        if (j + 1 < n && !(x[b * xs + j] <= x[b * xs + j + 1])) flags[b] = 0;
-    }
-}
-
-__global__ void fill_flags_kernel(int64_t B, int32_t *flags) {
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i < B) flags[i] = 1;
-}
 
 // First grid index t in [0, G) with pred(t * step), else G.  pred monotone (false.. true..).
 template <typename Pred>
@@ -48,148 +32,170 @@ __device__ __forceinline__ int64_t first_true(int64_t G, Pred pred) {
     return lo;
 }
 
-// Per (batch, row block): lb (first grid column within cutoff below the block's first row) and
-// ub (first grid column beyond cutoff above the block's last row), written to start / end as
-// scratch.  mode 0 = make_ranges, mode 1 = symmetric (only ub, predicate with >=).
-// `cutoffs` (device, B values) overrides the scalar when not null; x1s / x2s: elements between
-// batch rows (0: shared).
-__global__ void range_bounds_kernel(int64_t B, int64_t m, int64_t n, int64_t R, const float *x1, int64_t x1s,
-                                    const float *x2, int64_t x2s, float cutoff_scalar, const float *cutoffs, int block,
-                                    int step, int mode, const int32_t *flags, int32_t *start, int32_t *end) {
-    const int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (idx >= B * R) return;
-    const int64_t b = idx / R, i = idx % R;
-    if (!flags[b]) return;
-    const float cutoff = cutoffs ? cutoffs[b] : cutoff_scalar;
-    const float *a = x1 + b * x1s;
-    const float *c = x2 + b * x2s;
-    const int64_t G = (n + step - 1) / step;
-    const float last = a[min((i + 1) * (int64_t)block, m) - 1];
-    if (mode == 0) {
-        const float first = a[i * block];
+// One band construction.  mode 0 = make_ranges, mode 1 = symmetric (only upper bounds, predicate
+// with >=).  `cutoffs` (device, B values) overrides the scalar when not null; x1s / x2s: elements
+// between batch rows of x (0: one row shared by all).
+struct RangesArgs {
+    int64_t B, m, n, R;
+    const float *x1, *x2;
+    int64_t x1s, x2s;
+    float cutoff_scalar;
+    const float *cutoffs;
+    int block, step, mode;
+    int32_t *start, *end;
+    int32_t *unsorted;  // per batch row: non-zero if x2 is not non-decreasing
+};
+
+// lb (first grid column within cutoff below the block's first row) and ub (first grid column beyond
+// cutoff above the block's last row) of row block i, written to start / end as scratch.
+__device__ __forceinline__ void row_block_bounds(const RangesArgs &q, int64_t b, int64_t i) {
+    const float cutoff = q.cutoffs ? q.cutoffs[b] : q.cutoff_scalar;
+    const float *a = q.x1 + b * q.x1s;
+    const float *c = q.x2 + b * q.x2s;
+    const int64_t idx = b * q.R + i, step = q.step;
+    const int64_t G = (q.n + step - 1) / step;
+    const float last = a[min((i + 1) * (int64_t)q.block, q.m) - 1];
+    if (q.mode == 0) {
+        const float first = a[i * q.block];
         const int64_t tl = first_true(G, [&](int64_t t) { return first - c[t * step] <= cutoff; });
         const int64_t tu = first_true(G, [&](int64_t t) { return c[t * step] - last > cutoff; });
-        start[idx] = (int32_t)min(tl * step, n);
-        end[idx] = (int32_t)min(tu * step, n);
+        q.start[idx] = (int32_t)min(tl * step, q.n);
+        q.end[idx] = (int32_t)min(tu * step, q.n);
     } else {
         const int64_t tu = first_true(G, [&](int64_t t) { return c[t * step] - last >= cutoff; });
-        end[idx] = (int32_t)min(tu * step, n);
+        q.end[idx] = (int32_t)min(tu * step, q.n);
     }
 }
 
-// In-place inclusive prefix maximum over each batch row of `v` (R entries), one CTA per batch;
-// optionally a second array `w` becomes max(prefix-max(w), prefix-max(v)) (mode 0: end), or
-// v is floored at `floor_value` (mode 1: symmetric end).
-__global__ void __launch_bounds__(1024) prefix_max_kernel(int64_t R, const int32_t *flags, int32_t *v, int32_t *w,
-                                                           int mode, int floor_value) {
-    __shared__ int warp_max_v[32], warp_max_w[32];
-    __shared__ int carry_v, carry_w;
-    const int64_t b = blockIdx.x;
-    if (!flags[b]) return;
-    int32_t *pv = v + b * R;
-    int32_t *pw = w ? w + b * R : nullptr;
+// Inclusive-to-exclusive prefix maxima over the 1024 threads of the CTA of two values at once.
+__device__ __forceinline__ void block_exclusive_max2(int &v, int &w, int *warp_v, int *warp_w) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (threadIdx.x == 0) {
-        carry_v = mode == 1 ? floor_value : INT_MIN;
-        carry_w = INT_MIN;
-    }
-    __syncthreads();
-    for (int64_t base = 0; base < R; base += 1024) {
-        const int64_t i = base + threadIdx.x;
-        int xv = i < R ? pv[i] : INT_MIN;
-        int xw = (pw && i < R) ? pw[i] : INT_MIN;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int yv = __shfl_up_sync(0xffffffffu, xv, o);
-            const int yw = __shfl_up_sync(0xffffffffu, xw, o);
-            if (lane >= o) {
-                xv = max(xv, yv);
-                xw = max(xw, yw);
-            }
-        }
-        if (lane == 31) {
-            warp_max_v[warp] = xv;
-            warp_max_w[warp] = xw;
-        }
-        __syncthreads();
-        int pre_v = carry_v, pre_w = carry_w;
-        for (int q = 0; q < warp; q++) {
-            pre_v = max(pre_v, warp_max_v[q]);
-            pre_w = max(pre_w, warp_max_w[q]);
-        }
-        xv = max(xv, pre_v);
-        xw = max(xw, pre_w);
-        if (i < R) {
-            pv[i] = xv;
-            if (pw) pw[i] = max(xw, xv);
-        }
-        __syncthreads();
-        if (threadIdx.x == 1023) {
-            carry_v = xv;
-            carry_w = xw;
-        }
-        __syncthreads();
+    for (int o = 1; o < 32; o <<= 1) {
+        const int yv = __shfl_up_sync(0xffffffffu, v, o), yw = __shfl_up_sync(0xffffffffu, w, o);
+        if (lane >= o) v = max(v, yv), w = max(w, yw);
     }
+    if (lane == 31) warp_v[warp] = v, warp_w[warp] = w;
+    v = __shfl_up_sync(0xffffffffu, v, 1), w = __shfl_up_sync(0xffffffffu, w, 1);
+    if (lane == 0) v = w = INT_MIN;
+    __syncthreads();
+    for (int p = 0; p < warp; p++) v = max(v, warp_v[p]), w = max(w, warp_w[p]);
 }
 
-// Symmetric start from the (non-decreasing) end array.
-__global__ void symmetric_start_kernel(int64_t B, int64_t n, int64_t R, int block, const int32_t *flags,
-                                       const int32_t *end, int32_t *start) {
-    const int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (idx >= B * R) return;
-    const int64_t b = idx / R, k = idx % R;
-    if (!flags[b]) return;
-    const int32_t *e = end + b * R;
-    // first i in [0, R) with ceil(e[i] / block) > k
-    int64_t lo = 0, hi = R;
-    while (lo < hi) {
-        const int64_t mid = (lo + hi) >> 1;
-        const int64_t reach = ((int64_t)e[mid] + block - 1) / block;
-        if (reach > k) hi = mid; else lo = mid + 1;
+// Prefix maxima of a batch row and, in the symmetric mode, the starts, by one CTA of 1024 threads:
+// every thread owns R / 1024 consecutive row blocks.  The symmetric start of column block k is the
+// first row block whose end reaches past k: row block i therefore WRITES the starts of the column
+// blocks its end adds to those reached before, R writes altogether (a binary search per column
+// block over the finished ends took a launch of its own).
+__device__ __forceinline__ void finish_row(const RangesArgs &q, int64_t b, int *warp_v, int *warp_w) {
+    const int64_t R = q.R, chunk = (R + blockDim.x - 1) / blockDim.x;
+    const int64_t i0 = min(R, threadIdx.x * chunk), i1 = min(R, i0 + chunk);
+    int32_t *S = q.start + b * R, *E = q.end + b * R;
+    int v = INT_MIN, w = INT_MIN;
+    for (int64_t i = i0; i < i1; i++) {
+        w = max(w, E[i]);
+        if (q.mode == 0) v = max(v, S[i]);
     }
-    int32_t s = (lo <= k) ? (int32_t)(lo * block) : (int32_t)n;
-    if (k == 0) s = 0;
-    start[idx] = s;
+    block_exclusive_max2(v, w, warp_v, warp_w);
+    if (q.mode == 0) {
+        for (int64_t i = i0; i < i1; i++) {
+            v = max(v, S[i]);
+            w = max(w, E[i]);
+            S[i] = v;
+            E[i] = max(v, w);
+        }
+        return;
+    }
+    w = max(w, q.block);
+    const auto reach_of = [&](int e) { return ((int64_t)e + q.block - 1) / q.block; };
+    int64_t reach = i0 == 0 ? 0 : reach_of(w);
+    for (int64_t i = i0; i < i1; i++) {
+        w = max(w, E[i]);
+        E[i] = w;
+        const int64_t next = reach_of(w);
+        for (int64_t k = reach; k < min(next, R); k++) S[k] = k == 0 ? 0 : (i <= k ? (int32_t)(i * q.block) : (int32_t)q.n);
+        reach = next;
+    }
+    if (i0 < i1 && i1 == R)  // column blocks that no row block reaches
+        for (int64_t k = reach; k < R; k++) S[k] = k == 0 ? 0 : (int32_t)q.n;
 }
 
-// Sequential restatement of the reference scans for batch rows whose x2 is not sorted
-// (native/ranges/ranges.cpp:24-59 and :76-97).  One thread per batch row.
-__global__ void ranges_sequential_kernel(int64_t B, int64_t m, int64_t n, int64_t R, const float *x1, int64_t x1s,
-                                         const float *x2, int64_t x2s, float cutoff_scalar, const float *cutoffs,
-                                         int block, int step, int mode, const int32_t *flags, int32_t *start,
-                                         int32_t *end) {
-    const int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (b >= B || flags[b]) return;
-    const float cutoff = cutoffs ? cutoffs[b] : cutoff_scalar;
-    const float *a = x1 + b * x1s;
-    const float *c = x2 + b * x2s;
-    int32_t *S = start + b * R, *E = end + b * R;
-    if (mode == 0) {
+// Sequential restatement of the reference scans for a batch row whose x2 is not sorted
+// (native/ranges/ranges.cpp:24-59 and :76-97).  One thread.
+__device__ void sequential_row(const RangesArgs &q, int64_t b) {
+    const float cutoff = q.cutoffs ? q.cutoffs[b] : q.cutoff_scalar;
+    const float *a = q.x1 + b * q.x1s;
+    const float *c = q.x2 + b * q.x2s;
+    const int64_t R = q.R, m = q.m, n = q.n, block = q.block, step = q.step;
+    int32_t *S = q.start + b * R, *E = q.end + b * R;
+    if (q.mode == 0) {
         int64_t ps = 0, pe = 0;
         for (int64_t i = 0; i < R; i++) {
             const float first = a[i * block];
-            const float last = a[min((i + 1) * (int64_t)block, m) - 1];
+            const float last = a[min((i + 1) * block, m) - 1];
             int64_t j = ps;
             while (j < n && !(first - c[j] <= cutoff)) j = min(j + step, n);
-            int64_t q = max(pe, j);
-            while (q < n && !(c[q] - last > cutoff)) q = min(q + step, n);
+            int64_t t = max(pe, j);
+            while (t < n && !(c[t] - last > cutoff)) t = min(t + step, n);
             S[i] = (int32_t)j;
-            E[i] = (int32_t)q;
+            E[i] = (int32_t)t;
             ps = j;
-            pe = q;
+            pe = t;
         }
     } else {
         for (int64_t i = 0; i < R; i++) S[i] = (int32_t)n;
         if (R > 0) S[0] = 0;
         int64_t j = block;
         for (int64_t i = 0; i < R; i++) {
-            const float last = a[min((i + 1) * (int64_t)block, n) - 1];
+            const float last = a[min((i + 1) * block, n) - 1];
             while (j < n && !(c[j] - last >= cutoff)) j = min(j + block, n);
             E[i] = (int32_t)j;
             const int64_t reach = (j + block - 1) / block;
             for (int64_t t = i; t < reach && t < R; t++) S[t] = min(S[t], (int32_t)(i * block));
         }
     }
+}
+
+// The whole construction of one batch row by one CTA: what a training step on up to RANGES_ONE_CTA_N
+// points pays is launches, not work (five of them, 11 us of device time and as much host time,
+// before; one, about 5 us, now).
+__global__ void __launch_bounds__(1024) ranges_one_cta_kernel(const RangesArgs q) {
+    __shared__ int warp_v[32], warp_w[32];
+    const int64_t b = blockIdx.x;
+    const float *c = q.x2 + b * q.x2s;
+    int unsorted = 0;
+#pragma unroll 4
+    for (int64_t j = threadIdx.x; j + 1 < q.n; j += 1024) unsorted |= !(c[j] <= c[j + 1]);
+    for (int64_t i = threadIdx.x; i < q.R; i += 1024) row_block_bounds(q, b, i);
+    if (__syncthreads_or(unsorted)) {
+        if (threadIdx.x == 0) sequential_row(q, b);
+        return;
+    }
+    finish_row(q, b, warp_v, warp_w);
+}
+
+// Larger batch rows: sorted check and bounds by the whole GPU (q.unsorted is zero on entry), ...
+__global__ void __launch_bounds__(256) ranges_bounds_kernel(const RangesArgs q) {
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x, first = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    for (int64_t w = first; w < q.B * q.R; w += stride) row_block_bounds(q, w / q.R, w % q.R);
+    const int64_t rows = q.x2s == 0 ? 1 : q.B;  // a shared x2 is checked once, for all batch rows
+    for (int64_t b = 0; b < rows; b++) {
+        const float *c = q.x2 + b * q.x2s;
+        int unsorted = 0;
+        for (int64_t j = first; j + 1 < q.n; j += stride) unsorted |= !(c[j] <= c[j + 1]);
+        if (unsorted) q.unsorted[b] = 1;
+    }
+}
+
+// ... then one CTA per batch row.
+__global__ void __launch_bounds__(1024) ranges_finish_kernel(const RangesArgs q) {
+    __shared__ int warp_v[32], warp_w[32];
+    const int64_t b = blockIdx.x;
+    if (q.unsorted[q.x2s == 0 ? 0 : b]) {
+        if (threadIdx.x == 0) sequential_row(q, b);
+        return;
+    }
+    finish_row(q, b, warp_v, warp_w);
 }
 
 // transpose: every row block marks the column blocks it touches (integer atomic min / max
@@ -257,6 +263,9 @@ __global__ void __launch_bounds__(1024) transpose_fix_kernel(int64_t C, int x1_s
     }
 }
 
+// One CTA reads 65 536 points in about 3 us; from there on the whole GPU is the faster way.
+constexpr int64_t RANGES_ONE_CTA_N = 1 << 16;
+
 // One thread per item on at most 2^20 blocks of 256 threads: callers refuse more items.
 constexpr int64_t KM_RANGES_MAX_ITEMS = (1LL << 20) * 256;
 static inline unsigned grid_for(int64_t total, int threads) {
@@ -276,18 +285,16 @@ static int make_ranges_common(const char *name, int64_t B, int64_t m, int64_t n,
     // (the per-element kernels run one thread per (batch row, row block) on grids of at most 2^20 blocks)
     KM_REQUIRE(B <= KM_RANGES_MAX_ITEMS / R, KM_ERR_UNSUPPORTED, "%s: more than %lld (batch row, row block) pairs", name,
                (long long)KM_RANGES_MAX_ITEMS);
-    fill_flags_kernel<<<grid_for(B, 256), 256, 0, s>>>(B, flags);
-    if (n > 1) check_sorted_kernel<<<(unsigned)std::min<int64_t>(ceil_div(B * n, 256), 148 * 16), 256, 0, s>>>(B, n, x2, x2s, flags);
-    range_bounds_kernel<<<grid_for(B * R, 256), 256, 0, s>>>(B, m, n, R, x1, x1s, x2, x2s, cutoff, cutoffs, block, step,
-                                                             mode, flags, start, end);
-    if (mode == 0) {
-        prefix_max_kernel<<<(unsigned)B, 1024, 0, s>>>(R, flags, start, end, 0, 0);
+    const RangesArgs q = {B, m, n, R, x1, x2, x1s, x2s, cutoff, cutoffs, block, step, mode, start, end, flags};
+    if (n <= RANGES_ONE_CTA_N && R <= RANGES_ONE_CTA_N) {
+        ranges_one_cta_kernel<<<(unsigned)B, 1024, 0, s>>>(q);
     } else {
-        prefix_max_kernel<<<(unsigned)B, 1024, 0, s>>>(R, flags, end, nullptr, 1, block);
-        symmetric_start_kernel<<<grid_for(B * R, 256), 256, 0, s>>>(B, n, R, block, flags, end, start);
+        const cudaError_t err = cudaMemsetAsync(flags, 0, (size_t)B * sizeof(int32_t), s);
+        if (err != cudaSuccess) return cuda_fail(err, name);
+        const int64_t threads = std::max<int64_t>(B * R, n);
+        ranges_bounds_kernel<<<(unsigned)std::min<int64_t>(ceil_div(threads, 256), 148 * 8), 256, 0, s>>>(q);
+        ranges_finish_kernel<<<(unsigned)B, 1024, 0, s>>>(q);
     }
-    ranges_sequential_kernel<<<grid_for(B, 32), 32, 0, s>>>(B, m, n, R, x1, x1s, x2, x2s, cutoff, cutoffs, block, step,
-                                                            mode, flags, start, end);
     KM_CHECK_LAUNCH(name);
     return KM_OK;
 }
