@@ -16,9 +16,10 @@
  *    stride of 0 broadcasts the same data to every batch (the reference receives such views
  *    from `Tensor.expand`, kernel_matmul/linear_operator.py:170-183).
  *  - Inputs are borrowed and never written.  Outputs and workspaces are caller-allocated; the
- *    library never calls an allocator.  The only device state it holds is the fixed scratch
- *    array of km_bilinear_derivative_static_f32 (compiled into the library, 4 MiB per device)
- *    and the cached device address of that array; every other entry point is stateless.
+ *    library never calls a device allocator.  The state it holds is the fixed scratch array of
+ *    km_bilinear_derivative_static_f32 (compiled into the library, 4 MiB per device) with its
+ *    cached device address, and 256 bytes of mapped host memory (km_take_gave_up), allocated by
+ *    the first tensor-core launch; every other entry point is stateless.
  *  - Launches are asynchronous on the `stream` argument (a cudaStream_t passed as void*).
  *    The band-construction calls do not synchronise either.
  *  - Return value: KM_OK or an error code; km_last_error() gives a message for the calling
@@ -125,6 +126,12 @@ KM_API int km_matmul_tc_rows_f32(int kernel_type, const km_batch *batch, int64_t
                                  void *stream);
 
 KM_API int km_workspace_status(const void *workspace, int32_t *status_out, void *stream);
+
+/* What a launch that gave up has left for `device` since the last call: *what = 0 (nothing), 1 (a
+ * product) or 2 (a gradient), and clears it.  Reads one word of mapped host memory that the kernels
+ * write beside their status words: no copy, no event, no synchronisation (a launch that still runs
+ * has not reported yet). */
+KM_API int km_take_gave_up(int32_t device, int32_t *what);
 
 /* ---------------------------------------------------------------------------------------
  * The same product for a window of row blocks, optionally summed over the batch:
@@ -365,6 +372,20 @@ KM_API int km_make_ranges_symmetric_cutoffs_f32(int64_t B, int64_t n, const floa
 KM_API int km_transpose_ranges_i32(int64_t B, int64_t R, const int32_t *start, const int32_t *end,
                             int64_t x1_size, int64_t x2_size, int32_t block_size,
                             int32_t *start_t, int32_t *end_t, void *stream);
+
+/* ---------------------------------------------------------------------------------------
+ * Kernel parameters from raw values, as the kernel modules store them
+ * (kernel_matmul/gpytorch/base.py:47-84 stacks softplus-constrained parameters in native order):
+ *   params[e, q] = lower_bound + softplus(raw[q][e]),  e < count, q < P <= KM_MAX_PARAMS
+ * and, where `cutoff` is not null, *cutoff = cutoff_factor * max over e and the q whose bit is set in
+ * `lengthscales` of params[e, q] (fp64 product, rounded once).  raw: P device pointers (a host
+ * array), params (count, P) contiguous.  The second call is the gradient: grad_params element (e, q)
+ * at e * stride_batch + q * stride_param, grad_raw P device pointers of `count` values.
+ * ------------------------------------------------------------------------------------- */
+KM_API int km_positive_params_f32(int32_t P, int64_t count, const float *const *raw, float lower_bound, float *params,
+                                  uint32_t lengthscales, double cutoff_factor, float *cutoff, void *stream);
+KM_API int km_positive_params_bwd_f32(int32_t P, int64_t count, const float *const *raw, const float *grad_params,
+                                      int64_t stride_batch, int64_t stride_param, float *const *grad_raw, void *stream);
 
 /* Visited entries sum_b sum_r rows(r) * (end - start) (bands clamped), written to *count
  * (device int64).  No reference counterpart; used for throughput accounting. */

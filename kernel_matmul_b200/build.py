@@ -85,17 +85,19 @@ def build(force: bool = False, verbose: bool = False) -> str:
     return LIB
 
 
-TORCH_SRC = os.path.join(HERE, "csrc_torch", "km_torch.cpp")
+TORCH_CSRC = os.path.join(HERE, "csrc_torch")
 TORCH_EXT = os.path.join(HERE, "_C.so")
 
 
 def build_torch_extension(force: bool = False) -> str:
-    """Compile ``csrc_torch/km_torch.cpp`` into ``kernel_matmul_b200/_C.so``: the PyTorch C++
-    extension over the C ABI (needs the PyTorch headers of the running interpreter and g++; no
-    GPU).  It links against ``libkm_b200.so`` next to it (rpath ``$ORIGIN``)."""
+    """Compile ``csrc_torch/*.cpp`` into ``kernel_matmul_b200/_C.so``: the PyTorch C++ extension over
+    the C ABI, which the Python layer is built on (needs the PyTorch headers of the running
+    interpreter and g++; no GPU).  It links against ``libkm_b200.so`` next to it (rpath ``$ORIGIN``)."""
     build()
-    deps = [TORCH_SRC, HEADER, LIB, os.path.abspath(__file__)]
-    if not force and os.path.exists(TORCH_EXT) and all(os.path.getmtime(d) <= os.path.getmtime(TORCH_EXT) for d in deps):
+    srcs = sorted(os.path.join(TORCH_CSRC, f) for f in os.listdir(TORCH_CSRC) if f.endswith(".cpp"))
+    common = [os.path.join(TORCH_CSRC, f) for f in os.listdir(TORCH_CSRC) if f.endswith(".h")] + [HEADER, os.path.abspath(__file__)]
+    mtime = os.path.getmtime
+    if not force and os.path.exists(TORCH_EXT) and all(mtime(d) <= mtime(TORCH_EXT) for d in [*srcs, *common, LIB]):
         return TORCH_EXT
     import sysconfig
 
@@ -105,15 +107,26 @@ def build_torch_extension(force: bool = False) -> str:
     includes = cpp_extension.include_paths("cuda") + [sysconfig.get_paths()["include"]]
     torch_lib = os.path.join(os.path.dirname(torch.__file__), "lib")
     cuda_lib = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "lib64")
-    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-DTORCH_EXTENSION_NAME=_C",
-           "-DTORCH_API_INCLUDE_EXTENSION_H", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
-           *[f"-I{p}" for p in includes], TORCH_SRC, "-o", TORCH_EXT,
-           f"-L{HERE}", "-lkm_b200", f"-L{torch_lib}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch",
-           "-ltorch_python", f"-L{cuda_lib}", "-lcudart", "-Wl,-rpath,$ORIGIN", f"-Wl,-rpath,{torch_lib}"]
-    res = subprocess.run(cmd, capture_output=True, text=True)
-    if res.returncode != 0:
-        sys.stderr.write(res.stdout + res.stderr)
-        raise RuntimeError("build of the PyTorch extension kernel_matmul_b200/_C.so failed")
+    os.makedirs(OBJ_DIR, exist_ok=True)
+
+    def run(cmd: list[str]) -> None:
+        res = subprocess.run(cmd, capture_output=True, text=True)
+        if res.returncode != 0:
+            sys.stderr.write(res.stdout + res.stderr)
+            raise RuntimeError("build of the PyTorch extension kernel_matmul_b200/_C.so failed")
+
+    def compile_one(src: str) -> str:
+        obj = os.path.join(OBJ_DIR, "torch_" + os.path.basename(src)[:-4] + ".o")
+        if force or not os.path.exists(obj) or any(mtime(d) > mtime(obj) for d in [src, *common]):
+            run(["g++", "-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", "-DTORCH_EXTENSION_NAME=_C",
+                 "-DTORCH_API_INCLUDE_EXTENSION_H", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+                 *[f"-I{p}" for p in includes], "-c", src, "-o", obj])
+        return obj
+
+    with concurrent.futures.ThreadPoolExecutor(max_workers=len(srcs)) as pool:
+        objs = list(pool.map(compile_one, srcs))
+    run(["g++", "-shared", "-o", TORCH_EXT, *objs, f"-L{HERE}", "-lkm_b200", f"-L{torch_lib}", "-lc10", "-lc10_cuda", "-ltorch_cpu",
+         "-ltorch_cuda", "-ltorch", "-ltorch_python", f"-L{cuda_lib}", "-lcudart", "-Wl,-rpath,$ORIGIN", f"-Wl,-rpath,{torch_lib}"])
     return TORCH_EXT
 
 

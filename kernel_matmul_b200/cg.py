@@ -244,10 +244,6 @@ class ShardedOperator:
                 ws = phase_ws if (rb_begin >= begin and rb_begin + rb_count <= begin + count) else None
                 call = ops.prepare_matmul_rows(kernel_type, xb, xb, rhs, params, sb, eb, row_block_begin=rb_begin,
                                                row_block_count=rb_count, sum_batches=batched, out=out, phases=ws)
-                if call is None:  # (a product that needs a workspace: the unprepared call)
-                    def call(rhs=rhs, out=out, ws=ws):
-                        ops.matmul_rows(kernel_type, xb, xb, rhs, params, sb, eb, row_block_begin=rb_begin,
-                                        row_block_count=rb_count, sum_batches=batched, out=out, phases=ws)
                 if len(prepared) >= 8:
                     prepared.clear()
                 prepared[key] = call

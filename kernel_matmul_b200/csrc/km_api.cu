@@ -3,6 +3,8 @@
 #include <atomic>
 #include <cstdarg>
 #include <cstdio>
+#include <cstring>
+#include <mutex>
 
 #include "km_tcgen05.cuh"
 
@@ -42,6 +44,25 @@ int make_batch(const km_batch *in, Batch *out) {
 static std::atomic<unsigned> g_wait_polls{TC_WAIT_POLLS};
 
 unsigned current_wait_polls() { return g_wait_polls.load(std::memory_order_relaxed); }
+
+constexpr int KM_MAX_DEVICES = 64;
+static int32_t *g_gave_up = nullptr;  // KM_MAX_DEVICES words, mapped for every device
+static std::once_flag g_gave_up_once;
+
+int *gave_up_word() {
+    std::call_once(g_gave_up_once, [] {
+        void *p = nullptr;
+        if (cudaHostAlloc(&p, KM_MAX_DEVICES * sizeof(int32_t), cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+            (void)cudaGetLastError();  // without the words a give-up still shows in the status word and as NaN
+            return;
+        }
+        memset(p, 0, KM_MAX_DEVICES * sizeof(int32_t));
+        g_gave_up = static_cast<int32_t *>(p);
+    });
+    int dev = 0;
+    if (g_gave_up == nullptr || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= KM_MAX_DEVICES) return nullptr;
+    return g_gave_up + dev;  // unified addressing: the host pointer is valid on the device
+}
 
 // One CTA of one warp waits, with the given poll limit, on an mbarrier that nobody arrives at and
 // records whether the wait gave up: the hand-off failure of the tensor-core kernels in isolation.
@@ -114,6 +135,15 @@ extern "C" int km_num_params(int kernel_type) {
 }
 
 extern "C" const char *km_version(void) { return "km_b200 0.1 (sm_100a)"; }
+
+extern "C" int km_take_gave_up(int32_t device, int32_t *what) {
+    using namespace km;
+    KM_REQUIRE(what != nullptr && device >= 0, KM_ERR_INVALID_ARGUMENT, "km_take_gave_up: bad arguments");
+    *what = 0;
+    if (g_gave_up != nullptr && device < KM_MAX_DEVICES && *reinterpret_cast<volatile int32_t *>(g_gave_up + device) != 0)
+        *what = __atomic_exchange_n(g_gave_up + device, 0, __ATOMIC_ACQ_REL);
+    return KM_OK;
+}
 
 extern "C" int km_count_entries(const km_batch *batch, int64_t m, int64_t n, const km_view *start,
                                 const km_view *end, int64_t *count, void *stream) {

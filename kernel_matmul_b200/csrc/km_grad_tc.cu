@@ -48,6 +48,7 @@ struct GradTcArgs {
     int64_t image_slot_stride;  // floats between batch slots (0: right shared by all batches)
     float *partials;            // [batch.count][row_blocks][kblocks][KM_MAX_PARAMS]
     int *status;
+    int *gave_up;
     unsigned wait_polls;        // poll limit of every hand-off wait
 };
 
@@ -407,7 +408,7 @@ __global__ void __launch_bounds__(128 * G + 32, G == 4 ? 2 : GT_MIN_CTAS) grad_t
 
     tc_fence_before();
     __syncthreads();
-    if (tid == 0 && fail_flag) atomicExch(a.status, 1);
+    if (tid == 0 && fail_flag) report_gave_up(a.status, a.gave_up, GAVE_UP_GRADIENT);
     if (tid < KM_MAX_PARAMS) {
         float v = 0.0f;
         if (tid < NS) {
@@ -494,6 +495,7 @@ static int grad_tc_entry(const char *name, int kernel_type, const km_batch *batc
     a.kp = grad_tc_kp(k);
     a.kblocks = (int)grad_tc_kblocks(k);
     a.slots = a.kp <= 16 ? 4 : 3;
+    a.gave_up = gave_up_word();
     a.wait_polls = current_wait_polls();
     a.row_blocks = ceil_div(m, KM_BLOCK_SIZE);
     a.x1 = make_view<const float>(x1, a.batch);

@@ -550,7 +550,7 @@ __global__ void __launch_bounds__(TcCfg<N>::THREADS, TcCfg<N>::MIN_CTAS) matmul_
     if (fail_flag) {
         // a wait gave up: the status word says so, and the rows of this CTA become NaN so that the
         // failure also shows in whatever is computed from the result, without a host synchronisation
-        if (tid == 0) atomicExch(a.status, 1);
+        if (tid == 0) report_gave_up(a.status, a.gave_up, GAVE_UP_MATMUL);
         const int64_t row = r * KM_BLOCK_SIZE + row_local;
         if (is_gen && g == 0 && row < a.m) {
             float *orow = out + (row - a.rb_begin * KM_BLOCK_SIZE) * a.out.s0 + (int64_t)kb * N * a.out.s1;
@@ -650,6 +650,7 @@ static int tc_matmul(int kernel_type, TcArgs a, const View<const float> &rhs, vo
     a.tiles = supers;                         // 64-column groups per image
     a.n_pad = n_pad;
     a.col_inv_scale = reinterpret_cast<const float *>(scales) + TC_MAX_N;
+    a.gave_up = gave_up_word();
     a.wait_polls = current_wait_polls();
     cudaError_t err = cudaMemsetAsync(scales, 0, tc_scale_bytes(slots, kblocks), s);
     if (err != cudaSuccess) return cuda_fail(err, "km_matmul_tc_f32 cudaMemsetAsync");

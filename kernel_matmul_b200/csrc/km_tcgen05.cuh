@@ -23,6 +23,7 @@ struct TcArgs {
     int64_t image_slot_stride;   // non-zero: every batch has its own images (0: rhs shared by all batches)
     const float *col_inv_scale;  // per (image slot, column block): inverse of the per-column rhs scales
     int *status;
+    int *gave_up;                // the device's host-mapped give-up word (gave_up_word), or null
     unsigned wait_polls;         // poll limit of every hand-off wait (TC_WAIT_POLLS unless a self-test lowered it)
 };
 
@@ -37,6 +38,20 @@ constexpr unsigned TC_WAIT_POLLS = 1u << 18;  // each poll may block for a short
 // Poll limit the launchers put into the kernel arguments: TC_WAIT_POLLS, or what
 // km_selftest_set_wait_polls() set (km_api.cu).
 unsigned current_wait_polls();
+
+// A kernel that stopped at a hand-off wait says so in two places: the status word of its workspace
+// (km_workspace_status) and one word per device in mapped host memory, which the host reads without
+// a copy or an event per launch (km_take_gave_up).  gave_up_word(): that word for the current
+// device, null if the mapping could not be made.  `what` is one of the codes below.
+enum GaveUp : int { GAVE_UP_MATMUL = 1, GAVE_UP_GRADIENT = 2 };
+int *gave_up_word();
+__device__ __forceinline__ void report_gave_up(int *status, int *word, int what) {
+    atomicExch(status, 1);
+    if (word != nullptr) {
+        *reinterpret_cast<volatile int *>(word) = what;
+        __threadfence_system();
+    }
+}
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 

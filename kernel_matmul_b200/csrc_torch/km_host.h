@@ -1,0 +1,124 @@
+// Host side of the ops, shared by the bindings (km_torch.cpp), the autograd functions
+// (km_autograd.cpp) and the CG loop (km_cg_host.cpp): argument checks, broadcasting, choice of the
+// kernel, allocation, launch through the C ABI of libkm_b200.so.  No arithmetic happens here.
+//
+// All of this used to be Python (broadcast_shapes, expand, one ctypes structure per argument, a
+// device copy and an event per tensor-core launch): 70 - 150 us of host time per op call where the
+// smallest kernels take 5 us.  Here a call costs a few microseconds.
+#pragma once
+
+#include <ATen/ATen.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <c10/util/SmallVector.h>
+
+#include <stdexcept>
+#include <string>
+
+#include "../../include/km_b200.h"
+
+namespace kmh {
+
+using at::Tensor;
+using Shape = c10::SmallVector<int64_t, 6>;
+
+// An entry point of libkm_b200 returned a non-zero status (kernel_matmul_b200._lib.KmError in Python).
+struct StatusError : std::runtime_error {
+    using std::runtime_error::runtime_error;
+};
+// A tensor-core launch gave up at a hand-off wait (kernel_matmul_b200.ops.KernelGaveUpError).
+struct GaveUpError : std::runtime_error {
+    using std::runtime_error::runtime_error;
+};
+// Bad value of an argument (ValueError).
+struct ArgumentError : std::runtime_error {
+    using std::runtime_error::runtime_error;
+};
+
+enum Path : int64_t { PATH_AUTO = 0, PATH_FMA = 1, PATH_TC = 2 };
+
+// rhs widths from which a product, column counts from which a gradient runs on the tensor cores
+// (tcgen05) when it has at least TENSOR_CORE_MIN_ITEMS (batch, row block) items: the cost of those
+// kernels hardly depends on the width, and their pre-passes are two or three small launches.
+constexpr int64_t TENSOR_CORE_MIN_K = 9, GRAD_TENSOR_CORE_MIN_K = 8, TENSOR_CORE_MIN_ITEMS = 256;
+
+void check_f32(const Tensor &x);
+void check_i32(const Tensor &x);
+int num_params(int64_t kernel_type);
+inline void raise_on(int rc) {
+    if (rc != KM_OK) throw StatusError("[km status " + std::to_string(rc) + "] " + km_last_error());
+}
+// Raises GaveUpError if a tensor-core launch on `device` has reported a give-up.
+void poll_gave_up(int device);
+
+// One op call: the broadcast batch shape and the arguments as views of the C ABI.
+struct Problem {
+    int kid;
+    int device;
+    int64_t m, n, row_blocks;
+    Shape batch;
+    km_batch kb{};
+    km_view x1, x2, params, start, end;
+    c10::SmallVector<Tensor, 4> keep;  // copies made for more batch dims than the ABI carries
+
+    Problem(int64_t kernel_type, const Tensor &x1, const Tensor &x2, const Tensor &params, const Tensor &start, const Tensor &end,
+            std::initializer_list<std::pair<const Tensor *, int>> extra);
+    // `t` with its last `nonbatch` dims, broadcast over the batch
+    km_view view(const Tensor &t, int nonbatch);
+    Tensor empty(std::initializer_list<int64_t> tail, const Tensor &like) const;
+    int64_t items() const;
+    void *stream() const { return c10::cuda::getCurrentCUDAStream(device).stream(); }
+
+  private:
+    bool flat_ = false;
+};
+
+Tensor workspace(const Tensor &like, size_t bytes);
+
+// The ops (signatures of the reference's native modules).  `tc`: set to whether the tensor cores ran.
+Tensor matmul(int64_t kernel_type, const Tensor &x1, const Tensor &x2, const Tensor &rhs, const Tensor &params, const Tensor &start,
+              const Tensor &end, int64_t path, bool *tc = nullptr);
+// gradient of sum_c left[:, c]^T K right[:, c] with respect to params
+Tensor bilinear(int64_t kernel_type, const Tensor &x1, const Tensor &x2, const Tensor &left, const Tensor &right,
+                const Tensor &params, const Tensor &start, const Tensor &end, int64_t path, bool *tc = nullptr);
+Tensor dense(int64_t kernel_type, const Tensor &x1, const Tensor &x2, const Tensor &params, const Tensor &start, const Tensor &end);
+Tensor dense_bwd(int64_t kernel_type, const Tensor &x1, const Tensor &x2, const Tensor &params, const Tensor &start,
+                 const Tensor &end, const Tensor &out_grad);
+Tensor index(int64_t kernel_type, const Tensor &x1, const Tensor &x2, const Tensor &params, const Tensor &start, const Tensor &end,
+             const std::vector<Tensor> &batch_indices, const Tensor &row, const Tensor &col);
+Tensor index_bwd(int64_t kernel_type, const Tensor &x1, const Tensor &x2, const Tensor &params, const Tensor &start,
+                 const Tensor &end, const std::vector<Tensor> &batch_indices, const Tensor &row, const Tensor &col,
+                 const Tensor &out_grad);
+
+// matmul for a window of row blocks, optionally summed over the batch, with everything but the launch
+// done once: for loops that call the same product on the same buffers (whose contents change) many
+// times, as a CG solve does.
+class RowsProduct {
+  public:
+    RowsProduct(int64_t kernel_type, const Tensor &x1, const Tensor &x2, const Tensor &rhs, const Tensor &params, const Tensor &start,
+                const Tensor &end, int64_t row_block_begin, int64_t row_block_count, bool sum_batches,
+                const std::optional<Tensor> &out, int64_t path, const std::optional<Tensor> &phases);
+    void run();  // on the current stream
+    const Tensor &out() const { return out_; }
+    bool tensor_cores() const { return tc_; }
+
+  private:
+    Problem p_;
+    Tensor out_, phases_, workspace_;
+    std::vector<Tensor> keep_;
+    km_view rhs_, vout_;
+    int64_t k_, begin_, count_;
+    bool sum_, tc_;
+};
+
+// The differentiable forms (gradient for params only), km_autograd.cpp.
+Tensor matmul_ad(int64_t kernel_type, const Tensor &x1, const Tensor &x2, const Tensor &rhs, const Tensor &params,
+                 const Tensor &start, const Tensor &end);
+Tensor dense_ad(int64_t kernel_type, const Tensor &x1, const Tensor &x2, const Tensor &params, const Tensor &start, const Tensor &end);
+Tensor index_ad(int64_t kernel_type, const Tensor &x1, const Tensor &x2, const Tensor &params, const Tensor &start,
+                const Tensor &end, const std::vector<Tensor> &batch_indices, const Tensor &row, const Tensor &col);
+// (batch.., P) parameters lower_bound + softplus(raw[q]) and, where cutoff_factor > 0, the (1,) tensor
+// cutoff_factor * the largest value among the parameters whose bit is set in `lengthscales`
+std::pair<Tensor, Tensor> positive_params(const std::vector<Tensor> &raw, double lower_bound, int64_t lengthscales, double cutoff_factor);
+
+}  // namespace kmh

@@ -18,13 +18,15 @@ With both, ``forward`` + product + backward issue no host synchronisation.
 """
 from __future__ import annotations
 
+import functools
 import math
 
 import torch
 from torch import Tensor, nn
 
+from . import _BLOCK_SIZE, _C
 from .linear_operator import KernelMatmulOperator
-from .ranges import make_ranges, make_ranges_symmetric_cutoffs
+from .ranges import make_ranges
 
 
 def same_tensor(a: Tensor, b: Tensor) -> bool:
@@ -34,23 +36,34 @@ def same_tensor(a: Tensor, b: Tensor) -> bool:
                       and a.stride() == b.stride() and a.data_ptr() == b.data_ptr())
 
 
+@functools.lru_cache(maxsize=64)
+def cutoff_factor(epsilon: float) -> float:
+    """``sqrt(2) erfinv(1 - epsilon)``: the cutoff in lengthscales beyond which a Gaussian is below ``epsilon``."""
+    return math.sqrt(2.0) * torch.special.erfinv(torch.tensor(1.0 - epsilon, dtype=torch.float64)).item()
+
+
 def dynamic_cutoff(epsilon: float, lengthscales: list[Tensor]) -> Tensor:
     """``sqrt(2) erfinv(1 - epsilon) * max lengthscale`` as a 0-dim fp32 tensor on the lengthscales'
     device (double product, rounded once: the value the reference computes on the host)."""
-    z = math.sqrt(2.0) * torch.special.erfinv(torch.tensor(1.0 - epsilon, dtype=torch.float64)).item()
     largest = torch.stack([ls.detach().max() for ls in lengthscales]).max()
-    return (largest.double() * z).float()
+    return (largest.double() * cutoff_factor(epsilon)).float()
 
 
 def band_for(x1: Tensor, x2: Tensor, symmetric: bool, cutoff: float | None, epsilon: float | None,
              lengthscales: list[Tensor]) -> tuple[Tensor, Tensor]:
     """start / end for inputs ``(..., n, 1)``: fixed cutoff, or the epsilon rule."""
+    return _band(x1, x2, symmetric, cutoff if epsilon is None else dynamic_cutoff(epsilon, lengthscales).reshape(1))
+
+
+def _band(x1: Tensor, x2: Tensor, symmetric: bool, cutoff: float | Tensor | None) -> tuple[Tensor, Tensor]:
+    """start / end for inputs ``(..., n, 1)``; ``cutoff`` as a ``(1,)`` device tensor stays there
+    where the inputs are one symmetric set of points (batched or rectangular inputs take its host
+    value)."""
     xs = x1.squeeze(-1)
-    if epsilon is not None:
-        if symmetric and xs.is_cuda and xs.dim() == 1:
-            start, end = make_ranges_symmetric_cutoffs(dynamic_cutoff(epsilon, lengthscales).reshape(1), xs)
-            return start[0], end[0]
-        cutoff = float(dynamic_cutoff(epsilon, lengthscales))  # batched or rectangular inputs: host value
+    if isinstance(cutoff, Tensor):
+        if symmetric and xs.dim() == 1 and xs.is_cuda and xs.dtype == torch.float32:
+            return _C.band_cutoffs(cutoff.detach(), xs, _BLOCK_SIZE, True)
+        cutoff = float(cutoff)
     if symmetric:
         return make_ranges(cutoff, xs, align=True)
     return make_ranges(cutoff, xs, x2.squeeze(-1), align=True)
@@ -87,16 +100,29 @@ class KernelMatmulModule(nn.Module):
                 raw.copy_(v + torch.log(-torch.expm1(-v)))  # inverse softplus
         return self
 
+    def _params_and_cutoff(self) -> tuple[Tensor, float | Tensor | None]:
+        """The stacked parameters and the cutoff they imply, by one kernel on a CUDA device."""
+        raw = [getattr(self, f"raw_{name}") for name in self._PARAMS]
+        epsilon = self._epsilon
+        if type(self).value is KernelMatmulModule.value and all(r.is_cuda and r.dtype == torch.float32 for r in raw):
+            mask = sum(1 << i for i, name in enumerate(self._PARAMS) if name in self._LENGTHSCALES)
+            params, cutoff = _C.positive_params(raw, self.LOWER_BOUND, mask, 0.0 if epsilon is None else cutoff_factor(epsilon))
+            return params, (self._cutoff if epsilon is None else cutoff)
+        values = [self.value(name) for name in self._PARAMS]
+        cutoff = self._cutoff if epsilon is None else dynamic_cutoff(epsilon, [self.value(name) for name in self._LENGTHSCALES]).reshape(1)
+        return torch.stack(values, dim=-1), cutoff
+
     def params(self) -> Tensor:
         """``(*batch_shape, P)`` in the order the native ops expect."""
-        return torch.stack([self.value(name) for name in self._PARAMS], dim=-1)
+        return self._params_and_cutoff()[0]
 
     def forward(self, x1: Tensor, x2: Tensor | None = None) -> KernelMatmulOperator:
         if x2 is None:
             x2 = x1
         symmetric = same_tensor(x1, x2) or (x1.shape == x2.shape and torch.equal(x1, x2))
-        start, end = band_for(x1, x2, symmetric, self._cutoff, self._epsilon, [self.value(n) for n in self._LENGTHSCALES])
-        return KernelMatmulOperator(x1, x2, self.params(), start, end, kernel_type=self._KERNEL_TYPE, symmetric=symmetric)
+        params, cutoff = self._params_and_cutoff()
+        start, end = _band(x1, x2, symmetric, cutoff)
+        return KernelMatmulOperator(x1, x2, params, start, end, kernel_type=self._KERNEL_TYPE, symmetric=symmetric)
 
 
 class RBFKernelMatmulModule(KernelMatmulModule):

@@ -12,10 +12,9 @@ is that package's ``LinearOperator`` subclass with the same constructor and priv
 name is bound to ``KernelMatmulOperator`` so that code using only the operator-level methods
 still runs.
 
-The three autograd Functions give a gradient for ``params`` only, as in the reference
-(``linear_operator.py:22-76``).  Its index backward unpacks eight saved tensors into seven
-names (``:71-72``), which fails as soon as batch indices are present; here the split is
-seven / rest.
+Products, ``to_dense`` and ``get_indices`` are differentiable in ``params`` only, as the
+reference's three autograd Functions (``linear_operator.py:22-76``); the functions are in C++
+(``csrc_torch/km_autograd.cpp``), so that neither direction pays for the interpreter.
 """
 from __future__ import annotations
 
@@ -24,17 +23,8 @@ from typing import Any
 import torch
 from torch import Tensor
 
-from . import ranges
-from .configurations import (
-    BilinearDerivativeConfiguration,
-    DenseBwdConfiguration,
-    DenseConfiguration,
-    IndexBwdConfiguration,
-    IndexConfiguration,
-    MatmulAutotuneConfiguration,
-    MatmulBwdConfiguration,
-)
-from .native_function import NativeFunction
+from . import _C, ranges
+from ._lib import KERNEL_TYPES
 
 try:  # optional third-party base class
     from linear_operator import LinearOperator as _LinearOperator
@@ -44,50 +34,6 @@ try:  # optional third-party base class
 except Exception:  # noqa: BLE001 - absent or broken installation: operator-level API only
     _LinearOperator = None
     HAVE_LINEAR_OPERATOR = False
-
-
-class _MatmulOperator(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x1, x2, rhs, params, start, end, native_matmul, native_matmul_bwd):
-        ctx.save_for_backward(x1, x2, rhs, params, start, end)
-        ctx.native_matmul_bwd = native_matmul_bwd
-        return native_matmul(x1, x2, rhs, params, start, end)
-
-    @staticmethod
-    def backward(ctx, grad_output):
-        x1, x2, rhs, params, start, end = ctx.saved_tensors
-        grad = ctx.native_matmul_bwd(x1, x2, rhs, params, start, end, grad_output)
-        return None, None, None, grad, None, None, None, None
-
-
-class _DenseOperator(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x1, x2, params, start, end, native_dense, native_dense_bwd):
-        ctx.save_for_backward(x1, x2, params, start, end)
-        ctx.native_dense_bwd = native_dense_bwd
-        return native_dense(x1, x2, params, start, end)
-
-    @staticmethod
-    def backward(ctx, grad_output):
-        x1, x2, params, start, end = ctx.saved_tensors
-        grad = ctx.native_dense_bwd(x1, x2, params, start, end, grad_output)
-        return None, None, grad, None, None, None, None
-
-
-class _IndexOperator(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x1, x2, params, start, end, native_index, native_index_bwd, row_index, col_index, *batch_indices):
-        ctx.save_for_backward(x1, x2, params, start, end, row_index, col_index, *batch_indices)
-        ctx.native_index_bwd = native_index_bwd
-        return native_index(x1, x2, params, start, end, batch_indices, row_index, col_index)
-
-    @staticmethod
-    def backward(ctx, grad_output):
-        saved = ctx.saved_tensors
-        x1, x2, params, start, end, row_index, col_index = saved[:7]
-        batch_indices = saved[7:]
-        grad = ctx.native_index_bwd(x1, x2, params, start, end, batch_indices, row_index, col_index, grad_output)
-        return (None, None, grad, None, None, None, None, None, None, *[None for _ in batch_indices])
 
 
 class _OperatorCore:
@@ -100,76 +46,37 @@ class _OperatorCore:
             raise ValueError("x1 and x2 must have shapes (..., M, 1) and (..., N, 1), respectively")
         if symmetric is None:
             symmetric = x1.shape == x2.shape and torch.equal(x1, x2)
-        batch_shape = torch.broadcast_shapes(
-            x1.shape[:-2], x2.shape[:-2], params.shape[:-1], start.shape[:-1], end.shape[:-1]
-        )
-        self._x1 = x1.expand(*batch_shape, *x1.shape[-2:])
-        self._x2 = x2.expand(*batch_shape, *x2.shape[-2:])
-        self._params = params.expand(*batch_shape, params.shape[-1])
-        self._start = start.expand(*batch_shape, start.shape[-1])
-        self._end = end.expand(*batch_shape, end.shape[-1])
+        if kernel_type == "compact":
+            raise NotImplementedError("the 'compact' kernel is not part of this build")
+        self._kid = KERNEL_TYPES.get(kernel_type, -1)  # (-1: refused by the ops)
+        self._x1, self._x2, self._params, self._start, self._end, self._x1v, self._x2v = _C.expand_operator(
+            x1, x2, params, start, end)
         self._kernel_type = kernel_type
-        self._batch_shape = torch.Size(batch_shape)
+        self._batch_shape = self._x1.shape[:-2]
         self._symmetric = bool(symmetric)
-        self._native_matmul = NativeFunction("matmul", MatmulAutotuneConfiguration(kernel_type), compile_pool=compile_pool)
-        self._native_matmul_bwd = NativeFunction("matmul_bwd", MatmulBwdConfiguration(kernel_type))
-        self._native_dense = NativeFunction("dense", DenseConfiguration(kernel_type))
-        self._native_dense_bwd = NativeFunction("dense_bwd", DenseBwdConfiguration(kernel_type))
-        self._native_bilinear_derivative = NativeFunction(
-            "bilinear_derivative", BilinearDerivativeConfiguration(kernel_type)
-        )
-        self._native_index = NativeFunction("index", IndexConfiguration(kernel_type))
-        self._native_index_bwd = NativeFunction("index_bwd", IndexBwdConfiguration(kernel_type))
 
     # -- helpers ---------------------------------------------------------------------------
-    def _get_args_for_native(self, batch_shape) -> tuple[Tensor, Tensor, Tensor, Tensor, Tensor]:
-        def widen(t: Tensor) -> Tensor:
-            return t.expand(*batch_shape, t.shape[-1])
-
-        return (
-            widen(self._x1.squeeze(-1)),
-            widen(self._x2.squeeze(-1)),
-            widen(self._params),
-            widen(self._start),
-            widen(self._end),
-        )
-
     def _core_size(self) -> torch.Size:
         return torch.Size((*self._batch_shape, self._x1.size(-2), self._x2.size(-2)))
 
     def _core_matmul(self, rhs: Tensor) -> Tensor:
-        expected = torch.Size((*self._batch_shape, self._x2.size(-2), rhs.size(-1)))
-        full = torch.broadcast_shapes(expected, rhs.shape)
-        batch_shape = full[:-2]
-        x1, x2, params, start, end = self._get_args_for_native(batch_shape)
-        result = _MatmulOperator.apply(
-            x1, x2, rhs.expand(*full), params, start, end, self._native_matmul, self._native_matmul_bwd
-        )
-        return result.reshape(*batch_shape, *result.shape[-2:])
+        n = self._x2.size(-2)
+        if rhs.size(-2) != n:  # (a broadcast over the rows, or an error)
+            rhs = rhs.expand(*rhs.shape[:-2], n, rhs.size(-1))
+        return _C.matmul_ad(self._kid, self._x1v, self._x2v, rhs, self._params, self._start, self._end)
 
     def _core_to_dense(self) -> Tensor:
-        x1, x2, params, start, end = self._get_args_for_native(self._batch_shape)
-        return _DenseOperator.apply(x1, x2, params, start, end, self._native_dense, self._native_dense_bwd)
+        return _C.dense_ad(self._kid, self._x1v, self._x2v, self._params, self._start, self._end)
 
     def _core_bilinear_derivative(self, left_vecs: Tensor, right_vecs: Tensor) -> Tensor:
-        batch_shape = torch.broadcast_shapes(left_vecs.shape[:-2], right_vecs.shape[:-2], self._batch_shape)
-        left_vecs = left_vecs.expand(*batch_shape, *left_vecs.shape[-2:])
-        right_vecs = right_vecs.expand(*batch_shape, *right_vecs.shape[-2:])
-        x1, x2, params, start, end = self._get_args_for_native(batch_shape)
-        result = self._native_bilinear_derivative(x1, x2, left_vecs, right_vecs, params, start, end)
-        return result.reshape(*batch_shape, result.shape[-1])
+        return _C.op_bilinear(self._kid, self._x1v, self._x2v, left_vecs, right_vecs, self._params, self._start, self._end, 0)[0]
 
     def _core_get_indices(self, row_index: Tensor, col_index: Tensor, *batch_indices: Tensor) -> Tensor:
-        x1, x2, params, start, end = self._get_args_for_native(self._batch_shape)
-        shape = torch.broadcast_shapes(row_index.shape, col_index.shape, *(b.shape for b in batch_indices))
-
         def prepare(index: Tensor) -> Tensor:
-            return index.expand(*shape).to(device=x1.device, dtype=torch.int)
+            return index.to(device=self._x1.device, dtype=torch.int)
 
-        return _IndexOperator.apply(
-            x1, x2, params, start, end, self._native_index, self._native_index_bwd,
-            prepare(row_index), prepare(col_index), *(prepare(b) for b in batch_indices),
-        )
+        return _C.index_ad(self._kid, self._x1v, self._x2v, self._params, self._start, self._end,
+                           [prepare(b) for b in batch_indices], prepare(row_index), prepare(col_index))
 
     def _core_transpose_args(self):
         start_t, end_t = ranges.transpose_ranges(self._start, self._end, self._x1.size(-2), self._x2.size(-2))

@@ -13,7 +13,7 @@ import math
 import torch
 from torch import Tensor
 
-from . import _BLOCK_SIZE
+from . import _BLOCK_SIZE, _C
 from ._lib import check, lib
 
 
@@ -62,26 +62,11 @@ def make_ranges(
         return start, end
 
     dev = _device_for(x1)
-    x1d = x1.detach().to(device=dev, dtype=torch.float32).reshape(-1, m).contiguous()
-    B = x1d.shape[0]
-    start = torch.empty(B, rows, dtype=torch.int32, device=dev)
-    end = torch.empty(B, rows, dtype=torch.int32, device=dev)
-    flags = torch.empty(max(B, 1), dtype=torch.int32, device=dev)
-    stream = ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
-    with torch.cuda.device(dev):
-        if x2 is None:
-            check(lib.km_make_ranges_symmetric_f32(B, m, _ptr(x1d), float(cutoff), block_size, _ptr(start),
-                                                   _ptr(end), _ptr(flags), stream))
-        else:
-            if x2.shape[:-1] != batch_shape:
-                raise RuntimeError("x1 and x2 must share their batch dimensions")
-            n = x2.shape[-1]
-            x2d = x2.detach().to(device=dev, dtype=torch.float32).reshape(-1, n).contiguous()
-            check(lib.km_make_ranges_f32(B, m, n, _ptr(x1d), _ptr(x2d), float(cutoff), block_size,
-                                         1 if align else 0, _ptr(start), _ptr(end), _ptr(flags), stream))
-    start = start.reshape(*batch_shape, rows).to(out_device)
-    end = end.reshape(*batch_shape, rows).to(out_device)
-    return start, end
+    x1d = x1 if x1.is_cuda and x1.dtype == torch.float32 else x1.detach().to(device=dev, dtype=torch.float32)
+    if x2 is not None and not (x2.is_cuda and x2.dtype == torch.float32):
+        x2 = x2.detach().to(device=dev, dtype=torch.float32)
+    start, end = _C.band(float(cutoff), x1d, x2, block_size, align)
+    return (start, end) if x1.is_cuda else (start.to(out_device), end.to(out_device))
 
 
 def make_ranges_symmetric_cutoffs(cutoffs: Tensor, x: Tensor, *, block_size: int = _BLOCK_SIZE) -> tuple[Tensor, Tensor]:
@@ -95,20 +80,10 @@ def make_ranges_symmetric_cutoffs(cutoffs: Tensor, x: Tensor, *, block_size: int
     """
     if cutoffs.dim() != 1 or x.dim() not in (1, 2) or (x.dim() == 2 and x.shape[0] != cutoffs.shape[0]):
         raise RuntimeError("cutoffs must be (B,) and x (n,) or (B, n)")
-    out_device = x.device
     dev = _device_for(x)
-    B, n = cutoffs.shape[0], x.shape[-1]
-    rows = int(math.ceil(n / block_size))
-    xd = x.detach().to(device=dev, dtype=torch.float32).contiguous()
-    cd = cutoffs.detach().to(device=dev, dtype=torch.float32).contiguous()
-    start = torch.empty(B, rows, dtype=torch.int32, device=dev)
-    end = torch.empty(B, rows, dtype=torch.int32, device=dev)
-    flags = torch.empty(max(B, 1), dtype=torch.int32, device=dev)
-    stream = ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
-    with torch.cuda.device(dev):
-        check(lib.km_make_ranges_symmetric_cutoffs_f32(B, n, _ptr(xd), n if x.dim() == 2 else 0, _ptr(cd), block_size,
-                                                       _ptr(start), _ptr(end), _ptr(flags), stream))
-    return start.to(out_device), end.to(out_device)
+    xd = x.detach().to(device=dev, dtype=torch.float32)
+    start, end = _C.band_cutoffs(cutoffs.detach().to(device=dev, dtype=torch.float32), xd, block_size, False)
+    return start.to(x.device), end.to(x.device)
 
 
 def transpose_ranges(
