@@ -134,6 +134,22 @@ KM_API int km_workspace_status(const void *workspace, int32_t *status_out, void 
 KM_API int km_take_gave_up(int32_t device, int32_t *what);
 
 /* ---------------------------------------------------------------------------------------
+ * The same product by blockwise interpolation where its error bound allows: between blocks of 128
+ * sorted points kappa is a polynomial to fp32 rounding (error below 1e-8 of kappa's maximum, bounded
+ * from the block extents and the parameters on the device), so the product is taken between P = 4 .. 64
+ * Chebyshev points per block, with Lagrange matrices on both sides.  Calls whose bands are not
+ * aligned to blocks, or that would need more points, are evaluated directly (km_matmul_tc_f32 from 9
+ * columns, km_matmul_f32 below): the kernels of both ways are launched and the device decides.
+ * m, n, k >= 1.  workspace: ..._workspace_bytes (0: this call is too large for it), 256-byte aligned,
+ * contents irrelevant on entry.
+ * ------------------------------------------------------------------------------------- */
+KM_API size_t km_matmul_nodes_workspace_bytes(const km_batch *batch, int64_t m, int64_t n, int64_t k, const km_view *x1,
+                                              const km_view *x2, const km_view *rhs);
+KM_API int km_matmul_nodes_f32(int kernel_type, const km_batch *batch, int64_t m, int64_t n, int64_t k, const km_view *x1,
+                               const km_view *x2, const km_view *rhs, const km_view *params, const km_view *start,
+                               const km_view *end, const km_view *out, void *workspace, size_t workspace_bytes, void *stream);
+
+/* ---------------------------------------------------------------------------------------
  * The same product for a window of row blocks, optionally summed over the batch:
  *   rows [row_block_begin * 128, (row_block_begin + row_block_count) * 128) (clipped to m) only;
  *   out row 0 is row row_block_begin * 128, i.e. out is (B.., rows_in_window, k);
@@ -220,6 +236,16 @@ KM_API int km_matmul_bwd_f32(int kernel_type, const km_batch *batch, int64_t m, 
                       const km_view *params, const km_view *start, const km_view *end,
                       const km_view *out_grad, const km_view *grad, void *workspace,
                       size_t workspace_bytes, void *stream);
+
+/* The gradients by blockwise interpolation (see km_matmul_nodes_f32): left and right are taken to the
+ * blocks' Chebyshev points and the gradient is formed there.  Directly: km_bilinear_derivative_tc_f32
+ * from 8 columns, km_bilinear_derivative_f32 below. */
+KM_API size_t km_grad_nodes_workspace_bytes(int kernel_type, const km_batch *batch, int64_t m, int64_t n, int64_t k,
+                                            const km_view *x1, const km_view *x2, const km_view *left, const km_view *right);
+KM_API int km_bilinear_derivative_nodes_f32(int kernel_type, const km_batch *batch, int64_t m, int64_t n, int64_t k,
+                                            const km_view *x1, const km_view *x2, const km_view *left, const km_view *right,
+                                            const km_view *params, const km_view *start, const km_view *end,
+                                            const km_view *grad, void *workspace, size_t workspace_bytes, void *stream);
 
 /* ---------------------------------------------------------------------------------------
  * The same gradients with the coefficients <left[i, :], right[j, :]> computed on the tensor

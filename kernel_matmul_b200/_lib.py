@@ -100,6 +100,14 @@ def _load() -> ctypes.CDLL:
     lib.km_make_ranges_symmetric_cutoffs_f32.argtypes = [i64, i64, vp, i64, vp, i32, vp, vp, vp, vp]
     lib.km_transpose_ranges_i32.restype = ctypes.c_int
     lib.km_transpose_ranges_i32.argtypes = [i64, i64, vp, vp, i64, i64, i32, vp, vp, vp]
+    lib.km_matmul_nodes_workspace_bytes.restype = sz
+    lib.km_matmul_nodes_workspace_bytes.argtypes = [bp, i64, i64, i64, wp, wp, wp]
+    lib.km_matmul_nodes_f32.restype = ctypes.c_int
+    lib.km_matmul_nodes_f32.argtypes = [ctypes.c_int, bp, i64, i64, i64, wp, wp, wp, wp, wp, wp, wp, vp, sz, vp]
+    lib.km_grad_nodes_workspace_bytes.restype = sz
+    lib.km_grad_nodes_workspace_bytes.argtypes = [ctypes.c_int, bp, i64, i64, i64, wp, wp, wp, wp]
+    lib.km_bilinear_derivative_nodes_f32.restype = ctypes.c_int
+    lib.km_bilinear_derivative_nodes_f32.argtypes = [ctypes.c_int, bp, i64, i64, i64, wp, wp, wp, wp, wp, wp, wp, wp, vp, sz, vp]
     fp = ctypes.POINTER(ctypes.c_void_p)
     lib.km_take_gave_up.restype = ctypes.c_int
     lib.km_take_gave_up.argtypes = [i32, ctypes.POINTER(i32)]
@@ -137,7 +145,8 @@ lib = _load()
 
 EXPORTED = [
     "km_last_error", "km_version", "km_num_params", "km_matmul_f32", "km_matmul_rows_f32", "km_matmul_tc_workspace_bytes", "km_matmul_tc_f32", "km_matmul_tc_rows_f32",
-    "km_workspace_status", "km_take_gave_up", "km_positive_params_f32", "km_positive_params_bwd_f32", "km_grad_workspace_bytes", "km_grad_tc_workspace_bytes", "km_bilinear_derivative_tc_f32",
+    "km_workspace_status", "km_take_gave_up", "km_matmul_nodes_workspace_bytes", "km_matmul_nodes_f32", "km_grad_nodes_workspace_bytes",
+    "km_bilinear_derivative_nodes_f32", "km_positive_params_f32", "km_positive_params_bwd_f32", "km_grad_workspace_bytes", "km_grad_tc_workspace_bytes", "km_bilinear_derivative_tc_f32",
     "km_matmul_bwd_tc_f32",
     "km_bilinear_derivative_f32", "km_bilinear_derivative_static_f32", "km_matmul_bwd_f32", "km_dense_f32", "km_dense_bwd_f32",
     "km_index_f32", "km_index_bwd_workspace_bytes", "km_index_bwd_f32", "km_make_ranges_f32",

@@ -65,14 +65,37 @@ inline View<T> make_view(const km_view *v, const Batch &b) {
     return r;
 }
 
-inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
+__host__ __device__ inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
+
+// Runs a kernel only if *flag == want (always for a null flag): the choice between interpolation and
+// direct evaluation (km_nodes.cu) is made on the device.
+struct Gate {
+    const int *flag = nullptr;
+    int want = 0;
+    __device__ __forceinline__ bool closed() const { return flag != nullptr && *flag != want; }
+};
 
 // Second stage of every gradient op (km_grad.cu): per batch, add `units` partial records of
 // KM_MAX_PARAMS values (fp32 or fp64) in a fixed order in fp64, apply the chain rule
 // theta <- p and write grad[b, 0..P).
 int launch_grad_finish(int kernel_type, const Batch &batch, int64_t units, const void *partials,
                        bool partials_fp64, const View<const float> &params, const View<float> &grad,
-                       cudaStream_t stream);
+                       cudaStream_t stream, Gate gate = {});
+
+// The direct products and gradients behind a gate (km_matmul.cu, km_matmul_tc.cu, km_grad.cu,
+// km_grad_tc.cu): the C ABI's entry points with their arguments checked.
+int matmul_direct(int kernel_type, const km_batch *batch, int64_t m, int64_t n, int64_t k, const km_view *x1, const km_view *x2,
+                  const km_view *rhs, const km_view *params, const km_view *start, const km_view *end, const km_view *out,
+                  Gate gate, void *stream);
+int matmul_tc_direct(int kernel_type, const km_batch *batch, int64_t m, int64_t n, int64_t k, const km_view *x1, const km_view *x2,
+                     const km_view *rhs, const km_view *params, const km_view *start, const km_view *end, const km_view *out,
+                     void *workspace, size_t workspace_bytes, Gate gate, void *stream);
+int grad_direct(int kernel_type, const km_batch *batch, int64_t m, int64_t n, int64_t k, const km_view *x1, const km_view *x2,
+                const km_view *left, const km_view *right, const km_view *params, const km_view *start, const km_view *end,
+                const km_view *grad, void *workspace, size_t workspace_bytes, Gate gate, void *stream);
+int grad_tc_direct(int kernel_type, const km_batch *batch, int64_t m, int64_t n, int64_t k, const km_view *x1, const km_view *x2,
+                   const km_view *left, const km_view *right, const km_view *params, const km_view *start, const km_view *end,
+                   const km_view *grad, void *workspace, size_t workspace_bytes, Gate gate, void *stream);
 
 // ---------------------------------------------------------------------------- device side
 
@@ -238,6 +261,7 @@ struct KernelFn<KM_KERNEL_RBF> {
     }
     static constexpr bool PHASE = false;
     __device__ __forceinline__ float phase_w() const { return 0.0f; }
+    __device__ __forceinline__ float phase_half_turns() const { return 0.0f; }
     __device__ __forceinline__ f32x2 unscaled2_ph(f32x2 tau, f32x2, f32x2) const { return unscaled2(tau); }
     __device__ __forceinline__ void accumulate2_ph(f32x2 tau, f32x2, f32x2, f32x2 coeff, f32x2 *sums2) const {
         accumulate2(tau, coeff, sums2);
@@ -303,6 +327,7 @@ struct KernelFn<KM_KERNEL_SPECTRAL> {
     }
     static constexpr bool PHASE = true;
     __device__ __forceinline__ float phase_w() const { return w; }
+    __device__ __forceinline__ float phase_half_turns() const { return f2; }  // W / pi
     __device__ __forceinline__ f32x2 unscaled2_ph(f32x2 tau, f32x2 cs, f32x2) const {
         return mul2(ex2_approx2(mul2(splat2(c0), mul2(tau, tau))), cs);
     }
@@ -388,6 +413,7 @@ struct KernelFn<KM_KERNEL_LOCALLY_PERIODIC> {
     // with cs = cos(2 w tau), sn = sin(2 w tau): sin^2(w tau) = (1 - cs) / 2, sin cos = sn / 2
     static constexpr bool PHASE = true;
     __device__ __forceinline__ float phase_w() const { return 2.0f * w; }
+    __device__ __forceinline__ float phase_half_turns() const { return 2.0f / period; }
     // (the halves are folded into constants: c1 sin^2 = (c1 / 2) q with q = 1 - cs; the sums [1] and
     // [2] are accumulated as sum v q and sum v sn tau and halved once by rescale_ph)
     __device__ __forceinline__ f32x2 unscaled2_ph(f32x2 tau, f32x2 cs, f32x2) const {

@@ -28,6 +28,7 @@ struct GradArgs {
     View<float> grad;
     float *partials;  // [batch.count][row_blocks][KM_MAX_PARAMS]
     int right_vec_ok;
+    Gate gate;
 };
 
 template <int KT, int KB, int RPT, int WN>
@@ -39,6 +40,7 @@ __global__ void __launch_bounds__(32 * (128 / (32 * RPT)) * WN)
     constexpr int STAGE_FLOATS = TILE_N * KB + TILE_N;
     constexpr int NS = KernelFn<KT>::NSUMS;
 
+    if (a.gate.closed()) return;
     extern __shared__ __align__(16) float smem[];
     __shared__ float warp_sums[WARPS][KM_MAX_PARAMS];
 
@@ -176,7 +178,8 @@ __global__ void __launch_bounds__(32 * (128 / (32 * RPT)) * WN)
 // `units` partial records of KM_MAX_PARAMS values (float or double) per batch.
 template <int KT, typename PT>
 __global__ void __launch_bounds__(256) grad_finish_kernel(Batch batch, int64_t units, const PT *partials,
-                                                          View<const float> params, View<float> grad) {
+                                                          View<const float> params, View<float> grad, Gate gate) {
+    if (gate.closed()) return;
     constexpr int NS = KernelFn<KT>::NSUMS;
     __shared__ double red[256][KM_MAX_PARAMS];
     const int64_t b = blockIdx.x;
@@ -213,33 +216,33 @@ __global__ void __launch_bounds__(256) grad_finish_kernel(Batch batch, int64_t u
 
 template <typename PT>
 static void launch_finish_typed(int kernel_type, const Batch &batch, int64_t units, const PT *partials,
-                                const View<const float> &params, const View<float> &grad, cudaStream_t stream) {
+                                const View<const float> &params, const View<float> &grad, cudaStream_t stream, Gate gate) {
     const unsigned blocks = (unsigned)batch.count;
     switch (kernel_type) {
     case KM_KERNEL_RBF:
-        grad_finish_kernel<KM_KERNEL_RBF, PT><<<blocks, 256, 0, stream>>>(batch, units, partials, params, grad);
+        grad_finish_kernel<KM_KERNEL_RBF, PT><<<blocks, 256, 0, stream>>>(batch, units, partials, params, grad, gate);
         break;
     case KM_KERNEL_SPECTRAL:
-        grad_finish_kernel<KM_KERNEL_SPECTRAL, PT><<<blocks, 256, 0, stream>>>(batch, units, partials, params, grad);
+        grad_finish_kernel<KM_KERNEL_SPECTRAL, PT><<<blocks, 256, 0, stream>>>(batch, units, partials, params, grad, gate);
         break;
     default:
-        grad_finish_kernel<KM_KERNEL_LOCALLY_PERIODIC, PT><<<blocks, 256, 0, stream>>>(batch, units, partials, params, grad);
+        grad_finish_kernel<KM_KERNEL_LOCALLY_PERIODIC, PT><<<blocks, 256, 0, stream>>>(batch, units, partials, params, grad, gate);
         break;
     }
 }
 
 int launch_grad_finish(int kernel_type, const Batch &batch, int64_t units, const void *partials,
                        bool partials_fp64, const View<const float> &params, const View<float> &grad,
-                       cudaStream_t stream) {
+                       cudaStream_t stream, Gate gate) {
     if (batch.count == 0) return KM_OK;
     if (batch.count > 0x7fffffffLL) {
         set_error("too many batches (%lld)", (long long)batch.count);
         return KM_ERR_UNSUPPORTED;
     }
     if (partials_fp64)
-        launch_finish_typed(kernel_type, batch, units, static_cast<const double *>(partials), params, grad, stream);
+        launch_finish_typed(kernel_type, batch, units, static_cast<const double *>(partials), params, grad, stream, gate);
     else
-        launch_finish_typed(kernel_type, batch, units, static_cast<const float *>(partials), params, grad, stream);
+        launch_finish_typed(kernel_type, batch, units, static_cast<const float *>(partials), params, grad, stream, gate);
     KM_CHECK_LAUNCH("gradient finish launch");
     return KM_OK;
 }
@@ -273,7 +276,7 @@ static int dispatch_grad(const GradArgs &a, cudaStream_t stream) {
 static int grad_entry(const char *name, int kernel_type, const km_batch *batch, int64_t m, int64_t n, int64_t k,
                       const km_view *x1, const km_view *x2, const km_view *left, const km_view *right,
                       const km_view *params, const km_view *start, const km_view *end, const km_view *grad,
-                      void *workspace, size_t workspace_bytes, void *stream) {
+                      void *workspace, size_t workspace_bytes, void *stream, Gate gate = {}) {
     KM_REQUIRE(valid_kernel_type(kernel_type), KM_ERR_INVALID_ARGUMENT, "%s: unknown kernel type %d", name, kernel_type);
     KM_REQUIRE(batch && x1 && x2 && left && right && params && start && end && grad, KM_ERR_INVALID_ARGUMENT,
                "%s: null argument", name);
@@ -300,6 +303,7 @@ static int grad_entry(const char *name, int kernel_type, const km_batch *batch, 
     a.end = make_view<const int>(end, a.batch);
     a.grad = make_view<float>(grad, a.batch);
     a.partials = static_cast<float *>(workspace);
+    a.gate = gate;
     a.right_vec_ok = rows_vectorizable(a.right, a.batch) ? 1 : 0;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (a.row_blocks > 0) {
@@ -312,7 +316,14 @@ static int grad_entry(const char *name, int kernel_type, const km_batch *batch, 
         }
         if (rc != KM_OK) return rc;
     }
-    return launch_grad_finish(kernel_type, a.batch, a.row_blocks, a.partials, false, a.params, a.grad, s);
+    return launch_grad_finish(kernel_type, a.batch, a.row_blocks, a.partials, false, a.params, a.grad, s, gate);
+}
+
+int grad_direct(int kernel_type, const km_batch *batch, int64_t m, int64_t n, int64_t k, const km_view *x1, const km_view *x2,
+                const km_view *left, const km_view *right, const km_view *params, const km_view *start, const km_view *end,
+                const km_view *grad, void *workspace, size_t workspace_bytes, Gate gate, void *stream) {
+    return grad_entry("km_bilinear_derivative_f32", kernel_type, batch, m, n, k, x1, x2, left, right, params, start, end, grad,
+                      workspace, workspace_bytes, stream, gate);
 }
 
 // ---------------------------------------------------------------------------------------

@@ -49,6 +49,7 @@ struct GradTcArgs {
     float *partials;            // [batch.count][row_blocks][kblocks][KM_MAX_PARAMS]
     int *status;
     int *gave_up;
+    Gate gate;
     unsigned wait_polls;        // poll limit of every hand-off wait
 };
 
@@ -58,7 +59,8 @@ struct GradTcArgs {
 // columns past k are zero.  Also clears the status word.
 __global__ void __launch_bounds__(256) grad_tc_images_kernel(Batch batch, int64_t slots, int64_t n, int64_t k, int kp,
                                                              int kblocks, int64_t tiles, View<const float> right,
-                                                             float *images, int *status) {
+                                                             float *images, int *status, Gate gate) {
+    if (gate.closed()) return;
     if (blockIdx.x == 0 && threadIdx.x == 0) *status = 0;
     const int64_t img_floats = 2LL * kp * GT_COLS;
     const int64_t total = slots * kblocks * tiles * (int64_t)GT_COLS * kp;
@@ -93,6 +95,7 @@ __global__ void __launch_bounds__(256) grad_tc_images_kernel(Batch batch, int64_
 #endif
 template <int KT, int G>
 __global__ void __launch_bounds__(128 * G + 32, G == 4 ? 2 : GT_MIN_CTAS) grad_tc_kernel(const GradTcArgs a) {
+    if (a.gate.closed()) return;
     constexpr int WARPS = 4 * G;
     constexpr int NS = KernelFn<KT>::NSUMS;
     constexpr int CPT = GT_COLS / G;   // columns per thread and tile
@@ -475,7 +478,7 @@ static int dispatch_grad_tc(const GradTcArgs &a, cudaStream_t s) {
 static int grad_tc_entry(const char *name, int kernel_type, const km_batch *batch, int64_t m, int64_t n, int64_t k,
                          const km_view *x1, const km_view *x2, const km_view *left, const km_view *right,
                          const km_view *params, const km_view *start, const km_view *end, const km_view *grad,
-                         void *workspace, size_t workspace_bytes, void *stream) {
+                         void *workspace, size_t workspace_bytes, void *stream, Gate gate = {}) {
     KM_REQUIRE(valid_kernel_type(kernel_type), KM_ERR_INVALID_ARGUMENT, "%s: unknown kernel type %d", name, kernel_type);
     KM_REQUIRE(batch && x1 && x2 && left && right && params && start && end && grad, KM_ERR_INVALID_ARGUMENT,
                "%s: null argument", name);
@@ -496,6 +499,7 @@ static int grad_tc_entry(const char *name, int kernel_type, const km_batch *batc
     a.kblocks = (int)grad_tc_kblocks(k);
     a.slots = a.kp <= 16 ? 4 : 3;
     a.gave_up = gave_up_word();
+    a.gate = gate;
     a.wait_polls = current_wait_polls();
     a.row_blocks = ceil_div(m, KM_BLOCK_SIZE);
     a.x1 = make_view<const float>(x1, a.batch);
@@ -522,7 +526,7 @@ static int grad_tc_entry(const char *name, int kernel_type, const km_batch *batc
         KM_REQUIRE(n == 0 || (x2->data && right->data), KM_ERR_INVALID_ARGUMENT, "%s: null data pointer", name);
         const int64_t total = slots * a.kblocks * tiles * (int64_t)GT_COLS * a.kp;
         const unsigned blocks = (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(total, 256), 148 * 32));
-        grad_tc_images_kernel<<<blocks, 256, 0, s>>>(a.batch, slots, n, k, a.kp, a.kblocks, tiles, rv, images, a.status);
+        grad_tc_images_kernel<<<blocks, 256, 0, s>>>(a.batch, slots, n, k, a.kp, a.kblocks, tiles, rv, images, a.status, gate);
         KM_CHECK_LAUNCH("gradient (tensor cores) pre-pass launch");
         switch (kernel_type) {
         case KM_KERNEL_RBF: rc = dispatch_grad_tc<KM_KERNEL_RBF>(a, s); break;
@@ -531,7 +535,14 @@ static int grad_tc_entry(const char *name, int kernel_type, const km_batch *batc
         }
         if (rc != KM_OK) return rc;
     }
-    return launch_grad_finish(kernel_type, a.batch, a.row_blocks * a.kblocks, a.partials, false, a.params, gv, s);
+    return launch_grad_finish(kernel_type, a.batch, a.row_blocks * a.kblocks, a.partials, false, a.params, gv, s, gate);
+}
+
+int grad_tc_direct(int kernel_type, const km_batch *batch, int64_t m, int64_t n, int64_t k, const km_view *x1, const km_view *x2,
+                   const km_view *left, const km_view *right, const km_view *params, const km_view *start, const km_view *end,
+                   const km_view *grad, void *workspace, size_t workspace_bytes, Gate gate, void *stream) {
+    return grad_tc_entry("km_bilinear_derivative_tc_f32", kernel_type, batch, m, n, k, x1, x2, left, right, params, start, end,
+                         grad, workspace, workspace_bytes, stream, gate);
 }
 
 }  // namespace km

@@ -29,6 +29,7 @@ struct MatmulArgs {
     View<const float> x1, x2, rhs, params;
     View<const int> start, end;
     View<float> out;
+    Gate gate;
     int rhs_vec_ok;  // rhs rows may be copied 16 bytes at a time
     int out_vec_ok;  // out rows may be stored 16 bytes at a time
     int sum_shared_ok;  // batch sum: x1, x2, rhs, start, end are one copy shared by all batches
@@ -156,6 +157,7 @@ __device__ __forceinline__ void store_tile(const MatmulArgs<float> &a, float *ou
 template <int KT, int KB, int RPT, int WN>
 __global__ void __launch_bounds__(32 * (128 / (32 * RPT)) * WN, 384 / (32 * (128 / (32 * RPT)) * WN))
     matmul_fma_kernel(const MatmulArgs<float> a) {
+    if (a.gate.closed()) return;
     constexpr int WM = 128 / (32 * RPT);
     extern __shared__ __align__(16) float smem[];
 
@@ -567,7 +569,7 @@ static int matmul_entry(const char *name, int kernel_type, const km_batch *batch
                         const km_view *x1, const km_view *x2, const km_view *rhs, const km_view *params,
                         const km_view *start, const km_view *end, const km_view *out, int64_t rb_begin,
                         int64_t rb_count, bool sum_batches, void *stream, const void *phases = nullptr,
-                        size_t phases_bytes = 0) {
+                        size_t phases_bytes = 0, Gate gate = {}) {
     KM_REQUIRE(valid_kernel_type(kernel_type), KM_ERR_INVALID_ARGUMENT, "%s: unknown kernel type %d", name, kernel_type);
     KM_REQUIRE(batch && x1 && x2 && rhs && params && start && end && out, KM_ERR_INVALID_ARGUMENT, "%s: null argument", name);
     KM_REQUIRE(m >= 0 && n >= 0 && k >= 0 && n <= 0x7fffffffLL && m <= 0x7fffffffLL * 64, KM_ERR_INVALID_ARGUMENT,
@@ -602,6 +604,7 @@ static int matmul_entry(const char *name, int kernel_type, const km_batch *batch
     a.out = make_view<float>(out, a.batch);
     a.rhs_vec_ok = rows_vectorizable(a.rhs, a.batch) ? 1 : 0;
     a.out_vec_ok = 0;
+    a.gate = gate;
     a.sum_shared_ok = 1;
     a.sum_tc_launched = 0;
     for (int d = 0; d < a.batch.ndim; d++)
@@ -648,6 +651,13 @@ static int matmul_entry(const char *name, int kernel_type, const km_batch *batch
     case KM_KERNEL_SPECTRAL: return dispatch_matmul<KM_KERNEL_SPECTRAL, false>(a, s);
     default: return dispatch_matmul<KM_KERNEL_LOCALLY_PERIODIC, false>(a, s);
     }
+}
+
+int matmul_direct(int kernel_type, const km_batch *batch, int64_t m, int64_t n, int64_t k, const km_view *x1, const km_view *x2,
+                  const km_view *rhs, const km_view *params, const km_view *start, const km_view *end, const km_view *out,
+                  Gate gate, void *stream) {
+    return matmul_entry("km_matmul_f32", kernel_type, batch, m, n, k, x1, x2, rhs, params, start, end, out, 0, -1, false, stream,
+                        nullptr, 0, gate);
 }
 
 }  // namespace km

@@ -91,7 +91,8 @@ struct TcCfg {
 // The maxima words must be zero on entry.  Also clears the status word.
 __global__ void __launch_bounds__(256) tc_colmax_kernel(Batch batch, int64_t slots, int64_t n, int64_t k, int npad,
                                                          int kblocks, View<const float> rhs, unsigned *scales,
-                                                         int *status) {
+                                                         int *status, Gate gate) {
+    if (gate.closed()) return;
     if (blockIdx.x == 0 && threadIdx.x == 0) *status = 0;
     const int64_t rows_per_pass = (int64_t)gridDim.x * 16;
     for (int64_t slot = 0; slot < slots; slot++) {
@@ -124,7 +125,8 @@ __device__ __forceinline__ float tc_column_scale(unsigned max_bits) {
 // kind::f16 B operand); rows past n and columns past k are zero.  Also writes the inverse scales.
 __global__ void __launch_bounds__(256) tc_rhs_images_kernel(Batch batch, int64_t slots, int64_t n, int64_t k, int npad,
                                                              int kblocks, int64_t supers, View<const float> rhs,
-                                                             __half *images, unsigned *scales) {
+                                                             __half *images, unsigned *scales, Gate gate) {
+    if (gate.closed()) return;
     const int64_t total = slots * kblocks * supers * (int64_t)(TC_SCOLS * npad);
     for (int64_t idx = blockIdx.x * 256LL + threadIdx.x; idx < total; idx += (int64_t)gridDim.x * 256) {
         int64_t rem = idx;
@@ -157,6 +159,7 @@ __global__ void __launch_bounds__(256) tc_rhs_images_kernel(Batch batch, int64_t
 
 template <int KT, int N>
 __global__ void __launch_bounds__(TcCfg<N>::THREADS, TcCfg<N>::MIN_CTAS) matmul_tc_kernel(const TcArgs a) {
+    if (a.gate.closed()) return;
     using Cfg = TcCfg<N>;
     constexpr int G = Cfg::G;
     constexpr int NPT = N / G;  // accumulator columns per thread
@@ -655,11 +658,11 @@ static int tc_matmul(int kernel_type, TcArgs a, const View<const float> &rhs, vo
     cudaError_t err = cudaMemsetAsync(scales, 0, tc_scale_bytes(slots, kblocks), s);
     if (err != cudaSuccess) return cuda_fail(err, "km_matmul_tc_f32 cudaMemsetAsync");
     const unsigned max_blocks = (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(a.n, 16), 148 * 8));
-    tc_colmax_kernel<<<max_blocks, 256, 0, s>>>(a.batch, slots, a.n, a.k, n_pad, (int)kblocks, rhs, scales, a.status);
+    tc_colmax_kernel<<<max_blocks, 256, 0, s>>>(a.batch, slots, a.n, a.k, n_pad, (int)kblocks, rhs, scales, a.status, a.gate);
     KM_CHECK_LAUNCH("km_matmul_tc_f32 column-maximum launch");
     const int64_t total = slots * kblocks * supers * (int64_t)(TC_SCOLS * n_pad);
     const unsigned blocks = (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(total, 256), 148 * 32));
-    tc_rhs_images_kernel<<<blocks, 256, 0, s>>>(a.batch, slots, a.n, a.k, n_pad, (int)kblocks, supers, rhs, images, scales);
+    tc_rhs_images_kernel<<<blocks, 256, 0, s>>>(a.batch, slots, a.n, a.k, n_pad, (int)kblocks, supers, rhs, images, scales, a.gate);
     KM_CHECK_LAUNCH("km_matmul_tc_f32 pre-pass launch");
     switch (kernel_type) {
     case KM_KERNEL_RBF: return launch_tc<KM_KERNEL_RBF>(a, n_pad, s);
@@ -680,7 +683,7 @@ extern "C" size_t km_matmul_tc_workspace_bytes(const km_batch *batch, int64_t n,
 static int km_matmul_tc_entry(const char *name, int kernel_type, const km_batch *batch, int64_t m, int64_t n, int64_t k,
                               const km_view *x1, const km_view *x2, const km_view *rhs, const km_view *params,
                               const km_view *start, const km_view *end, const km_view *out, int64_t rb_begin,
-                              int64_t rb_count, void *workspace, size_t workspace_bytes, void *stream) {
+                              int64_t rb_count, void *workspace, size_t workspace_bytes, void *stream, km::Gate gate = {}) {
     using namespace km;
     KM_REQUIRE(valid_kernel_type(kernel_type), KM_ERR_INVALID_ARGUMENT, "%s: unknown kernel type %d", name, kernel_type);
     KM_REQUIRE(batch && x1 && x2 && rhs && params && start && end && out, KM_ERR_INVALID_ARGUMENT, "%s: null argument", name);
@@ -713,7 +716,15 @@ static int km_matmul_tc_entry(const char *name, int kernel_type, const km_batch 
     a.start = make_view<const int>(start, a.batch);
     a.end = make_view<const int>(end, a.batch);
     a.out = make_view<float>(out, a.batch);
+    a.gate = gate;
     return tc_matmul(kernel_type, a, make_view<const float>(rhs, a.batch), workspace, static_cast<cudaStream_t>(stream));
+}
+
+int km::matmul_tc_direct(int kernel_type, const km_batch *batch, int64_t m, int64_t n, int64_t k, const km_view *x1, const km_view *x2,
+                         const km_view *rhs, const km_view *params, const km_view *start, const km_view *end, const km_view *out,
+                         void *workspace, size_t workspace_bytes, Gate gate, void *stream) {
+    return km_matmul_tc_entry("km_matmul_tc_f32", kernel_type, batch, m, n, k, x1, x2, rhs, params, start, end, out, 0, -1,
+                              workspace, workspace_bytes, stream, gate);
 }
 
 extern "C" int km_matmul_tc_f32(int kernel_type, const km_batch *batch, int64_t m, int64_t n, int64_t k,

@@ -24,6 +24,7 @@ struct TcArgs {
     const float *col_inv_scale;  // per (image slot, column block): inverse of the per-column rhs scales
     int *status;
     int *gave_up;                // the device's host-mapped give-up word (gave_up_word), or null
+    Gate gate;
     unsigned wait_polls;         // poll limit of every hand-off wait (TC_WAIT_POLLS unless a self-test lowered it)
 };
 

@@ -35,12 +35,16 @@ struct ArgumentError : std::runtime_error {
     using std::runtime_error::runtime_error;
 };
 
-enum Path : int64_t { PATH_AUTO = 0, PATH_FMA = 1, PATH_TC = 2 };
+enum Path : int64_t { PATH_AUTO = 0, PATH_FMA = 1, PATH_TC = 2, PATH_NODES = 3 };
 
 // rhs widths from which a product, column counts from which a gradient runs on the tensor cores
 // (tcgen05) when it has at least TENSOR_CORE_MIN_ITEMS (batch, row block) items: the cost of those
 // kernels hardly depends on the width, and their pre-passes are two or three small launches.
 constexpr int64_t TENSOR_CORE_MIN_K = 9, GRAD_TENSOR_CORE_MIN_K = 8, TENSOR_CORE_MIN_ITEMS = 256;
+
+// (batch, row block) items from which the automatic path tries blockwise interpolation
+// (km_matmul_nodes_f32): its four small passes take about 10 us more than they save below.
+constexpr int64_t NODES_MIN_ITEMS = 512;
 
 void check_f32(const Tensor &x);
 void check_i32(const Tensor &x);

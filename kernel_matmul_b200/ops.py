@@ -32,7 +32,7 @@ def _kernel_id(kernel_type: str) -> int:
         raise ValueError(f"Unknown kernel type: {kernel_type}") from None
 
 
-_PATHS = {"auto": 0, "fma": 1, "tc": 2}
+_PATHS = {"auto": 0, "fma": 1, "tc": 2, "nodes": 3}
 
 
 def _path_id(path: str) -> int:
