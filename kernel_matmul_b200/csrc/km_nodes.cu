@@ -8,20 +8,31 @@
 // return at once if it was; the interpolation kernels return at once if not.  So no call waits for
 // the host, and inputs without short intervals (unsorted points without a cutoff, frequencies of many
 // periods per block) are computed as they always were.
+#include <cstddef>
 #include <type_traits>
 
 #include "km_nodes.cuh"
 
 namespace km {
 
-// First bytes of the workspace, zero on entry to the plan kernel.
+constexpr int NODES_CLASSES_PER_LEVEL = 8;
+constexpr int NODES_CLASSES = NODES_LEVELS * NODES_CLASSES_PER_LEVEL;
+
+// A class is a number of nodes at one of the half-lengths.  First bytes of the workspace; the first
+// three words are zero on entry to the plan kernel.
 struct NodesHeader {
     int max_h_bits;  // largest half-length of any block (bits of a non-negative float)
     int bad;         // some band is not aligned to blocks, or an input is not finite
     int done;        // CTAs of the plan kernel that have finished
-    int P;
     int use;         // 1: interpolate, 0: evaluate directly
+    float h[NODES_LEVELS];
+    int first[NODES_LEVELS + 1];  // classes of level l: first[l] .. first[l + 1] - 1
+    int P[NODES_CLASSES];
+    int off[NODES_CLASSES];       // nodes of smaller classes of the level: place in the arrays shared by all batches
+    float delta[NODES_CLASSES][NODES_MAX];   // node offsets from a block's centre
+    float weight[NODES_CLASSES][NODES_MAX];  // barycentric weights
 };
+constexpr size_t NODES_ZEROED = offsetof(NodesHeader, use);
 
 struct NodesArgs {
     Batch batch;
@@ -29,13 +40,31 @@ struct NodesArgs {
     int64_t R, C;       // row and column blocks
     int64_t slots1, slots2;  // distinct x1 / x2 rows: batch.count, or 1 if all batches share one
     int same;           // x1 and x2 are the same points
-    int max_p;
+    int max_p;          // most nodes of a block
+    int cap;            // most nodes of a block over all classes of its level, where batches share x
     View<const float> x1, x2, params;
     View<const int> start, end;
     NodesHeader *hdr;
-    NodeBox *box1, *box2;    // [slot][block]
-    float *lambda1, *lambda2;  // [slot][block][P][128]
+    int *classes;              // [batch][level]
+    float *centre1, *centre2;  // [slot][block]
+    float *half1, *half2;      // [slot][block] half-lengths
+    float *lambda1, *lambda2;  // [slot][block][cap or max_p][128]
 };
+
+__device__ __forceinline__ int level_of(const NodesHeader *hdr, float half) {
+    int l = 0;
+#pragma unroll
+    for (int i = 1; i < NODES_LEVELS; i++) l += half <= hdr->h[i];
+    return l;
+}
+
+// Rows (of 128 or kq floats) between blocks, and first row of a class within its block, of an array
+// with one copy for all batches (classes side by side) or one per batch.
+__device__ __forceinline__ int64_t node_rows(const NodesArgs &a, int64_t slots) { return slots == 1 && a.batch.count > 1 ? a.cap : a.max_p; }
+__device__ __forceinline__ int node_first(const NodesArgs &a, int64_t slots, int cls) { return slots == 1 && a.batch.count > 1 ? a.hdr->off[cls] : 0; }
+
+template <int V>
+using Int = std::integral_constant<int, V>;
 
 __device__ __forceinline__ int nodes_needed_for(int kt, const float *theta, int64_t stride, float h, int lane) {
     if (kt == KM_KERNEL_RBF) return nodes_needed<KM_KERNEL_RBF>(theta, stride, h, lane);
@@ -44,7 +73,7 @@ __device__ __forceinline__ int nodes_needed_for(int kt, const float *theta, int6
 }
 
 // Extents of every block (a warp each), alignment of every band, and -- the CTA that finishes last --
-// the number of nodes for the longest interval over all kernels of the batch.
+// the number of nodes of every kernel of the batch at every half-length.
 __global__ void __launch_bounds__(256) nodes_plan_kernel(const NodesArgs a, int kernel_type) {
     const int lane = threadIdx.x & 31;
     const int64_t warps = (int64_t)gridDim.x * 8, first = blockIdx.x * 8LL + (threadIdx.x >> 5);
@@ -77,7 +106,7 @@ __global__ void __launch_bounds__(256) nodes_plan_kernel(const NodesArgs a, int 
         const float c = 0.5f * lo + 0.5f * hi, h = fmaxf(fmaxf(hi - c, c - lo), NODES_MIN_H);
         bad |= nan || !(h < INFINITY);
         longest = fmaxf(longest, h);
-        if (lane == 0) (one ? a.box1 : a.box2)[v] = NodeBox{c, h};
+        if (lane == 0) (one ? a.centre1 : a.centre2)[v] = c, (one ? a.half1 : a.half2)[v] = h;
     }
     const int64_t threads = (int64_t)gridDim.x * blockDim.x;
     for (int64_t w = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; w < a.batch.count * a.R; w += threads) {
@@ -87,263 +116,533 @@ __global__ void __launch_bounds__(256) nodes_plan_kernel(const NodesArgs a, int 
         if (s >= e) continue;  // an empty band
         bad |= s < 0 || s % KM_BLOCK_SIZE != 0 || (e < a.n && e % KM_BLOCK_SIZE != 0);
     }
-    __shared__ int s_last, s_p;
+    __shared__ int s_last, s_fits;
+    __shared__ int s_class[NODES_LEVELS][NODES_MAX / 2 + 1];  // by P / 2: needed, then its class
+    __shared__ int s_nodes, s_P[NODES_CLASSES], s_node_first[NODES_CLASSES];
+    __shared__ float s_h[NODES_CLASSES], s_delta[NODES_CLASSES * NODES_MAX];
+    __shared__ unsigned char s_node_class[NODES_CLASSES * NODES_MAX];
     if (lane == 0) atomicMax(&a.hdr->max_h_bits, __float_as_int(longest));
     bad = __syncthreads_or(bad);
     if (threadIdx.x == 0) {
         if (bad) a.hdr->bad = 1;
         __threadfence();
         s_last = atomicAdd(&a.hdr->done, 1) == (int)gridDim.x - 1;
-        s_p = 0;
+        s_fits = 1;
     }
+    for (int i = threadIdx.x; i < NODES_LEVELS * (NODES_MAX / 2 + 1); i += 256) (&s_class[0][0])[i] = 0;
     __syncthreads();
     if (!s_last) return;
     __threadfence();
-    const float h = __int_as_float(*reinterpret_cast<volatile int *>(&a.hdr->max_h_bits));
+    float h[NODES_LEVELS];
+    h[0] = __int_as_float(*reinterpret_cast<volatile int *>(&a.hdr->max_h_bits));
+#pragma unroll
+    for (int l = 1; l < NODES_LEVELS; l++) h[l] = h[l - 1] * (1.0f / NODES_RATIO);
     const bool any_bad = *reinterpret_cast<volatile int *>(&a.hdr->bad) != 0;
-    for (int64_t b = threadIdx.x >> 5; b < a.batch.count; b += 8) {
-        const int p = nodes_needed_for(kernel_type, batch_ptr(a.params, decompose(a.batch, b)), a.params.s0, h, lane);
-        if (lane == 0) atomicMax(&s_p, p);
+    for (int64_t w = threadIdx.x >> 5; w < a.batch.count * NODES_LEVELS; w += 8) {
+        const int l = (int)(w % NODES_LEVELS);
+        const float *theta = batch_ptr(a.params, decompose(a.batch, w / NODES_LEVELS));
+        // (fewer classes where batches share the points: every class has its own Lagrange matrices)
+        const int unit = a.batch.count > 1 && (a.slots1 == 1 || a.slots2 == 1) ? 4 : 2;
+        const int p = max(4, (min(nodes_needed_for(kernel_type, theta, a.params.s0, h[l], lane), 4096) + unit - 1) & -unit);
+        if (lane == 0) {
+            if (p > a.max_p) {
+                s_fits = 0;
+            } else {
+                a.classes[w] = p;
+                s_class[l][p / 2] = 1;
+            }
+        }
+    }
+    __syncthreads();
+    const bool use = !any_bad && s_fits;
+    // warp l lists the classes of level l (NODES_LEVELS <= 8 warps): counted from the largest node count
+    // down while they fit; smaller ones are served by the smallest that does (the largest always fits)
+    __shared__ int s_count[NODES_LEVELS], s_smallest[NODES_LEVELS];
+    const int l = threadIdx.x >> 5;
+    if (l < NODES_LEVELS && lane == 0 && use) {
+        int count = 0, total = 0, smallest = 0;
+        for (int i = NODES_MAX / 2; i >= 2; i--) {
+            if (!s_class[l][i]) continue;
+            if (count == NODES_CLASSES_PER_LEVEL || total + 2 * i > a.cap) break;
+            count++, total += 2 * i, smallest = i;
+        }
+        s_count[l] = count, s_smallest[l] = smallest;
+    }
+    __syncthreads();
+    if (l < NODES_LEVELS && lane == 0 && use) {
+        int at = 0, off = 0;
+        for (int i = 0; i < l; i++) at += s_count[i];
+        a.hdr->h[l] = h[l];
+        a.hdr->first[l] = at;
+        if (l == NODES_LEVELS - 1) a.hdr->first[NODES_LEVELS] = at + s_count[l];
+        for (int i = 2; i < s_smallest[l]; i++) s_class[l][i] = at;
+        for (int i = s_smallest[l]; i <= NODES_MAX / 2; i++) {
+            if (!s_class[l][i]) continue;
+            a.hdr->P[at] = s_P[at] = 2 * i;
+            a.hdr->off[at] = off;
+            s_h[at] = h[l];
+            s_class[l][i] = at++;
+            off += 2 * i;
+        }
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-        const int P = max(4, (min(s_p, 4096) + 3) & ~3);
-        a.hdr->P = P;
-        a.hdr->use = !any_bad && P <= a.max_p;
+        a.hdr->use = use;
+        int at = 0;
+        if (use)
+            for (int c = 0; c < s_count[0] + s_count[1] + s_count[2] + s_count[3]; c++) s_node_first[c] = at, at += s_P[c];
+        s_nodes = at;
+    }
+    __syncthreads();
+    if (!use) return;
+    for (int c = threadIdx.x >> 5; c < s_count[0] + s_count[1] + s_count[2] + s_count[3]; c += 8)
+        for (int q = lane; q < s_P[c]; q += 32) s_node_class[s_node_first[c] + q] = (unsigned char)c;
+    __syncthreads();
+    for (int64_t w = threadIdx.x; w < a.batch.count * NODES_LEVELS; w += 256) a.classes[w] = s_class[w % NODES_LEVELS][a.classes[w] / 2];
+    // offsets, then weights, of all classes: one node per thread and round
+    for (int i = threadIdx.x; i < s_nodes; i += 256) {
+        const int c = s_node_class[i], q = i - s_node_first[c];
+        s_delta[i] = a.hdr->delta[c][q] = node_offset(s_h[c], q, s_P[c]);
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < s_nodes; i += 256) {
+        const int c = s_node_class[i], q = i - s_node_first[c];
+        a.hdr->weight[c][q] = node_weight(s_delta + s_node_first[c], s_h[c], q, s_P[c]);
     }
 }
 
-// Lagrange matrix of one block: thread = row, lambda[q][row] = (w_q / (x - xi_q)) / sum of the same.
+// Lagrange matrices of one block, one per class in use for it: thread = row,
+// lambda[q][row] = (w_q / (x - xi_q)) / sum of the same.
 __global__ void __launch_bounds__(128) nodes_lambda_kernel(const NodesArgs a) {
-    if (!a.hdr->use) return;
-    const int P = a.hdr->P;
+    const NodesHeader *hdr = a.hdr;
+    if (!hdr->use) return;
     __shared__ float delta[NODES_MAX], weight[NODES_MAX];
     const int64_t boxes1 = a.slots1 * a.R;
     const bool one = blockIdx.x < boxes1;
     const int64_t v = one ? blockIdx.x : blockIdx.x - boxes1, blocks = one ? a.R : a.C, rows = one ? a.m : a.n;
-    const NodeBox box = (one ? a.box1 : a.box2)[v];
+    const int64_t slots = one ? a.slots1 : a.slots2;
     const View<const float> &x = one ? a.x1 : a.x2;
     const int t = threadIdx.x;
-    if (t < P) delta[t] = node_offset(box.h, t, P);
-    __syncthreads();
-    if (t < P) weight[t] = node_weight(delta, box.h, t, P);
-    __syncthreads();
-    const int64_t row = (v % blocks) * KM_BLOCK_SIZE + t;
-    float *out = (one ? a.lambda1 : a.lambda2) + v * P * KM_BLOCK_SIZE + t;
-    if (row >= rows) {
-        for (int q = 0; q < P; q++) out[q * KM_BLOCK_SIZE] = 0.0f;
-        return;
-    }
-    const float d = batch_ptr(x, decompose(a.batch, v / blocks))[row * x.s0] - box.c;
+    const int level = level_of(hdr, (one ? a.half1 : a.half2)[v]);
     // (differences in units of h: an interval may be as short as NODES_MIN_H)
-    const float inv_h = 1.0f / box.h;
-    float sum = 0.0f;
-    int hit = -1;
-    for (int q = 0; q < P; q++) {
-        const float e = (d - delta[q]) * inv_h;
-        if (e == 0.0f) hit = q;
-        sum += weight[q] / e;
-    }
-    const float inv = 1.0f / sum;
-    for (int q = 0; q < P; q++) {
-        const float e = (d - delta[q]) * inv_h;
-        out[q * KM_BLOCK_SIZE] = hit >= 0 ? (q == hit ? 1.0f : 0.0f) : (weight[q] / e) * inv;
+    const float inv_h = 1.0f / hdr->h[level];
+    const int64_t row = (v % blocks) * KM_BLOCK_SIZE + t;
+    const float d = row < rows ? batch_ptr(x, decompose(a.batch, v / blocks))[row * x.s0] - (one ? a.centre1 : a.centre2)[v] : 0.0f;
+    const bool shared = slots == 1;
+    const int c0 = shared ? hdr->first[level] : a.classes[v / blocks * NODES_LEVELS + level], c1 = shared ? hdr->first[level + 1] : c0 + 1;
+    for (int cls = c0; cls < c1; cls++) {
+        const int P = hdr->P[cls];
+        __syncthreads();
+        if (t < P) delta[t] = hdr->delta[cls][t], weight[t] = hdr->weight[cls][t];
+        __syncthreads();
+        float *out = (one ? a.lambda1 : a.lambda2) + (v * node_rows(a, slots) + node_first(a, slots, cls)) * KM_BLOCK_SIZE + t;
+        if (row >= rows) {
+            for (int q = 0; q < P; q++) out[q * KM_BLOCK_SIZE] = 0.0f;
+            continue;
+        }
+        float sum = 0.0f;
+        int hit = -1;
+#pragma unroll 4
+        for (int q = 0; q < P; q++) {
+            const float e = (d - delta[q]) * inv_h;
+            if (e == 0.0f) hit = q;
+            sum += __fdividef(weight[q], e);
+        }
+        const float inv = 1.0f / sum;
+#pragma unroll 4
+        for (int q = 0; q < P; q++) {
+            const float e = (d - delta[q]) * inv_h;
+            out[q * KM_BLOCK_SIZE] = hit >= 0 ? (q == hit ? 1.0f : 0.0f) : __fdividef(weight[q], e) * inv;
+        }
     }
 }
 
 // Lambda^T of one operand: out[slot][block][q][c] = sum_row lambda[q][row] * v[row][c], columns padded
-// to kq = a multiple of 4 with zeros.
+// to kq = a multiple of 4 with zeros; an operand that all batches share is taken to the nodes of every
+// class in use for its block.
 struct CompressArgs {
-    Batch batch;
-    int64_t rows, k, kq, blocks, slots;
-    int64_t lambda_slots;  // 1: one Lagrange matrix per block for all batches
+    NodesArgs a;
+    int64_t rows, kq, blocks;
+    int64_t slots;     // distinct (operand, points) rows
+    int64_t x_slots;   // distinct points: one Lagrange matrix per block for all batches if 1
+    int vec;           // rows may be read 16 bytes at a time
     View<const float> v;
-    const float *lambda;
+    const float *half, *lambda;
     float *out;
-    const NodesHeader *hdr;
 };
 
-constexpr int CP_ROWS = 64, CP_COLS = 32;
+constexpr int CP_ROWS = 32;              // rows per stage
+constexpr int CP_NODES = 40;             // nodes per pass
+constexpr int CP_LS = CP_ROWS + 1;
+template <int COLS>
+struct CompressShape {
+    static constexpr int STAGE = CP_ROWS * COLS + CP_NODES * CP_LS + 3 & ~3;  // floats: operand rows, then Lagrange matrix
+    static constexpr size_t SMEM = 4 * 2 * STAGE * sizeof(float);
+};
 
-// One CTA per (slot, block, 32 columns).  A thread owns (node, 4 columns) pairs; rows are staged
-// 64 at a time.  Bound by the shared-memory reads (two per four FMAs); the whole pass is a few per cent
-// of the direct evaluation it replaces.
-__global__ void __launch_bounds__(128) nodes_compress_kernel(const CompressArgs a) {
+// A warp per (slot, block, COLS columns), no synchronisation beyond the warp: the block's 128 rows pass
+// through two stages of 32 rows (operand and Lagrange matrix, cp.async), a lane owning 4 nodes x 4 columns
+// (8 shared-memory words read for 8 packed FMAs).  More than 40 nodes, or more units than lanes, take
+// further passes over the rows.
+template <int COLS>
+__global__ void __launch_bounds__(128) nodes_compress_kernel(const CompressArgs p) {
+    const NodesArgs &a = p.a;
     if (!a.hdr->use) return;
-    const int P = a.hdr->P;
-    __shared__ float ls[NODES_MAX][CP_ROWS + 1];
-    __shared__ __align__(16) float vs[CP_ROWS][CP_COLS];
-    const int64_t chunks = ceil_div(a.kq, CP_COLS);
-    const int64_t chunk = blockIdx.x % chunks, box = blockIdx.x / chunks, slot = box / a.blocks, block = box % a.blocks;
-    const int k0 = (int)chunk * CP_COLS, kc = (int)min((int64_t)CP_COLS, a.kq - k0);  // a multiple of 4
-    const float *v = batch_ptr(a.v, decompose(a.batch, slot));
-    const float *lambda = a.lambda + ((a.lambda_slots == 1 ? 0 : slot) * a.blocks + block) * P * KM_BLOCK_SIZE;
-    float *out = a.out + box * P * a.kq + k0;
-    const int t = threadIdx.x;
-    constexpr int UNITS = NODES_MAX * (CP_COLS / 4) / 128;
-    float acc[UNITS][4] = {};
-    const int groups = kc / 4, units = P * groups;
-    for (int half = 0; half < KM_BLOCK_SIZE / CP_ROWS; half++) {
-        const int64_t row0 = block * KM_BLOCK_SIZE + half * CP_ROWS;
-        if (row0 >= a.rows) break;
-        __syncthreads();
-        for (int e = t; e < P * CP_ROWS; e += 128) ls[e / CP_ROWS][e % CP_ROWS] = lambda[(e / CP_ROWS) * KM_BLOCK_SIZE + half * CP_ROWS + e % CP_ROWS];
-        for (int e = t; e < CP_ROWS * kc; e += 128) {
-            const int i = e / kc, c = e % kc;
-            vs[i][c] = (row0 + i < a.rows && k0 + c < a.k) ? v[(row0 + i) * a.v.s0 + (k0 + c) * a.v.s1] : 0.0f;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int u = 0; u < UNITS; u++) {
-            const int unit = t + 128 * u;
-            if (unit >= units) break;
-            const int q = unit % P, c = (unit / P) * 4;
+    constexpr int STAGE = CompressShape<COLS>::STAGE;
+    extern __shared__ __align__(16) float smem[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float *stages = smem + warp * 2 * STAGE;
+    const int64_t chunks = (p.kq + COLS - 1) / COLS;
+    const int64_t item = blockIdx.x * 4LL + warp;
+    if (item >= chunks * p.slots * p.blocks) return;
+    const int64_t chunk = item % chunks, box = item / chunks, slot = box / p.blocks, block = box % p.blocks;
+    const int k0 = (int)chunk * COLS, kc = (int)min((int64_t)COLS, p.kq - k0);  // a multiple of 4
+    const float *v = batch_ptr(p.v, decompose(a.batch, slot));
+    const int64_t row0 = block * KM_BLOCK_SIZE, x_slot = p.x_slots == 1 ? 0 : slot;
+    const int groups = kc / 4;
+    const int level = level_of(a.hdr, p.half[x_slot * p.blocks + block]);
+    const bool shared = p.slots == 1;
+    const int c0 = shared ? a.hdr->first[level] : a.classes[slot * NODES_LEVELS + level], c1 = shared ? a.hdr->first[level + 1] : c0 + 1;
+    const int row_count = (int)min((int64_t)KM_BLOCK_SIZE, p.rows - row0), steps = (row_count + CP_ROWS - 1) / CP_ROWS;
+
+    for (int cls = c0; cls < c1; cls++) {
+        const int P = a.hdr->P[cls];
+        const float *lambda_cls =
+            p.lambda + ((x_slot * p.blocks + block) * node_rows(a, p.x_slots) + node_first(a, p.x_slots, cls)) * KM_BLOCK_SIZE;
+        float *out_cls = p.out + (box * node_rows(a, p.slots) + node_first(a, p.slots, cls)) * p.kq + k0;
+        for (int p0 = 0; p0 < P; p0 += CP_NODES) {
+            const int Pn = min(CP_NODES, P - p0);
+            const float *lambda = lambda_cls + p0 * KM_BLOCK_SIZE;
+            float *out = out_cls + p0 * p.kq;
+            const auto load = [&](int step, int which) {
+                float *vs = stages + which * STAGE, *ls = vs + CP_ROWS * COLS;
+                const int r = step * CP_ROWS, count = min(CP_ROWS, row_count - r);
+                if (p.vec) {
+                    for (int e = lane; e < CP_ROWS * groups; e += 32) {
+                        const int i = e / groups, c = (e - i * groups) * 4;
+                        if (i < count)
+                            cp_async16(vs + i * COLS + c, v + (row0 + r + i) * p.v.s0 + k0 + c);
+                        else
+                            *reinterpret_cast<float4 *>(vs + i * COLS + c) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    }
+                } else {
+                    for (int e = lane; e < CP_ROWS * kc; e += 32) {
+                        const int i = e / kc, c = e - i * kc;
+                        if (i < count && k0 + c < a.k)
+                            cp_async4(vs + i * COLS + c, v + (row0 + r + i) * p.v.s0 + (k0 + c) * p.v.s1);
+                        else
+                            vs[i * COLS + c] = 0.0f;
+                    }
+                }
+                for (int q = 0; q < Pn; q++) cp_async4(ls + q * CP_LS + lane, lambda + q * KM_BLOCK_SIZE + r + lane);
+                cp_async_commit();
+            };
+            const int quads = (Pn + 3) / 4, units = quads * groups;
+            for (int u0 = 0; u0 < units; u0 += 32) {
+                const int unit = u0 + lane;
+                const bool mine = unit < units;
+                const int q = mine ? (unit % quads) * 4 : 0, c = mine ? (unit / quads) * 4 : 0;
+                const int last = Pn - 1 - q;  // (P is even, not always a multiple of 4)
+                const int at0 = q * CP_LS, at1 = at0 + CP_LS, at2 = at0 + (last >= 2 ? 2 : 0) * CP_LS, at3 = at0 + (last >= 3 ? 3 : 0) * CP_LS;
+                f32x2 acc[4][2] = {};
+                load(0, 0);
+                for (int step = 0; step < steps; step++) {
+                    if (step + 1 < steps) {
+                        load(step + 1, (step + 1) & 1);
+                        cp_async_wait<1>();
+                    } else {
+                        cp_async_wait<0>();
+                    }
+                    __syncwarp();
+                    const float *w0 = stages + (step & 1) * STAGE + c, *ls = stages + (step & 1) * STAGE + CP_ROWS * COLS;
 #pragma unroll 8
-            for (int i = 0; i < CP_ROWS; i++) {
-                const float l = ls[q][i];
-                const float4 w = *reinterpret_cast<const float4 *>(&vs[i][c]);
-                acc[u][0] = fmaf(l, w.x, acc[u][0]);
-                acc[u][1] = fmaf(l, w.y, acc[u][1]);
-                acc[u][2] = fmaf(l, w.z, acc[u][2]);
-                acc[u][3] = fmaf(l, w.w, acc[u][3]);
+                    for (int i = 0; i < CP_ROWS; i++) {
+                        const ulonglong2 w = *reinterpret_cast<const ulonglong2 *>(w0 + i * COLS);
+                        const f32x2 a0 = splat2(ls[at0 + i]), a1 = splat2(ls[at1 + i]), a2 = splat2(ls[at2 + i]), a3 = splat2(ls[at3 + i]);
+                        acc[0][0] = fma2(a0, w.x, acc[0][0]), acc[0][1] = fma2(a0, w.y, acc[0][1]);
+                        acc[1][0] = fma2(a1, w.x, acc[1][0]), acc[1][1] = fma2(a1, w.y, acc[1][1]);
+                        acc[2][0] = fma2(a2, w.x, acc[2][0]), acc[2][1] = fma2(a2, w.y, acc[2][1]);
+                        acc[3][0] = fma2(a3, w.x, acc[3][0]), acc[3][1] = fma2(a3, w.y, acc[3][1]);
+                    }
+                    __syncwarp();
+                }
+                if (mine) {
+#pragma unroll
+                    for (int j = 0; j < 4; j++)
+                        if (j <= last) *reinterpret_cast<ulonglong2 *>(out + (q + j) * p.kq + c) = make_ulonglong2(acc[j][0], acc[j][1]);
+                }
             }
         }
     }
-#pragma unroll
-    for (int u = 0; u < UNITS; u++) {
-        const int unit = t + 128 * u;
-        if (unit >= units) break;
-        *reinterpret_cast<float4 *>(out + (unit % P) * a.kq + (unit / P) * 4) = make_float4(acc[u][0], acc[u][1], acc[u][2], acc[u][3]);
-    }
 }
 
-// The kernel values of node rows against the nodes of one column block.  Per pair of blocks a lane
-// keeps, for its node rows, the distance to the column block's centre and the cosine and sine of its
-// phase; per node of the column block the offset and the phase factors lie in shared memory, so an
-// entry costs one SFU exponential (as in the tensor-core kernels).  The factors are evaluated with
-// full precision, the distance of the centres reduced to half turns in fp64: a few values per pair.
-template <int KT>
-struct NodePair {
-    using Fn = KernelFn<KT>;
-    static __device__ __forceinline__ void column_factors(const Fn &fn, float delta, float &c, float &s) {
-        c = 1.0f, s = 0.0f;
-        if constexpr (Fn::PHASE) sincospif(fn.phase_half_turns() * delta, &s, &c);
+// What the product and the gradient at the nodes share.  A CTA of four warps works on one batch and KC
+// columns: on four row blocks, a warp each -- then nothing but the tables of phase factors is shared and no
+// warp waits for another --, or, in problems with too few row blocks for that, on one, of whose band
+// every warp takes every fourth column block.  Lanes own node rows:
+// LANES lanes x RPT rows cover the P rows of the block and 32 / LANES column subsets share the warp, so
+// that a shared-memory read of an operand row serves LANES * RPT entries per subset and no lane idles
+// at the common P.  Per pair of blocks a lane keeps, for its rows, the distance to the column block's
+// centre and cosine and sine of its phase; the phase factors of the column nodes are the same for every
+// half-length, so an entry costs one SFU exponential and no sine or cosine.  All phase factors are
+// evaluated with full precision, the distance of two centres reduced to half turns in fp64.
+template <int KC>
+struct NodeShape {
+    static constexpr int QS = KC + 4;  // floats per staged operand row: column subsets fall into different banks
+    // most rows per lane (registers: RPT * KC accumulators or left values)
+    static constexpr int CTAS = KC <= 16 ? 4 : 3;  // per SM
+    static constexpr int MAX_ROWS = KC <= 16 ? 4 : (KC == 24 ? 3 : 2);
+    // shared memory for the warps' operand tiles: two stages while they fit, else one
+    static constexpr int TILE_FLOATS = 4 * NODES_MAX * QS;
+    // per half-length: offset, cos and sin of W offset of the nodes
+    static constexpr int TABLE_FLOATS = NODES_LEVELS * 3 * NODES_MAX;
+    static constexpr size_t SMEM = (TILE_FLOATS + TABLE_FLOATS) * sizeof(float);
+};
+
+// f(LANES, RPT) for the smallest layout that holds P rows.
+template <int MAX_ROWS, typename F>
+__device__ __forceinline__ void with_row_layout(int P, F f) {
+    if (P <= 16) return f(Int<8>(), Int<2>());
+    if constexpr (MAX_ROWS >= 3)
+        if (P <= 24) return f(Int<8>(), Int<3>());
+    if constexpr (MAX_ROWS >= 4) {
+        if (P <= 32) return f(Int<8>(), Int<4>());
+        if (P <= 48) return f(Int<16>(), Int<3>());
+        if (P <= 64) return f(Int<16>(), Int<4>());
+        return f(Int<32>(), Int<3>());
     }
-    // cos, sin of W (D + delta)
-    static __device__ __forceinline__ void row_factors(const Fn &fn, float D, float delta, float &c, float &s) {
-        c = 1.0f, s = 0.0f;
-        if constexpr (Fn::PHASE) {
+    if (P <= 32) return f(Int<16>(), Int<2>());
+    if constexpr (MAX_ROWS >= 3)
+        if (P <= 48) return f(Int<16>(), Int<3>());
+    if (P <= 64) return f(Int<32>(), Int<2>());
+    return f(Int<32>(), Int<3>());
+}
+
+// Distance, phase factors and half-length of 32 of a warp's column blocks at a time, one per lane.
+template <int KT>
+struct NodePairs {
+    float D = 0.0f, c = 1.0f, s = 0.0f;
+    int level = 0;
+    __device__ __forceinline__ void load(const KernelFn<KT> &fn, const NodesHeader *hdr, float row_centre, const float *centre2,
+                                         const float *half2, int cb, int c_hi) {
+        if (cb >= c_hi) return;
+        D = row_centre - centre2[cb];
+        level = level_of(hdr, half2[cb]);
+        if constexpr (KernelFn<KT>::PHASE) {
             const double t = (double)fn.phase_half_turns() * (double)D;
-            sincospif((float)(t - 2.0 * rint(0.5 * t)) + fn.phase_half_turns() * delta, &s, &c);
+            sincospif((float)(t - 2.0 * rint(0.5 * t)), &s, &c);
         }
     }
 };
+
+// Per node row of a lane: offset from the row block's centre, cos and sin of W times it; and, for the
+// current column block, distance to its centre (y) and cos and sin of W times that (rc, rs).
+template <int KT, int LANES, int RPT>
+struct NodeRows {
+    float d[RPT], cw[RPT], sw[RPT];
+    f32x2 y[RPT], rc[RPT], rs[RPT];
+    __device__ __forceinline__ void init(const float *table, int row, int P) {
+#pragma unroll
+        for (int i = 0; i < RPT; i++) {
+            const int q = row + LANES * i;
+            d[i] = q < P ? table[q] : 0.0f;
+            cw[i] = q < P ? table[NODES_MAX + q] : 1.0f;
+            sw[i] = q < P ? table[2 * NODES_MAX + q] : 0.0f;
+        }
+    }
+    __device__ __forceinline__ void pair(float D, float c, float s) {
+#pragma unroll
+        for (int i = 0; i < RPT; i++) {
+            y[i] = splat2(D + d[i]);
+            if constexpr (KernelFn<KT>::PHASE) {
+                rc[i] = splat2(c * cw[i] - s * sw[i]);
+                rs[i] = splat2(s * cw[i] + c * sw[i]);
+            }
+        }
+    }
+};
+
+// Everything about a CTA's work item.
+template <int KT, int KC>
+struct NodeItem {
+    int64_t b, r;
+    int chunk, k0, kc, c_lo, c_hi, c_step, P, row_class, stages, stage_floats;
+    bool idle;  // a warp of the last CTA without a row block
+    int col_P[NODES_LEVELS], col_class[NODES_LEVELS];
+    KernelFn<KT> fn;
+    float row_centre;
+    const NodesHeader *hdr;
+    const float *centre2, *half2;
+    float *tiles, *tables, *row_table;
+
+    // `wpr`: warps per row block, 1 or 4
+    __device__ __forceinline__ void init(const NodesArgs &a, int64_t kq, int wpr, float *smem, BatchIndex *bi_out) {
+        hdr = a.hdr;
+        const int warp = threadIdx.x >> 5;
+        int64_t item = blockIdx.x;
+        b = item % a.batch.count;
+        item /= a.batch.count;
+        const int64_t groups = wpr == 1 ? (a.R + 3) / 4 : a.R;
+        r = item % groups;
+        chunk = (int)(item / groups);
+        if (wpr == 1) r = r * 4 + warp;
+        idle = r >= a.R;
+        if (idle) r = a.R - 1;
+        const BatchIndex bi = decompose(a.batch, b);
+        *bi_out = bi;
+        k0 = chunk * KC;
+        kc = (int)min((int64_t)KC, kq - k0);  // a multiple of 4
+        fn.init(batch_ptr(a.params, bi), a.params.s0);
+        const int s = batch_ptr(a.start, bi)[r * a.start.s0], e = batch_ptr(a.end, bi)[r * a.end.s0];
+        c_lo = s < e ? s / KM_BLOCK_SIZE : 0;
+        c_hi = s < e && !idle ? (int)((min((int64_t)e, a.n) + KM_BLOCK_SIZE - 1) / KM_BLOCK_SIZE) : 0;
+        c_step = wpr;
+        if (wpr > 1) c_lo += warp;
+        const int64_t row_box = (a.slots1 == 1 ? 0 : b) * a.R + r;
+        row_centre = a.centre1[row_box];
+        const int row_level = level_of(hdr, a.half1[row_box]);
+        centre2 = a.centre2 + (a.slots2 == 1 ? 0 : b) * a.C;
+        half2 = a.half2 + (a.slots2 == 1 ? 0 : b) * a.C;
+        tables = smem + NodeShape<KC>::TILE_FLOATS;
+        row_table = tables + row_level * 3 * NODES_MAX;
+#pragma unroll
+        for (int l = 0; l < NODES_LEVELS; l++) {
+            col_class[l] = a.classes[b * NODES_LEVELS + l];
+            col_P[l] = hdr->P[col_class[l]];
+            float *t = tables + l * 3 * NODES_MAX;
+            for (int q = threadIdx.x; q < col_P[l]; q += 128) {
+                const float d = hdr->delta[col_class[l]][q];
+                float c = 1.0f, sn = 0.0f;
+                if constexpr (KernelFn<KT>::PHASE) sincospif(fn.phase_half_turns() * d, &sn, &c);
+                t[q] = d, t[NODES_MAX + q] = c, t[2 * NODES_MAX + q] = sn;
+            }
+            if (l == row_level) P = col_P[l], row_class = col_class[l];
+        }
+        stage_floats = max(col_P[0], P) * NodeShape<KC>::QS;  // (the longest half-length has the most nodes)
+        stages = 8 * stage_floats <= NodeShape<KC>::TILE_FLOATS ? 2 : 1;
+        tiles = smem + (threadIdx.x >> 5) * stages * stage_floats;
+        __syncthreads();
+    }
+
+    // One column block's operand rows (Pc x KC of an array with rows of kq) into this warp's stage.
+    __device__ __forceinline__ void stage(const float *src, int64_t kq, int Pc, int which) const {
+        const int lane = threadIdx.x & 31;
+        float *to = tiles + which * stage_floats;
+        for (int q = lane; q < Pc * (KC / 4); q += 32) {
+            const int j = q / (KC / 4), c4 = (q % (KC / 4)) * 4;
+            if (c4 < kc)
+                cp_async16(to + j * NodeShape<KC>::QS + c4, src + j * kq + c4);
+            else
+                *reinterpret_cast<float4 *>(to + j * NodeShape<KC>::QS + c4) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+        cp_async_commit();
+    }
+
+    // Calls body(D, c, s, Pc, table, tile) for each of this warp's column blocks; `operand`: column k0 of
+    // an array [column block][block_rows][kq] that has this kernel's nodes of level l at row first[l].
+    template <typename Body>
+    __device__ __forceinline__ void walk(const NodesArgs &a, const float *operand, int64_t slots, int64_t kq, Body body) const {
+        const int lane = threadIdx.x & 31;
+        const int64_t block = node_rows(a, slots) * kq;
+        int first[NODES_LEVELS];
+#pragma unroll
+        for (int l = 0; l < NODES_LEVELS; l++) first[l] = node_first(a, slots, col_class[l]);
+        const auto pick = [](const int (&v)[NODES_LEVELS], int l) { return l == 0 ? v[0] : (l == 1 ? v[1] : (l == 2 ? v[2] : v[3])); };
+        static_assert(NODES_LEVELS == 4, "pick");
+        const auto fetch = [&](int cb, int level, int which) { stage(operand + cb * block + pick(first, level) * kq, kq, pick(col_P, level), which); };
+        NodePairs<KT> now, next;  // this group of 32 column blocks and the one after it
+        next.load(fn, hdr, row_centre, centre2, half2, c_lo + c_step * lane, c_hi);
+        int at = 0;
+        for (int cb = c_lo; cb < c_hi; cb += c_step, at++) {
+            if (at % 32 == 0) {
+                now = next;
+                next.load(fn, hdr, row_centre, centre2, half2, cb + c_step * (lane + 32), c_hi);
+                if (at == 0) fetch(cb, __shfl_sync(0xffffffffu, now.level, 0), 0);
+            }
+            const bool more = cb + c_step < c_hi;
+            const int ahead = at % 32 == 31 ? __shfl_sync(0xffffffffu, next.level, 0) : __shfl_sync(0xffffffffu, now.level, (at + 1) % 32);
+            if (stages == 2 && more) {
+                fetch(cb + c_step, ahead, (at + 1) & 1);
+                cp_async_wait<1>();
+            } else {
+                cp_async_wait<0>();
+            }
+            __syncwarp();
+            const float D = __shfl_sync(0xffffffffu, now.D, at % 32), c = __shfl_sync(0xffffffffu, now.c, at % 32),
+                        s = __shfl_sync(0xffffffffu, now.s, at % 32);
+            const int level = __shfl_sync(0xffffffffu, now.level, at % 32);
+            body(D, c, s, pick(col_P, level), tables + level * 3 * NODES_MAX, tiles + (stages == 2 ? (at & 1) : 0) * stage_floats);
+            __syncwarp();
+            if (stages == 1 && more) fetch(cb + c_step, ahead, 0);
+        }
+    }
+};
+
+// One operand row of a tile as packed pairs.
+template <int KC>
+__device__ __forceinline__ void load_node_row(const float *tile, int j, f32x2 (&rv)[KC / 2]) {
+#pragma unroll
+    for (int c4 = 0; c4 < KC / 4; c4++) {
+        const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(tile + j * NodeShape<KC>::QS + c4 * 4);
+        rv[2 * c4] = v.x, rv[2 * c4 + 1] = v.y;
+    }
+}
 
 struct NodesProductArgs {
     NodesArgs a;
     int64_t kq;
     int64_t q_slots;   // 1: one compressed rhs for all batches
-    int k_chunks;
-    const float *Q;    // [slot][column block][P][kq]
+    int k_chunks, wpr;
+    const float *Q;    // [slot][column block][nodes][kq]
     View<float> out;
     int out_vec;
 };
 
-// Product at the nodes and back to the rows: one CTA of four warps per (batch, row block, KC columns).
-// Each warp takes every fourth column block of the band: it stages the block's compressed rhs
-// (P x KC) in its own part of shared memory, its lanes hold node rows (two rows each beyond 32 nodes; two
-// or four column subsets per warp up to 16 or 8) and accumulate KC sums per row with packed FMAs.  The four
-// warps' sums meet in shared memory, and thread = row forms lambda_1 times them.
-// Per entry: about 4.5 issue slots of kernel value, KC / 2 of FMA and KC / 4 + 1 shared-memory reads.
+// Product at the nodes and back to the rows.  The lanes accumulate KC sums per row with packed FMAs, the
+// four warps' sums meet in shared memory, and thread = row forms lambda_1 times them.
 template <int KT, int KC>
-__global__ void __launch_bounds__(128) nodes_product_kernel(const NodesProductArgs p) {
+__global__ void __launch_bounds__(128, NodeShape<KC>::CTAS) nodes_product_kernel(const NodesProductArgs p) {
     const NodesArgs &a = p.a;
     if (!a.hdr->use) return;
-    const int P = a.hdr->P;
     using Fn = KernelFn<KT>;
-    constexpr int KC2 = KC / 2;
+    constexpr int KC2 = KC / 2, QS = NodeShape<KC>::QS;
     extern __shared__ __align__(16) float smem[];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    float *qs = smem + warp * (NODES_MAX * KC);                     // [P][KC]; later this warp's sums
-    float *cf = smem + 4 * NODES_MAX * KC + warp * (3 * NODES_MAX);  // offset, cosine, sine of the column nodes
-    float *unit = smem + 4 * NODES_MAX * KC + 4 * 3 * NODES_MAX;     // offsets for h = 1
+    const int tid = threadIdx.x, lane = tid & 31;
+    NodeItem<KT, KC> it;
+    BatchIndex bi;
+    it.init(a, p.kq, p.wpr, smem, &bi);
+    const Fn fn = it.fn;
+    const int P = it.P;
+    const float *Q = p.Q + (p.q_slots == 1 ? 0 : it.b) * a.C * node_rows(a, p.q_slots) * p.kq + it.k0;
 
-    int64_t item = blockIdx.x;
-    const int64_t b = item % a.batch.count;
-    item /= a.batch.count;
-    const int64_t r = item % a.R;
-    const int k0 = (int)(item / a.R) * KC;
-    const BatchIndex bi = decompose(a.batch, b);
-    Fn fn;
-    fn.init(batch_ptr(a.params, bi), a.params.s0);
-    const int s = batch_ptr(a.start, bi)[r * a.start.s0], e = batch_ptr(a.end, bi)[r * a.end.s0];
-    const int c_lo = s < e ? s / KM_BLOCK_SIZE : 0;
-    const int c_hi = s < e ? (int)((min((int64_t)e, a.n) + KM_BLOCK_SIZE - 1) / KM_BLOCK_SIZE) : 0;
-    const NodeBox rbox = a.box1[(a.slots1 == 1 ? 0 : b) * a.R + r];
-    const NodeBox *cbox = a.box2 + (a.slots2 == 1 ? 0 : b) * a.C;
-    const float *Q = p.Q + (p.q_slots == 1 ? 0 : b) * a.C * P * p.kq + k0;
-    const int kc = (int)min((int64_t)KC, p.kq - k0);  // a multiple of 4
-
-    if (tid < P) unit[tid] = node_offset(1.0f, tid, P);
-    __syncthreads();
-
-    auto walk = [&](auto rows_per_lane) {
-        constexpr int RPT = decltype(rows_per_lane)::value;
-        const int width = P <= 8 ? 8 : (P <= 16 ? 16 : 32);  // lanes per column subset
-        const int row = lane & (width - 1), subset = lane / width, subsets = 32 / width;
-        float dr[RPT];
-#pragma unroll
-        for (int i = 0; i < RPT; i++) dr[i] = row + 32 * i < P ? rbox.h * unit[row + 32 * i] : 0.0f;
+    with_row_layout<NodeShape<KC>::MAX_ROWS>(P, [&](auto lanes, auto rows_per_lane) {
+        constexpr int LANES = decltype(lanes)::value, RPT = decltype(rows_per_lane)::value, SUBSETS = 32 / LANES;
+        const int row = lane % LANES, subset = lane / LANES;
+        NodeRows<KT, LANES, RPT> rows;
+        rows.init(it.row_table, row, P);
         f32x2 acc[RPT][KC2];
 #pragma unroll
         for (int i = 0; i < RPT; i++)
 #pragma unroll
             for (int c = 0; c < KC2; c++) acc[i][c] = 0ull;
-        for (int cb = c_lo + warp; cb < c_hi; cb += 4) {
-            const NodeBox box = cbox[cb];
-            const float *src = Q + (int64_t)cb * P * p.kq;
-            __syncwarp();
-            for (int q = lane; q < P * (KC / 4); q += 32) {
-                const int j = q / (KC / 4), c4 = (q % (KC / 4)) * 4;
-                if (c4 < kc)
-                    cp_async16(qs + j * KC + c4, src + j * p.kq + c4);
-                else
-                    *reinterpret_cast<float4 *>(qs + j * KC + c4) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            }
-            cp_async_commit();
-            for (int j = lane; j < P; j += 32) {
-                const float dj = box.h * unit[j];
-                float c, sn;
-                NodePair<KT>::column_factors(fn, dj, c, sn);
-                cf[j] = dj;
-                if constexpr (Fn::PHASE) cf[NODES_MAX + j] = c, cf[2 * NODES_MAX + j] = sn;
-            }
-            const float D = rbox.c - box.c;
-            f32x2 y[RPT], rc[RPT], rs[RPT];
-#pragma unroll
-            for (int i = 0; i < RPT; i++) {
-                float c, sn;
-                NodePair<KT>::row_factors(fn, D, dr[i], c, sn);
-                y[i] = splat2(D + dr[i]), rc[i] = splat2(c), rs[i] = splat2(sn);
-            }
-            cp_async_wait<0>();
-            __syncwarp();
-#pragma unroll 2
-            for (int j = 2 * subset; j < P; j += 2 * subsets) {
-                const f32x2 dj = *reinterpret_cast<const f32x2 *>(cf + j);
+        it.walk(a, Q, p.q_slots, p.kq, [&](float D, float c, float s, int Pc, const float *table, const float *tile) {
+            rows.pair(D, c, s);
+            for (int j = 2 * subset; j < Pc; j += 2 * SUBSETS) {
+                const f32x2 dj = *reinterpret_cast<const f32x2 *>(table + j);
                 [[maybe_unused]] f32x2 cj = 0ull, sj = 0ull;
                 if constexpr (Fn::PHASE) {
-                    cj = *reinterpret_cast<const f32x2 *>(cf + NODES_MAX + j);
-                    sj = *reinterpret_cast<const f32x2 *>(cf + 2 * NODES_MAX + j);
+                    cj = *reinterpret_cast<const f32x2 *>(table + NODES_MAX + j);
+                    sj = *reinterpret_cast<const f32x2 *>(table + 2 * NODES_MAX + j);
                 }
                 f32x2 kv[RPT];
 #pragma unroll
                 for (int i = 0; i < RPT; i++) {
-                    const f32x2 cs = Fn::PHASE ? fma2(rc[i], cj, mul2(rs[i], sj)) : 0ull;
-                    kv[i] = fn.unscaled2_ph(sub2(y[i], dj), cs, 0ull);
+                    f32x2 cs = 0ull;
+                    if constexpr (Fn::PHASE) cs = fma2(rows.rc[i], cj, mul2(rows.rs[i], sj));
+                    kv[i] = fn.unscaled2_ph(sub2(rows.y[i], dj), cs, 0ull);
                 }
                 f32x2 rv[KC2];
-                load_staged_row2<KC>(qs, j, rv);
+                load_node_row<KC>(tile, j, rv);
 #pragma unroll
                 for (int i = 0; i < RPT; i++) {
                     float k_even, k_odd;
@@ -352,7 +651,7 @@ __global__ void __launch_bounds__(128) nodes_product_kernel(const NodesProductAr
 #pragma unroll
                     for (int c = 0; c < KC2; c++) acc[i][c] = fma2(kk, rv[c], acc[i][c]);
                 }
-                load_staged_row2<KC>(qs, j + 1, rv);
+                load_node_row<KC>(tile, j + 1, rv);
 #pragma unroll
                 for (int i = 0; i < RPT; i++) {
                     float k_even, k_odd;
@@ -362,174 +661,158 @@ __global__ void __launch_bounds__(128) nodes_product_kernel(const NodesProductAr
                     for (int c = 0; c < KC2; c++) acc[i][c] = fma2(kk, rv[c], acc[i][c]);
                 }
             }
-        }
-        __syncwarp();
+        });
 #pragma unroll
         for (int i = 0; i < RPT; i++) {
 #pragma unroll
             for (int c = 0; c < KC2; c++) {
                 float v0, v1;
                 unpack2(acc[i][c], v0, v1);
-                for (int o = width; o < 32; o <<= 1) {
+#pragma unroll
+                for (int o = LANES; o < 32; o <<= 1) {
                     v0 += __shfl_xor_sync(0xffffffffu, v0, o);
                     v1 += __shfl_xor_sync(0xffffffffu, v1, o);
                 }
-                if (subset == 0 && row + 32 * i < P) {
-                    qs[(row + 32 * i) * KC + 2 * c] = v0;
-                    qs[(row + 32 * i) * KC + 2 * c + 1] = v1;
+                if (subset == 0 && row + LANES * i < P)
+                    *reinterpret_cast<float2 *>(it.tiles + (row + LANES * i) * QS + 2 * c) = make_float2(v0, v1);
+            }
+        }
+    });
+    const float *sums = it.tiles;  // [P][QS]
+    if (p.wpr == 1) {
+        __syncwarp();
+    } else {
+        __syncthreads();
+        const int warp_floats = it.stages * it.stage_floats;
+        for (int q = tid; q < P * KC; q += 128) {
+            const int e = (q / KC) * QS + q % KC;
+            smem[e] = (smem[e] + smem[warp_floats + e]) + (smem[2 * warp_floats + e] + smem[3 * warp_floats + e]);
+        }
+        sums = smem;
+        __syncthreads();
+    }
+    if (it.idle) return;
+
+    // rows: out[row] = sum_q lambda[q][row] * sums[q].  A lane forms OC columns of its rows at a time: the
+    // sums come from shared memory as broadcasts, whose cost is the registers they fill, so that
+    // each one read should serve several rows.
+    const float *lambda = a.lambda1 + (((a.slots1 == 1 ? 0 : it.b) * a.R + it.r) * node_rows(a, a.slots1) +
+                                       node_first(a, a.slots1, it.row_class)) * KM_BLOCK_SIZE;
+    const auto expand = [&](auto rows_per_lane, int row0) {
+        constexpr int OR = decltype(rows_per_lane)::value, OC = KC >= 8 ? 8 : 4;
+        for (int g = 0; g < KC / OC; g++) {
+            const int k_here = (int)min((int64_t)OC, a.k - it.k0 - g * OC);
+            if (k_here <= 0) break;
+            f32x2 o2[OR][OC / 2];
+#pragma unroll
+            for (int i = 0; i < OR; i++)
+#pragma unroll
+                for (int c = 0; c < OC / 2; c++) o2[i][c] = 0ull;
+#pragma unroll 4
+            for (int q = 0; q < P; q++) {
+                f32x2 rv[OC / 2];
+#pragma unroll
+                for (int c4 = 0; c4 < OC / 4; c4++) {
+                    const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(sums + q * QS + g * OC + c4 * 4);
+                    rv[2 * c4] = v.x, rv[2 * c4 + 1] = v.y;
+                }
+#pragma unroll
+                for (int i = 0; i < OR; i++) {
+                    const f32x2 l = splat2(lambda[q * KM_BLOCK_SIZE + row0 + lane + 32 * i] * fn.scale);
+#pragma unroll
+                    for (int c = 0; c < OC / 2; c++) o2[i][c] = fma2(l, rv[c], o2[i][c]);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < OR; i++) {
+                const int64_t row = it.r * KM_BLOCK_SIZE + row0 + lane + 32 * i;
+                if (row >= a.m) break;
+                float *out = batch_ptr(p.out, bi) + row * p.out.s0 + (it.k0 + g * OC) * p.out.s1;
+#pragma unroll
+                for (int c4 = 0; c4 < OC / 4; c4++) {
+                    float4 v;
+                    unpack2(o2[i][2 * c4], v.x, v.y);
+                    unpack2(o2[i][2 * c4 + 1], v.z, v.w);
+                    if (p.out_vec && c4 * 4 + 4 <= k_here) {
+                        *reinterpret_cast<float4 *>(out + c4 * 4) = v;
+                    } else {
+                        const float w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                        for (int u = 0; u < 4; u++)
+                            if (c4 * 4 + u < k_here) out[(c4 * 4 + u) * p.out.s1] = w[u];
+                    }
                 }
             }
         }
     };
-    if (P <= 32)
-        walk(std::integral_constant<int, 1>());
+    if (p.wpr == 1)
+        expand(Int<4>(), 0);
     else
-        walk(std::integral_constant<int, 2>());
-    __syncthreads();
-    for (int q = tid; q < P * KC; q += 128)
-        smem[q] = ((smem[q] + smem[NODES_MAX * KC + q]) + (smem[2 * NODES_MAX * KC + q] + smem[3 * NODES_MAX * KC + q])) * fn.scale;
-    __syncthreads();
-
-    // rows: out[row] = sum_q lambda[q][row] * sums[q]
-    const int64_t row = r * KM_BLOCK_SIZE + tid;
-    if (row >= a.m) return;
-    const float *lambda = a.lambda1 + ((a.slots1 == 1 ? 0 : b) * a.R + r) * P * KM_BLOCK_SIZE + tid;
-    f32x2 o2[KC2];
-#pragma unroll
-    for (int c = 0; c < KC2; c++) o2[c] = 0ull;
-#pragma unroll 4
-    for (int q = 0; q < P; q++) {
-        const f32x2 l = splat2(lambda[q * KM_BLOCK_SIZE]);
-        f32x2 rv[KC2];
-        load_staged_row2<KC>(smem, q, rv);
-#pragma unroll
-        for (int c = 0; c < KC2; c++) o2[c] = fma2(l, rv[c], o2[c]);
-    }
-    float *out = batch_ptr(p.out, bi) + row * p.out.s0 + k0 * p.out.s1;
-    const int k_here = (int)min((int64_t)KC, a.k - k0);
-#pragma unroll
-    for (int c4 = 0; c4 < KC / 4; c4++) {
-        float4 v;
-        unpack2(o2[2 * c4], v.x, v.y);
-        unpack2(o2[2 * c4 + 1], v.z, v.w);
-        if (p.out_vec && c4 * 4 + 4 <= k_here) {
-            *reinterpret_cast<float4 *>(out + c4 * 4) = v;
-        } else {
-            const float w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-            for (int u = 0; u < 4; u++)
-                if (c4 * 4 + u < k_here) out[(c4 * 4 + u) * p.out.s1] = w[u];
-        }
-    }
+        expand(Int<1>(), 32 * (tid >> 5));
 }
 
 struct NodesGradArgs {
     NodesArgs a;
     int64_t kq;
     int64_t l_slots, r_slots;
-    int k_chunks;
-    const float *L, *Rt;  // compressed left [slot][row block][P][kq], right [slot][column block][P][kq]
+    int k_chunks, wpr;
+    const float *L, *Rt;  // compressed left [slot][row block][nodes][kq], right [slot][column block][nodes][kq]
     float *partials;      // [batch][row block][chunk][KM_MAX_PARAMS]
 };
 
-// The gradient's sums at the nodes: the same walk, with the left values of a lane's node rows in
-// registers, the coefficient of an entry KC / 2 packed FMAs, and the factors of d kappa / d p added up
-// as in the direct kernels.
+// The gradient's sums at the nodes: the left values of a lane's node rows stay in registers, the
+// coefficient of an entry is KC / 2 packed FMAs, and the factors of d kappa / d p are added up as in the
+// direct kernels.
 template <int KT, int KC>
-__global__ void __launch_bounds__(128) nodes_grad_kernel(const NodesGradArgs p) {
+__global__ void __launch_bounds__(128, NodeShape<KC>::CTAS) nodes_grad_kernel(const NodesGradArgs p) {
     const NodesArgs &a = p.a;
     if (!a.hdr->use) return;
-    const int P = a.hdr->P;
     using Fn = KernelFn<KT>;
     constexpr int KC2 = KC / 2, NS = Fn::NSUMS;
     extern __shared__ __align__(16) float smem[];
     __shared__ float warp_sums[4][KM_MAX_PARAMS];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    float *qs = smem + warp * (NODES_MAX * KC);
-    float *cf = smem + 4 * NODES_MAX * KC + warp * (3 * NODES_MAX);
-    float *unit = smem + 4 * NODES_MAX * KC + 4 * 3 * NODES_MAX;
-
-    int64_t item = blockIdx.x;
-    const int64_t b = item % a.batch.count;
-    item /= a.batch.count;
-    const int64_t r = item % a.R;
-    const int chunk = (int)(item / a.R), k0 = chunk * KC;
-    const BatchIndex bi = decompose(a.batch, b);
-    Fn fn;
-    fn.init(batch_ptr(a.params, bi), a.params.s0);
-    const int s = batch_ptr(a.start, bi)[r * a.start.s0], e = batch_ptr(a.end, bi)[r * a.end.s0];
-    const int c_lo = s < e ? s / KM_BLOCK_SIZE : 0;
-    const int c_hi = s < e ? (int)((min((int64_t)e, a.n) + KM_BLOCK_SIZE - 1) / KM_BLOCK_SIZE) : 0;
-    const NodeBox rbox = a.box1[(a.slots1 == 1 ? 0 : b) * a.R + r];
-    const NodeBox *cbox = a.box2 + (a.slots2 == 1 ? 0 : b) * a.C;
-    const float *L = p.L + ((p.l_slots == 1 ? 0 : b) * a.R + r) * P * p.kq + k0;
-    const float *Rt = p.Rt + (p.r_slots == 1 ? 0 : b) * a.C * P * p.kq + k0;
-    const int kc = (int)min((int64_t)KC, p.kq - k0);
-
-    if (tid < P) unit[tid] = node_offset(1.0f, tid, P);
-    __syncthreads();
+    NodeItem<KT, KC> it;
+    BatchIndex bi;
+    it.init(a, p.kq, p.wpr, smem, &bi);
+    const Fn fn = it.fn;
+    const int P = it.P;
+    const float *L = p.L + (((p.l_slots == 1 ? 0 : it.b) * a.R + it.r) * node_rows(a, p.l_slots) + node_first(a, p.l_slots, it.row_class)) * p.kq + it.k0;
+    const float *Rt = p.Rt + (p.r_slots == 1 ? 0 : it.b) * a.C * node_rows(a, p.r_slots) * p.kq + it.k0;
 
     f32x2 sums2[NS];
 #pragma unroll
     for (int q = 0; q < NS; q++) sums2[q] = 0ull;
-    auto walk = [&](auto rows_per_lane) {
-        constexpr int RPT = decltype(rows_per_lane)::value;
-        const int width = P <= 8 ? 8 : (P <= 16 ? 16 : 32);
-        const int row = lane & (width - 1), subset = lane / width, subsets = 32 / width;
-        float dr[RPT];
-        f32x2 lv[RPT][KC2];
+    with_row_layout<NodeShape<KC>::MAX_ROWS>(P, [&](auto lanes, auto rows_per_lane) {
+        constexpr int LANES = decltype(lanes)::value, RPT = decltype(rows_per_lane)::value, SUBSETS = 32 / LANES;
+        const int row = lane % LANES, subset = lane / LANES;
+        NodeRows<KT, LANES, RPT> rows;
+        rows.init(it.row_table, row, P);
+        f32x2 lv[RPT][KC2];  // (zero for rows past P: their coefficients vanish)
 #pragma unroll
         for (int i = 0; i < RPT; i++) {
-            const bool valid = row + 32 * i < P;
-            dr[i] = valid ? rbox.h * unit[row + 32 * i] : 0.0f;
+            const bool valid = row + LANES * i < P;
 #pragma unroll
             for (int c4 = 0; c4 < KC / 4; c4++) {
                 ulonglong2 v = make_ulonglong2(0ull, 0ull);
-                if (valid && c4 * 4 < kc) v = *reinterpret_cast<const ulonglong2 *>(L + (row + 32 * i) * p.kq + c4 * 4);
+                if (valid && c4 * 4 < it.kc) v = *reinterpret_cast<const ulonglong2 *>(L + (row + LANES * i) * p.kq + c4 * 4);
                 lv[i][2 * c4] = v.x, lv[i][2 * c4 + 1] = v.y;
             }
         }
-        for (int cb = c_lo + warp; cb < c_hi; cb += 4) {
-            const NodeBox box = cbox[cb];
-            const float *src = Rt + (int64_t)cb * P * p.kq;
-            __syncwarp();
-            for (int q = lane; q < P * (KC / 4); q += 32) {
-                const int j = q / (KC / 4), c4 = (q % (KC / 4)) * 4;
-                if (c4 < kc)
-                    cp_async16(qs + j * KC + c4, src + j * p.kq + c4);
-                else
-                    *reinterpret_cast<float4 *>(qs + j * KC + c4) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            }
-            cp_async_commit();
-            for (int j = lane; j < P; j += 32) {
-                const float dj = box.h * unit[j];
-                float c, sn;
-                NodePair<KT>::column_factors(fn, dj, c, sn);
-                cf[j] = dj;
-                if constexpr (Fn::PHASE) cf[NODES_MAX + j] = c, cf[2 * NODES_MAX + j] = sn;
-            }
-            const float D = rbox.c - box.c;
-            f32x2 y[RPT], rc[RPT], rs[RPT];
-#pragma unroll
-            for (int i = 0; i < RPT; i++) {
-                float c, sn;
-                NodePair<KT>::row_factors(fn, D, dr[i], c, sn);
-                y[i] = splat2(D + dr[i]), rc[i] = splat2(c), rs[i] = splat2(sn);
-            }
-            cp_async_wait<0>();
-            __syncwarp();
-            for (int j = 2 * subset; j < P; j += 2 * subsets) {
-                const f32x2 dj = *reinterpret_cast<const f32x2 *>(cf + j);
+        it.walk(a, Rt, p.r_slots, p.kq, [&](float D, float c, float s, int Pc, const float *table, const float *tile) {
+            rows.pair(D, c, s);
+            for (int j = 2 * subset; j < Pc; j += 2 * SUBSETS) {
+                const f32x2 dj = *reinterpret_cast<const f32x2 *>(table + j);
                 [[maybe_unused]] f32x2 cj = 0ull, sj = 0ull;
                 if constexpr (Fn::PHASE) {
-                    cj = *reinterpret_cast<const f32x2 *>(cf + NODES_MAX + j);
-                    sj = *reinterpret_cast<const f32x2 *>(cf + 2 * NODES_MAX + j);
+                    cj = *reinterpret_cast<const f32x2 *>(table + NODES_MAX + j);
+                    sj = *reinterpret_cast<const f32x2 *>(table + 2 * NODES_MAX + j);
                 }
                 float co[RPT][2];
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
                     f32x2 rv[KC2];
-                    load_staged_row2<KC>(qs, j + h, rv);
+                    load_node_row<KC>(tile, j + h, rv);
 #pragma unroll
                     for (int i = 0; i < RPT; i++) {
                         f32x2 t = mul2(lv[i][0], rv[0]);
@@ -544,18 +827,14 @@ __global__ void __launch_bounds__(128) nodes_grad_kernel(const NodesGradArgs p) 
                 for (int i = 0; i < RPT; i++) {
                     f32x2 cs = 0ull, sn = 0ull;
                     if constexpr (Fn::PHASE) {
-                        cs = fma2(rc[i], cj, mul2(rs[i], sj));
-                        sn = sub2(mul2(rs[i], cj), mul2(rc[i], sj));
+                        cs = fma2(rows.rc[i], cj, mul2(rows.rs[i], sj));
+                        sn = sub2(mul2(rows.rs[i], cj), mul2(rows.rc[i], sj));
                     }
-                    fn.accumulate2_ph(sub2(y[i], dj), cs, sn, pack2(co[i][0], co[i][1]), sums2);
+                    fn.accumulate2_ph(sub2(rows.y[i], dj), cs, sn, pack2(co[i][0], co[i][1]), sums2);
                 }
             }
-        }
-    };
-    if (P <= 32)
-        walk(std::integral_constant<int, 1>());
-    else
-        walk(std::integral_constant<int, 2>());
+        });
+    });
     fn.rescale_ph(sums2);
 #pragma unroll
     for (int q = 0; q < NS; q++) {
@@ -566,11 +845,17 @@ __global__ void __launch_bounds__(128) nodes_grad_kernel(const NodesGradArgs p) 
         for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
         if (lane == 0) warp_sums[warp][q] = v;
     }
+    float *record = p.partials + ((it.b * a.R + it.r) * p.k_chunks + it.chunk) * KM_MAX_PARAMS;
+    if (p.wpr == 1) {
+        __syncwarp();
+        if (!it.idle && lane < KM_MAX_PARAMS) record[lane] = lane < NS ? warp_sums[warp][lane] : 0.0f;
+        return;
+    }
     __syncthreads();
     if (tid < KM_MAX_PARAMS) {
         float v = 0.0f;
         if (tid < NS) v = (warp_sums[0][tid] + warp_sums[1][tid]) + (warp_sums[2][tid] + warp_sums[3][tid]);
-        p.partials[((b * a.R + r) * p.k_chunks + chunk) * KM_MAX_PARAMS + tid] = v;
+        record[tid] = v;
     }
 }
 
@@ -587,7 +872,7 @@ static bool shared_by_batches(const View<T> &v, const Batch &b) {
 // The node counts for which interpolation is the faster way.  Per entry the kernels here take about
 // 4.5 + 0.75 k issue slots per 32 entries; the tensor-core kernels 11 - 15, whatever k.  (128 / P)^2 fewer entries make
 // up for that up to P = 64 at 32 columns and up to P = 48 beyond.
-static int nodes_limit(int64_t k) { return k <= 32 ? 64 : 48; }
+static int nodes_limit(int64_t k) { return k <= 16 ? NODES_MAX : (k <= 32 ? 64 : 48); }
 
 // Columns per CTA: chunks of at most 32, all of one width.
 static int nodes_kc(int64_t k) {
@@ -598,11 +883,14 @@ static int nodes_kc(int64_t k) {
     return per <= 16 ? 16 : (per <= 24 ? 24 : 32);
 }
 
+// A warp per row block once that gives every SM its 12 - 16 warps; four warps below.
+static int nodes_warps_per_row_block(int64_t items) { return items >= 148 * 12 ? 1 : 4; }
+
 struct NodesLayout {
     int64_t slots1, slots2, R, C, kq;
     bool same;
-    int max_p;
-    size_t box1, box2, lambda1, lambda2, ops[2], partials, direct, total;
+    int max_p, cap;
+    size_t classes, centre1, centre2, half1, half2, lambda1, lambda2, ops[2], partials, direct, total;
     int64_t op_slots[2];
 
     static size_t up(size_t v) { return (v + 255) / 256 * 256; }
@@ -615,44 +903,68 @@ struct NodesLayout {
         C = ceil_div(n, KM_BLOCK_SIZE);
         kq = ceil_div(k, 4) * 4;
         max_p = nodes_limit(k);
+        // Where batches share their points every class needs its own Lagrange matrices and operands: room
+        // for several node counts, as long as it is not much memory.
+        cap = std::max<int>(max_p, R + C <= 16384 ? 160 : 96);
         same = m == n && x1.data == x2.data && x1.s0 == x2.s0;
         for (int d = 0; d < b.ndim; d++) same = same && (b.size[d] == 1 || x1.bs[d] == x2.bs[d]);
         op_slots[1] = shared_by_batches(right, b) && slots2 == 1 ? 1 : b.count;
         op_slots[0] = left == nullptr ? 0 : (shared_by_batches(*left, b) && slots1 == 1 ? 1 : b.count);
-        size_t at = 256;
+        size_t at = up(sizeof(NodesHeader));
         const auto take = [&](size_t bytes) {
             const size_t here = at;
             at += up(bytes);
             return here;
         };
-        const size_t per_block = (size_t)max_p * KM_BLOCK_SIZE * sizeof(float);
-        box1 = take((size_t)(slots1 * R) * sizeof(NodeBox));
-        box2 = same ? box1 : take((size_t)(slots2 * C) * sizeof(NodeBox));
-        lambda1 = take((size_t)(slots1 * R) * per_block);
-        lambda2 = same ? lambda1 : take((size_t)(slots2 * C) * per_block);
-        ops[0] = take((size_t)(op_slots[0] * R * max_p * kq) * sizeof(float));
-        ops[1] = take((size_t)(op_slots[1] * C * max_p * kq) * sizeof(float));
+        const auto nodes = [&](int64_t slots) { return (size_t)(slots == 1 && b.count > 1 ? cap : max_p) * slots; };
+        classes = take((size_t)(b.count * NODES_LEVELS) * sizeof(int));
+        centre1 = take((size_t)(slots1 * R) * sizeof(float));
+        centre2 = same ? centre1 : take((size_t)(slots2 * C) * sizeof(float));
+        half1 = take((size_t)(slots1 * R) * sizeof(float));
+        half2 = same ? half1 : take((size_t)(slots2 * C) * sizeof(float));
+        lambda1 = take(nodes(slots1) * R * KM_BLOCK_SIZE * sizeof(float));
+        lambda2 = same ? lambda1 : take(nodes(slots2) * C * KM_BLOCK_SIZE * sizeof(float));
+        ops[0] = take(op_slots[0] == 0 ? 0 : nodes(op_slots[0]) * R * kq * sizeof(float));
+        ops[1] = take(nodes(op_slots[1]) * C * kq * sizeof(float));
         partials = take(left == nullptr ? 0 : (size_t)(b.count * R * ceil_div(k, nodes_kc(k))) * KM_MAX_PARAMS * sizeof(float));
         direct = take(direct_bytes);
         total = at;
     }
 };
 
-static int nodes_compress(const NodesArgs &a, const View<const float> &v, int64_t rows, int64_t blocks, int64_t kq, int64_t slots,
-                          int64_t lambda_slots, const float *lambda, float *out, cudaStream_t s) {
-    const CompressArgs c = {a.batch, rows, a.k, kq, blocks, slots, lambda_slots, v, lambda, out, a.hdr};
-    const int64_t ctas = slots * blocks * ceil_div(kq, CP_COLS);
-    nodes_compress_kernel<<<(unsigned)ctas, 128, 0, s>>>(c);
+// `side` 0: left / row blocks, 1: right / column blocks.
+static int nodes_compress(const NodesArgs &a, const NodesLayout &l, const View<const float> &v, int side, float *out, cudaStream_t s) {
+    CompressArgs c;
+    c.a = a;
+    c.rows = side == 0 ? a.m : a.n, c.kq = l.kq, c.blocks = side == 0 ? l.R : l.C;
+    c.slots = l.op_slots[side], c.x_slots = side == 0 ? l.slots1 : l.slots2;
+    c.vec = a.k % 4 == 0 && rows_vectorizable(v, a.batch);
+    c.v = v;
+    c.half = side == 0 ? a.half1 : a.half2, c.lambda = side == 0 ? a.lambda1 : a.lambda2;
+    c.out = out;
+    const auto launch = [&](auto cols) {
+        constexpr int COLS = decltype(cols)::value;
+        const cudaError_t err = cudaFuncSetAttribute(nodes_compress_kernel<COLS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                     (int)CompressShape<COLS>::SMEM);
+        if (err != cudaSuccess) return cuda_fail(err, "cudaFuncSetAttribute(interpolation)");
+        const int64_t ctas = ceil_div(c.slots * c.blocks * ceil_div(l.kq, COLS), 4);
+        nodes_compress_kernel<COLS><<<(unsigned)ctas, 128, CompressShape<COLS>::SMEM, s>>>(c);
+        return (int)KM_OK;
+    };
+    const int rc = l.kq <= 16 ? launch(Int<16>()) : launch(Int<32>());
+    if (rc != KM_OK) return rc;
     KM_CHECK_LAUNCH("interpolation: operand launch");
     return KM_OK;
 }
 
 static int nodes_begin(NodesArgs &a, const NodesLayout &l, int kernel_type, unsigned char *ws, cudaStream_t s) {
-    a.R = l.R, a.C = l.C, a.slots1 = l.slots1, a.slots2 = l.slots2, a.same = l.same ? 1 : 0, a.max_p = l.max_p;
+    a.R = l.R, a.C = l.C, a.slots1 = l.slots1, a.slots2 = l.slots2, a.same = l.same ? 1 : 0, a.max_p = l.max_p, a.cap = l.cap;
+    a.classes = reinterpret_cast<int *>(ws + l.classes);
+    a.half1 = reinterpret_cast<float *>(ws + l.half1), a.half2 = reinterpret_cast<float *>(ws + l.half2);
     a.hdr = reinterpret_cast<NodesHeader *>(ws);
-    a.box1 = reinterpret_cast<NodeBox *>(ws + l.box1), a.box2 = reinterpret_cast<NodeBox *>(ws + l.box2);
+    a.centre1 = reinterpret_cast<float *>(ws + l.centre1), a.centre2 = reinterpret_cast<float *>(ws + l.centre2);
     a.lambda1 = reinterpret_cast<float *>(ws + l.lambda1), a.lambda2 = reinterpret_cast<float *>(ws + l.lambda2);
-    cudaError_t err = cudaMemsetAsync(ws, 0, sizeof(NodesHeader), s);
+    cudaError_t err = cudaMemsetAsync(ws, 0, NODES_ZEROED, s);
     if (err != cudaSuccess) return cuda_fail(err, "interpolation: cudaMemsetAsync");
     const int64_t boxes = l.slots1 * l.R + (l.same ? 0 : l.slots2 * l.C), work = std::max(ceil_div(boxes, 8), ceil_div(a.batch.count * l.R, 256));
     nodes_plan_kernel<<<(unsigned)std::min<int64_t>(work, 148 * 4), 256, 0, s>>>(a, kernel_type);
@@ -662,24 +974,21 @@ static int nodes_begin(NodesArgs &a, const NodesLayout &l, int kernel_type, unsi
     return KM_OK;
 }
 
-template <int KC>
-constexpr size_t nodes_smem() { return (size_t)(4 * NODES_MAX * KC + 4 * 3 * NODES_MAX + NODES_MAX) * sizeof(float); }
-
 template <int KT, int KC>
 static int launch_nodes_product(const NodesProductArgs &p, cudaStream_t s) {
     auto kernel = nodes_product_kernel<KT, KC>;
-    const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)nodes_smem<KC>());
+    const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)NodeShape<KC>::SMEM);
     if (err != cudaSuccess) return cuda_fail(err, "cudaFuncSetAttribute(interpolation)");
-    kernel<<<(unsigned)(p.a.batch.count * p.a.R * p.k_chunks), 128, nodes_smem<KC>(), s>>>(p);
+    kernel<<<(unsigned)(p.a.batch.count * (p.wpr == 1 ? ceil_div(p.a.R, 4) : p.a.R) * p.k_chunks), 128, NodeShape<KC>::SMEM, s>>>(p);
     KM_CHECK_LAUNCH("interpolation: product launch");
     return KM_OK;
 }
 template <int KT, int KC>
 static int launch_nodes_grad(const NodesGradArgs &p, cudaStream_t s) {
     auto kernel = nodes_grad_kernel<KT, KC>;
-    const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)nodes_smem<KC>());
+    const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)NodeShape<KC>::SMEM);
     if (err != cudaSuccess) return cuda_fail(err, "cudaFuncSetAttribute(interpolation)");
-    kernel<<<(unsigned)(p.a.batch.count * p.a.R * p.k_chunks), 128, nodes_smem<KC>(), s>>>(p);
+    kernel<<<(unsigned)(p.a.batch.count * (p.wpr == 1 ? ceil_div(p.a.R, 4) : p.a.R) * p.k_chunks), 128, NodeShape<KC>::SMEM, s>>>(p);
     KM_CHECK_LAUNCH("interpolation: gradient launch");
     return KM_OK;
 }
@@ -784,13 +1093,14 @@ extern "C" int km_matmul_nodes_f32(int kernel_type, const km_batch *batch, int64
     p.kq = l.kq, p.q_slots = l.op_slots[1];
     float *Q = reinterpret_cast<float *>(ws + l.ops[1]);
     p.Q = Q;
-    rc = nodes_compress(p.a, make_view<const float>(rhs, b), n, l.C, l.kq, l.op_slots[1], l.slots2, p.a.lambda2, Q, s);
+    rc = nodes_compress(p.a, l, make_view<const float>(rhs, b), 1, Q, s);
     if (rc != KM_OK) return rc;
     p.out = make_view<float>(out, b);
     p.out_vec = p.out.s1 == 1 && p.out.s0 % 4 == 0 && (uintptr_t)p.out.data % 16 == 0;
     for (int d = 0; d < b.ndim; d++) p.out_vec = p.out_vec && p.out.bs[d] % 4 == 0;
     const int kc = nodes_kc(k);
     p.k_chunks = (int)ceil_div(k, kc);
+    p.wpr = nodes_warps_per_row_block(b.count * l.R * p.k_chunks);
     rc = KM_NODES_DISPATCH(launch_nodes_product, p)(kernel_type, kc);
     if (rc != KM_OK) return rc;
     const Gate gate = {&p.a.hdr->use, 0};
@@ -833,12 +1143,13 @@ extern "C" int km_bilinear_derivative_nodes_f32(int kernel_type, const km_batch 
     p.kq = l.kq, p.l_slots = l.op_slots[0], p.r_slots = l.op_slots[1];
     float *L = reinterpret_cast<float *>(ws + l.ops[0]), *Rt = reinterpret_cast<float *>(ws + l.ops[1]);
     p.L = L, p.Rt = Rt;
-    rc = nodes_compress(p.a, make_view<const float>(left, b), m, l.R, l.kq, l.op_slots[0], l.slots1, p.a.lambda1, L, s);
+    rc = nodes_compress(p.a, l, make_view<const float>(left, b), 0, L, s);
     if (rc != KM_OK) return rc;
-    rc = nodes_compress(p.a, make_view<const float>(right, b), n, l.C, l.kq, l.op_slots[1], l.slots2, p.a.lambda2, Rt, s);
+    rc = nodes_compress(p.a, l, make_view<const float>(right, b), 1, Rt, s);
     if (rc != KM_OK) return rc;
     const int kc = nodes_kc(k);
     p.k_chunks = (int)ceil_div(k, kc);
+    p.wpr = nodes_warps_per_row_block(b.count * l.R * p.k_chunks);
     p.partials = reinterpret_cast<float *>(ws + l.partials);
     rc = KM_NODES_DISPATCH(launch_nodes_grad, p)(kernel_type, kc);
     if (rc != KM_OK) return rc;

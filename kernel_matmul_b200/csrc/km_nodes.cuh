@@ -5,11 +5,15 @@
 // into an interval that is short against what kappa varies over.  On a pair of such intervals kappa(x - y)
 // is, to fp32 rounding, a polynomial of low degree in x and in y, so with P Chebyshev points xi of
 // every block's interval and the Lagrange polynomials lambda on them
-//     kappa(x_i - x_j) = sum_pq lambda_p(x_i) kappa(xi_p - xi_q) lambda_q(x_j) + O(eps),   P = 8 .. 64,
-// and  K rhs = Lambda_1 ( K(xi, xi) ( Lambda_2^T rhs ) ):  (128 / P)^2 = 4 .. 256 times fewer kernel entries.
+//     kappa(x_i - x_j) = sum_pq lambda_p(x_i) kappa(xi_p - xi_q) lambda_q(x_j) + O(eps),   P = 8 .. 80,
+// and  K rhs = Lambda_1 ( K(xi, xi) ( Lambda_2^T rhs ) ):  (128 / P)^2 = 2.5 .. 256 times fewer kernel entries.
 // The band is kept exactly (ranges aligned to blocks; others are left to the direct kernels), and a
 // gradient is the same gradient of the small problem with left and right replaced by Lambda^T left and
 // Lambda^T right.
+//
+// Each block has an interval around its own centre whose half-length is one of four (the longest
+// block's, and that divided by 1.15, 1.32 and 1.52); P follows from half-length and kernel.  Node offsets,
+// weights and phase factors are then the same for all blocks of one half-length.
 //
 // P follows from the inputs (nodes_needed): for f analytic in the Bernstein ellipse with parameter rho
 // around an interval of half-length h, the interpolation error on P Chebyshev points is at most
@@ -18,8 +22,8 @@
 //     |exp(-z^2 / 2 l^2)| <= exp(b^2 / 2 l^2),   |cos(W z)| <= cosh(W b) <= exp(W b),
 //     |exp(-2 sin^2(W z / 2) / l_p)| <= exp((cosh(W b) - 1) / l_p)
 // and a factor (1 + b^2 / l^2) for the gradients' powers of tau.  The bound is evaluated on the device for
-// the longest interval and every kernel of the call, and P taken so that it is below 1e-8 of
-// kappa's maximum: less than the rounding of an fp32 value near 1 (6e-8), than the SFU's exp and cos
+// the four half-lengths and every kernel of the call, and P taken so that it is below 3e-8 of
+// kappa's maximum: half an ulp of an fp32 value near 1, less than the SFU's exp and cos
 // (1e-7 and 5e-7) and than the fp16 pairs of the tensor-core kernels (3e-8).
 #pragma once
 
@@ -27,14 +31,13 @@
 
 namespace km {
 
-constexpr int NODES_MAX = 64;           // P of a call is a multiple of 4 up to this
-constexpr float NODES_EPS = 1e-8f;      // bound on the interpolation error, relative to kappa's maximum
+constexpr int NODES_MAX = 80;           // most nodes of a block; P is even
+constexpr float NODES_EPS = 3e-8f;      // bound on the interpolation error, relative to kappa's maximum: half an ulp of 1
+// The blocks of a call use intervals of one of NODES_LEVELS half-lengths: the longest block's, divided
+// by powers of NODES_RATIO.  The longest of some hundred blocks of uniform points is 1.3 times the mean.
+constexpr int NODES_LEVELS = 4;
+constexpr float NODES_RATIO = 1.15f;
 constexpr float NODES_MIN_H = 1e-18f;   // half-length given to an interval of coincident points
-
-// Interval of one block: points c + h t, |t| <= 1.
-struct NodeBox {
-    float c, h;
-};
 
 // Smallest P whose error bound is below NODES_EPS on an interval of half-length h; > NODES_MAX if
 // none (or for non-finite arguments).  `lane` of 32 lanes tries one rho; the result is in every lane.
@@ -55,12 +58,11 @@ __device__ __forceinline__ int nodes_needed(const float *theta, int64_t stride, 
     return (int)ceilf(p);
 }
 
-// Offset of node q of P from the centre of its interval.  Every kernel calls this one function, so
-// that positions agree to the bit with those the Lagrange polynomials were formed for.
+// Node q of P on an interval of half-length h, as an offset from its centre.
 __device__ __forceinline__ float node_offset(float h, int q, int P) { return h * cospif((2.0f * q + 1.0f) / (2.0f * P)); }
 
-// Barycentric weights of the rounded offsets `delta` (shared memory, P values), scaled by (2 / h)^P:
-// thread q < P forms 1 / prod_r (delta_q - delta_r) in fp64.
+// Barycentric weight of node q, scaled by (2 / h)^P: 1 / prod_r (delta_q - delta_r) of the ROUNDED
+// offsets, in fp64, so that the Lagrange polynomials are those of the very points kappa is taken at.
 __device__ __forceinline__ float node_weight(const float *delta, float h, int q, int P) {
     const double s = 2.0 / (double)h;
     double w = 1.0;
