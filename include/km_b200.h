@@ -488,6 +488,51 @@ KM_API int km_cg_update_p_f32(int64_t k, float *p, const float *r, int64_t lo, i
                               const float *rs_old, float *rs_new, const float *ynorm, float *history_row,
                               float *beta_row, void *stream);
 
+/* Stochastic Lanczos quadrature from the coefficients of a batched CG run (what linear_operator's
+ * inv_quad_logdet does): out[c] = z_c^T log(A) z_c for the columns of A V = Z solved from zero, with
+ * alphas, betas (iterations, k), residual_norms (iterations + 1, k) and z_norm2 (k) = |z_c|^2.  A column is cut
+ * where its residual norm is not above `converged` (its later coefficients are rounding noise). */
+KM_API int km_cg_log_forms_f32(int64_t iterations, int64_t k, const float *alphas, const float *betas,
+                               const float *residual_norms, const float *z_norm2, float converged, double *out,
+                               void *stream);
+
+
+/* ---------------------------------------------------------------------------------------
+ * The operator of a CG solve by blockwise interpolation (see km_matmul_nodes_f32), laid out once and
+ * applied many times.  K = sum over the batch of params of kernels that share the points x (n values,
+ * x_stride elements apart) and the band start / end (contiguous, one per row block).
+ *  - plan: looks at points, band and parameters; `plan` (KM_NODE_PLAN_BYTES, 8-byte aligned) begins with
+ *    five int64: first and last column the row blocks of the window read, a checksum of the whole
+ *    band, the nodes per block (0: this operator cannot be laid out so) and the widest band of the
+ *    window in blocks; `centre` receives one value per row block.
+ *  - build, with these as `nodes` and `max_blocks`: lambda (row blocks x nodes x 128 floats) and
+ *    matrix (row blocks of the window x max_blocks x nodes x nodes floats).
+ *  - compress: nodes (row blocks x nodes x ceil4(k)) = lambda^T v for blocks [block_begin, block_end).
+ *  - update_p: the same behind p = r + beta p on these blocks (arguments as km_cg_update_p_f32).
+ *  - product: the window's rows of K v from its nodes; with p not null of K v + sigma2 p, and the
+ *    row blocks' partial sums of p . (K v + sigma2 p) (as km_cg_q_dots_f32).
+ * No reference counterpart (its solves call matmul once per iteration).
+ * ------------------------------------------------------------------------------------- */
+#define KM_NODE_PLAN_BYTES 128
+KM_API int km_node_operator_plan_f32(int kernel_type, const km_batch *batch, int64_t n, const float *x, int64_t x_stride,
+                                     const km_view *params, const int32_t *start, const int32_t *end, int64_t row_block_begin,
+                                     int64_t row_block_count, float *centre, void *plan, void *stream);
+KM_API int km_node_operator_build_f32(int kernel_type, const km_batch *batch, int64_t n, const float *x, int64_t x_stride,
+                                      const km_view *params, const int32_t *start, const int32_t *end, int64_t row_block_begin,
+                                      int64_t row_block_count, const float *centre, const void *plan, int64_t nodes,
+                                      int64_t max_blocks, float *lambda, float *matrix, void *stream);
+KM_API int km_node_compress_f32(int64_t k, int64_t n, int64_t nodes_per_block, const float *lambda, const float *v, float *nodes,
+                                int64_t block_begin, int64_t block_end, void *stream);
+KM_API int km_node_update_p_f32(int64_t k, int64_t n, int64_t nodes_per_block, const float *lambda, float *p, const float *r,
+                                float *nodes, int64_t block_begin, int64_t block_end, const void *rr_seg_sums,
+                                int64_t seg_rank_stride_bytes, int32_t seg_ranks, int32_t seg_slots, const float *rs_old,
+                                float *rs_new, const float *ynorm, float *history_row, float *beta_row, void *stream);
+KM_API int km_node_product_f32(int64_t k, int64_t n, int64_t nodes_per_block, int64_t max_blocks, const int32_t *start,
+                               const int32_t *end, const float *lambda, const float *matrix, const float *nodes,
+                               int64_t row_block_begin, int64_t row_block_count, float *out, const float *p, float sigma2,
+                               float *block_partials, void *stream);
+
+
 /* ---------------------------------------------------------------------------------------
  * Self-tests of the give-up path of the tensor-core kernels.  No reference counterpart (the
  * reference's debug build synchronises and throws on a CUDA error,

@@ -53,6 +53,13 @@ BLOCK_SIZE = 128
 MAX_SEGMENTS = 64
 
 
+#: points from which a solve lays its operator out as a node matrix; below, the kernels are evaluated in
+#: every product
+NODE_OPERATOR_MIN_ROWS = 4096
+#: most memory for the node matrix of a rank
+NODE_OPERATOR_MAX_BYTES = 16 << 30
+
+
 def segment_layout(num_row_blocks: int, world_size: int) -> tuple[int, int, int]:
     """``(row blocks per segment, segments, segments per rank)``: at most ``MAX_SEGMENTS`` segments
     of equal length (the last may be shorter), dealt out in equal counts (the last ranks may get
@@ -214,13 +221,21 @@ class ShardedOperator:
         """Operator backed by ``ops.matmul_rows`` (sum over the batch of ``params`` if batched);
         ``start`` / ``end`` are one band ``(R,)`` shared by all components.
 
+        From ``NODE_OPERATOR_MIN_ROWS`` points, where the points' blocks are short enough against what
+        the kernel varies over (sorted points; bands aligned to blocks), the operator is laid out as a
+        matrix between the nodes of blockwise interpolation (``km_node_operator_build_f32``), summed over
+        all components, once; a product then reads it instead of evaluating kernels.
+
         ``phases``: for a sum of spectral components, write the per-point phase vectors once now
         (``ops.prepare_sum_phases``: about ``16 B n`` bytes for ``B`` components) so that every product
-        of the solve copies them instead of evaluating them again; default: yes, unless the
-        environment variable ``KM_SUM_PHASES`` is ``0``."""
+        of the solve copies them instead of evaluating them again (``True``), or evaluate them in every
+        product (``False``; also with the environment variable ``KM_SUM_PHASES`` ``0``); both evaluate the
+        kernels of every product directly.  Default: the node operator where it can be had, else
+        ``True``."""
         import os
 
-        from . import ops
+        from . import _C, ops
+        from ._lib import KERNEL_TYPES
 
         n = x.shape[-1]
         batched = params.dim() > 1
@@ -229,12 +244,14 @@ class ShardedOperator:
         sb = start.expand(*B, start.shape[-1]) if batched else start
         eb = end.expand(*B, end.shape[-1]) if batched else end
 
+        direct = phases is not None or os.environ.get("KM_SUM_PHASES") is not None
         if phases is None:
             phases = os.environ.get("KM_SUM_PHASES", "1") != "0"
         phase_ws = None  # set below, once this rank's rows and columns are known
+        nodes = None  # likewise
         prepared: dict = {}  # (buffers, window) -> launch with all arguments already marshalled
 
-        def matvec_rows(v: Tensor, rb_begin: int, rb_count: int, out: Tensor) -> None:
+        def rows_product(v: Tensor, rb_begin: int, rb_count: int, out: Tensor):
             # a solve calls this with the same two buffers every iteration: validate and marshal once
             key = (v.data_ptr(), tuple(v.shape), tuple(v.stride()), out.data_ptr(), tuple(out.shape), rb_begin, rb_count)
             call = prepared.get(key)
@@ -247,7 +264,13 @@ class ShardedOperator:
                 if len(prepared) >= 8:
                     prepared.clear()
                 prepared[key] = call
-            call()
+            return call
+
+        def matvec_rows(v: Tensor, rb_begin: int, rb_count: int, out: Tensor) -> None:
+            if nodes is not None and (rb_begin, rb_count) == (begin, count) and v.is_contiguous() and out.is_contiguous():
+                nodes.matvec(v, out)
+            else:
+                rows_product(v, rb_begin, rb_count, out)()
 
         import torch.distributed as dist
 
@@ -255,22 +278,23 @@ class ShardedOperator:
         rank = dist.get_rank(group) if world > 1 else 0
         R = -(-n // BLOCK_SIZE)
         begin, count = row_block_window(R, rank, world)
-        # the columns this rank's row blocks read, and a checksum of the whole band (one host
-        # synchronisation, at set-up only)
-        s64, e64 = start.reshape(-1)[:R].to(torch.int64), end.reshape(-1)[:R].to(torch.int64)
-        weights = torch.arange(1, R + 1, device=start.device, dtype=torch.int64)
-        checksum = ((s64 * weights).sum() * 31 + (e64 * weights).sum()) % (2**61 - 1)
-        if count > 0:
-            mine = torch.stack([s64[begin:begin + count].min(), e64[begin:begin + count].max(), checksum])
-        else:
-            mine = torch.stack([torch.zeros((), dtype=torch.int64, device=start.device)] * 2 + [checksum])
-        lo, hi, checksum = (int(v) for v in mine.tolist())
-        if phases and batched and count > 0:
+        # the columns this rank's row blocks read, a checksum of the whole band, and how many nodes
+        # per block and blocks per band a node operator would have (one host synchronisation, at
+        # set-up only)
+        plan = _C.NodeOperator(KERNEL_TYPES.get(kernel_type, -1), x, params, start.reshape(-1)[:R], end.reshape(-1)[:R], begin, count)
+        lo, hi, checksum, node_count, widest = (int(v) for v in plan.plan().tolist())
+        if (not direct and n >= NODE_OPERATOR_MIN_ROWS and node_count > 0
+                and 4 * count * widest * node_count**2 <= NODE_OPERATOR_MAX_BYTES):
+            plan.build(lo, hi, node_count, widest)
+            nodes = plan
+        elif phases and batched and count > 0:
             phase_ws = ops.prepare_sum_phases(kernel_type, x, x, params, rows=(begin * BLOCK_SIZE, min(n, (begin + count) * BLOCK_SIZE)),
                                               cols=(max(0, min(lo, n)), max(0, min(hi, n))))
         op = cls(n, sigma2, matvec_rows, group=group, device=x.device, col_range=(lo, hi) if count > 0 else (0, 0),
                  band_checksum=checksum, mode=mode)
         op.phase_workspace = phase_ws  # (None: the products evaluate the phase vectors themselves)
+        op.node_operator = nodes
+        op.rows_product = rows_product
         return op
 
     # ---- the operator applied to a full vector (tests, diagnostics)
@@ -384,6 +408,26 @@ class CGSolver:
         if self.op.world > 1:
             self.op.dist.all_gather_into_tensor(full, mine, group=self.op.group)
 
+    def run(self, iterations: int) -> Tensor:
+        """``iterations`` steps; on one GPU they are launched without the interpreter in between."""
+        op = self.op
+        if self.it + iterations > self.max_iterations:
+            raise RuntimeError(f"more than max_iterations = {self.max_iterations} steps")
+        if iterations > 0 and op.world == 1 and op.rows > 0 and self.mark is None and isinstance(self.V, CudaVectorOps) and \
+                getattr(op, "rows_product", None) is not None:
+            from . import _C
+
+            nodes = op.node_operator
+            rows = None if nodes is not None else op.rows_product(self.p[: op.n], op.begin, op.count, self.kp[op.row0: op.row1])
+            state = _C.CgState(self.x, self.r, self.p, self.kp, self.bp, self.rs, self.ynorm, self.history, self.alphas, self.betas,
+                               self.send1, self.send2, op.n, self.k, op.count, op.seg_blocks, op.segs_per_rank, op.sigma2)
+            _C.cg_run(state, nodes, rows, self.it, iterations)
+            self.it += iterations
+        else:
+            for _ in range(iterations):
+                self.step()
+        return self.history[self.it]
+
     def step(self) -> Tensor:
         """One iteration; returns the relative residual norms ``(k,)`` (a view of the history)."""
         op, V, k = self.op, self.V, self.k
@@ -451,10 +495,14 @@ def conjugate_gradient(op: ShardedOperator, y: Tensor, iterations: int, tol: flo
     ``tol``, which costs one host synchronisation per iteration and is off for ``tol == 0``)."""
     solver = CGSolver(op, y, max_iterations=max(iterations, 1))
     done = 0
-    for _ in range(iterations):
-        res = solver.step()
-        done += 1
-        if tol > 0 and bool((res <= tol).all()):
-            break
+    if tol <= 0:
+        solver.run(iterations)
+        done = iterations
+    else:
+        for _ in range(iterations):
+            res = solver.step()
+            done += 1
+            if bool((res <= tol).all()):
+                break
     return CGResult(solver.solution(), solver.residual_norms().clone(), done, solver.alphas[:done].clone(),
                     solver.betas[:done].clone(), solver.ynorm.clone())

@@ -20,69 +20,9 @@
 // Rows a rank does not own but needs as right-hand side of its next product (the band's halo)
 // are updated redundantly by that rank: it receives the owner's q rows and applies the same
 // alpha and beta, so p never has to be exchanged itself.
-#include "km_common.cuh"
+#include "km_cg.cuh"
 
 namespace km {
-
-constexpr int CG_THREADS = 128;  // = rows of a row block
-
-// Adds `v[c]`, c < KC, over the 128 threads of the CTA in a fixed order; the totals arrive in
-// thread c (c < KC) of warp 0 as the return value.
-template <int KC>
-__device__ __forceinline__ float cg_block_reduce(float (&v)[KC], float (*warp_part)[32]) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int c = 0; c < KC; c++) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v[c] += __shfl_xor_sync(0xffffffffu, v[c], o);
-    }
-    if (lane == 0) {
-#pragma unroll
-        for (int c = 0; c < KC; c++) warp_part[warp][c] = v[c];
-    }
-    __syncthreads();
-    float total = 0.0f;
-    if (warp == 0 && lane < KC) total = (warp_part[0][lane] + warp_part[1][lane]) + (warp_part[2][lane] + warp_part[3][lane]);
-    __syncthreads();
-    return total;
-}
-
-// k columns of one row, starting at column c0: 16-byte accesses when `vec`.
-template <int KC>
-__device__ __forceinline__ void cg_load_row(const float *row, int c0, int k, bool vec, float (&v)[KC]) {
-    if (KC >= 4 && vec && c0 + KC <= k) {
-#pragma unroll
-        for (int c = 0; c < KC; c += 4) {
-            const float4 t = *reinterpret_cast<const float4 *>(row + c0 + c);
-            v[c] = t.x, v[c + 1] = t.y, v[c + 2] = t.z, v[c + 3] = t.w;
-        }
-    } else {
-#pragma unroll
-        for (int c = 0; c < KC; c++) v[c] = c0 + c < k ? row[c0 + c] : 0.0f;
-    }
-}
-template <int KC>
-__device__ __forceinline__ void cg_store_row(float *row, int c0, int k, bool vec, const float (&v)[KC]) {
-    if (KC >= 4 && vec && c0 + KC <= k) {
-#pragma unroll
-        for (int c = 0; c < KC; c += 4) *reinterpret_cast<float4 *>(row + c0 + c) = make_float4(v[c], v[c + 1], v[c + 2], v[c + 3]);
-    } else {
-#pragma unroll
-        for (int c = 0; c < KC; c++)
-            if (c0 + c < k) row[c0 + c] = v[c];
-    }
-}
-
-// Sum of the gathered segment sums, in slot order: base[rank * rank_stride_bytes + slot * k + c].
-__device__ __forceinline__ double cg_total(const unsigned char *base, int64_t rank_stride_bytes, int ranks, int slots,
-                                           int64_t k, int c) {
-    double t = 0.0;
-    for (int rk = 0; rk < ranks; rk++) {
-        const double *seg = reinterpret_cast<const double *>(base + rk * rank_stride_bytes);
-        for (int s = 0; s < slots; s++) t += seg[s * k + c];
-    }
-    return t;
-}
 
 struct CgDotsArgs {
     int64_t k, row0, row1;       // rows [row0, row1) of this rank (row0 a multiple of 128)
@@ -160,9 +100,7 @@ struct CgUpdateArgs {
     const float *q_own;             // q of own rows, indexed by global row
     const float *q_below, *q_above; // q(row) = q_below[(row - below_origin) * k + c] for row < row0, etc.
     int64_t below_origin, above_origin;
-    const unsigned char *seg_base;  // gathered segment sums (p . q for update_xr, r . r for update_p)
-    int64_t seg_rank_stride;        // bytes
-    int seg_ranks, seg_slots;
+    CgTotals totals;                // gathered segment sums (p . q for update_xr, r . r for update_p)
     const float *rs_in;             // [k] r . r of the current residual
     float *rs_out;                  // update_p: [k] r . r of the new residual
     float *history;                 // update_p: [k] sqrt(rs_new) / ynorm
@@ -185,7 +123,7 @@ __global__ void __launch_bounds__(CG_THREADS) cg_update_xr_kernel(const CgUpdate
         __syncthreads();
         if (threadIdx.x < KC && c0 + threadIdx.x < k) {
             const int c = c0 + threadIdx.x;
-            const double pq = cg_total(g.seg_base, g.seg_rank_stride, g.seg_ranks, g.seg_slots, k, c);
+            const double pq = cg_total(g.totals, k, c);
             alpha_s[threadIdx.x] = g.rs_in[c] / fmaxf((float)pq, g.tiny);
             if (blockIdx.x == 0 && g.coeff_out != nullptr) g.coeff_out[c] = alpha_s[threadIdx.x];
         }
@@ -242,7 +180,7 @@ __global__ void __launch_bounds__(CG_THREADS) cg_update_p_kernel(const CgUpdateA
         __syncthreads();
         if (threadIdx.x < KC && c0 + threadIdx.x < k) {
             const int c = c0 + threadIdx.x;
-            const float rs_new = (float)cg_total(g.seg_base, g.seg_rank_stride, g.seg_ranks, g.seg_slots, k, c);
+            const float rs_new = (float)cg_total(g.totals, k, c);
             beta_s[threadIdx.x] = rs_new / fmaxf(g.rs_in[c], g.tiny);
             if (blockIdx.x == 0) {
                 if (g.coeff_out != nullptr) g.coeff_out[c] = beta_s[threadIdx.x];
@@ -272,10 +210,86 @@ __global__ void __launch_bounds__(CG_THREADS) cg_update_p_kernel(const CgUpdateA
 __global__ void cg_init_scalars_kernel(int64_t k, const unsigned char *seg_base, int64_t seg_rank_stride, int seg_ranks,
                                        int seg_slots, float *rs, float *ynorm, float tiny) {
     for (int64_t c = threadIdx.x; c < k; c += blockDim.x) {
-        const float t = (float)cg_total(seg_base, seg_rank_stride, seg_ranks, seg_slots, k, (int)c);
+        const float t = (float)cg_total(CgTotals{seg_base, seg_rank_stride, seg_ranks, seg_slots}, k, (int)c);
         rs[c] = t;
         ynorm[c] = fmaxf(sqrtf(t), tiny);
     }
+}
+
+// z_c^T log(A) z_c from the coefficients of a CG run A v = z_c from v = 0 (km_cg_log_forms_f32): with T the
+// Lanczos tridiagonal they are the entries of, |z_c|^2 e_1^T log(T) e_1.
+//
+// No eigenvalues: log x = int_0^inf 1 / (1 + s) - 1 / (x + s) ds, so e_1^T log(T) e_1 is the same integral over the
+// first entry of (T + s)^-1, which is a continued fraction of T's entries -- m divisions, all of its
+// denominators positive for a positive definite T.  With s = e^u the integrand is analytic in the
+// strip |Im u| < pi and decays like e^-|u| (below the smallest eigenvalue and above the largest), so
+// the trapezoid rule with step 0.36 is exact to e^(-2 pi^2 / 0.36) = 1e-24 and 256 points, one per thread, reach from e^-62
+// to e^30 times the largest eigenvalue.  One CTA per column: 100 steps of 15 columns take 15 us, where the
+// eigenvalues of 15 matrices on the host took 40 ms with the copies and the assembly of the matrices.
+constexpr int LOG_POINTS = 256;
+constexpr double LOG_STEP = 0.36, LOG_FIRST = -62.0;
+
+__global__ void __launch_bounds__(LOG_POINTS) cg_log_forms_kernel(int64_t m, int64_t k, const float *alphas, const float *betas,
+                                                                  const float *residuals, const float *z_norm2, float converged,
+                                                                  double *out) {
+    __shared__ double red[LOG_POINTS];
+    __shared__ int s_steps;
+    constexpr int CHUNK = 512;
+    __shared__ double diag[CHUNK], off2[CHUNK];  // d_j and e_j^2 of a chunk of rows, last rows first
+    const int64_t c = blockIdx.x;
+    const int t = threadIdx.x;
+    if (t == 0) s_steps = (int)m;
+    __syncthreads();
+    for (int64_t j = 1 + t; j <= m; j += LOG_POINTS) {
+        const float res = residuals[j * k + c];
+        if (!(fabsf(res) < INFINITY) || res <= converged) atomicMin(&s_steps, (int)j);
+    }
+    __syncthreads();
+    const int steps = max(1, s_steps);
+    const auto entry = [&](int j, double &d, double &e2) {
+        const double a = (double)alphas[j * k + c];
+        d = 1.0 / a;
+        if (j > 0) d += (double)betas[(j - 1) * k + c] / (double)alphas[(j - 1) * k + c];
+        e2 = j + 1 < steps ? (double)betas[j * k + c] / (a * a) : 0.0;
+    };
+    // an upper bound on the eigenvalues (Gershgorin)
+    double top = 0.0;
+    for (int j = t; j < steps; j += LOG_POINTS) {
+        double d, e2, d0, b2 = 0.0;
+        entry(j, d, e2);
+        if (j > 0) entry(j - 1, d0, b2);
+        top = fmax(top, d + sqrt(e2) + sqrt(b2));
+    }
+    red[t] = top;
+    __syncthreads();
+    for (int o = LOG_POINTS / 2; o > 0; o >>= 1) {
+        if (t < o) red[t] = fmax(red[t], red[t + o]);
+        __syncthreads();
+    }
+    top = red[0];
+    const double s = exp(LOG_FIRST + LOG_STEP * t), inv = 1.0 / top;
+    double f = 0.0;  // the fraction from row j on: d_j + s - e_j^2 / f
+    for (int j1 = steps; j1 > 0; j1 -= CHUNK) {
+        const int j0 = max(0, j1 - CHUNK);
+        __syncthreads();
+        for (int j = j0 + t; j < j1; j += LOG_POINTS) {
+            double d, e2;
+            entry(j, d, e2);
+            diag[j - j0] = d * inv, off2[j - j0] = e2 * inv * inv;
+        }
+        __syncthreads();
+        for (int j = j1 - 1; j >= j0; j--) {
+            const double next = diag[j - j0] + s;
+            f = j == steps - 1 ? next : next - off2[j - j0] / f;
+        }
+    }
+    red[t] = LOG_STEP * s * (1.0 / (1.0 + s) - 1.0 / f);
+    __syncthreads();
+    for (int o = LOG_POINTS / 2; o > 0; o >>= 1) {
+        if (t < o) red[t] += red[t + o];
+        __syncthreads();
+    }
+    if (t == 0) out[c] = (double)z_norm2[c] * (log(top) + red[0]);
 }
 
 static int cg_grid(int64_t blocks) {
@@ -388,8 +402,8 @@ extern "C" int km_cg_update_xr_f32(int64_t k, float *x, float *r, const float *p
     CgUpdateArgs g{};
     g.k = k, g.row0 = row0, g.row1 = row1, g.lo = lo, g.hi = hi, g.x = x, g.r = r, g.p = const_cast<float *>(p);
     g.q_own = q_own, g.q_below = q_below, g.q_above = q_above, g.below_origin = below_origin, g.above_origin = above_origin;
-    g.seg_base = static_cast<const unsigned char *>(pq_seg_sums), g.seg_rank_stride = seg_rank_stride_bytes;
-    g.seg_ranks = seg_ranks, g.seg_slots = seg_slots, g.rs_in = rs, g.block_partials = block_partials;
+    g.totals = {static_cast<const unsigned char *>(pq_seg_sums), seg_rank_stride_bytes, seg_ranks, seg_slots};
+    g.rs_in = rs, g.block_partials = block_partials;
     g.coeff_out = alpha_row;
     g.tiny = 1.17549435e-38f;
     g.vec = cg_vec_ok(k, {x, r, p, q_own, q_below, q_above}) ? 1 : 0;
@@ -413,8 +427,8 @@ extern "C" int km_cg_update_p_f32(int64_t k, float *p, const float *r, int64_t l
                KM_ERR_INVALID_ARGUMENT, "km_cg_update_p_f32: bad arguments (rs_old and rs_new must differ)");
     CgUpdateArgs g{};
     g.k = k, g.lo = lo, g.hi = hi, g.p = p, g.r = const_cast<float *>(r);
-    g.seg_base = static_cast<const unsigned char *>(rr_seg_sums), g.seg_rank_stride = seg_rank_stride_bytes;
-    g.seg_ranks = seg_ranks, g.seg_slots = seg_slots, g.rs_in = rs_old, g.rs_out = rs_new, g.history = history_row;
+    g.totals = {static_cast<const unsigned char *>(rr_seg_sums), seg_rank_stride_bytes, seg_ranks, seg_slots};
+    g.rs_in = rs_old, g.rs_out = rs_new, g.history = history_row;
     g.ynorm = ynorm, g.tiny = 1.17549435e-38f, g.coeff_out = beta_row;
     g.vec = cg_vec_ok(k, {p, r}) ? 1 : 0;
     const int64_t blocks = std::max<int64_t>(1, ceil_div(hi, KM_BLOCK_SIZE) - lo / KM_BLOCK_SIZE);  // CTA 0 always runs
@@ -424,4 +438,15 @@ extern "C" int km_cg_update_p_f32(int64_t k, float *p, const float *r, int64_t l
         KM_CHECK_LAUNCH("km_cg_update_p_f32 launch");
         return KM_OK;
     });
+}
+
+extern "C" int km_cg_log_forms_f32(int64_t iterations, int64_t k, const float *alphas, const float *betas, const float *residual_norms,
+                                   const float *z_norm2, float converged, double *out, void *stream) {
+    using namespace km;
+    KM_REQUIRE(iterations >= 1 && iterations <= 1 << 24 && k >= 1 && k <= 0x7fffffffLL && alphas && betas && residual_norms && z_norm2 && out,
+               KM_ERR_INVALID_ARGUMENT, "km_cg_log_forms_f32: bad arguments");
+    cg_log_forms_kernel<<<(unsigned)k, LOG_POINTS, 0, static_cast<cudaStream_t>(stream)>>>(iterations, k, alphas, betas, residual_norms,
+                                                                                          z_norm2, converged, out);
+    KM_CHECK_LAUNCH("km_cg_log_forms_f32 launch");
+    return KM_OK;
 }

@@ -1,0 +1,650 @@
+// The operator of a CG solve by blockwise interpolation (km_nodes.cuh has the method and its bound).
+//
+// A solve applies ONE operator many times, so what the products of km_nodes.cu form on every call is
+// laid out once here: P nodes per block of 128 points (one interval length for all blocks), the
+// Lagrange matrices, and the kernel matrix between the nodes,
+//     G[r][c - c_lo(r)][q][p] = sum_b scale_b kappa_b(xi_{r,p} - xi_{c,q}),
+// summed over all components of the operator: whatever their number, a product then reads
+// P^2 values per pair of blocks instead of evaluating 128^2 x components.  With P = 14 that is 0.56 GB for
+// 4 million points and a band of 22 blocks; a product is 85 us of HBM time for it, 135 us for the vectors
+// and Lagrange matrices, where the sum of 64 components took 11 ms on the tensor cores.
+//
+// An iteration is: p = r + beta p and Lambda^T p (node_compress_kernel), G times that, Lambda times the
+// result, q = K p + sigma^2 p and p . q (node_product_kernel), then the updates of x and r (km_cg.cu).
+#include <type_traits>
+
+#include "km_cg.cuh"
+#include "km_nodes.cuh"
+
+namespace km {
+
+constexpr int NODE_OP_MAX = 32;  // most nodes per block of an operator
+
+struct NodePlan {
+    long long lo, hi;        // columns read by the row blocks of the window
+    long long checksum;      // of the whole band
+    long long P;             // nodes per block; 0: not this way (band not aligned, or too many nodes)
+    long long max_blocks;    // widest band of the window, in blocks
+    int max_h_bits, done, bad, width;
+    int lo_bits, hi_bits;
+};
+
+struct NodePlanArgs {
+    Batch batch;
+    int64_t n, R, rb0, rb1;
+    const float *x;
+    int64_t xs;
+    View<const float> params;
+    const int *start, *end;
+    float *centre;
+    NodePlan *plan;
+};
+
+template <int KT>
+__global__ void __launch_bounds__(256) node_plan_kernel(const NodePlanArgs a) {
+    const int lane = threadIdx.x & 31;
+    float longest = 0.0f;
+    int bad = 0;
+    for (int64_t v = blockIdx.x * 8LL + (threadIdx.x >> 5); v < a.R; v += gridDim.x * 8LL) {
+        float lo = INFINITY, hi = -INFINITY;
+        bool nan = false;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int64_t row = v * KM_BLOCK_SIZE + lane + 32 * i;
+            if (row < a.n) {
+                const float e = a.x[row * a.xs];
+                lo = fminf(lo, e), hi = fmaxf(hi, e);
+                nan = nan || !(fabsf(e) < INFINITY);
+            }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+            hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+        }
+        const float c = 0.5f * lo + 0.5f * hi, h = fmaxf(fmaxf(hi - c, c - lo), NODES_MIN_H);
+        bad |= nan || !(h < INFINITY);
+        longest = fmaxf(longest, h);
+        if (lane == 0) a.centre[v] = c;
+    }
+    int first = INT_MAX, last = 0, width = 0;
+    unsigned long long sum = 0;
+    for (int64_t r = blockIdx.x * 256LL + threadIdx.x; r < a.R; r += gridDim.x * 256LL) {
+        const int s = a.start[r], e = a.end[r];
+        sum += (unsigned long long)(r + 1) * (31ull * (unsigned long long)s + (unsigned long long)e);
+        if (r >= a.rb0 && r < a.rb1) first = min(first, s), last = max(last, e);
+        if (s >= e) continue;
+        bad |= s < 0 || s % KM_BLOCK_SIZE != 0 || (e < a.n && e % KM_BLOCK_SIZE != 0);
+        if (r >= a.rb0 && r < a.rb1) width = max(width, (int)((min((int64_t)e, a.n) - s + KM_BLOCK_SIZE - 1) / KM_BLOCK_SIZE));
+    }
+    first = __reduce_min_sync(0xffffffffu, first);
+    last = __reduce_max_sync(0xffffffffu, last);
+    width = __reduce_max_sync(0xffffffffu, width);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    __shared__ int s_last, s_p;
+    bad = __syncthreads_or(bad);
+    if (lane == 0) {
+        atomicMax(&a.plan->max_h_bits, __float_as_int(longest));
+        atomicMax(&a.plan->lo_bits, INT_MAX - first);
+        atomicMax(&a.plan->hi_bits, last);
+        atomicMax(&a.plan->width, width);
+        atomicAdd(reinterpret_cast<unsigned long long *>(&a.plan->checksum), sum);
+        __threadfence();
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        if (bad) a.plan->bad = 1;
+        __threadfence();
+        s_last = atomicAdd(&a.plan->done, 1) == (int)gridDim.x - 1;
+        s_p = 0;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    volatile NodePlan *plan = a.plan;
+    const float h = __int_as_float(plan->max_h_bits);
+    for (int64_t b = threadIdx.x >> 5; b < a.batch.count; b += 8) {
+        const int p = nodes_needed<KT>(batch_ptr(a.params, decompose(a.batch, b)), a.params.s0, h, lane);
+        if (lane == 0) atomicMax(&s_p, p);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const int P = max(4, (min(s_p, 4096) + 1) & ~1);
+        plan->lo = a.rb1 > a.rb0 ? INT_MAX - plan->lo_bits : 0;
+        plan->hi = a.rb1 > a.rb0 ? plan->hi_bits : 0;
+        plan->checksum = plan->checksum & ((1ll << 61) - 1);
+        plan->P = (plan->bad == 0 && P <= NODE_OP_MAX) ? P : 0;
+        plan->max_blocks = plan->width;
+    }
+}
+
+struct NodeOpArgs {
+    Batch batch;
+    int64_t n, R, rb0, rb1;
+    const float *x;
+    int64_t xs;
+    View<const float> params;
+    const int *start, *end;
+    const NodePlan *plan;
+    const float *centre;
+    float *lambda;  // [R][P][128]
+    float *G;       // [rb1 - rb0][max_blocks][P (column node)][P (row node)]
+    int P, max_blocks;
+};
+
+// Lagrange matrix of every block: thread = row.
+__global__ void __launch_bounds__(128) node_lambda_kernel(const NodeOpArgs a) {
+    __shared__ float delta[NODE_OP_MAX], weight[NODE_OP_MAX];
+    const int t = threadIdx.x, P = a.P;
+    const float h = __int_as_float(a.plan->max_h_bits), inv_h = 1.0f / h;
+    if (t < P) delta[t] = node_offset(h, t, P);
+    __syncthreads();
+    if (t < P) weight[t] = node_weight(delta, h, t, P);
+    __syncthreads();
+    for (int64_t v = blockIdx.x; v < a.R; v += gridDim.x) {
+        const int64_t row = v * KM_BLOCK_SIZE + t;
+        float *out = a.lambda + v * P * KM_BLOCK_SIZE + t;
+        if (row >= a.n) {
+            for (int q = 0; q < P; q++) out[q * KM_BLOCK_SIZE] = 0.0f;
+            continue;
+        }
+        const float d = a.x[row * a.xs] - a.centre[v];
+        float sum = 0.0f;
+        int hit = -1;
+#pragma unroll 4
+        for (int q = 0; q < P; q++) {
+            const float e = (d - delta[q]) * inv_h;
+            if (e == 0.0f) hit = q;
+            sum += __fdividef(weight[q], e);
+        }
+        const float inv = 1.0f / sum;
+#pragma unroll 4
+        for (int q = 0; q < P; q++) {
+            const float e = (d - delta[q]) * inv_h;
+            out[q * KM_BLOCK_SIZE] = hit >= 0 ? (q == hit ? 1.0f : 0.0f) : __fdividef(weight[q], e) * inv;
+        }
+    }
+}
+
+// G: a warp per (row block, GB_PAIRS column blocks).  A lane owns row node p = lane mod 16 (or 32) and 8
+// column nodes at a time of each pair of blocks; the halves of a warp take alternate groups of 8 where 16 lanes
+// hold all rows.  Components are the outer loop: the phase factors of the nodes are the same for
+// all pairs and lie in shared memory, all that changes from pair to pair is the phase of the centres'
+// distance (reduced in fp64), so a component costs 4 FMAs per pair to rotate the row's factors and 2 per
+// entry; where all spectral components share a lengthscale the envelope multiplies the finished sum.
+constexpr int GB_PAIRS = 6;
+constexpr int GB_COMPS = 32;  // components per chunk
+
+template <int KT>
+__global__ void __launch_bounds__(128) node_matrix_kernel(const NodeOpArgs a) {
+    using Fn = KernelFn<KT>;
+    constexpr bool SPECTRAL = KT == KM_KERNEL_SPECTRAL;
+    __shared__ float delta[NODE_OP_MAX + 8];
+    __shared__ __align__(16) float2 node_phase[GB_COMPS][NODE_OP_MAX + 8];  // cos, sin of W delta
+    __shared__ float2 pair_phase[4][GB_PAIRS][GB_COMPS];
+    __shared__ float scales[GB_COMPS];
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5, P = a.P;
+    const float h = __int_as_float(a.plan->max_h_bits);
+    if (t < NODE_OP_MAX + 8) delta[t] = t < P ? node_offset(h, t, P) : 0.0f;
+    const int64_t groups = (a.max_blocks + GB_PAIRS - 1) / GB_PAIRS;
+    const int64_t item = blockIdx.x * 4LL + warp;
+    const bool live = item < (a.rb1 - a.rb0) * groups;
+    const int64_t r = a.rb0 + (live ? item / groups : 0);
+    const int s = a.start[r], e = a.end[r];
+    const int c_lo = s < e ? s / KM_BLOCK_SIZE : 0;
+    const int blocks = s < e ? (int)((min((int64_t)e, a.n) + KM_BLOCK_SIZE - 1) / KM_BLOCK_SIZE) - c_lo : 0;
+    const int first = (int)(item % groups) * GB_PAIRS, pairs = live ? max(0, min(GB_PAIRS, blocks - first)) : 0;
+    __syncthreads();
+    const int width = P <= 16 ? 16 : 32, p = min(lane % width, P - 1);
+    const float dp = delta[p], centre = a.centre[r];
+    float D[GB_PAIRS];
+#pragma unroll
+    for (int i = 0; i < GB_PAIRS; i++) D[i] = i < pairs ? centre - a.centre[c_lo + first + i] : 0.0f;
+    bool one_ell = SPECTRAL;
+    if constexpr (SPECTRAL)
+        for (int64_t b = lane; b < a.batch.count; b += 32) one_ell = one_ell && batch_ptr(a.params, decompose(a.batch, b))[0] == a.params.data[0];
+    one_ell = __all_sync(0xffffffffu, one_ell);
+
+    const int q_step = 8 * (32 / width);
+    for (int round = 0; round * q_step < P; round++) {
+        const int q0 = round * q_step + (lane / width) * 8;  // (may lie past P in one half: computed, not stored)
+        const int qs = min(q0, NODE_OP_MAX);
+        float acc[GB_PAIRS][8];
+#pragma unroll
+        for (int i = 0; i < GB_PAIRS; i++)
+#pragma unroll
+            for (int j = 0; j < 8; j++) acc[i][j] = 0.0f;
+        for (int64_t b0 = 0; b0 < a.batch.count; b0 += GB_COMPS) {
+            const int comps = (int)min((int64_t)GB_COMPS, a.batch.count - b0);
+            __syncthreads();
+            for (int i = t; i < comps * P; i += 128) {
+                const int b = i / P, q = i % P;
+                Fn fn;
+                fn.init(batch_ptr(a.params, decompose(a.batch, b0 + b)), a.params.s0);
+                float c = 1.0f, sn = 0.0f;
+                if constexpr (Fn::PHASE) sincospif(fn.phase_half_turns() * delta[q], &sn, &c);
+                node_phase[b][q] = make_float2(c, sn);
+                if (q == 0) scales[b] = fn.scale;
+            }
+            if constexpr (Fn::PHASE) {
+                if (lane < comps) {
+                    Fn fn;
+                    fn.init(batch_ptr(a.params, decompose(a.batch, b0 + lane)), a.params.s0);
+#pragma unroll
+                    for (int i = 0; i < GB_PAIRS; i++) {
+                        const double turns = (double)fn.phase_half_turns() * (double)D[i];
+                        float c, sn;
+                        sincospif((float)(turns - 2.0 * rint(0.5 * turns)), &sn, &c);
+                        pair_phase[warp][i][lane] = make_float2(c, sn);
+                    }
+                }
+            }
+            __syncthreads();
+            for (int b = 0; b < comps; b++) {
+                const float scale = scales[b];
+                const float2 row_phase = node_phase[b][p];
+                float2 col[8];
+#pragma unroll
+                for (int j = 0; j < 8; j++) col[j] = node_phase[b][qs + j];
+                if (SPECTRAL && one_ell) {
+#pragma unroll
+                    for (int i = 0; i < GB_PAIRS; i++) {
+                        if (i >= pairs) break;
+                        const float2 ph = pair_phase[warp][i][b];
+                        const float rc = scale * (ph.x * row_phase.x - ph.y * row_phase.y), rs = scale * (ph.y * row_phase.x + ph.x * row_phase.y);
+#pragma unroll
+                        for (int j = 0; j < 8; j++) acc[i][j] = fmaf(rc, col[j].x, fmaf(rs, col[j].y, acc[i][j]));
+                    }
+                } else {
+                    Fn fn;
+                    fn.init(batch_ptr(a.params, decompose(a.batch, b0 + b)), a.params.s0);
+#pragma unroll
+                    for (int i = 0; i < GB_PAIRS; i++) {
+                        if (i >= pairs) break;
+                        float rc = 1.0f, rs = 0.0f;
+                        if constexpr (Fn::PHASE) {
+                            const float2 ph = pair_phase[warp][i][b];
+                            rc = ph.x * row_phase.x - ph.y * row_phase.y, rs = ph.y * row_phase.x + ph.x * row_phase.y;
+                        }
+                        const float y = D[i] + dp;
+#pragma unroll
+                        for (int j = 0; j < 8; j += 2) {
+                            f32x2 cs = 0ull;
+                            if constexpr (Fn::PHASE) cs = pack2(rc * col[j].x + rs * col[j].y, rc * col[j + 1].x + rs * col[j + 1].y);
+                            float k0, k1;
+                            unpack2(fn.unscaled2_ph(pack2(y - delta[qs + j], y - delta[qs + j + 1]), cs, 0ull), k0, k1);
+                            acc[i][j] = fmaf(scale, k0, acc[i][j]);
+                            acc[i][j + 1] = fmaf(scale, k1, acc[i][j + 1]);
+                        }
+                    }
+                }
+            }
+        }
+        if (lane % width < P) {
+            const float ell = a.params.data[0], c0 = -(0.5f / (ell * ell)) * KM_LOG2E_F;
+#pragma unroll
+            for (int i = 0; i < GB_PAIRS; i++) {
+                if (i >= pairs) break;
+                float *out = a.G + ((r - a.rb0) * a.max_blocks + first + i) * P * P + p;
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    if (q0 + j >= P) break;
+                    float v = acc[i][j];
+                    if (SPECTRAL && one_ell) {
+                        const float tau = (D[i] + dp) - delta[q0 + j];
+                        v *= exp2f(c0 * tau * tau);
+                    }
+                    out[(q0 + j) * P] = v;
+                }
+            }
+        }
+    }
+}
+
+struct NodeVectorArgs {
+    int64_t n, k, kq;
+    int P;
+    int64_t blk0, blk1;   // row blocks
+    const float *lambda;  // [R][P][128]
+    float *v;             // (n, k): the vector; updated first (v = r + beta v) where r is not null
+    const float *r;
+    float *nodes;         // [R][P][kq]
+    // beta and the bookkeeping of an update (as cg_update_p_kernel)
+    CgTotals totals;
+    const float *rs_in;
+    float *rs_out, *history, *coeff_out;
+    const float *ynorm;
+    float tiny;
+    int vec;
+};
+
+// [v = r + beta v on whole blocks, and] nodes = Lambda^T v.  One CTA per row block at a time: thread =
+// row for the update, whose result stays in shared memory for the second part; there a warp adds up
+// its own 32 rows, a lane owning 4 nodes x 4 columns, and the warps' sums are added in order.
+constexpr int NV_COLS = 16;
+template <int KC>
+__global__ void __launch_bounds__(128) node_compress_kernel(const NodeVectorArgs g) {
+    __shared__ __align__(16) float vs[KM_BLOCK_SIZE][NV_COLS];
+    __shared__ float ls[NODE_OP_MAX][KM_BLOCK_SIZE + 1];
+    __shared__ __align__(16) float part[4][4][32][4];
+    __shared__ float beta_s[NV_COLS];
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5, P = g.P;
+    const int64_t k = g.k;
+    for (int c0 = 0; c0 < g.kq; c0 += KC < 4 ? 4 : KC) {
+        if (g.r != nullptr) {
+            __syncthreads();
+            if (t < KC && c0 + t < k) {
+                const int c = c0 + t;
+                const float rs_new = (float)cg_total(g.totals, k, c);
+                beta_s[t] = rs_new / fmaxf(g.rs_in[c], g.tiny);
+                if (blockIdx.x == 0) {
+                    if (g.coeff_out != nullptr) g.coeff_out[c] = beta_s[t];
+                    g.rs_out[c] = rs_new;
+                    if (g.history != nullptr) g.history[c] = sqrtf(rs_new) / g.ynorm[c];
+                }
+            }
+            __syncthreads();
+        }
+        for (int64_t blk = g.blk0 + blockIdx.x; blk < g.blk1; blk += gridDim.x) {
+            const int64_t row = blk * KM_BLOCK_SIZE + t;
+            float v[KC];
+#pragma unroll
+            for (int c = 0; c < KC; c++) v[c] = 0.0f;
+            if (row < g.n) {
+                cg_load_row<KC>(g.v + row * k, c0, (int)k, g.vec, v);
+                if (g.r != nullptr) {
+                    float rv[KC];
+                    cg_load_row<KC>(g.r + row * k, c0, (int)k, g.vec, rv);
+#pragma unroll
+                    for (int c = 0; c < KC; c++) v[c] = fmaf(c0 + c < k ? beta_s[c] : 0.0f, v[c], rv[c]);
+                    cg_store_row<KC>(g.v + row * k, c0, (int)k, g.vec, v);
+                }
+            }
+            const float *lambda = g.lambda + blk * P * KM_BLOCK_SIZE + t;
+#pragma unroll 8
+            for (int q = 0; q < P; q++) ls[q][t] = lambda[q * KM_BLOCK_SIZE];
+            if constexpr (KC >= 4) {
+#pragma unroll
+                for (int c = 0; c < KC; c += 4) *reinterpret_cast<float4 *>(&vs[t][c]) = make_float4(v[c], v[c + 1], v[c + 2], v[c + 3]);
+            } else {
+#pragma unroll
+                for (int c = 0; c < 4; c++) vs[t][c] = c < KC ? v[c < KC ? c : 0] : 0.0f;
+            }
+            __syncthreads();
+            const int groups = (int)min((int64_t)(KC < 4 ? 4 : KC), g.kq - c0) / 4;
+            const int quads = (P + 3) / 4, units = quads * groups;  // <= 32
+            const bool mine = lane < units;
+            const int q = mine ? (lane % quads) * 4 : 0, c = mine ? (lane / quads) * 4 : 0;
+            f32x2 acc[4][2] = {};
+#pragma unroll 8
+            for (int i = 0; i < 32; i++) {
+                const ulonglong2 w = *reinterpret_cast<const ulonglong2 *>(&vs[warp * 32 + i][c]);
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    const f32x2 l = splat2(ls[min(q + j, P - 1)][warp * 32 + i]);
+                    acc[j][0] = fma2(l, w.x, acc[j][0]), acc[j][1] = fma2(l, w.y, acc[j][1]);
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < 4; j++) *reinterpret_cast<ulonglong2 *>(part[warp][j][lane]) = make_ulonglong2(acc[j][0], acc[j][1]);
+            __syncthreads();
+            if (mine && q + warp < P) {
+                float4 o = *reinterpret_cast<const float4 *>(part[0][warp][lane]);
+#pragma unroll
+                for (int w = 1; w < 4; w++) {
+                    const float4 x = *reinterpret_cast<const float4 *>(part[w][warp][lane]);
+                    o.x += x.x, o.y += x.y, o.z += x.z, o.w += x.w;
+                }
+                *reinterpret_cast<float4 *>(g.nodes + (blk * P + q + warp) * g.kq + c0 + c) = o;
+            }
+        }
+    }
+}
+
+struct NodeProductArgs {
+    int64_t n, k, kq, rb0, rb1;
+    int P, max_blocks;
+    const int *start, *end;
+    const float *lambda, *G, *nodes;
+    float *out;          // row rb0 * 128 of the window first
+    const float *p;      // not null: out = K v + sigma2 p, and partials of p . out
+    float sigma2;
+    float *block_partials;
+    int vec;
+};
+
+// K v of one row block per CTA: 8 (or 4) slices of threads take every 8th (4th) column node of the band,
+// lanes the P row nodes, and the slices' sums go through shared memory to thread = row.
+template <int KC>
+__global__ void __launch_bounds__(128) node_product_kernel(const NodeProductArgs g) {
+    constexpr int KC4 = KC < 4 ? 4 : KC, KC2 = KC4 / 2;
+    __shared__ __align__(16) float sums[8][16 * (KC4 + 4)];
+    __shared__ float warp_part[4][32];
+    const int t = threadIdx.x, P = g.P;
+    const int64_t k = g.k, r = g.rb0 + blockIdx.x;
+    const int width = P <= 16 ? 16 : 32, slices = 128 / width, p = t % width, slice = t / width;
+    const int s = g.start[r], e = g.end[r];
+    const int64_t c_lo = s < e ? s / KM_BLOCK_SIZE : 0;
+    const int count = s < e ? (int)((min((int64_t)e, g.n) + KM_BLOCK_SIZE - 1) / KM_BLOCK_SIZE - c_lo) * P : 0;
+    const float *G = g.G + (int64_t)blockIdx.x * g.max_blocks * P * P + min(p, P - 1);
+    const int64_t row = r * KM_BLOCK_SIZE + t;
+    for (int c0 = 0; c0 < g.kq; c0 += KC4) {
+        const float *nodes = g.nodes + c_lo * P * g.kq + c0;
+        f32x2 acc[KC2];
+#pragma unroll
+        for (int c = 0; c < KC2; c++) acc[c] = 0ull;
+        const int valid = (int)min((int64_t)KC4, g.kq - c0);
+#pragma unroll 4
+        for (int j = slice; j < count; j += slices) {
+            const f32x2 m = splat2(__ldg(G + (int64_t)j * P));
+            const float *v = nodes + j * g.kq;
+#pragma unroll
+            for (int c4 = 0; c4 < KC4 / 4; c4++) {
+                if (c4 * 4 < valid) {
+                    const ulonglong2 w = __ldg(reinterpret_cast<const ulonglong2 *>(v + c4 * 4));
+                    acc[2 * c4] = fma2(m, w.x, acc[2 * c4]), acc[2 * c4 + 1] = fma2(m, w.y, acc[2 * c4 + 1]);
+                }
+            }
+        }
+        // sums[slice (two per array of 32 lanes)][row node][column]
+        __syncthreads();
+        float *flat = &sums[0][0];
+        constexpr int QS = KC4 + 4;
+#pragma unroll
+        for (int c4 = 0; c4 < KC4 / 4; c4++)
+            *reinterpret_cast<ulonglong2 *>(flat + (slice * width + p) * QS + c4 * 4) = make_ulonglong2(acc[2 * c4], acc[2 * c4 + 1]);
+        __syncthreads();
+        for (int i = t; i < P * KC4; i += 128) {
+            const int q = i / KC4, c = i % KC4;
+            float v = 0.0f;
+            for (int sl = 0; sl < slices; sl++) v += flat[(sl * width + q) * QS + c];
+            flat[q * QS + c] = v;
+        }
+        __syncthreads();
+        f32x2 o2[KC2];
+#pragma unroll
+        for (int c = 0; c < KC2; c++) o2[c] = 0ull;
+        const float *lambda = g.lambda + r * P * KM_BLOCK_SIZE + t;
+#pragma unroll 4
+        for (int q = 0; q < P; q++) {
+            const f32x2 l = splat2(lambda[q * KM_BLOCK_SIZE]);
+#pragma unroll
+            for (int c4 = 0; c4 < KC4 / 4; c4++) {
+                const ulonglong2 w = *reinterpret_cast<const ulonglong2 *>(flat + q * QS + c4 * 4);
+                o2[2 * c4] = fma2(l, w.x, o2[2 * c4]), o2[2 * c4 + 1] = fma2(l, w.y, o2[2 * c4 + 1]);
+            }
+        }
+        float o[KC4], acc_dot[KC];
+#pragma unroll
+        for (int c = 0; c < KC2; c++) unpack2(o2[c], o[2 * c], o[2 * c + 1]);
+        float u[KC];
+#pragma unroll
+        for (int c = 0; c < KC; c++) u[c] = o[c], acc_dot[c] = 0.0f;
+        if (row < g.n) {
+            if (g.p != nullptr) {
+                float w[KC];
+                cg_load_row<KC>(g.p + row * k, c0, (int)k, g.vec, w);
+#pragma unroll
+                for (int c = 0; c < KC; c++) {
+                    u[c] = fmaf(g.sigma2, w[c], u[c]);
+                    acc_dot[c] = w[c] * u[c];
+                }
+            }
+            cg_store_row<KC>(g.out + (row - g.rb0 * KM_BLOCK_SIZE) * k, c0, (int)k, g.vec, u);
+        }
+        if (g.p != nullptr) {
+            const float total = cg_block_reduce<KC>(acc_dot, warp_part);
+            if (t < KC && c0 + t < k) g.block_partials[(int64_t)blockIdx.x * k + c0 + t] = total;
+        }
+    }
+}
+
+template <typename F>
+static int node_dispatch_kt(int kernel_type, F f) {
+    switch (kernel_type) {
+    case KM_KERNEL_RBF: return f(std::integral_constant<int, KM_KERNEL_RBF>());
+    case KM_KERNEL_SPECTRAL: return f(std::integral_constant<int, KM_KERNEL_SPECTRAL>());
+    default: return f(std::integral_constant<int, KM_KERNEL_LOCALLY_PERIODIC>());
+    }
+}
+
+template <int MAX_KC, typename F>
+static int node_dispatch_kc(int64_t k, F f) {
+    if (k <= 1) return f(std::integral_constant<int, 1>());
+    if (k <= 2) return f(std::integral_constant<int, 2>());
+    if (k <= 4) return f(std::integral_constant<int, 4>());
+    if (k <= 8) return f(std::integral_constant<int, 8>());
+    if (k <= 16 || MAX_KC == 16) return f(std::integral_constant<int, 16>());
+    return f(std::integral_constant<int, MAX_KC>());
+}
+
+static int node_compress(NodeVectorArgs g, cudaStream_t s) {
+    g.kq = ceil_div(g.k, 4) * 4;
+    g.tiny = 1.17549435e-38f;
+    g.vec = g.k % 4 == 0 && (uintptr_t)g.v % 16 == 0 && (uintptr_t)g.r % 16 == 0;
+    if (g.blk1 <= g.blk0 && g.r == nullptr) return KM_OK;
+    // (an update always runs one CTA: it keeps the residual history)
+    const unsigned ctas = (unsigned)std::max<int64_t>(1, std::min<int64_t>(g.blk1 - g.blk0, 148 * 6));
+    return node_dispatch_kc<16>(g.k, [&](auto kc) {
+        node_compress_kernel<decltype(kc)::value><<<ctas, 128, 0, s>>>(g);
+        KM_CHECK_LAUNCH("node compression launch");
+        return (int)KM_OK;
+    });
+}
+
+}  // namespace km
+
+extern "C" int km_node_operator_plan_f32(int kernel_type, const km_batch *batch, int64_t n, const float *x, int64_t x_stride,
+                                         const km_view *params, const int32_t *start, const int32_t *end, int64_t row_block_begin,
+                                         int64_t row_block_count, float *centre, void *plan, void *stream) {
+    using namespace km;
+    KM_REQUIRE(valid_kernel_type(kernel_type) && batch && params, KM_ERR_INVALID_ARGUMENT, "km_node_operator_plan_f32: bad arguments");
+    NodePlanArgs a;
+    const int rc = make_batch(batch, &a.batch);
+    if (rc != KM_OK) return rc;
+    const int64_t R = ceil_div(n, KM_BLOCK_SIZE);
+    KM_REQUIRE(n >= 1 && n <= 0x7fffffffLL - 256 && a.batch.count >= 1 && row_block_begin >= 0 && row_block_count >= 0 &&
+                   row_block_begin + row_block_count <= R,
+               KM_ERR_INVALID_ARGUMENT, "km_node_operator_plan_f32: bad sizes");
+    KM_REQUIRE(x && params->data && start && end && centre && plan && (uintptr_t)plan % 8 == 0, KM_ERR_INVALID_ARGUMENT,
+               "km_node_operator_plan_f32: null pointer");
+    a.n = n, a.R = R, a.rb0 = row_block_begin, a.rb1 = row_block_begin + row_block_count;
+    a.x = x, a.xs = x_stride, a.params = make_view<const float>(params, a.batch), a.start = start, a.end = end;
+    a.centre = centre, a.plan = static_cast<NodePlan *>(plan);
+    static_assert(sizeof(NodePlan) <= KM_NODE_PLAN_BYTES, "plan size");
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    const cudaError_t err = cudaMemsetAsync(plan, 0, sizeof(NodePlan), s);
+    if (err != cudaSuccess) return cuda_fail(err, "km_node_operator_plan_f32");
+    const unsigned ctas = (unsigned)std::min<int64_t>(ceil_div(R, 8), 148 * 4);
+    return node_dispatch_kt(kernel_type, [&](auto kt) {
+        node_plan_kernel<decltype(kt)::value><<<ctas, 256, 0, s>>>(a);
+        KM_CHECK_LAUNCH("km_node_operator_plan_f32 launch");
+        return (int)KM_OK;
+    });
+}
+
+extern "C" int km_node_operator_build_f32(int kernel_type, const km_batch *batch, int64_t n, const float *x, int64_t x_stride,
+                                          const km_view *params, const int32_t *start, const int32_t *end, int64_t row_block_begin,
+                                          int64_t row_block_count, const float *centre, const void *plan, int64_t nodes,
+                                          int64_t max_blocks, float *lambda, float *matrix, void *stream) {
+    using namespace km;
+    KM_REQUIRE(valid_kernel_type(kernel_type) && batch && params, KM_ERR_INVALID_ARGUMENT, "km_node_operator_build_f32: bad arguments");
+    NodeOpArgs a;
+    const int rc = make_batch(batch, &a.batch);
+    if (rc != KM_OK) return rc;
+    const int64_t R = ceil_div(n, KM_BLOCK_SIZE);
+    KM_REQUIRE(n >= 1 && n <= 0x7fffffffLL - 256 && a.batch.count >= 1 && row_block_begin >= 0 && row_block_count >= 0 &&
+                   row_block_begin + row_block_count <= R && nodes >= 4 && nodes <= NODE_OP_MAX && nodes % 2 == 0 && max_blocks >= 0 &&
+                   max_blocks <= R,
+               KM_ERR_INVALID_ARGUMENT, "km_node_operator_build_f32: bad sizes");
+    KM_REQUIRE(x && params->data && start && end && centre && plan && lambda && (matrix || row_block_count * max_blocks == 0),
+               KM_ERR_INVALID_ARGUMENT, "km_node_operator_build_f32: null pointer");
+    a.n = n, a.R = R, a.rb0 = row_block_begin, a.rb1 = row_block_begin + row_block_count;
+    a.x = x, a.xs = x_stride, a.params = make_view<const float>(params, a.batch), a.start = start, a.end = end;
+    a.plan = static_cast<const NodePlan *>(plan), a.centre = centre, a.lambda = lambda, a.G = matrix;
+    a.P = (int)nodes, a.max_blocks = (int)max_blocks;
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    node_lambda_kernel<<<(unsigned)std::min<int64_t>(R, 148 * 16), 128, 0, s>>>(a);
+    KM_CHECK_LAUNCH("km_node_operator_build_f32 launch");
+    const int64_t items = row_block_count * ceil_div(max_blocks, GB_PAIRS);
+    if (items == 0) return KM_OK;
+    KM_REQUIRE(items <= 0x7fffffffLL, KM_ERR_UNSUPPORTED, "km_node_operator_build_f32: too many blocks");
+    return node_dispatch_kt(kernel_type, [&](auto kt) {
+        node_matrix_kernel<decltype(kt)::value><<<(unsigned)ceil_div(items, 4), 128, 0, s>>>(a);
+        KM_CHECK_LAUNCH("km_node_operator_build_f32 launch");
+        return (int)KM_OK;
+    });
+}
+
+extern "C" int km_node_compress_f32(int64_t k, int64_t n, int64_t nodes_per_block, const float *lambda, const float *v, float *nodes,
+                                    int64_t block_begin, int64_t block_end, void *stream) {
+    using namespace km;
+    KM_REQUIRE(k >= 1 && n >= 1 && nodes_per_block >= 4 && nodes_per_block <= NODE_OP_MAX && block_begin >= 0 && block_end >= block_begin &&
+                   block_end <= ceil_div(n, KM_BLOCK_SIZE) && lambda && v && nodes,
+               KM_ERR_INVALID_ARGUMENT, "km_node_compress_f32: bad arguments");
+    NodeVectorArgs g{};
+    g.n = n, g.k = k, g.P = (int)nodes_per_block, g.blk0 = block_begin, g.blk1 = block_end, g.lambda = lambda;
+    g.v = const_cast<float *>(v), g.nodes = nodes;
+    return node_compress(g, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int km_node_update_p_f32(int64_t k, int64_t n, int64_t nodes_per_block, const float *lambda, float *p, const float *r,
+                                    float *nodes, int64_t block_begin, int64_t block_end, const void *rr_seg_sums,
+                                    int64_t seg_rank_stride_bytes, int32_t seg_ranks, int32_t seg_slots, const float *rs_old,
+                                    float *rs_new, const float *ynorm, float *history_row, float *beta_row, void *stream) {
+    using namespace km;
+    KM_REQUIRE(k >= 1 && n >= 1 && nodes_per_block >= 4 && nodes_per_block <= NODE_OP_MAX && block_begin >= 0 && block_end >= block_begin &&
+                   block_end <= ceil_div(n, KM_BLOCK_SIZE) && lambda && p && r && nodes && rr_seg_sums && rs_old && rs_new &&
+                   rs_old != rs_new && (history_row == nullptr || ynorm) && seg_ranks >= 1 && seg_slots >= 0 && seg_rank_stride_bytes % 8 == 0,
+               KM_ERR_INVALID_ARGUMENT, "km_node_update_p_f32: bad arguments");
+    NodeVectorArgs g{};
+    g.n = n, g.k = k, g.P = (int)nodes_per_block, g.blk0 = block_begin, g.blk1 = block_end, g.lambda = lambda;
+    g.v = p, g.r = r, g.nodes = nodes;
+    g.totals = {static_cast<const unsigned char *>(rr_seg_sums), seg_rank_stride_bytes, seg_ranks, seg_slots};
+    g.rs_in = rs_old, g.rs_out = rs_new, g.ynorm = ynorm, g.history = history_row, g.coeff_out = beta_row;
+    return node_compress(g, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int km_node_product_f32(int64_t k, int64_t n, int64_t nodes_per_block, int64_t max_blocks, const int32_t *start,
+                                   const int32_t *end, const float *lambda, const float *matrix, const float *nodes,
+                                   int64_t row_block_begin, int64_t row_block_count, float *out, const float *p, float sigma2,
+                                   float *block_partials, void *stream) {
+    using namespace km;
+    KM_REQUIRE(k >= 1 && n >= 1 && nodes_per_block >= 4 && nodes_per_block <= NODE_OP_MAX && row_block_begin >= 0 && row_block_count >= 0 &&
+                   row_block_begin + row_block_count <= ceil_div(n, KM_BLOCK_SIZE) && row_block_count <= 0x7fffffffLL && start && end &&
+                   lambda && nodes && out && (matrix || max_blocks == 0) && (p == nullptr || block_partials),
+               KM_ERR_INVALID_ARGUMENT, "km_node_product_f32: bad arguments");
+    if (row_block_count == 0) return KM_OK;
+    NodeProductArgs g{};
+    g.n = n, g.k = k, g.kq = ceil_div(k, 4) * 4, g.rb0 = row_block_begin, g.rb1 = row_block_begin + row_block_count;
+    g.P = (int)nodes_per_block, g.max_blocks = (int)max_blocks, g.start = start, g.end = end, g.lambda = lambda, g.G = matrix;
+    g.nodes = nodes, g.out = out, g.p = p, g.sigma2 = sigma2, g.block_partials = block_partials;
+    g.vec = k % 4 == 0 && (uintptr_t)out % 16 == 0 && (uintptr_t)p % 16 == 0;
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    return node_dispatch_kc<32>(k, [&](auto kc) {
+        node_product_kernel<decltype(kc)::value><<<(unsigned)row_block_count, 128, 0, s>>>(g);
+        KM_CHECK_LAUNCH("km_node_product_f32 launch");
+        return (int)KM_OK;
+    });
+}

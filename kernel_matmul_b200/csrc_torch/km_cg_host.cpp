@@ -1,0 +1,126 @@
+// The CG solve's operator by blockwise interpolation, and whole runs of iterations without the
+// interpreter: an iteration on a few thousand points is five kernels of 2 us, and their launches from
+// Python took 350 us.
+#include "km_cg_host.h"
+
+namespace kmh {
+
+NodeOperator::NodeOperator(int64_t kernel_type, const Tensor &x, const Tensor &params, const Tensor &start, const Tensor &end,
+                           int64_t row_block_begin, int64_t row_block_count)
+    : kid_((int)kernel_type), begin_(row_block_begin), count_(row_block_count), x_(x), params_(params) {
+    check_f32(x), check_f32(params), check_i32(start), check_i32(end);
+    TORCH_CHECK(x.dim() == 1 && params.dim() >= 1 && params.size(-1) == num_params(kernel_type), "x must be (n,) and params (.., P)");
+    n_ = x.size(0);
+    R_ = (n_ + KM_BLOCK_SIZE - 1) / KM_BLOCK_SIZE;
+    TORCH_CHECK(start.numel() >= R_ && end.numel() >= R_, "start / end must have ", R_, " entries");
+    start_ = start.reshape({-1}).contiguous(), end_ = end.reshape({-1}).contiguous();
+    if (params_.dim() - 1 > KM_MAX_BATCH_DIMS) params_ = params_.reshape({-1, params_.size(-1)});
+    const int nb = (int)params_.dim() - 1;
+    kb_.ndim = nb;
+    for (int d = 0; d < nb; d++) kb_.size[d] = params_.size(d), vparams_.batch_stride[d] = params_.stride(d);
+    vparams_.data = params_.data_ptr();
+    vparams_.stride[0] = params_.stride(nb);
+    const c10::cuda::CUDAGuard guard(x.device());
+    const auto opt = x.options().requires_grad(false);
+    centre_ = at::empty({std::max<int64_t>(R_, 1)}, opt);
+    plan_ = at::empty({KM_NODE_PLAN_BYTES / 8}, opt.dtype(at::kLong));
+    raise_on(km_node_operator_plan_f32(kid_, &kb_, n_, x_.const_data_ptr<float>(), x_.stride(0), &vparams_, start_.const_data_ptr<int32_t>(),
+                                       end_.const_data_ptr<int32_t>(), begin_, count_, centre_.data_ptr<float>(), plan_.data_ptr(), stream()));
+}
+
+void NodeOperator::build(int64_t lo, int64_t hi, int64_t nodes, int64_t max_blocks) {
+    const c10::cuda::CUDAGuard guard(x_.device());
+    const auto opt = x_.options().requires_grad(false);
+    P_ = nodes, max_blocks_ = max_blocks;
+    blk0_ = std::max<int64_t>(0, lo) / KM_BLOCK_SIZE, blk1_ = (std::min(hi, n_) + KM_BLOCK_SIZE - 1) / KM_BLOCK_SIZE;
+    blk0_ = std::min(blk0_, blk1_);
+    lambda_ = at::empty({R_ * P_ * KM_BLOCK_SIZE}, opt);
+    matrix_ = at::empty({std::max<int64_t>(1, count_ * max_blocks * P_ * P_)}, opt);
+    raise_on(km_node_operator_build_f32(kid_, &kb_, n_, x_.const_data_ptr<float>(), x_.stride(0), &vparams_, start_.const_data_ptr<int32_t>(),
+                                        end_.const_data_ptr<int32_t>(), begin_, count_, centre_.const_data_ptr<float>(), plan_.data_ptr(),
+                                        P_, max_blocks_, lambda_.data_ptr<float>(), matrix_.data_ptr<float>(), stream()));
+}
+
+float *NodeOperator::nodes(int64_t k) {
+    const int64_t need = R_ * P_ * ((k + 3) / 4 * 4);
+    if (!nodes_.defined() || nodes_.numel() < need) nodes_ = at::empty({need}, x_.options().requires_grad(false));
+    return nodes_.data_ptr<float>();
+}
+
+void NodeOperator::compress(const Tensor &v, int64_t k) {
+    raise_on(km_node_compress_f32(k, n_, P_, lambda_.const_data_ptr<float>(), v.const_data_ptr<float>(), nodes(k), blk0_, blk1_, stream()));
+}
+
+void NodeOperator::update_p(const CgState &s, int64_t it) {
+    const int64_t k = s.k;
+    raise_on(km_node_update_p_f32(k, n_, P_, lambda_.const_data_ptr<float>(), s.p.data_ptr<float>(), s.r.const_data_ptr<float>(), nodes(k), 0, R_,
+                                  s.send2.data_ptr(), s.send2.numel(), 1, (int32_t)s.slots, s.rs_row(it), s.rs_row(it + 1),
+                                  s.ynorm.const_data_ptr<float>(), s.row(s.history, it + 1), s.row(s.betas, it), stream()));
+}
+
+void NodeOperator::product(int64_t k, float *out, const float *p, double sigma2, float *block_partials) {
+    raise_on(km_node_product_f32(k, n_, P_, max_blocks_, start_.const_data_ptr<int32_t>(), end_.const_data_ptr<int32_t>(),
+                                 lambda_.const_data_ptr<float>(), matrix_.const_data_ptr<float>(), nodes(k), begin_, count_, out, p, (float)sigma2,
+                                 block_partials, stream()));
+}
+
+void NodeOperator::matvec(const Tensor &v, const Tensor &out) {
+    check_f32(v), check_f32(out);
+    TORCH_CHECK(v.dim() == 2 && v.size(0) == n_ && v.is_contiguous() && out.dim() == 2 && out.is_contiguous() && out.size(1) == v.size(1),
+                "v must be a contiguous (n, k) tensor and out (rows, k)");
+    const int64_t rows = std::max<int64_t>(0, std::min(n_, (begin_ + count_) * KM_BLOCK_SIZE) - begin_ * KM_BLOCK_SIZE);
+    TORCH_CHECK(out.size(0) == rows, "out must have ", rows, " rows");
+    const c10::cuda::CUDAGuard guard(x_.device());
+    compress(v, v.size(1));
+    product(v.size(1), out.data_ptr<float>(), nullptr, 0.0, nullptr);
+}
+
+// Iterations first .. first + count - 1 of a solve on one GPU: what CGSolver.step() does, from here.  With
+// `nodes` the product, q and the partial sums of p . q are one kernel, and the update of p and its
+// compression another; otherwise `rows` is the product.
+void cg_run(const CgState &s, NodeOperator *nodes, RowsProduct *rows, int64_t first, int64_t count) {
+    const c10::cuda::CUDAGuard guard(s.p.device());
+    void *stream = c10::cuda::getCurrentCUDAStream(s.p.device().index()).stream();
+    const int64_t k = s.k, n = s.n;
+    float *x = s.x.data_ptr<float>(), *r = s.r.data_ptr<float>(), *p = s.p.data_ptr<float>(), *q = s.kp.data_ptr<float>();
+    float *bp = s.bp.data_ptr<float>();
+    const auto totals = [&](const Tensor &to) {
+        raise_on(km_cg_segment_sums_f32(k, bp, s.blocks, s.seg_blocks, static_cast<double *>(to.data_ptr()), stream));
+    };
+    TORCH_CHECK((nodes != nullptr) != (rows != nullptr), "one kind of product");
+    for (int64_t it = first; it < first + count; it++) {
+        if (nodes != nullptr) {
+            if (it == first) nodes->compress(s.p, k);
+            nodes->product(k, q, p, s.sigma2, bp);
+        } else {
+            rows->run();
+            raise_on(km_cg_q_dots_f32(k, q, p, (float)s.sigma2, 0, n, bp, nullptr, 0, nullptr, 0, stream));
+        }
+        totals(s.send1);
+        raise_on(km_cg_update_xr_f32(k, x, r, p, q, nullptr, 0, nullptr, 0, 0, n, 0, n, s.send1.data_ptr(), s.send1.numel(), 1, (int32_t)s.slots,
+                                     s.rs_row(it), bp, s.row(s.alphas, it), stream));
+        totals(s.send2);
+        if (nodes != nullptr && it + 1 < first + count)
+            nodes->update_p(s, it);
+        else
+            raise_on(km_cg_update_p_f32(k, p, r, 0, n, s.send2.data_ptr(), s.send2.numel(), 1, (int32_t)s.slots, s.rs_row(it), s.rs_row(it + 1),
+                                        s.ynorm.const_data_ptr<float>(), s.row(s.history, it + 1), s.row(s.betas, it), stream));
+    }
+}
+
+Tensor log_forms(const Tensor &alphas, const Tensor &betas, const Tensor &residual_norms, const Tensor &z_norm2, double converged) {
+    for (const Tensor *t : {&alphas, &betas, &residual_norms, &z_norm2}) check_f32(*t);
+    TORCH_CHECK(alphas.dim() == 2 && betas.sizes() == alphas.sizes() && residual_norms.dim() == 2 &&
+                    residual_norms.size(0) == alphas.size(0) + 1 && residual_norms.size(1) == alphas.size(1) && z_norm2.dim() == 1 &&
+                    z_norm2.size(0) == alphas.size(1),
+                "alphas and betas must be (m, k), residual_norms (m + 1, k) and z_norm2 (k,)");
+    const c10::cuda::CUDAGuard guard(alphas.device());
+    const Tensor a = alphas.contiguous(), b = betas.contiguous(), r = residual_norms.contiguous(), z = z_norm2.contiguous();
+    Tensor out = at::empty({alphas.size(1)}, alphas.options().dtype(at::kDouble).requires_grad(false));
+    raise_on(km_cg_log_forms_f32(a.size(0), a.size(1), a.const_data_ptr<float>(), b.const_data_ptr<float>(), r.const_data_ptr<float>(),
+                                 z.const_data_ptr<float>(), (float)converged, out.data_ptr<double>(),
+                                 c10::cuda::getCurrentCUDAStream(alphas.device().index()).stream()));
+    return out;
+}
+
+}  // namespace kmh

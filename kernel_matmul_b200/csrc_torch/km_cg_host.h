@@ -1,0 +1,46 @@
+#pragma once
+
+#include "km_host.h"
+
+namespace kmh {
+
+// The buffers of a solve on one GPU (kernel_matmul_b200.cg.CGSolver).
+struct CgState {
+    Tensor x, r, p, kp, bp, rs, ynorm, history, alphas, betas, send1, send2;
+    int64_t n, k, blocks, seg_blocks, slots;
+    double sigma2;
+    float *row(const Tensor &t, int64_t i) const { return t.data_ptr<float>() + i * k; }
+    float *rs_row(int64_t it) const { return row(rs, it & 1); }
+};
+
+class NodeOperator {
+  public:
+    // Looks at points, band and parameters of a window of row blocks; `plan()` tells what came of it.
+    NodeOperator(int64_t kernel_type, const Tensor &x, const Tensor &params, const Tensor &start, const Tensor &end,
+                 int64_t row_block_begin, int64_t row_block_count);
+    // int64 on the device: lo, hi, checksum, nodes per block (0: not this way), widest band in blocks
+    Tensor plan() const { return plan_.slice(0, 0, 5); }
+    void build(int64_t lo, int64_t hi, int64_t nodes, int64_t max_blocks);
+    // out = the window's rows of K v
+    void matvec(const Tensor &v, const Tensor &out);
+
+    void compress(const Tensor &v, int64_t k);
+    void update_p(const CgState &s, int64_t it);
+    void product(int64_t k, float *out, const float *p, double sigma2, float *block_partials);
+
+  private:
+    float *nodes(int64_t k);
+    void *stream() const { return c10::cuda::getCurrentCUDAStream(x_.device().index()).stream(); }
+    int kid_;
+    int64_t n_, R_, begin_, count_, P_ = 0, max_blocks_ = 0, blk0_ = 0, blk1_ = 0;
+    Tensor x_, params_, start_, end_, centre_, plan_, lambda_, matrix_, nodes_;
+    km_batch kb_{};
+    km_view vparams_{};
+};
+
+void cg_run(const CgState &s, NodeOperator *nodes, RowsProduct *rows, int64_t first, int64_t count);
+
+// z_c^T log(A) z_c for every column of a CG run, fp64 on the device
+Tensor log_forms(const Tensor &alphas, const Tensor &betas, const Tensor &residual_norms, const Tensor &z_norm2, double converged);
+
+}  // namespace kmh

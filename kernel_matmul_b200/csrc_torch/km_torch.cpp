@@ -13,7 +13,7 @@
 
 #include <vector>
 
-#include "km_host.h"
+#include "km_cg_host.h"
 
 namespace {
 
@@ -214,6 +214,22 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         .def("__call__", &kmh::RowsProduct::run, nogil())
         .def_property_readonly("out", &kmh::RowsProduct::out)
         .def_property_readonly("tensor_cores", &kmh::RowsProduct::tensor_cores);
+    py::class_<kmh::NodeOperator>(m, "NodeOperator")
+        .def(py::init<int64_t, const Tensor &, const Tensor &, const Tensor &, const Tensor &, int64_t, int64_t>())
+        .def("plan", &kmh::NodeOperator::plan)
+        .def("build", &kmh::NodeOperator::build, nogil())
+        .def("matvec", &kmh::NodeOperator::matvec, nogil());
+    py::class_<kmh::CgState>(m, "CgState")
+        .def(py::init([](const Tensor &x, const Tensor &r, const Tensor &p, const Tensor &kp, const Tensor &bp, const Tensor &rs,
+                         const Tensor &ynorm, const Tensor &history, const Tensor &alphas, const Tensor &betas, const Tensor &send1,
+                         const Tensor &send2, int64_t n, int64_t k, int64_t blocks, int64_t seg_blocks, int64_t slots, double sigma2) {
+            return kmh::CgState{x, r, p, kp, bp, rs, ynorm, history, alphas, betas, send1, send2, n, k, blocks, seg_blocks, slots, sigma2};
+        }));
+    m.def("cg_run", [](const kmh::CgState &s, kmh::NodeOperator *nodes, kmh::RowsProduct *rows, int64_t first, int64_t count) {
+        py::gil_scoped_release release;
+        kmh::cg_run(s, nodes, rows, first, count);
+    });
+    m.def("log_forms", &kmh::log_forms, nogil());
     m.def("matmul_ad", &kmh::matmul_ad, nogil());
     m.def("dense_ad", &kmh::dense_ad, nogil());
     m.def("index_ad", &kmh::index_ad, nogil());

@@ -29,7 +29,7 @@ from dataclasses import dataclass
 import torch
 from torch import Tensor
 
-from . import ops, ranges
+from . import _C, ops, ranges
 from .cg import ShardedOperator, conjugate_gradient
 
 
@@ -40,7 +40,10 @@ def lanczos_log_quadratic_forms(alphas: Tensor, betas: Tensor, residual_norms: T
     ``alphas``, ``betas`` ``(m, k)`` and ``residual_norms`` ``(m + 1, k)`` are what the solve recorded,
     ``z_norm2 (k,)`` the squared norms of the right-hand sides.  A column's recurrence is cut where
     its relative residual falls below ``converged`` (its later coefficients are rounding noise).
-    Runs in fp64 on the CPU: the tridiagonals are ``m x m`` with ``m`` the iteration count."""
+    Returns fp64 values on the CPU; coefficients on a CUDA device are evaluated there
+    (``km_cg_log_forms_f32``), others with the eigenvalues of the ``m x m`` tridiagonals."""
+    if alphas.is_cuda:
+        return _C.log_forms(alphas.detach(), betas.detach(), residual_norms.detach(), z_norm2.detach(), converged).cpu()
     a = alphas.detach().double().cpu()
     b = betas.detach().double().cpu()
     res = residual_norms.detach().double().cpu()
@@ -102,8 +105,7 @@ def mll_gradient(kernel_type: str, x: Tensor, params: Tensor, sigma2: float, y: 
     grad_sigma2 = -0.5 * (u * u).sum() + (0.5 / t) * (w * probes).sum()
     inv_quad = (y * u).sum()
     # log det Khat from the Lanczos coefficients of the probe columns (columns 1 .. t of the solve)
-    quad = lanczos_log_quadratic_forms(res.alphas[:, 1:], res.betas[:, 1:], res.residual_norms[:, 1:],
-                                       (probes * probes).sum(dim=0))
-    logdet = quad.mean().to(device=x.device, dtype=torch.float32)
+    quad = _C.log_forms(res.alphas[:, 1:], res.betas[:, 1:], res.residual_norms[:, 1:], (probes * probes).sum(dim=0), 1e-7)
+    logdet = quad.mean().to(torch.float32)
     nll = 0.5 * inv_quad + 0.5 * logdet + 0.5 * n * math.log(2.0 * math.pi)
     return MllGradient(grad_params, grad_sigma2, inv_quad, logdet, nll, u, w, res.residual_norms)

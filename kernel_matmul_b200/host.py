@@ -120,8 +120,7 @@ def cg_solve_from_host(
     start, end = ranges.make_ranges(cutoff, dx)
     op = ShardedOperator.from_kernel(kernel_type, dx, dp, start, end, sigma2, group=group, mode=mode)
     solver = CGSolver(op, y, max_iterations=max(iterations, 1))
-    for _ in range(iterations):
-        solver.step()
+    solver.run(iterations)
     if op.rows > 0:
         out[op.row0: op.row1].copy_(solver.solution_rows(), non_blocking=True)
     return solver, (op.row0, op.row1)
