@@ -13,8 +13,8 @@
 //   * per SEGMENT of `seg_blocks` consecutive row blocks the partials are added in fp64 in a
 //     fixed order (km_cg_segment_sums_f32); segments are aligned at row block 0 and a rank owns
 //     whole segments,
-//   * the segment sums of all ranks, gathered in rank order (= segment order), are added in that
-//     order in fp64 by every CTA that needs alpha or beta.
+//   * the segment sums of all ranks, gathered in rank order (= segment order), are added in fp64, in
+//     an order that only depends on the segments' numbers, by every CTA that needs alpha or beta.
 // The same numbers therefore come out for 1, 2, 4 or 8 ranks.
 //
 // Rows a rank does not own but needs as right-hand side of its next product (the band's halo)
@@ -39,6 +39,7 @@ struct CgDotsArgs {
 // else : partial of a . b.
 template <int KC, bool QFORM>
 __global__ void __launch_bounds__(CG_THREADS) cg_dots_kernel(const CgDotsArgs g) {
+    grid_wait();
     __shared__ float warp_part[4][32];
     const int64_t blocks = (g.row1 - g.row0 + KM_BLOCK_SIZE - 1) / KM_BLOCK_SIZE;
     const int64_t k = g.k;
@@ -80,6 +81,7 @@ __global__ void __launch_bounds__(CG_THREADS) cg_dots_kernel(const CgDotsArgs g)
 // lanes per column take the blocks lane, lane + 32, ... in order, then a fixed tree over the lanes.
 __global__ void __launch_bounds__(512) cg_segment_sums_kernel(int64_t k, const float *block_partials, int64_t blocks,
                                                               int64_t seg_blocks, double *seg_sums) {
+    grid_wait();
     const int64_t s = blockIdx.x;
     const int64_t b0 = s * seg_blocks, b1 = min(b0 + seg_blocks, blocks);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;  // warp = column inside a chunk of 16
@@ -114,16 +116,19 @@ struct CgUpdateArgs {
 // x += alpha p (own rows), r -= alpha q (rows [lo, hi)), partials of r . r (own row blocks).
 template <int KC>
 __global__ void __launch_bounds__(CG_THREADS) cg_update_xr_kernel(const CgUpdateArgs g) {
+    grid_wait();
     __shared__ float warp_part[4][32];
     __shared__ float alpha_s[KC];
+    __shared__ double total_s[KC];
     const int64_t k = g.k;
     const int64_t blk_lo = g.lo / KM_BLOCK_SIZE, blk_hi = (g.hi + KM_BLOCK_SIZE - 1) / KM_BLOCK_SIZE;
     const int64_t own_blk0 = g.row0 / KM_BLOCK_SIZE;
     for (int c0 = 0; c0 < k; c0 += KC) {
         __syncthreads();
+        cg_totals<KC>(g.totals, k, c0, total_s);
         if (threadIdx.x < KC && c0 + threadIdx.x < k) {
             const int c = c0 + threadIdx.x;
-            const double pq = cg_total(g.totals, k, c);
+            const double pq = total_s[threadIdx.x];
             alpha_s[threadIdx.x] = g.rs_in[c] / fmaxf((float)pq, g.tiny);
             if (blockIdx.x == 0 && g.coeff_out != nullptr) g.coeff_out[c] = alpha_s[threadIdx.x];
         }
@@ -173,14 +178,17 @@ __global__ void __launch_bounds__(CG_THREADS) cg_update_xr_kernel(const CgUpdate
 // residual norm.
 template <int KC>
 __global__ void __launch_bounds__(CG_THREADS) cg_update_p_kernel(const CgUpdateArgs g) {
+    grid_wait();
     __shared__ float beta_s[KC];
+    __shared__ double total_s[KC];
     const int64_t k = g.k;
     const int64_t blk_lo = g.lo / KM_BLOCK_SIZE, blk_hi = (g.hi + KM_BLOCK_SIZE - 1) / KM_BLOCK_SIZE;
     for (int c0 = 0; c0 < k; c0 += KC) {
         __syncthreads();
+        cg_totals<KC>(g.totals, k, c0, total_s);
         if (threadIdx.x < KC && c0 + threadIdx.x < k) {
             const int c = c0 + threadIdx.x;
-            const float rs_new = (float)cg_total(g.totals, k, c);
+            const float rs_new = (float)total_s[threadIdx.x];
             beta_s[threadIdx.x] = rs_new / fmaxf(g.rs_in[c], g.tiny);
             if (blockIdx.x == 0) {
                 if (g.coeff_out != nullptr) g.coeff_out[c] = beta_s[threadIdx.x];
@@ -207,12 +215,16 @@ __global__ void __launch_bounds__(CG_THREADS) cg_update_p_kernel(const CgUpdateA
 }
 
 // rs[c] = total of the gathered segment sums, ynorm[c] = max(sqrt(rs[c]), tiny): the start of a solve.
-__global__ void cg_init_scalars_kernel(int64_t k, const unsigned char *seg_base, int64_t seg_rank_stride, int seg_ranks,
-                                       int seg_slots, float *rs, float *ynorm, float tiny) {
-    for (int64_t c = threadIdx.x; c < k; c += blockDim.x) {
-        const float t = (float)cg_total(CgTotals{seg_base, seg_rank_stride, seg_ranks, seg_slots}, k, (int)c);
-        rs[c] = t;
-        ynorm[c] = fmaxf(sqrtf(t), tiny);
+__global__ void __launch_bounds__(CG_THREADS) cg_init_scalars_kernel(int64_t k, CgTotals totals, float *rs, float *ynorm, float tiny) {
+    __shared__ double total_s[32];
+    for (int64_t c0 = 0; c0 < k; c0 += 32) {
+        cg_totals<32>(totals, k, (int)c0, total_s);
+        if (threadIdx.x < 32 && c0 + threadIdx.x < k) {
+            const float t = (float)total_s[threadIdx.x];
+            rs[c0 + threadIdx.x] = t;
+            ynorm[c0 + threadIdx.x] = fmaxf(sqrtf(t), tiny);
+        }
+        __syncthreads();
     }
 }
 
@@ -331,9 +343,7 @@ extern "C" int km_cg_block_dots_f32(int64_t k, const float *a, const float *b, i
     const int64_t blocks = ceil_div(row1 - row0, KM_BLOCK_SIZE);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     return cg_dispatch_kc(k, [&](auto kc) {
-        cg_dots_kernel<decltype(kc)::value, false><<<cg_grid(blocks), CG_THREADS, 0, s>>>(g);
-        KM_CHECK_LAUNCH("km_cg_block_dots_f32 launch");
-        return KM_OK;
+        return launch_chained("km_cg_block_dots_f32 launch", cg_dots_kernel<decltype(kc)::value, false>, cg_grid(blocks), CG_THREADS, 0, s, g);
     });
 }
 
@@ -354,9 +364,7 @@ extern "C" int km_cg_q_dots_f32(int64_t k, float *kp, const float *p, float sigm
     const int64_t blocks = ceil_div(row1 - row0, KM_BLOCK_SIZE);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     return cg_dispatch_kc(k, [&](auto kc) {
-        cg_dots_kernel<decltype(kc)::value, true><<<cg_grid(blocks), CG_THREADS, 0, s>>>(g);
-        KM_CHECK_LAUNCH("km_cg_q_dots_f32 launch");
-        return KM_OK;
+        return launch_chained("km_cg_q_dots_f32 launch", cg_dots_kernel<decltype(kc)::value, true>, cg_grid(blocks), CG_THREADS, 0, s, g);
     });
 }
 
@@ -368,10 +376,8 @@ extern "C" int km_cg_segment_sums_f32(int64_t k, const float *block_partials, in
     KM_REQUIRE(block_partials && seg_sums, KM_ERR_INVALID_ARGUMENT, "km_cg_segment_sums_f32: null pointer");
     const int64_t segs = ceil_div(blocks, seg_blocks);
     KM_REQUIRE(segs <= 0x7fffffffLL, KM_ERR_UNSUPPORTED, "km_cg_segment_sums_f32: too many segments");
-    cg_segment_sums_kernel<<<(unsigned)segs, 512, 0, static_cast<cudaStream_t>(stream)>>>(k, block_partials, blocks,
-                                                                                          seg_blocks, seg_sums);
-    KM_CHECK_LAUNCH("km_cg_segment_sums_f32 launch");
-    return KM_OK;
+    return launch_chained("km_cg_segment_sums_f32 launch", cg_segment_sums_kernel, (unsigned)segs, 512, 0, static_cast<cudaStream_t>(stream),
+                          k, block_partials, blocks, seg_blocks, seg_sums);
 }
 
 extern "C" int km_cg_init_scalars_f32(int64_t k, const void *seg_sums, int64_t seg_rank_stride_bytes, int32_t seg_ranks,
@@ -380,7 +386,8 @@ extern "C" int km_cg_init_scalars_f32(int64_t k, const void *seg_sums, int64_t s
     KM_REQUIRE(k >= 1 && seg_sums && rs && ynorm && seg_ranks >= 1 && seg_slots >= 0 && seg_rank_stride_bytes % 8 == 0,
                KM_ERR_INVALID_ARGUMENT, "km_cg_init_scalars_f32: bad arguments");
     cg_init_scalars_kernel<<<1, 128, 0, static_cast<cudaStream_t>(stream)>>>(
-        k, static_cast<const unsigned char *>(seg_sums), seg_rank_stride_bytes, seg_ranks, seg_slots, rs, ynorm, 1.17549435e-38f);
+        k, CgTotals{static_cast<const unsigned char *>(seg_sums), seg_rank_stride_bytes, seg_ranks, seg_slots}, rs, ynorm,
+        1.17549435e-38f);
     KM_CHECK_LAUNCH("km_cg_init_scalars_f32 launch");
     return KM_OK;
 }
@@ -410,9 +417,7 @@ extern "C" int km_cg_update_xr_f32(int64_t k, float *x, float *r, const float *p
     const int64_t blocks = ceil_div(hi, KM_BLOCK_SIZE) - lo / KM_BLOCK_SIZE;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     return cg_dispatch_kc(k, [&](auto kc) {
-        cg_update_xr_kernel<decltype(kc)::value><<<cg_grid(blocks), CG_THREADS, 0, s>>>(g);
-        KM_CHECK_LAUNCH("km_cg_update_xr_f32 launch");
-        return KM_OK;
+        return launch_chained("km_cg_update_xr_f32 launch", cg_update_xr_kernel<decltype(kc)::value>, cg_grid(blocks), CG_THREADS, 0, s, g);
     });
 }
 
@@ -434,9 +439,7 @@ extern "C" int km_cg_update_p_f32(int64_t k, float *p, const float *r, int64_t l
     const int64_t blocks = std::max<int64_t>(1, ceil_div(hi, KM_BLOCK_SIZE) - lo / KM_BLOCK_SIZE);  // CTA 0 always runs
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     return cg_dispatch_kc(k, [&](auto kc) {
-        cg_update_p_kernel<decltype(kc)::value><<<cg_grid(blocks), CG_THREADS, 0, s>>>(g);
-        KM_CHECK_LAUNCH("km_cg_update_p_f32 launch");
-        return KM_OK;
+        return launch_chained("km_cg_update_p_f32 launch", cg_update_p_kernel<decltype(kc)::value>, cg_grid(blocks), CG_THREADS, 0, s, g);
     });
 }
 

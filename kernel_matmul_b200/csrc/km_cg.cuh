@@ -63,14 +63,25 @@ struct CgTotals {
     int ranks, slots;
 };
 
-// Their sum, in slot order.
-__device__ __forceinline__ double cg_total(const CgTotals &g, int64_t k, int c) {
-    double t = 0.0;
-    for (int rk = 0; rk < g.ranks; rk++) {
-        const double *seg = reinterpret_cast<const double *>(g.base + rk * g.rank_stride);
-        for (int s = 0; s < g.slots; s++) t += seg[s * k + c];
+// Their sums for columns c0 .. c0 + KC - 1, by all 128 threads of a CTA, in to[0 .. KC).  The order does not
+// depend on how segments are dealt out to ranks: lane l of a warp adds segments l, l + 32, .. (segments past
+// the last are zero), then a fixed tree over the lanes.  (Added one after the other by one thread they
+// took 5 us of every update: 64 loads, none of which waits for the one before.)
+template <int KC>
+__device__ __forceinline__ void cg_totals(const CgTotals &g, int64_t k, int c0, double (&to)[KC]) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int segments = g.ranks * g.slots;
+    for (int c = warp; c < KC && c0 + c < k; c += 4) {
+        double t = 0.0;
+        for (int s = lane; s < segments; s += 32) {
+            const int rank = g.ranks == 1 ? 0 : s / g.slots, slot = g.ranks == 1 ? s : s - rank * g.slots;
+            t += reinterpret_cast<const double *>(g.base + rank * g.rank_stride)[slot * k + c0 + c];
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (lane == 0) to[c] = t;
     }
-    return t;
+    __syncthreads();
 }
 
 }  // namespace km

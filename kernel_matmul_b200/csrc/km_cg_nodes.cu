@@ -319,24 +319,44 @@ struct NodeVectorArgs {
     int vec;
 };
 
-// [v = r + beta v on whole blocks, and] nodes = Lambda^T v.  One CTA per row block at a time: thread =
-// row for the update, whose result stays in shared memory for the second part; there a warp adds up
-// its own 32 rows, a lane owning 4 nodes x 4 columns, and the warps' sums are added in order.
-constexpr int NV_COLS = 16;
+// [v = r + beta v on whole blocks, and] nodes = Lambda^T v.  One CTA per row block: thread = row for the
+// update, whose result stays in shared memory for the second part; there a warp adds up its own 32
+// rows -- a lane owns 4 nodes x 4 columns of every 1st, 2nd, .. 32nd of them, however many lanes that takes to
+// fill the warp --, and the warps' sums are added in order.
 template <int KC>
 __global__ void __launch_bounds__(128) node_compress_kernel(const NodeVectorArgs g) {
-    __shared__ __align__(16) float vs[KM_BLOCK_SIZE][NV_COLS];
-    __shared__ float ls[NODE_OP_MAX][KM_BLOCK_SIZE + 1];
+    constexpr int KC4 = KC < 4 ? 4 : KC, VS = KC4 + 4;
+    __shared__ __align__(16) float vs[KM_BLOCK_SIZE * VS];
+    __shared__ float ls[NODE_OP_MAX * (KM_BLOCK_SIZE + 1)];
     __shared__ __align__(16) float part[4][4][32][4];
-    __shared__ float beta_s[NV_COLS];
+    __shared__ float beta_s[KC];
+    __shared__ double total_s[KC];
+    constexpr int LS = KM_BLOCK_SIZE + 1;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5, P = g.P;
-    const int64_t k = g.k;
-    for (int c0 = 0; c0 < g.kq; c0 += KC < 4 ? 4 : KC) {
+    const int64_t k = g.k, blk = g.blk0 + blockIdx.x, row = blk * KM_BLOCK_SIZE + t;
+    const bool any = blk < g.blk1;  // (an update with no blocks keeps the history all the same)
+    if (!any) grid_wait();
+    for (int c0 = 0; c0 < g.kq; c0 += KC4) {
+        float v[KC], rv[KC];
+#pragma unroll
+        for (int c = 0; c < KC; c++) v[c] = rv[c] = 0.0f;
+        if (any) {
+            if (c0 == 0) {
+                const float *lambda = g.lambda + blk * P * KM_BLOCK_SIZE + t;
+                for (int q = 0; q < P; q++) cp_async4(ls + q * LS + t, lambda + q * KM_BLOCK_SIZE);
+                cp_async_commit();
+                grid_wait();  // (the Lagrange matrices were there before)
+            }
+            if (row < g.n) {
+                cg_load_row<KC>(g.v + row * k, c0, (int)k, g.vec, v);
+                if (g.r != nullptr) cg_load_row<KC>(g.r + row * k, c0, (int)k, g.vec, rv);
+            }
+        }
         if (g.r != nullptr) {
-            __syncthreads();
+            cg_totals<KC>(g.totals, k, c0, total_s);
             if (t < KC && c0 + t < k) {
                 const int c = c0 + t;
-                const float rs_new = (float)cg_total(g.totals, k, c);
+                const float rs_new = (float)total_s[t];
                 beta_s[t] = rs_new / fmaxf(g.rs_in[c], g.tiny);
                 if (blockIdx.x == 0) {
                     if (g.coeff_out != nullptr) g.coeff_out[c] = beta_s[t];
@@ -345,59 +365,58 @@ __global__ void __launch_bounds__(128) node_compress_kernel(const NodeVectorArgs
                 }
             }
             __syncthreads();
+            if (row < g.n && any) {
+#pragma unroll
+                for (int c = 0; c < KC; c++) v[c] = fmaf(c0 + c < k ? beta_s[c] : 0.0f, v[c], rv[c]);
+                cg_store_row<KC>(g.v + row * k, c0, (int)k, g.vec, v);
+            }
         }
-        for (int64_t blk = g.blk0 + blockIdx.x; blk < g.blk1; blk += gridDim.x) {
-            const int64_t row = blk * KM_BLOCK_SIZE + t;
-            float v[KC];
+        if (!any) continue;
+        if constexpr (KC >= 4) {
 #pragma unroll
-            for (int c = 0; c < KC; c++) v[c] = 0.0f;
-            if (row < g.n) {
-                cg_load_row<KC>(g.v + row * k, c0, (int)k, g.vec, v);
-                if (g.r != nullptr) {
-                    float rv[KC];
-                    cg_load_row<KC>(g.r + row * k, c0, (int)k, g.vec, rv);
+            for (int c = 0; c < KC; c += 4) *reinterpret_cast<float4 *>(vs + t * VS + c) = make_float4(v[c], v[c + 1], v[c + 2], v[c + 3]);
+        } else {
+            *reinterpret_cast<float4 *>(vs + t * VS) = make_float4(v[0], KC > 1 ? v[KC - 1] : 0.0f, 0.0f, 0.0f);
+        }
+        cp_async_wait<0>();
+        __syncthreads();
+        const int groups = (int)min((int64_t)KC4, g.kq - c0) / 4, quads = (P + 3) / 4, units = quads * groups;  // <= 32
+        const int span = units <= 4 ? 4 : (units <= 8 ? 8 : (units <= 16 ? 16 : 32)), unit = lane & (span - 1), step = 32 / span;
+        const bool mine = unit < units;
+        const int q = mine ? (unit % quads) * 4 : 0, c = mine ? (unit / quads) * 4 : 0;
+        f32x2 acc[4][2] = {};
+        const float *l[4];
 #pragma unroll
-                    for (int c = 0; c < KC; c++) v[c] = fmaf(c0 + c < k ? beta_s[c] : 0.0f, v[c], rv[c]);
-                    cg_store_row<KC>(g.v + row * k, c0, (int)k, g.vec, v);
-                }
+        for (int j = 0; j < 4; j++) l[j] = ls + min(q + j, P - 1) * LS + warp * 32;
+#pragma unroll 4
+        for (int i = lane / span; i < 32; i += step) {
+            const ulonglong2 w = *reinterpret_cast<const ulonglong2 *>(vs + (warp * 32 + i) * VS + c);
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const f32x2 f = splat2(l[j][i]);
+                acc[j][0] = fma2(f, w.x, acc[j][0]), acc[j][1] = fma2(f, w.y, acc[j][1]);
             }
-            const float *lambda = g.lambda + blk * P * KM_BLOCK_SIZE + t;
-#pragma unroll 8
-            for (int q = 0; q < P; q++) ls[q][t] = lambda[q * KM_BLOCK_SIZE];
-            if constexpr (KC >= 4) {
+        }
+        for (int o = span; o < 32; o <<= 1) {
 #pragma unroll
-                for (int c = 0; c < KC; c += 4) *reinterpret_cast<float4 *>(&vs[t][c]) = make_float4(v[c], v[c + 1], v[c + 2], v[c + 3]);
-            } else {
-#pragma unroll
-                for (int c = 0; c < 4; c++) vs[t][c] = c < KC ? v[c < KC ? c : 0] : 0.0f;
+            for (int j = 0; j < 4; j++) {
+                acc[j][0] = add2(acc[j][0], __shfl_xor_sync(0xffffffffu, acc[j][0], o));
+                acc[j][1] = add2(acc[j][1], __shfl_xor_sync(0xffffffffu, acc[j][1], o));
             }
-            __syncthreads();
-            const int groups = (int)min((int64_t)(KC < 4 ? 4 : KC), g.kq - c0) / 4;
-            const int quads = (P + 3) / 4, units = quads * groups;  // <= 32
-            const bool mine = lane < units;
-            const int q = mine ? (lane % quads) * 4 : 0, c = mine ? (lane / quads) * 4 : 0;
-            f32x2 acc[4][2] = {};
-#pragma unroll 8
-            for (int i = 0; i < 32; i++) {
-                const ulonglong2 w = *reinterpret_cast<const ulonglong2 *>(&vs[warp * 32 + i][c]);
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    const f32x2 l = splat2(ls[min(q + j, P - 1)][warp * 32 + i]);
-                    acc[j][0] = fma2(l, w.x, acc[j][0]), acc[j][1] = fma2(l, w.y, acc[j][1]);
-                }
-            }
+        }
+        if (lane < span) {
 #pragma unroll
             for (int j = 0; j < 4; j++) *reinterpret_cast<ulonglong2 *>(part[warp][j][lane]) = make_ulonglong2(acc[j][0], acc[j][1]);
-            __syncthreads();
-            if (mine && q + warp < P) {
-                float4 o = *reinterpret_cast<const float4 *>(part[0][warp][lane]);
+        }
+        __syncthreads();
+        if (lane < span && mine && q + warp < P) {
+            float4 o = *reinterpret_cast<const float4 *>(part[0][warp][lane]);
 #pragma unroll
-                for (int w = 1; w < 4; w++) {
-                    const float4 x = *reinterpret_cast<const float4 *>(part[w][warp][lane]);
-                    o.x += x.x, o.y += x.y, o.z += x.z, o.w += x.w;
-                }
-                *reinterpret_cast<float4 *>(g.nodes + (blk * P + q + warp) * g.kq + c0 + c) = o;
+            for (int w = 1; w < 4; w++) {
+                const float4 x = *reinterpret_cast<const float4 *>(part[w][warp][lane]);
+                o.x += x.x, o.y += x.y, o.z += x.z, o.w += x.w;
             }
+            *reinterpret_cast<float4 *>(g.nodes + (blk * P + q + warp) * g.kq + c0 + c) = o;
         }
     }
 }
@@ -405,6 +424,7 @@ __global__ void __launch_bounds__(128) node_compress_kernel(const NodeVectorArgs
 struct NodeProductArgs {
     int64_t n, k, kq, rb0, rb1;
     int P, max_blocks;
+    int chunk;           // column nodes staged at a time, a multiple of 16
     const int *start, *end;
     const float *lambda, *G, *nodes;
     float *out;          // row rb0 * 128 of the window first
@@ -414,88 +434,147 @@ struct NodeProductArgs {
     int vec;
 };
 
-// K v of one row block per CTA: 8 (or 4) slices of threads take every 8th (4th) column node of the band,
-// lanes the P row nodes, and the slices' sums go through shared memory to thread = row.
-template <int KC>
+// K v of one row block per CTA.  Everything a block needs is contiguous -- its part of G, the nodes of
+// its band, its Lagrange matrix -- and is fetched at once into shared memory, several CTAs per SM
+// overlapping each other's fetches.  Lanes own two row nodes, 8 (16 beyond 16 nodes) lanes a column node; the sums
+// over column nodes end in shared memory, and a thread forms two rows x half of the columns of
+// Lambda times them.  Inner products are those of cg_q_dots to the bit (rows of a warp in a shuffle
+// tree, then the four warps).
+template <int KC4>
 __global__ void __launch_bounds__(128) node_product_kernel(const NodeProductArgs g) {
-    constexpr int KC4 = KC < 4 ? 4 : KC, KC2 = KC4 / 2;
-    __shared__ __align__(16) float sums[8][16 * (KC4 + 4)];
+    constexpr int KC2 = KC4 / 2, HC = KC4 / 2;  // pairs of columns; columns of a thread in the second part
+    extern __shared__ __align__(16) float smem[];
     __shared__ float warp_part[4][32];
-    const int t = threadIdx.x, P = g.P;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5, P = g.P;
     const int64_t k = g.k, r = g.rb0 + blockIdx.x;
-    const int width = P <= 16 ? 16 : 32, slices = 128 / width, p = t % width, slice = t / width;
+    float *ls = smem;                       // [P][128]
+    float *gs = ls + P * KM_BLOCK_SIZE;     // [chunk][P]; later the warps' sums [4][P][KC4]
+    float *qs = gs + max(g.chunk * P, 4 * P * KC4);  // [chunk][KC4]
     const int s = g.start[r], e = g.end[r];
     const int64_t c_lo = s < e ? s / KM_BLOCK_SIZE : 0;
     const int count = s < e ? (int)((min((int64_t)e, g.n) + KM_BLOCK_SIZE - 1) / KM_BLOCK_SIZE - c_lo) * P : 0;
-    const float *G = g.G + (int64_t)blockIdx.x * g.max_blocks * P * P + min(p, P - 1);
-    const int64_t row = r * KM_BLOCK_SIZE + t;
+    const float *G = g.G + (int64_t)blockIdx.x * g.max_blocks * P * P;
+    const float *lambda = g.lambda + r * P * KM_BLOCK_SIZE;
+    for (int i = t; i < P * (KM_BLOCK_SIZE / 4); i += 128) cp_async16(ls + i * 4, lambda + i * 4);
+    // second part: rows (t & 63) and that + 64, columns of half t >> 6
+    const int row_in = t & 63, half = t >> 6;
+    const int64_t row0 = r * KM_BLOCK_SIZE + row_in;
+
+    const int width = P <= 16 ? 8 : 16, pair = min(lane & (width - 1), P / 2 - 1), slices = 128 / width, slice = t / width;
     for (int c0 = 0; c0 < g.kq; c0 += KC4) {
+        const int valid = (int)min((int64_t)KC4, g.kq - c0);  // a multiple of 4
         const float *nodes = g.nodes + c_lo * P * g.kq + c0;
-        f32x2 acc[KC2];
+        f32x2 acc[2][KC2];
 #pragma unroll
-        for (int c = 0; c < KC2; c++) acc[c] = 0ull;
-        const int valid = (int)min((int64_t)KC4, g.kq - c0);
-#pragma unroll 4
-        for (int j = slice; j < count; j += slices) {
-            const f32x2 m = splat2(__ldg(G + (int64_t)j * P));
-            const float *v = nodes + j * g.kq;
+        for (int c = 0; c < KC2; c++) acc[0][c] = acc[1][c] = 0ull;
+        float w[2][HC];
+        for (int j0 = 0; j0 < count; j0 += g.chunk) {
+            const int here = min(g.chunk, count - j0);
+            if (j0 > 0 || c0 > 0) __syncthreads();
+            for (int i = t; i < here * P / 4; i += 128) cp_async16(gs + i * 4, G + (int64_t)j0 * P + i * 4);
+            if (j0 == 0 && c0 == 0) grid_wait();  // (the matrix was there before)
+            if (valid == KC4 && g.kq == KC4) {
+                for (int i = t; i < here * (KC4 / 4); i += 128) cp_async16(qs + i * 4, nodes + (int64_t)j0 * KC4 + i * 4);
+            } else {
+                for (int i = t; i < here * (KC4 / 4); i += 128) {
+                    const int j = i / (KC4 / 4), c = (i % (KC4 / 4)) * 4;
+                    if (c < valid)
+                        cp_async16(qs + j * KC4 + c, nodes + (int64_t)(j0 + j) * g.kq + c);
+                    else
+                        *reinterpret_cast<float4 *>(qs + j * KC4 + c) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                }
+            }
+            cp_async_commit();
+            if (j0 == 0 && g.p != nullptr) {  // on the way with the rest
 #pragma unroll
-            for (int c4 = 0; c4 < KC4 / 4; c4++) {
-                if (c4 * 4 < valid) {
-                    const ulonglong2 w = __ldg(reinterpret_cast<const ulonglong2 *>(v + c4 * 4));
-                    acc[2 * c4] = fma2(m, w.x, acc[2 * c4]), acc[2 * c4 + 1] = fma2(m, w.y, acc[2 * c4 + 1]);
+                for (int i = 0; i < 2; i++)
+                    if (row0 + 64 * i < g.n) cg_load_row<HC>(g.p + (row0 + 64 * i) * k, c0 + half * HC, (int)k, g.vec && HC >= 4, w[i]);
+            }
+            cp_async_wait<0>();
+            __syncthreads();
+#pragma unroll 2
+            for (int j = slice; j < here; j += slices) {
+                const float2 m = *reinterpret_cast<const float2 *>(gs + j * P + 2 * pair);
+                const f32x2 m0 = splat2(m.x), m1 = splat2(m.y);
+#pragma unroll
+                for (int c4 = 0; c4 < KC4 / 4; c4++) {
+                    const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(qs + j * KC4 + c4 * 4);
+                    acc[0][2 * c4] = fma2(m0, v.x, acc[0][2 * c4]), acc[0][2 * c4 + 1] = fma2(m0, v.y, acc[0][2 * c4 + 1]);
+                    acc[1][2 * c4] = fma2(m1, v.x, acc[1][2 * c4]), acc[1][2 * c4 + 1] = fma2(m1, v.y, acc[1][2 * c4 + 1]);
                 }
             }
         }
-        // sums[slice (two per array of 32 lanes)][row node][column]
-        __syncthreads();
-        float *flat = &sums[0][0];
-        constexpr int QS = KC4 + 4;
+        if (count == 0) {
+            if (c0 == 0) grid_wait();
+            cp_async_commit();
+            cp_async_wait<0>();
+            if (g.p != nullptr)
 #pragma unroll
-        for (int c4 = 0; c4 < KC4 / 4; c4++)
-            *reinterpret_cast<ulonglong2 *>(flat + (slice * width + p) * QS + c4 * 4) = make_ulonglong2(acc[2 * c4], acc[2 * c4 + 1]);
-        __syncthreads();
-        for (int i = t; i < P * KC4; i += 128) {
-            const int q = i / KC4, c = i % KC4;
-            float v = 0.0f;
-            for (int sl = 0; sl < slices; sl++) v += flat[(sl * width + q) * QS + c];
-            flat[q * QS + c] = v;
+                for (int i = 0; i < 2; i++)
+                    if (row0 + 64 * i < g.n) cg_load_row<HC>(g.p + (row0 + 64 * i) * k, c0 + half * HC, (int)k, g.vec && HC >= 4, w[i]);
+        }
+        for (int o = width; o < 32; o <<= 1) {
+#pragma unroll
+            for (int c = 0; c < KC2; c++) {
+                acc[0][c] = add2(acc[0][c], __shfl_xor_sync(0xffffffffu, acc[0][c], o));
+                acc[1][c] = add2(acc[1][c], __shfl_xor_sync(0xffffffffu, acc[1][c], o));
+            }
+        }
+        __syncthreads();  // every warp is done with gs
+        if (lane < P / 2) {
+#pragma unroll
+            for (int i = 0; i < 2; i++)
+#pragma unroll
+                for (int c4 = 0; c4 < KC4 / 4; c4++)
+                    *reinterpret_cast<ulonglong2 *>(gs + (warp * P + 2 * lane + i) * KC4 + c4 * 4) = make_ulonglong2(acc[i][2 * c4], acc[i][2 * c4 + 1]);
         }
         __syncthreads();
-        f32x2 o2[KC2];
+        for (int i = t; i < P * KC4; i += 128) gs[i] = (gs[i] + gs[P * KC4 + i]) + (gs[2 * P * KC4 + i] + gs[3 * P * KC4 + i]);
+        __syncthreads();
+        float u[2][HC];
 #pragma unroll
-        for (int c = 0; c < KC2; c++) o2[c] = 0ull;
-        const float *lambda = g.lambda + r * P * KM_BLOCK_SIZE + t;
-#pragma unroll 4
+        for (int c = 0; c < HC; c++) u[0][c] = u[1][c] = 0.0f;
+#pragma unroll 2
         for (int q = 0; q < P; q++) {
-            const f32x2 l = splat2(lambda[q * KM_BLOCK_SIZE]);
+            const float l0 = ls[q * KM_BLOCK_SIZE + row_in], l1 = ls[q * KM_BLOCK_SIZE + row_in + 64];
+            const float *sums = gs + q * KC4 + half * HC;
 #pragma unroll
-            for (int c4 = 0; c4 < KC4 / 4; c4++) {
-                const ulonglong2 w = *reinterpret_cast<const ulonglong2 *>(flat + q * QS + c4 * 4);
-                o2[2 * c4] = fma2(l, w.x, o2[2 * c4]), o2[2 * c4 + 1] = fma2(l, w.y, o2[2 * c4 + 1]);
+            for (int c = 0; c < HC; c += 2) {
+                const float2 v = *reinterpret_cast<const float2 *>(sums + c);
+                u[0][c] = fmaf(l0, v.x, u[0][c]), u[0][c + 1] = fmaf(l0, v.y, u[0][c + 1]);
+                u[1][c] = fmaf(l1, v.x, u[1][c]), u[1][c + 1] = fmaf(l1, v.y, u[1][c + 1]);
             }
         }
-        float o[KC4], acc_dot[KC];
+        float dot[2][HC];
 #pragma unroll
-        for (int c = 0; c < KC2; c++) unpack2(o2[c], o[2 * c], o[2 * c + 1]);
-        float u[KC];
+        for (int i = 0; i < 2; i++) {
+            const int64_t row = row0 + 64 * i;
 #pragma unroll
-        for (int c = 0; c < KC; c++) u[c] = o[c], acc_dot[c] = 0.0f;
-        if (row < g.n) {
-            if (g.p != nullptr) {
-                float w[KC];
-                cg_load_row<KC>(g.p + row * k, c0, (int)k, g.vec, w);
+            for (int c = 0; c < HC; c++) dot[i][c] = 0.0f;
+            if (row < g.n) {
+                if (g.p != nullptr) {
 #pragma unroll
-                for (int c = 0; c < KC; c++) {
-                    u[c] = fmaf(g.sigma2, w[c], u[c]);
-                    acc_dot[c] = w[c] * u[c];
+                    for (int c = 0; c < HC; c++) {
+                        u[i][c] = fmaf(g.sigma2, w[i][c], u[i][c]);
+                        dot[i][c] = w[i][c] * u[i][c];
+                    }
                 }
+                cg_store_row<HC>(g.out + (row - g.rb0 * KM_BLOCK_SIZE) * k, c0 + half * HC, (int)k, g.vec && HC >= 4, u[i]);
             }
-            cg_store_row<KC>(g.out + (row - g.rb0 * KM_BLOCK_SIZE) * k, c0, (int)k, g.vec, u);
         }
         if (g.p != nullptr) {
-            const float total = cg_block_reduce<KC>(acc_dot, warp_part);
-            if (t < KC && c0 + t < k) g.block_partials[(int64_t)blockIdx.x * k + c0 + t] = total;
+            // rows 32 w .. 32 w + 31 of the block are those of one warp and one i: w = (warp & 1) + 2 i
+#pragma unroll
+            for (int i = 0; i < 2; i++)
+#pragma unroll
+                for (int c = 0; c < HC; c++) {
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) dot[i][c] += __shfl_xor_sync(0xffffffffu, dot[i][c], o);
+                    if (lane == 0) warp_part[(warp & 1) + 2 * i][half * HC + c] = dot[i][c];
+                }
+            __syncthreads();
+            if (t < KC4 && c0 + t < k)
+                g.block_partials[(int64_t)blockIdx.x * k + c0 + t] = (warp_part[0][t] + warp_part[1][t]) + (warp_part[2][t] + warp_part[3][t]);
         }
     }
 }
@@ -525,11 +604,9 @@ static int node_compress(NodeVectorArgs g, cudaStream_t s) {
     g.vec = g.k % 4 == 0 && (uintptr_t)g.v % 16 == 0 && (uintptr_t)g.r % 16 == 0;
     if (g.blk1 <= g.blk0 && g.r == nullptr) return KM_OK;
     // (an update always runs one CTA: it keeps the residual history)
-    const unsigned ctas = (unsigned)std::max<int64_t>(1, std::min<int64_t>(g.blk1 - g.blk0, 148 * 6));
+    const unsigned ctas = (unsigned)std::max<int64_t>(1, g.blk1 - g.blk0);
     return node_dispatch_kc<16>(g.k, [&](auto kc) {
-        node_compress_kernel<decltype(kc)::value><<<ctas, 128, 0, s>>>(g);
-        KM_CHECK_LAUNCH("node compression launch");
-        return (int)KM_OK;
+        return launch_chained("node compression launch", node_compress_kernel<decltype(kc)::value>, ctas, 128, 0, s, g);
     });
 }
 
@@ -642,9 +719,19 @@ extern "C" int km_node_product_f32(int64_t k, int64_t n, int64_t nodes_per_block
     g.nodes = nodes, g.out = out, g.p = p, g.sigma2 = sigma2, g.block_partials = block_partials;
     g.vec = k % 4 == 0 && (uintptr_t)out % 16 == 0 && (uintptr_t)p % 16 == 0;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    return node_dispatch_kc<32>(k, [&](auto kc) {
-        node_product_kernel<decltype(kc)::value><<<(unsigned)row_block_count, 128, 0, s>>>(g);
-        KM_CHECK_LAUNCH("km_node_product_f32 launch");
-        return (int)KM_OK;
-    });
+    const auto launch = [&](auto cols) {
+        constexpr int KC4 = decltype(cols)::value;
+        // 32 KB of matrix and operand at a time: four CTAs per SM with the Lagrange matrices
+        const int P = g.P;
+        g.chunk = std::max(16, (int)std::min<int64_t>(8192 / (P + KC4), max_blocks * P) / 16 * 16);
+        const size_t smem = (size_t)(P * KM_BLOCK_SIZE + std::max(g.chunk * P, 4 * P * KC4) + g.chunk * KC4) * sizeof(float);
+        auto kernel = node_product_kernel<KC4>;
+        const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
+        if (err != cudaSuccess) return cuda_fail(err, "cudaFuncSetAttribute(node product)");
+        return launch_chained("km_node_product_f32 launch", kernel, (unsigned)row_block_count, 128, smem, s, g);
+    };
+    if (k <= 4) return launch(std::integral_constant<int, 4>());
+    if (k <= 8) return launch(std::integral_constant<int, 8>());
+    if (k <= 16) return launch(std::integral_constant<int, 16>());
+    return launch(std::integral_constant<int, 32>());
 }
