@@ -140,14 +140,18 @@ KM_API int km_take_gave_up(int32_t device, int32_t *what);
  * Chebyshev points per block, with Lagrange matrices on both sides.  Calls whose bands are not
  * aligned to blocks, or that would need more points, are evaluated directly (km_matmul_tc_f32 from 9
  * columns, km_matmul_f32 below): the kernels of both ways are launched and the device decides.
+ * all_columns != 0: the caller expects every row block to see all columns (no cutoff); the points, shared by
+ * all batches, are then put in order first and taken in larger blocks (a band that does exclude
+ * something, or points that cannot be ordered quickly, are evaluated directly).
  * m, n, k >= 1.  workspace: ..._workspace_bytes (0: this call is too large for it), 256-byte aligned,
  * contents irrelevant on entry.
  * ------------------------------------------------------------------------------------- */
 KM_API size_t km_matmul_nodes_workspace_bytes(const km_batch *batch, int64_t m, int64_t n, int64_t k, const km_view *x1,
-                                              const km_view *x2, const km_view *rhs);
+                                              const km_view *x2, const km_view *rhs, int32_t all_columns);
 KM_API int km_matmul_nodes_f32(int kernel_type, const km_batch *batch, int64_t m, int64_t n, int64_t k, const km_view *x1,
                                const km_view *x2, const km_view *rhs, const km_view *params, const km_view *start,
-                               const km_view *end, const km_view *out, void *workspace, size_t workspace_bytes, void *stream);
+                               const km_view *end, const km_view *out, int32_t all_columns, void *workspace,
+                               size_t workspace_bytes, void *stream);
 
 /* ---------------------------------------------------------------------------------------
  * The same product for a window of row blocks, optionally summed over the batch:
@@ -241,11 +245,13 @@ KM_API int km_matmul_bwd_f32(int kernel_type, const km_batch *batch, int64_t m, 
  * blocks' Chebyshev points and the gradient is formed there.  Directly: km_bilinear_derivative_tc_f32
  * from 8 columns, km_bilinear_derivative_f32 below. */
 KM_API size_t km_grad_nodes_workspace_bytes(int kernel_type, const km_batch *batch, int64_t m, int64_t n, int64_t k,
-                                            const km_view *x1, const km_view *x2, const km_view *left, const km_view *right);
+                                            const km_view *x1, const km_view *x2, const km_view *left, const km_view *right,
+                                            int32_t all_columns);
 KM_API int km_bilinear_derivative_nodes_f32(int kernel_type, const km_batch *batch, int64_t m, int64_t n, int64_t k,
                                             const km_view *x1, const km_view *x2, const km_view *left, const km_view *right,
                                             const km_view *params, const km_view *start, const km_view *end,
-                                            const km_view *grad, void *workspace, size_t workspace_bytes, void *stream);
+                                            const km_view *grad, int32_t all_columns, void *workspace, size_t workspace_bytes,
+                                            void *stream);
 
 /* ---------------------------------------------------------------------------------------
  * The same gradients with the coefficients <left[i, :], right[j, :]> computed on the tensor

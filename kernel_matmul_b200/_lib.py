@@ -101,13 +101,13 @@ def _load() -> ctypes.CDLL:
     lib.km_transpose_ranges_i32.restype = ctypes.c_int
     lib.km_transpose_ranges_i32.argtypes = [i64, i64, vp, vp, i64, i64, i32, vp, vp, vp]
     lib.km_matmul_nodes_workspace_bytes.restype = sz
-    lib.km_matmul_nodes_workspace_bytes.argtypes = [bp, i64, i64, i64, wp, wp, wp]
+    lib.km_matmul_nodes_workspace_bytes.argtypes = [bp, i64, i64, i64, wp, wp, wp, i32]
     lib.km_matmul_nodes_f32.restype = ctypes.c_int
-    lib.km_matmul_nodes_f32.argtypes = [ctypes.c_int, bp, i64, i64, i64, wp, wp, wp, wp, wp, wp, wp, vp, sz, vp]
+    lib.km_matmul_nodes_f32.argtypes = [ctypes.c_int, bp, i64, i64, i64, wp, wp, wp, wp, wp, wp, wp, i32, vp, sz, vp]
     lib.km_grad_nodes_workspace_bytes.restype = sz
-    lib.km_grad_nodes_workspace_bytes.argtypes = [ctypes.c_int, bp, i64, i64, i64, wp, wp, wp, wp]
+    lib.km_grad_nodes_workspace_bytes.argtypes = [ctypes.c_int, bp, i64, i64, i64, wp, wp, wp, wp, i32]
     lib.km_bilinear_derivative_nodes_f32.restype = ctypes.c_int
-    lib.km_bilinear_derivative_nodes_f32.argtypes = [ctypes.c_int, bp, i64, i64, i64, wp, wp, wp, wp, wp, wp, wp, wp, vp, sz, vp]
+    lib.km_bilinear_derivative_nodes_f32.argtypes = [ctypes.c_int, bp, i64, i64, i64, wp, wp, wp, wp, wp, wp, wp, wp, i32, vp, sz, vp]
     fp = ctypes.POINTER(ctypes.c_void_p)
     lib.km_take_gave_up.restype = ctypes.c_int
     lib.km_take_gave_up.argtypes = [i32, ctypes.POINTER(i32)]

@@ -40,6 +40,8 @@ struct NodesArgs {
     int64_t R, C;       // row and column blocks
     int64_t slots1, slots2;  // distinct x1 / x2 rows: batch.count, or 1 if all batches share one
     int same;           // x1 and x2 are the same points
+    int block;          // points per block: KM_BLOCK_SIZE, or more where all rows see all columns
+    const int *order1, *order2;  // the points in order (not null where block > KM_BLOCK_SIZE)
     int max_p;          // most nodes of a block
     int cap;            // most nodes of a block over all classes of its level, where batches share x
     View<const float> x1, x2, params;
@@ -48,8 +50,11 @@ struct NodesArgs {
     int *classes;              // [batch][level]
     float *centre1, *centre2;  // [slot][block]
     float *half1, *half2;      // [slot][block] half-lengths
-    float *lambda1, *lambda2;  // [slot][block][cap or max_p][128]
+    float *lambda1, *lambda2;  // [slot][block][cap or max_p][points per block]
 };
+
+// Row of the caller's arrays that holds point i of the blocks.
+__device__ __forceinline__ int64_t point_row(const int *order, int64_t i) { return order == nullptr ? i : (int64_t)order[i]; }
 
 __device__ __forceinline__ int level_of(const NodesHeader *hdr, float half) {
     int l = 0;
@@ -88,11 +93,12 @@ __global__ void __launch_bounds__(256) nodes_plan_kernel(const NodesArgs a, int 
         const float *base = batch_ptr(x, decompose(a.batch, slot));
         float lo = INFINITY, hi = -INFINITY;
         bool nan = false;
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const int64_t row = block * KM_BLOCK_SIZE + lane + 32 * i;
+        const int *order = one ? a.order1 : a.order2;
+#pragma unroll 4
+        for (int i = lane; i < a.block; i += 32) {
+            const int64_t row = block * a.block + i;
             if (row < rows) {
-                const float e = base[row * x.s0];
+                const float e = base[point_row(order, row) * x.s0];
                 lo = fminf(lo, e);
                 hi = fmaxf(hi, e);
                 nan = nan || !(fabsf(e) < INFINITY);
@@ -109,10 +115,15 @@ __global__ void __launch_bounds__(256) nodes_plan_kernel(const NodesArgs a, int 
         if (lane == 0) (one ? a.centre1 : a.centre2)[v] = c, (one ? a.half1 : a.half2)[v] = h;
     }
     const int64_t threads = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t w = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; w < a.batch.count * a.R; w += threads) {
-        const BatchIndex bi = decompose(a.batch, w / a.R);
-        const int64_t r = w % a.R;
+    const int64_t bands = (a.m + KM_BLOCK_SIZE - 1) / KM_BLOCK_SIZE;  // row blocks of the band
+    for (int64_t w = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; w < a.batch.count * bands; w += threads) {
+        const BatchIndex bi = decompose(a.batch, w / bands);
+        const int64_t r = w % bands;
         const int s = batch_ptr(a.start, bi)[r * a.start.s0], e = batch_ptr(a.end, bi)[r * a.end.s0];
+        if (a.order1 != nullptr) {  // all rows must see all columns
+            bad |= s > 0 || e < a.n;
+            continue;
+        }
         if (s >= e) continue;  // an empty band
         bad |= s < 0 || s % KM_BLOCK_SIZE != 0 || (e < a.n && e % KM_BLOCK_SIZE != 0);
     }
@@ -211,23 +222,24 @@ __global__ void __launch_bounds__(256) nodes_plan_kernel(const NodesArgs a, int 
     }
 }
 
-// Lagrange matrices of one block, one per class in use for it: thread = row,
+// Lagrange matrices of 128 rows of one block, one per class in use for it: thread = row,
 // lambda[q][row] = (w_q / (x - xi_q)) / sum of the same.
 __global__ void __launch_bounds__(128) nodes_lambda_kernel(const NodesArgs a) {
     const NodesHeader *hdr = a.hdr;
     if (!hdr->use) return;
     __shared__ float delta[NODES_MAX], weight[NODES_MAX];
     const int64_t boxes1 = a.slots1 * a.R;
-    const bool one = blockIdx.x < boxes1;
-    const int64_t v = one ? blockIdx.x : blockIdx.x - boxes1, blocks = one ? a.R : a.C, rows = one ? a.m : a.n;
+    const int parts = a.block / 128, part = blockIdx.x % parts;
+    const bool one = blockIdx.x / parts < boxes1;
+    const int64_t v = blockIdx.x / parts - (one ? 0 : boxes1), blocks = one ? a.R : a.C, rows = one ? a.m : a.n;
     const int64_t slots = one ? a.slots1 : a.slots2;
     const View<const float> &x = one ? a.x1 : a.x2;
     const int t = threadIdx.x;
     const int level = level_of(hdr, (one ? a.half1 : a.half2)[v]);
     // (differences in units of h: an interval may be as short as NODES_MIN_H)
     const float inv_h = 1.0f / hdr->h[level];
-    const int64_t row = (v % blocks) * KM_BLOCK_SIZE + t;
-    const float d = row < rows ? batch_ptr(x, decompose(a.batch, v / blocks))[row * x.s0] - (one ? a.centre1 : a.centre2)[v] : 0.0f;
+    const int64_t row = (v % blocks) * a.block + part * 128 + t;
+    const float d = row < rows ? batch_ptr(x, decompose(a.batch, v / blocks))[point_row(one ? a.order1 : a.order2, row) * x.s0] - (one ? a.centre1 : a.centre2)[v] : 0.0f;
     const bool shared = slots == 1;
     const int c0 = shared ? hdr->first[level] : a.classes[v / blocks * NODES_LEVELS + level], c1 = shared ? hdr->first[level + 1] : c0 + 1;
     for (int cls = c0; cls < c1; cls++) {
@@ -235,9 +247,9 @@ __global__ void __launch_bounds__(128) nodes_lambda_kernel(const NodesArgs a) {
         __syncthreads();
         if (t < P) delta[t] = hdr->delta[cls][t], weight[t] = hdr->weight[cls][t];
         __syncthreads();
-        float *out = (one ? a.lambda1 : a.lambda2) + (v * node_rows(a, slots) + node_first(a, slots, cls)) * KM_BLOCK_SIZE + t;
+        float *out = (one ? a.lambda1 : a.lambda2) + (v * node_rows(a, slots) + node_first(a, slots, cls)) * a.block + part * 128 + t;
         if (row >= rows) {
-            for (int q = 0; q < P; q++) out[q * KM_BLOCK_SIZE] = 0.0f;
+            for (int q = 0; q < P; q++) out[q * a.block] = 0.0f;
             continue;
         }
         float sum = 0.0f;
@@ -252,9 +264,133 @@ __global__ void __launch_bounds__(128) nodes_lambda_kernel(const NodesArgs a) {
 #pragma unroll 4
         for (int q = 0; q < P; q++) {
             const float e = (d - delta[q]) * inv_h;
-            out[q * KM_BLOCK_SIZE] = hit >= 0 ? (q == hit ? 1.0f : 0.0f) : __fdividef(weight[q], e) * inv;
+            out[q * a.block] = hit >= 0 ? (q == hit ? 1.0f : 0.0f) : __fdividef(weight[q], e) * inv;
         }
     }
+}
+
+// Order of points that no band orders: a counting sort into equal intervals between the smallest and the
+// largest point, then every interval (16 points on average) sorted by (value, index) by a warp, so that
+// the order, and with it every sum, is the same on every run.  Inputs that fill an interval with more
+// than SORT_MOST points are evaluated directly.
+constexpr int SORT_BUCKETS = 8192;
+constexpr int SORT_MOST = 1024;
+struct SortTables {
+    unsigned lo, hi;             // smallest and largest point as ordered integers (zero on entry: of ~lo, hi)
+    int counts[SORT_BUCKETS];    // zero on entry; later the points placed so far
+    int first[SORT_BUCKETS + 1];
+};
+
+__device__ __forceinline__ unsigned ordered_bits(float v) {
+    const unsigned b = __float_as_uint(v);
+    return (b & 0x80000000u) ? ~b : b | 0x80000000u;
+}
+__device__ __forceinline__ float ordered_value(unsigned b) { return __uint_as_float((b & 0x80000000u) ? b & 0x7fffffffu : ~b); }
+__device__ __forceinline__ int sort_bucket(float v, float lo, float scale) { return min(max((int)((v - lo) * scale), 0), SORT_BUCKETS - 1); }
+__device__ __forceinline__ float sort_scale(float lo, float hi) { return hi > lo ? (float)SORT_BUCKETS / (hi - lo) : 0.0f; }
+
+__global__ void __launch_bounds__(256) sort_bounds_kernel(View<const float> x, int64_t n, SortTables *t) {
+    unsigned lo = 0u, hi = 0u;  // of the complement, so that zero is neutral for both
+    for (int64_t i = blockIdx.x * 256LL + threadIdx.x; i < n; i += gridDim.x * 256LL) {
+        const unsigned b = ordered_bits(x.data[i * x.s0]);
+        lo = max(lo, ~b);
+        hi = max(hi, b);
+    }
+    lo = __reduce_max_sync(0xffffffffu, lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    if ((threadIdx.x & 31) == 0) atomicMax(&t->lo, lo), atomicMax(&t->hi, hi);
+}
+
+__global__ void __launch_bounds__(256) sort_count_kernel(View<const float> x, int64_t n, SortTables *t) {
+    const float lo = ordered_value(~t->lo), scale = sort_scale(lo, ordered_value(t->hi));
+    for (int64_t i = blockIdx.x * 256LL + threadIdx.x; i < n; i += gridDim.x * 256LL)
+        atomicAdd(&t->counts[sort_bucket(x.data[i * x.s0], lo, scale)], 1);
+}
+
+__global__ void __launch_bounds__(1024) sort_scan_kernel(SortTables *t, int *bad) {
+    constexpr int PER = SORT_BUCKETS / 1024;
+    __shared__ int warp_sum[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int c[PER], sum = 0;
+    bool over = false;
+#pragma unroll
+    for (int i = 0; i < PER; i++) {
+        c[i] = t->counts[threadIdx.x * PER + i];
+        over = over || c[i] > SORT_MOST;
+        sum += c[i];
+    }
+    int run = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, run, o);
+        if (lane >= o) run += y;
+    }
+    if (lane == 31) warp_sum[warp] = run;
+    __syncthreads();
+    int before = run - sum;
+    for (int w = 0; w < warp; w++) before += warp_sum[w];
+#pragma unroll
+    for (int i = 0; i < PER; i++) {
+        t->first[threadIdx.x * PER + i] = before;
+        t->counts[threadIdx.x * PER + i] = 0;
+        before += c[i];
+    }
+    if (threadIdx.x == 1023) t->first[SORT_BUCKETS] = before;
+    if (over) *bad = 1;
+}
+
+__global__ void __launch_bounds__(256) sort_place_kernel(View<const float> x, int64_t n, SortTables *t, int *order) {
+    const float lo = ordered_value(~t->lo), scale = sort_scale(lo, ordered_value(t->hi));
+    for (int64_t i = blockIdx.x * 256LL + threadIdx.x; i < n; i += gridDim.x * 256LL) {
+        const int b = sort_bucket(x.data[i * x.s0], lo, scale);
+        order[t->first[b] + atomicAdd(&t->counts[b], 1)] = (int)i;
+    }
+}
+
+// Bitonic sort of each interval's (value, index) pairs in shared memory, a warp per interval.
+__global__ void __launch_bounds__(128) sort_intervals_kernel(View<const float> x, const SortTables *t, int *order, const int *bad) {
+    if (*bad) return;
+    __shared__ unsigned long long keys[4][SORT_MOST];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int b = blockIdx.x * 4 + warp; b < SORT_BUCKETS; b += gridDim.x * 4) {
+        const int first = t->first[b], count = t->first[b + 1] - first;
+        if (count < 2) continue;
+        int size = 2;
+        while (size < count) size *= 2;
+        for (int i = lane; i < size; i += 32) {
+            unsigned long long key = ~0ull;
+            if (i < count) {
+                const int p = order[first + i];
+                key = ((unsigned long long)ordered_bits(x.data[p * x.s0]) << 32) | (unsigned)p;
+            }
+            keys[warp][i] = key;
+        }
+        __syncwarp();
+        for (int span = 2; span <= size; span *= 2)
+            for (int d = span / 2; d > 0; d /= 2) {
+                for (int i = lane; i < size / 2; i += 32) {
+                    const int u = 2 * d * (i / d) + i % d, v = u + d;
+                    const unsigned long long p = keys[warp][u], q = keys[warp][v];
+                    if ((p > q) == ((u & span) == 0)) keys[warp][u] = q, keys[warp][v] = p;
+                }
+                __syncwarp();
+            }
+        for (int i = lane; i < count; i += 32) order[first + i] = (int)(unsigned)keys[warp][i];
+        __syncwarp();
+    }
+}
+
+static int sort_points(const View<const float> &x, int64_t n, SortTables *t, int *order, int *bad, cudaStream_t s) {
+    const cudaError_t err = cudaMemsetAsync(t, 0, offsetof(SortTables, first), s);
+    if (err != cudaSuccess) return cuda_fail(err, "interpolation: cudaMemsetAsync");
+    const unsigned ctas = (unsigned)std::min<int64_t>((n + 255) / 256, 148 * 4);
+    sort_bounds_kernel<<<ctas, 256, 0, s>>>(x, n, t);
+    sort_count_kernel<<<ctas, 256, 0, s>>>(x, n, t);
+    sort_scan_kernel<<<1, 1024, 0, s>>>(t, bad);
+    sort_place_kernel<<<ctas, 256, 0, s>>>(x, n, t, order);
+    sort_intervals_kernel<<<148 * 4, 128, 0, s>>>(x, t, order, bad);
+    KM_CHECK_LAUNCH("interpolation: sort launch");
+    return KM_OK;
 }
 
 // Lambda^T of one operand: out[slot][block][q][c] = sum_row lambda[q][row] * v[row][c], columns padded
@@ -267,6 +403,7 @@ struct CompressArgs {
     int64_t x_slots;   // distinct points: one Lagrange matrix per block for all batches if 1
     int vec;           // rows may be read 16 bytes at a time
     View<const float> v;
+    const int *order;
     const float *half, *lambda;
     float *out;
 };
@@ -280,7 +417,7 @@ struct CompressShape {
     static constexpr size_t SMEM = 4 * 2 * STAGE * sizeof(float);
 };
 
-// A warp per (slot, block, COLS columns), no synchronisation beyond the warp: the block's 128 rows pass
+// A warp per (slot, block, COLS columns), no synchronisation beyond the warp: the block's rows pass
 // through two stages of 32 rows (operand and Lagrange matrix, cp.async), a lane owning 4 nodes x 4 columns
 // (8 shared-memory words read for 8 packed FMAs).  More than 40 nodes, or more units than lanes, take
 // further passes over the rows.
@@ -298,21 +435,21 @@ __global__ void __launch_bounds__(128) nodes_compress_kernel(const CompressArgs 
     const int64_t chunk = item % chunks, box = item / chunks, slot = box / p.blocks, block = box % p.blocks;
     const int k0 = (int)chunk * COLS, kc = (int)min((int64_t)COLS, p.kq - k0);  // a multiple of 4
     const float *v = batch_ptr(p.v, decompose(a.batch, slot));
-    const int64_t row0 = block * KM_BLOCK_SIZE, x_slot = p.x_slots == 1 ? 0 : slot;
+    const int64_t row0 = block * a.block, x_slot = p.x_slots == 1 ? 0 : slot;
     const int groups = kc / 4;
     const int level = level_of(a.hdr, p.half[x_slot * p.blocks + block]);
     const bool shared = p.slots == 1;
     const int c0 = shared ? a.hdr->first[level] : a.classes[slot * NODES_LEVELS + level], c1 = shared ? a.hdr->first[level + 1] : c0 + 1;
-    const int row_count = (int)min((int64_t)KM_BLOCK_SIZE, p.rows - row0), steps = (row_count + CP_ROWS - 1) / CP_ROWS;
+    const int row_count = (int)min((int64_t)a.block, p.rows - row0), steps = (row_count + CP_ROWS - 1) / CP_ROWS;
 
     for (int cls = c0; cls < c1; cls++) {
         const int P = a.hdr->P[cls];
         const float *lambda_cls =
-            p.lambda + ((x_slot * p.blocks + block) * node_rows(a, p.x_slots) + node_first(a, p.x_slots, cls)) * KM_BLOCK_SIZE;
+            p.lambda + ((x_slot * p.blocks + block) * node_rows(a, p.x_slots) + node_first(a, p.x_slots, cls)) * a.block;
         float *out_cls = p.out + (box * node_rows(a, p.slots) + node_first(a, p.slots, cls)) * p.kq + k0;
         for (int p0 = 0; p0 < P; p0 += CP_NODES) {
             const int Pn = min(CP_NODES, P - p0);
-            const float *lambda = lambda_cls + p0 * KM_BLOCK_SIZE;
+            const float *lambda = lambda_cls + p0 * a.block;
             float *out = out_cls + p0 * p.kq;
             const auto load = [&](int step, int which) {
                 float *vs = stages + which * STAGE, *ls = vs + CP_ROWS * COLS;
@@ -321,7 +458,7 @@ __global__ void __launch_bounds__(128) nodes_compress_kernel(const CompressArgs 
                     for (int e = lane; e < CP_ROWS * groups; e += 32) {
                         const int i = e / groups, c = (e - i * groups) * 4;
                         if (i < count)
-                            cp_async16(vs + i * COLS + c, v + (row0 + r + i) * p.v.s0 + k0 + c);
+                            cp_async16(vs + i * COLS + c, v + point_row(p.order, row0 + r + i) * p.v.s0 + k0 + c);
                         else
                             *reinterpret_cast<float4 *>(vs + i * COLS + c) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                     }
@@ -329,12 +466,12 @@ __global__ void __launch_bounds__(128) nodes_compress_kernel(const CompressArgs 
                     for (int e = lane; e < CP_ROWS * kc; e += 32) {
                         const int i = e / kc, c = e - i * kc;
                         if (i < count && k0 + c < a.k)
-                            cp_async4(vs + i * COLS + c, v + (row0 + r + i) * p.v.s0 + (k0 + c) * p.v.s1);
+                            cp_async4(vs + i * COLS + c, v + point_row(p.order, row0 + r + i) * p.v.s0 + (k0 + c) * p.v.s1);
                         else
                             vs[i * COLS + c] = 0.0f;
                     }
                 }
-                for (int q = 0; q < Pn; q++) cp_async4(ls + q * CP_LS + lane, lambda + q * KM_BLOCK_SIZE + r + lane);
+                for (int q = 0; q < Pn; q++) cp_async4(ls + q * CP_LS + lane, lambda + q * a.block + r + lane);
                 cp_async_commit();
             };
             const int quads = (Pn + 3) / 4, units = quads * groups;
@@ -493,9 +630,14 @@ struct NodeItem {
         k0 = chunk * KC;
         kc = (int)min((int64_t)KC, kq - k0);  // a multiple of 4
         fn.init(batch_ptr(a.params, bi), a.params.s0);
-        const int s = batch_ptr(a.start, bi)[r * a.start.s0], e = batch_ptr(a.end, bi)[r * a.end.s0];
-        c_lo = s < e ? s / KM_BLOCK_SIZE : 0;
-        c_hi = s < e && !idle ? (int)((min((int64_t)e, a.n) + KM_BLOCK_SIZE - 1) / KM_BLOCK_SIZE) : 0;
+        if (a.order1 != nullptr) {
+            c_lo = 0;
+            c_hi = idle ? 0 : (int)a.C;
+        } else {
+            const int s = batch_ptr(a.start, bi)[r * a.start.s0], e = batch_ptr(a.end, bi)[r * a.end.s0];
+            c_lo = s < e ? s / KM_BLOCK_SIZE : 0;
+            c_hi = s < e && !idle ? (int)((min((int64_t)e, a.n) + KM_BLOCK_SIZE - 1) / KM_BLOCK_SIZE) : 0;
+        }
         c_step = wpr;
         if (wpr > 1) c_lo += warp;
         const int64_t row_box = (a.slots1 == 1 ? 0 : b) * a.R + r;
@@ -697,7 +839,7 @@ __global__ void __launch_bounds__(128, NodeShape<KC>::CTAS) nodes_product_kernel
     // sums come from shared memory as broadcasts, whose cost is the registers they fill, so that
     // each one read should serve several rows.
     const float *lambda = a.lambda1 + (((a.slots1 == 1 ? 0 : it.b) * a.R + it.r) * node_rows(a, a.slots1) +
-                                       node_first(a, a.slots1, it.row_class)) * KM_BLOCK_SIZE;
+                                       node_first(a, a.slots1, it.row_class)) * a.block;
     const auto expand = [&](auto rows_per_lane, int row0) {
         constexpr int OR = decltype(rows_per_lane)::value, OC = KC >= 8 ? 8 : 4;
         for (int g = 0; g < KC / OC; g++) {
@@ -718,16 +860,16 @@ __global__ void __launch_bounds__(128, NodeShape<KC>::CTAS) nodes_product_kernel
                 }
 #pragma unroll
                 for (int i = 0; i < OR; i++) {
-                    const f32x2 l = splat2(lambda[q * KM_BLOCK_SIZE + row0 + lane + 32 * i] * fn.scale);
+                    const f32x2 l = splat2(lambda[q * a.block + row0 + lane + 32 * i] * fn.scale);
 #pragma unroll
                     for (int c = 0; c < OC / 2; c++) o2[i][c] = fma2(l, rv[c], o2[i][c]);
                 }
             }
 #pragma unroll
             for (int i = 0; i < OR; i++) {
-                const int64_t row = it.r * KM_BLOCK_SIZE + row0 + lane + 32 * i;
+                const int64_t row = it.r * a.block + row0 + lane + 32 * i;
                 if (row >= a.m) break;
-                float *out = batch_ptr(p.out, bi) + row * p.out.s0 + (it.k0 + g * OC) * p.out.s1;
+                float *out = batch_ptr(p.out, bi) + point_row(a.order1, row) * p.out.s0 + (it.k0 + g * OC) * p.out.s1;
 #pragma unroll
                 for (int c4 = 0; c4 < OC / 4; c4++) {
                     float4 v;
@@ -746,9 +888,11 @@ __global__ void __launch_bounds__(128, NodeShape<KC>::CTAS) nodes_product_kernel
         }
     };
     if (p.wpr == 1)
-        expand(Int<4>(), 0);
-    else
+        for (int row0 = 0; row0 < a.block; row0 += 128) expand(Int<4>(), row0);
+    else if (a.block == 128)
         expand(Int<1>(), 32 * (tid >> 5));
+    else
+        for (int row0 = 128 * (tid >> 5); row0 < a.block; row0 += 512) expand(Int<4>(), row0);
 }
 
 struct NodesGradArgs {
@@ -886,21 +1030,28 @@ static int nodes_kc(int64_t k) {
 // A warp per row block once that gives every SM its 12 - 16 warps; four warps below.
 static int nodes_warps_per_row_block(int64_t items) { return items >= 148 * 12 ? 1 : 4; }
 
+// Points per block where all rows see all columns: enough blocks for the GPU, few enough nodes.
+static int nodes_sorted_block(int64_t points) { return points >= (1 << 16) ? 1024 : (points >= (1 << 14) ? 512 : 256); }
+
 struct NodesLayout {
     int64_t slots1, slots2, R, C, kq;
     bool same;
-    int max_p, cap;
+    int max_p, cap, block;
+    bool sorted;
+    size_t sort1, sort2, order1, order2;
     size_t classes, centre1, centre2, half1, half2, lambda1, lambda2, ops[2], partials, direct, total;
     int64_t op_slots[2];
 
     static size_t up(size_t v) { return (v + 255) / 256 * 256; }
     // operands: rhs of a product (right[0] null), or left and right of a gradient
     NodesLayout(const Batch &b, int64_t m, int64_t n, int64_t k, const View<const float> &x1, const View<const float> &x2,
-                const View<const float> *left, const View<const float> &right, size_t direct_bytes) {
+                const View<const float> *left, const View<const float> &right, bool all_columns, size_t direct_bytes) {
         slots1 = shared_by_batches(x1, b) ? 1 : b.count;
         slots2 = shared_by_batches(x2, b) ? 1 : b.count;
-        R = ceil_div(m, KM_BLOCK_SIZE);
-        C = ceil_div(n, KM_BLOCK_SIZE);
+        sorted = all_columns && slots1 == 1 && slots2 == 1;
+        block = sorted ? nodes_sorted_block(std::max(m, n)) : KM_BLOCK_SIZE;
+        R = ceil_div(m, block);
+        C = ceil_div(n, block);
         kq = ceil_div(k, 4) * 4;
         max_p = nodes_limit(k);
         // Where batches share their points every class needs its own Lagrange matrices and operands: room
@@ -922,8 +1073,12 @@ struct NodesLayout {
         centre2 = same ? centre1 : take((size_t)(slots2 * C) * sizeof(float));
         half1 = take((size_t)(slots1 * R) * sizeof(float));
         half2 = same ? half1 : take((size_t)(slots2 * C) * sizeof(float));
-        lambda1 = take(nodes(slots1) * R * KM_BLOCK_SIZE * sizeof(float));
-        lambda2 = same ? lambda1 : take(nodes(slots2) * C * KM_BLOCK_SIZE * sizeof(float));
+        lambda1 = take(nodes(slots1) * R * block * sizeof(float));
+        lambda2 = same ? lambda1 : take(nodes(slots2) * C * block * sizeof(float));
+        sort1 = take(sorted ? sizeof(SortTables) : 0);
+        sort2 = same ? sort1 : take(sorted ? sizeof(SortTables) : 0);
+        order1 = take(sorted ? (size_t)m * sizeof(int) : 0);
+        order2 = same ? order1 : take(sorted ? (size_t)n * sizeof(int) : 0);
         ops[0] = take(op_slots[0] == 0 ? 0 : nodes(op_slots[0]) * R * kq * sizeof(float));
         ops[1] = take(nodes(op_slots[1]) * C * kq * sizeof(float));
         partials = take(left == nullptr ? 0 : (size_t)(b.count * R * ceil_div(k, nodes_kc(k))) * KM_MAX_PARAMS * sizeof(float));
@@ -940,6 +1095,7 @@ static int nodes_compress(const NodesArgs &a, const NodesLayout &l, const View<c
     c.slots = l.op_slots[side], c.x_slots = side == 0 ? l.slots1 : l.slots2;
     c.vec = a.k % 4 == 0 && rows_vectorizable(v, a.batch);
     c.v = v;
+    c.order = side == 0 ? a.order1 : a.order2;
     c.half = side == 0 ? a.half1 : a.half2, c.lambda = side == 0 ? a.lambda1 : a.lambda2;
     c.out = out;
     const auto launch = [&](auto cols) {
@@ -966,10 +1122,19 @@ static int nodes_begin(NodesArgs &a, const NodesLayout &l, int kernel_type, unsi
     a.lambda1 = reinterpret_cast<float *>(ws + l.lambda1), a.lambda2 = reinterpret_cast<float *>(ws + l.lambda2);
     cudaError_t err = cudaMemsetAsync(ws, 0, NODES_ZEROED, s);
     if (err != cudaSuccess) return cuda_fail(err, "interpolation: cudaMemsetAsync");
-    const int64_t boxes = l.slots1 * l.R + (l.same ? 0 : l.slots2 * l.C), work = std::max(ceil_div(boxes, 8), ceil_div(a.batch.count * l.R, 256));
+    a.block = l.block;
+    a.order1 = a.order2 = nullptr;
+    if (l.sorted) {
+        int rc = sort_points(a.x1, a.m, reinterpret_cast<SortTables *>(ws + l.sort1), reinterpret_cast<int *>(ws + l.order1), &a.hdr->bad, s);
+        if (rc == KM_OK && !l.same)
+            rc = sort_points(a.x2, a.n, reinterpret_cast<SortTables *>(ws + l.sort2), reinterpret_cast<int *>(ws + l.order2), &a.hdr->bad, s);
+        if (rc != KM_OK) return rc;
+        a.order1 = reinterpret_cast<const int *>(ws + l.order1), a.order2 = reinterpret_cast<const int *>(ws + l.order2);
+    }
+    const int64_t boxes = l.slots1 * l.R + (l.same ? 0 : l.slots2 * l.C), work = std::max(ceil_div(boxes, 8), ceil_div(a.batch.count * ceil_div(a.m, KM_BLOCK_SIZE), 256));
     nodes_plan_kernel<<<(unsigned)std::min<int64_t>(work, 148 * 4), 256, 0, s>>>(a, kernel_type);
     KM_CHECK_LAUNCH("interpolation: plan launch");
-    nodes_lambda_kernel<<<(unsigned)boxes, 128, 0, s>>>(a);
+    nodes_lambda_kernel<<<(unsigned)(boxes * (l.block / 128)), 128, 0, s>>>(a);
     KM_CHECK_LAUNCH("interpolation: Lagrange matrices launch");
     return KM_OK;
 }
@@ -1042,11 +1207,11 @@ static size_t grad_direct_bytes(int kernel_type, const NodesCall &c) {
     return c.k >= 8 ? km_grad_tc_workspace_bytes(c.kb, c.m, c.n, c.k, c.right) : km_grad_workspace_bytes(kernel_type, c.kb, c.m);
 }
 
-static NodesLayout nodes_layout(const NodesCall &c, const Batch &b, size_t direct_bytes) {
+static NodesLayout nodes_layout(const NodesCall &c, const Batch &b, bool all_columns, size_t direct_bytes) {
     View<const float> left;
     if (c.left) left = make_view<const float>(c.left, b);
     return NodesLayout(b, c.m, c.n, c.k, make_view<const float>(c.x1, b), make_view<const float>(c.x2, b), c.left ? &left : nullptr,
-                       make_view<const float>(c.right, b), direct_bytes);
+                       make_view<const float>(c.right, b), all_columns, direct_bytes);
 }
 
 static NodesArgs nodes_args(const NodesCall &c, const Batch &b) {
@@ -1062,25 +1227,25 @@ static NodesArgs nodes_args(const NodesCall &c, const Batch &b) {
 }  // namespace km
 
 extern "C" size_t km_matmul_nodes_workspace_bytes(const km_batch *batch, int64_t m, int64_t n, int64_t k, const km_view *x1,
-                                                  const km_view *x2, const km_view *rhs) {
+                                                  const km_view *x2, const km_view *rhs, int32_t all_columns) {
     using namespace km;
     Batch b;
     if (!batch || !x1 || !x2 || !rhs || m < 1 || n < 1 || k < 1 || make_batch(batch, &b) != KM_OK || b.count < 1) return 0;
     const NodesCall c = {m, n, k, batch, x1, x2, nullptr, rhs, nullptr, nullptr, nullptr};
-    const NodesLayout l = nodes_layout(c, b, product_direct_bytes(c));
+    const NodesLayout l = nodes_layout(c, b, all_columns != 0, product_direct_bytes(c));
     return nodes_fit(b, m, n, k, l) ? l.total : 0;
 }
 
 extern "C" int km_matmul_nodes_f32(int kernel_type, const km_batch *batch, int64_t m, int64_t n, int64_t k, const km_view *x1,
                                    const km_view *x2, const km_view *rhs, const km_view *params, const km_view *start,
-                                   const km_view *end, const km_view *out, void *workspace, size_t workspace_bytes, void *stream) {
+                                   const km_view *end, const km_view *out, int32_t all_columns, void *workspace, size_t workspace_bytes, void *stream) {
     using namespace km;
     Batch b;
     const NodesCall c = {m, n, k, batch, x1, x2, nullptr, rhs, params, start, end};
     int rc = nodes_arguments("km_matmul_nodes_f32", kernel_type, c, &b);
     if (rc != KM_OK) return rc;
     KM_REQUIRE(out && out->data, KM_ERR_INVALID_ARGUMENT, "km_matmul_nodes_f32: null argument");
-    const NodesLayout l = nodes_layout(c, b, product_direct_bytes(c));
+    const NodesLayout l = nodes_layout(c, b, all_columns != 0, product_direct_bytes(c));
     KM_REQUIRE(nodes_fit(b, m, n, k, l), KM_ERR_UNSUPPORTED, "km_matmul_nodes_f32: too large");
     KM_REQUIRE(workspace != nullptr && workspace_bytes >= l.total && (uintptr_t)workspace % 256 == 0, KM_ERR_WORKSPACE,
                "km_matmul_nodes_f32: workspace of %zu bytes needed (256-byte aligned), %zu given", l.total, workspace_bytes);
@@ -1111,26 +1276,27 @@ extern "C" int km_matmul_nodes_f32(int kernel_type, const km_batch *batch, int64
 }
 
 extern "C" size_t km_grad_nodes_workspace_bytes(int kernel_type, const km_batch *batch, int64_t m, int64_t n, int64_t k,
-                                                const km_view *x1, const km_view *x2, const km_view *left, const km_view *right) {
+                                                const km_view *x1, const km_view *x2, const km_view *left, const km_view *right,
+                                                int32_t all_columns) {
     using namespace km;
     Batch b;
     if (!batch || !x1 || !x2 || !left || !right || m < 1 || n < 1 || k < 1 || make_batch(batch, &b) != KM_OK || b.count < 1) return 0;
     const NodesCall c = {m, n, k, batch, x1, x2, left, right, nullptr, nullptr, nullptr};
-    const NodesLayout l = nodes_layout(c, b, grad_direct_bytes(kernel_type, c));
+    const NodesLayout l = nodes_layout(c, b, all_columns != 0, grad_direct_bytes(kernel_type, c));
     return nodes_fit(b, m, n, k, l) ? l.total : 0;
 }
 
 extern "C" int km_bilinear_derivative_nodes_f32(int kernel_type, const km_batch *batch, int64_t m, int64_t n, int64_t k,
                                                 const km_view *x1, const km_view *x2, const km_view *left, const km_view *right,
                                                 const km_view *params, const km_view *start, const km_view *end,
-                                                const km_view *grad, void *workspace, size_t workspace_bytes, void *stream) {
+                                                const km_view *grad, int32_t all_columns, void *workspace, size_t workspace_bytes, void *stream) {
     using namespace km;
     Batch b;
     const NodesCall c = {m, n, k, batch, x1, x2, left, right, params, start, end};
     KM_REQUIRE(left != nullptr && grad && grad->data, KM_ERR_INVALID_ARGUMENT, "km_bilinear_derivative_nodes_f32: null argument");
     int rc = nodes_arguments("km_bilinear_derivative_nodes_f32", kernel_type, c, &b);
     if (rc != KM_OK) return rc;
-    const NodesLayout l = nodes_layout(c, b, grad_direct_bytes(kernel_type, c));
+    const NodesLayout l = nodes_layout(c, b, all_columns != 0, grad_direct_bytes(kernel_type, c));
     KM_REQUIRE(nodes_fit(b, m, n, k, l), KM_ERR_UNSUPPORTED, "km_bilinear_derivative_nodes_f32: too large");
     KM_REQUIRE(workspace != nullptr && workspace_bytes >= l.total && (uintptr_t)workspace % 256 == 0, KM_ERR_WORKSPACE,
                "km_bilinear_derivative_nodes_f32: workspace of %zu bytes needed (256-byte aligned), %zu given", l.total, workspace_bytes);

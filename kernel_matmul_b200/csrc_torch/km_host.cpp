@@ -136,12 +136,12 @@ Tensor matmul(int64_t kernel_type, const Tensor &x1, const Tensor &x2, const Ten
     const c10::cuda::CUDAGuard guard(x1.device());
     Tensor out = p.empty({p.m, k}, x1);
     const km_view vr = p.view(rhs, 2), vo = p.view(out, 2);
-    if (path == PATH_NODES || (path == PATH_AUTO && p.items() >= NODES_MIN_ITEMS)) {
-        const size_t bytes = km_matmul_nodes_workspace_bytes(&p.kb, p.m, p.n, k, &p.x1, &p.x2, &vr);
+    if (p.try_nodes(path)) {
+        const size_t bytes = km_matmul_nodes_workspace_bytes(&p.kb, p.m, p.n, k, &p.x1, &p.x2, &vr, p.one_range());
         if (bytes > 0) {
             Tensor ws = workspace(x1, bytes);
-            raise_on(km_matmul_nodes_f32(p.kid, &p.kb, p.m, p.n, k, &p.x1, &p.x2, &vr, &p.params, &p.start, &p.end, &vo, ws.data_ptr(),
-                                         ws.numel(), p.stream()));
+            raise_on(km_matmul_nodes_f32(p.kid, &p.kb, p.m, p.n, k, &p.x1, &p.x2, &vr, &p.params, &p.start, &p.end, &vo, p.one_range(),
+                                         ws.data_ptr(), ws.numel(), p.stream()));
             return out;
         }
     }
@@ -167,12 +167,12 @@ Tensor bilinear(int64_t kernel_type, const Tensor &x1, const Tensor &x2, const T
     const c10::cuda::CUDAGuard guard(x1.device());
     Tensor grad = p.empty({num_params(kernel_type)}, x1);
     const km_view vl = p.view(left, 2), vr = p.view(right, 2), vg = p.view(grad, 1);
-    if (path == PATH_NODES || (path == PATH_AUTO && p.items() >= NODES_MIN_ITEMS)) {
-        const size_t bytes = km_grad_nodes_workspace_bytes(p.kid, &p.kb, p.m, p.n, k, &p.x1, &p.x2, &vl, &vr);
+    if (p.try_nodes(path)) {
+        const size_t bytes = km_grad_nodes_workspace_bytes(p.kid, &p.kb, p.m, p.n, k, &p.x1, &p.x2, &vl, &vr, p.one_range());
         if (bytes > 0) {
             Tensor ws = workspace(x1, bytes);
             raise_on(km_bilinear_derivative_nodes_f32(p.kid, &p.kb, p.m, p.n, k, &p.x1, &p.x2, &vl, &vr, &p.params, &p.start, &p.end, &vg,
-                                                      ws.data_ptr(), ws.numel(), p.stream()));
+                                                      p.one_range(), ws.data_ptr(), ws.numel(), p.stream()));
             return grad;
         }
     }

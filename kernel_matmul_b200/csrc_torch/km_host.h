@@ -45,6 +45,8 @@ constexpr int64_t TENSOR_CORE_MIN_K = 9, GRAD_TENSOR_CORE_MIN_K = 8, TENSOR_CORE
 // (batch, row block) items from which the automatic path tries blockwise interpolation
 // (km_matmul_nodes_f32): its four small passes take about 10 us more than they save below.
 constexpr int64_t NODES_MIN_ITEMS = 512;
+// Without a cutoff: kernel entries from which it does (the points have to be put in order first).
+constexpr int64_t NODES_MIN_ENTRIES = 1LL << 27;
 
 void check_f32(const Tensor &x);
 void check_i32(const Tensor &x);
@@ -71,6 +73,14 @@ struct Problem {
     km_view view(const Tensor &t, int nonbatch);
     Tensor empty(std::initializer_list<int64_t> tail, const Tensor &like) const;
     int64_t items() const;
+    // Every row block has the same range (ranges.make_ranges without a cutoff says so by the stride of
+    // start and end): all columns, presumably.
+    bool one_range() const { return row_blocks > 1 && start.stride[0] == 0 && end.stride[0] == 0; }
+    bool try_nodes(int64_t path) const {
+        if (path == PATH_NODES) return true;
+        if (path != PATH_AUTO) return false;
+        return one_range() ? m * n * (items() / row_blocks) >= NODES_MIN_ENTRIES : items() >= NODES_MIN_ITEMS;
+    }
     void *stream() const { return c10::cuda::getCurrentCUDAStream(device).stream(); }
 
   private:

@@ -57,8 +57,9 @@ def make_ranges(
     rows = int(math.ceil(m / block_size))
     if cutoff is None:
         n = x2.shape[-1] if x2 is not None else m
-        start = torch.zeros(*batch_shape, rows, dtype=torch.int32, device=out_device)
-        end = torch.full((*batch_shape, rows), n, dtype=torch.int32, device=out_device)
+        # one value for all row blocks: its stride tells the products that there is only one range
+        start = torch.zeros(1, dtype=torch.int32, device=out_device).expand(*batch_shape, rows)
+        end = torch.full((1,), n, dtype=torch.int32, device=out_device).expand(*batch_shape, rows)
         return start, end
 
     dev = _device_for(x1)
