@@ -2,7 +2,9 @@
 // autograd Functions (kernel_matmul/linear_operator.py:22-76; its index backward unpacks eight saved
 // tensors into seven names, :71-72, which fails as soon as batch indices are present).  In C++ the
 // backward of a training step runs without the interpreter.
+#include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <torch/csrc/autograd/custom_function.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 
 #include "km_host.h"
 
@@ -67,10 +69,10 @@ struct IndexFunction : torch::autograd::Function<IndexFunction> {
     }
 };
 
-// params (batch.., P) and, with `cutoff_factor` > 0, the cutoff of the largest lengthscale.
+// params (batch.., P) and, with a `cutoff_factor`, the cutoff of the largest lengthscale.
 struct PositiveParams : torch::autograd::Function<PositiveParams> {
     static variable_list forward(AutogradContext *ctx, at::TensorList raw_in, double lower_bound, int64_t lengthscales,
-                                 double cutoff_factor) {
+                                 std::optional<double> cutoff_factor) {
         std::vector<Tensor> raw;
         const float *ptr[KM_MAX_PARAMS];
         TORCH_CHECK(raw_in.size() >= 1 && raw_in.size() <= KM_MAX_PARAMS, "1 to ", KM_MAX_PARAMS, " raw parameters");
@@ -86,7 +88,7 @@ struct PositiveParams : torch::autograd::Function<PositiveParams> {
         const auto opt = raw[0].options().requires_grad(false);
         Tensor params = at::empty(shape, opt), cutoff = at::empty({1}, opt);
         raise_on(km_positive_params_f32((int32_t)raw.size(), raw[0].numel(), ptr, (float)lower_bound, params.data_ptr<float>(),
-                                        (uint32_t)lengthscales, cutoff_factor, cutoff_factor > 0 ? cutoff.data_ptr<float>() : nullptr,
+                                        (uint32_t)lengthscales, cutoff_factor.value_or(0.0), cutoff_factor ? cutoff.data_ptr<float>() : nullptr,
                                         c10::cuda::getCurrentCUDAStream(raw[0].device().index()).stream()));
         ctx->save_for_backward(raw);
         ctx->mark_non_differentiable({cutoff});
@@ -98,6 +100,11 @@ struct PositiveParams : torch::autograd::Function<PositiveParams> {
         const c10::cuda::CUDAGuard guard(raw[0].device());
         variable_list out(raw.size() + 3);
         if (!g.defined()) return out;
+        if (at::GradMode::is_enabled()) {  // (create_graph: the gradient itself is differentiable)
+            for (size_t q = 0; q < raw.size(); q++)
+                out[q] = at::where(raw[q] > 20.0, g.select(-1, (int64_t)q), g.select(-1, (int64_t)q) * at::sigmoid(raw[q]));
+            return out;
+        }
         const float *ptr[KM_MAX_PARAMS];
         float *to[KM_MAX_PARAMS];
         Tensor flat = g.reshape({-1, (int64_t)raw.size()});
@@ -112,10 +119,11 @@ struct PositiveParams : torch::autograd::Function<PositiveParams> {
     }
 };
 
+// Whether a call has to go through the autograd function: for a gradient, or -- so that it is refused
+// there, not ignored -- for a forward-mode tangent.
 static bool recording(std::initializer_list<const Tensor *> inputs) {
-    if (!at::GradMode::is_enabled()) return false;
     for (const Tensor *t : inputs)
-        if (t->requires_grad()) return true;
+        if ((t->requires_grad() && at::GradMode::is_enabled()) || t->_fw_grad(0).defined()) return true;
     return false;
 }
 
@@ -136,10 +144,31 @@ Tensor index_ad(int64_t kernel_type, const Tensor &x1, const Tensor &x2, const T
     return IndexFunction::apply(x1, x2, params, start, end, batch_indices, row, col, kernel_type);
 }
 
+// Tensors on which the kernels of PositiveParams cannot stand in for tensor expressions: under jit
+// tracing, forward-mode differentiation, torch.func transforms, dispatch modes and subclasses, or empty.
+static bool needs_expressions(const std::vector<Tensor> &raw) {
+    constexpr c10::DispatchKeySet wrapped({c10::DispatchKey::Python, c10::DispatchKey::FuncTorchBatched,
+                                           c10::DispatchKey::FuncTorchGradWrapper, c10::DispatchKey::Functionalize});
+    if (torch::jit::tracer::isTracing() || c10::impl::TorchDispatchModeTLS::any_modes_set()) return true;
+    for (const Tensor &t : raw)
+        if (t.key_set().has_any(wrapped) || t.numel() == 0 || t._fw_grad(0).defined()) return true;
+    return false;
+}
+
 std::pair<Tensor, Tensor> positive_params(const std::vector<Tensor> &raw, double lower_bound, int64_t lengthscales,
-                                          double cutoff_factor) {
-    variable_list r = PositiveParams::apply(at::TensorList(raw), lower_bound, lengthscales, cutoff_factor);
-    return {r[0], r[1]};
+                                          std::optional<double> cutoff_factor) {
+    if (!needs_expressions(raw)) {
+        variable_list r = PositiveParams::apply(at::TensorList(raw), lower_bound, lengthscales, cutoff_factor);
+        return {r[0], r[1]};
+    }
+    std::vector<Tensor> values, largest;
+    for (size_t q = 0; q < raw.size(); q++) {
+        values.push_back(at::softplus(raw[q]) + lower_bound);
+        if (cutoff_factor && ((lengthscales >> q) & 1)) largest.push_back(values.back().detach().max());
+    }
+    Tensor cutoff;
+    if (!largest.empty()) cutoff = (at::stack(largest).max().to(at::kDouble) * *cutoff_factor).to(at::kFloat).reshape({1});
+    return {at::stack(values, -1), cutoff};
 }
 
 }  // namespace kmh

@@ -131,8 +131,9 @@ Tensor matmul_ad(int64_t kernel_type, const Tensor &x1, const Tensor &x2, const 
 Tensor dense_ad(int64_t kernel_type, const Tensor &x1, const Tensor &x2, const Tensor &params, const Tensor &start, const Tensor &end);
 Tensor index_ad(int64_t kernel_type, const Tensor &x1, const Tensor &x2, const Tensor &params, const Tensor &start,
                 const Tensor &end, const std::vector<Tensor> &batch_indices, const Tensor &row, const Tensor &col);
-// (batch.., P) parameters lower_bound + softplus(raw[q]) and, where cutoff_factor > 0, the (1,) tensor
+// (batch.., P) parameters lower_bound + softplus(raw[q]) and, with a cutoff_factor, the (1,) tensor
 // cutoff_factor * the largest value among the parameters whose bit is set in `lengthscales`
-std::pair<Tensor, Tensor> positive_params(const std::vector<Tensor> &raw, double lower_bound, int64_t lengthscales, double cutoff_factor);
+std::pair<Tensor, Tensor> positive_params(const std::vector<Tensor> &raw, double lower_bound, int64_t lengthscales,
+                                          std::optional<double> cutoff_factor);
 
 }  // namespace kmh

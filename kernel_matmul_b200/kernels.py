@@ -106,7 +106,7 @@ class KernelMatmulModule(nn.Module):
         epsilon = self._epsilon
         if type(self).value is KernelMatmulModule.value and all(r.is_cuda and r.dtype == torch.float32 for r in raw):
             mask = sum(1 << i for i, name in enumerate(self._PARAMS) if name in self._LENGTHSCALES)
-            params, cutoff = _C.positive_params(raw, self.LOWER_BOUND, mask, 0.0 if epsilon is None else cutoff_factor(epsilon))
+            params, cutoff = _C.positive_params(raw, self.LOWER_BOUND, mask, None if epsilon is None else cutoff_factor(epsilon))
             return params, (self._cutoff if epsilon is None else cutoff)
         values = [self.value(name) for name in self._PARAMS]
         cutoff = self._cutoff if epsilon is None else dynamic_cutoff(epsilon, [self.value(name) for name in self._LENGTHSCALES]).reshape(1)

@@ -36,6 +36,49 @@ except Exception:  # noqa: BLE001 - absent or broken installation: operator-leve
     HAVE_LINEAR_OPERATOR = False
 
 
+class _TracedProduct(torch.autograd.Function):
+    """The op calls as calls that ``torch.jit.trace`` records (it sees nothing of the C++ functions, and
+    would keep their results as constants)."""
+
+    @staticmethod
+    def forward(ctx, x1v, x2v, rhs, params, start, end, kid):
+        ctx.save_for_backward(x1v, x2v, rhs, params, start, end)
+        ctx.kid = kid
+        return _C.op_matmul(kid, x1v, x2v, rhs, params, start, end, 0)[0]
+
+    @staticmethod
+    def backward(ctx, grad):
+        x1v, x2v, rhs, params, start, end = ctx.saved_tensors
+        g = _C.op_bilinear(ctx.kid, x1v, x2v, grad, rhs, params, start, end, 0)[0]
+        return None, None, None, g.sum_to_size(params.shape), None, None, None
+
+
+class _TracedDense(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x1v, x2v, params, start, end, kid):
+        ctx.save_for_backward(x1v, x2v, params, start, end)
+        ctx.kid = kid
+        return _C.dense(kid, x1v, x2v, params, start, end)
+
+    @staticmethod
+    def backward(ctx, grad):
+        return None, None, _C.dense_bwd(ctx.kid, *ctx.saved_tensors, grad), None, None, None
+
+
+class _TracedIndex(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x1v, x2v, params, start, end, kid, row, col, *batch):
+        ctx.save_for_backward(x1v, x2v, params, start, end, row, col, *batch)
+        ctx.kid = kid
+        return _C.index(kid, x1v, x2v, params, start, end, list(batch), row, col)
+
+    @staticmethod
+    def backward(ctx, grad):
+        x1v, x2v, params, start, end, row, col, *batch = ctx.saved_tensors
+        g = _C.index_bwd(ctx.kid, x1v, x2v, params, start, end, batch, row, col, grad)
+        return None, None, g, None, None, None, None, None, *[None for _ in batch]
+
+
 class _OperatorCore:
     """State and arithmetic shared by the plain operator and the LinearOperator subclass."""
 
@@ -63,9 +106,13 @@ class _OperatorCore:
         n = self._x2.size(-2)
         if rhs.size(-2) != n:  # (a broadcast over the rows, or an error)
             rhs = rhs.expand(*rhs.shape[:-2], n, rhs.size(-1))
+        if torch.jit.is_tracing():
+            return _TracedProduct.apply(self._x1v, self._x2v, rhs, self._params, self._start, self._end, self._kid)
         return _C.matmul_ad(self._kid, self._x1v, self._x2v, rhs, self._params, self._start, self._end)
 
     def _core_to_dense(self) -> Tensor:
+        if torch.jit.is_tracing():
+            return _TracedDense.apply(self._x1v, self._x2v, self._params, self._start, self._end, self._kid)
         return _C.dense_ad(self._kid, self._x1v, self._x2v, self._params, self._start, self._end)
 
     def _core_bilinear_derivative(self, left_vecs: Tensor, right_vecs: Tensor) -> Tensor:
@@ -75,8 +122,10 @@ class _OperatorCore:
         def prepare(index: Tensor) -> Tensor:
             return index.to(device=self._x1.device, dtype=torch.int)
 
-        return _C.index_ad(self._kid, self._x1v, self._x2v, self._params, self._start, self._end,
-                           [prepare(b) for b in batch_indices], prepare(row_index), prepare(col_index))
+        row, col, batch = prepare(row_index), prepare(col_index), [prepare(b) for b in batch_indices]
+        if torch.jit.is_tracing():
+            return _TracedIndex.apply(self._x1v, self._x2v, self._params, self._start, self._end, self._kid, row, col, *batch)
+        return _C.index_ad(self._kid, self._x1v, self._x2v, self._params, self._start, self._end, batch, row, col)
 
     def _core_transpose_args(self):
         start_t, end_t = ranges.transpose_ranges(self._start, self._end, self._x1.size(-2), self._x2.size(-2))
