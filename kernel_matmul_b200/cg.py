@@ -267,8 +267,9 @@ class ShardedOperator:
             return call
 
         def matvec_rows(v: Tensor, rb_begin: int, rb_count: int, out: Tensor) -> None:
-            if nodes is not None and (rb_begin, rb_count) == (begin, count) and v.is_contiguous() and out.is_contiguous():
-                nodes.matvec(v, out)
+            by_nodes = current_nodes() if (rb_begin, rb_count) == (begin, count) and v.is_contiguous() and out.is_contiguous() else None
+            if by_nodes is not None:
+                by_nodes.matvec(v, out)
             else:
                 rows_product(v, rb_begin, rb_count, out)()
 
@@ -281,19 +282,42 @@ class ShardedOperator:
         # the columns this rank's row blocks read, a checksum of the whole band, and how many nodes
         # per block and blocks per band a node operator would have (one host synchronisation, at
         # set-up only)
-        plan = _C.NodeOperator(KERNEL_TYPES.get(kernel_type, -1), x, params, start.reshape(-1)[:R], end.reshape(-1)[:R], begin, count)
-        lo, hi, checksum, node_count, widest = (int(v) for v in plan.plan().tolist())
-        if (not direct and n >= NODE_OPERATOR_MIN_ROWS and node_count > 0
-                and 4 * count * widest * node_count**2 <= NODE_OPERATOR_MAX_BYTES):
+        def plan_nodes():
+            plan = _C.NodeOperator(KERNEL_TYPES.get(kernel_type, -1), x, params, start.reshape(-1)[:R], end.reshape(-1)[:R], begin, count)
+            return (plan, *(int(v) for v in plan.plan().tolist()))
+
+        def versions():
+            return tuple(None if t.is_inference() else t._version for t in (x, params, start, end))
+
+        def usable(node_count: int, widest: int) -> bool:
+            return (not direct and n >= NODE_OPERATOR_MIN_ROWS and node_count > 0
+                    and 4 * count * widest * node_count**2 <= NODE_OPERATOR_MAX_BYTES)
+
+        laid_out = versions()
+        plan, lo, hi, checksum, node_count, widest = plan_nodes()
+        if usable(node_count, widest):
             plan.build(lo, hi, node_count, widest)
             nodes = plan
         elif phases and batched and count > 0:
             phase_ws = ops.prepare_sum_phases(kernel_type, x, x, params, rows=(begin * BLOCK_SIZE, min(n, (begin + count) * BLOCK_SIZE)),
                                               cols=(max(0, min(lo, n)), max(0, min(hi, n))))
+
+        def current_nodes():
+            """The node operator, laid out again if points, parameters or band were written to since;
+            ``None``: the products evaluate the kernels."""
+            nonlocal nodes, laid_out
+            if nodes is not None and versions() != laid_out:
+                laid_out = versions()
+                again, now_lo, now_hi, _, node_count, widest = plan_nodes()
+                if usable(node_count, widest):
+                    again.build(now_lo, now_hi, node_count, widest)
+                nodes = again if usable(node_count, widest) else None
+            return nodes
+
         op = cls(n, sigma2, matvec_rows, group=group, device=x.device, col_range=(lo, hi) if count > 0 else (0, 0),
                  band_checksum=checksum, mode=mode)
         op.phase_workspace = phase_ws  # (None: the products evaluate the phase vectors themselves)
-        op.node_operator = nodes
+        op.current_nodes = current_nodes
         op.rows_product = rows_product
         return op
 
@@ -417,7 +441,7 @@ class CGSolver:
                 getattr(op, "rows_product", None) is not None:
             from . import _C
 
-            nodes = op.node_operator
+            nodes = op.current_nodes()
             rows = None if nodes is not None else op.rows_product(self.p[: op.n], op.begin, op.count, self.kp[op.row0: op.row1])
             state = _C.CgState(self.x, self.r, self.p, self.kp, self.bp, self.rs, self.ynorm, self.history, self.alphas, self.betas,
                                self.send1, self.send2, op.n, self.k, op.count, op.seg_blocks, op.segs_per_rank, op.sigma2)

@@ -41,44 +41,45 @@ void NodeOperator::build(int64_t lo, int64_t hi, int64_t nodes, int64_t max_bloc
                                         P_, max_blocks_, lambda_.data_ptr<float>(), matrix_.data_ptr<float>(), stream()));
 }
 
-float *NodeOperator::nodes(int64_t k) {
-    const int64_t need = R_ * P_ * ((k + 3) / 4 * 4);
-    if (!nodes_.defined() || nodes_.numel() < need) nodes_ = at::empty({need}, x_.options().requires_grad(false));
-    return nodes_.data_ptr<float>();
+// Scratch of a product: one per call or run, on its stream, so that an operator may be applied on several
+// streams and threads at a time.
+Tensor NodeOperator::nodes(int64_t k) const {
+    return at::empty({R_ * P_ * ((k + 3) / 4 * 4)}, x_.options().requires_grad(false));
 }
 
-void NodeOperator::compress(const Tensor &v, int64_t k) {
-    raise_on(km_node_compress_f32(k, n_, P_, lambda_.const_data_ptr<float>(), v.const_data_ptr<float>(), nodes(k), blk0_, blk1_, stream()));
+void NodeOperator::compress(const Tensor &v, int64_t k, float *nodes) const {
+    raise_on(km_node_compress_f32(k, n_, P_, lambda_.const_data_ptr<float>(), v.const_data_ptr<float>(), nodes, blk0_, blk1_, stream()));
 }
 
-void NodeOperator::update_p(const CgState &s, int64_t it) {
+void NodeOperator::update_p(const CgState &s, int64_t it, float *nodes) const {
     const int64_t k = s.k;
-    raise_on(km_node_update_p_f32(k, n_, P_, lambda_.const_data_ptr<float>(), s.p.data_ptr<float>(), s.r.const_data_ptr<float>(), nodes(k), 0, R_,
+    raise_on(km_node_update_p_f32(k, n_, P_, lambda_.const_data_ptr<float>(), s.p.data_ptr<float>(), s.r.const_data_ptr<float>(), nodes, 0, R_,
                                   s.send2.data_ptr(), s.send2.numel(), 1, (int32_t)s.slots, s.rs_row(it), s.rs_row(it + 1),
                                   s.ynorm.const_data_ptr<float>(), s.row(s.history, it + 1), s.row(s.betas, it), stream()));
 }
 
-void NodeOperator::product(int64_t k, float *out, const float *p, double sigma2, float *block_partials) {
+void NodeOperator::product(int64_t k, const float *nodes, float *out, const float *p, double sigma2, float *block_partials) const {
     raise_on(km_node_product_f32(k, n_, P_, max_blocks_, start_.const_data_ptr<int32_t>(), end_.const_data_ptr<int32_t>(),
-                                 lambda_.const_data_ptr<float>(), matrix_.const_data_ptr<float>(), nodes(k), begin_, count_, out, p, (float)sigma2,
+                                 lambda_.const_data_ptr<float>(), matrix_.const_data_ptr<float>(), nodes, begin_, count_, out, p, (float)sigma2,
                                  block_partials, stream()));
 }
 
-void NodeOperator::matvec(const Tensor &v, const Tensor &out) {
+void NodeOperator::matvec(const Tensor &v, const Tensor &out) const {
     check_f32(v), check_f32(out);
     TORCH_CHECK(v.dim() == 2 && v.size(0) == n_ && v.is_contiguous() && out.dim() == 2 && out.is_contiguous() && out.size(1) == v.size(1),
                 "v must be a contiguous (n, k) tensor and out (rows, k)");
     const int64_t rows = std::max<int64_t>(0, std::min(n_, (begin_ + count_) * KM_BLOCK_SIZE) - begin_ * KM_BLOCK_SIZE);
     TORCH_CHECK(out.size(0) == rows, "out must have ", rows, " rows");
     const c10::cuda::CUDAGuard guard(x_.device());
-    compress(v, v.size(1));
-    product(v.size(1), out.data_ptr<float>(), nullptr, 0.0, nullptr);
+    const Tensor scratch = nodes(v.size(1));
+    compress(v, v.size(1), scratch.data_ptr<float>());
+    product(v.size(1), scratch.const_data_ptr<float>(), out.data_ptr<float>(), nullptr, 0.0, nullptr);
 }
 
 // Iterations first .. first + count - 1 of a solve on one GPU: what CGSolver.step() does, from here.  With
 // `nodes` the product, q and the partial sums of p . q are one kernel, and the update of p and its
 // compression another; otherwise `rows` is the product.
-void cg_run(const CgState &s, NodeOperator *nodes, RowsProduct *rows, int64_t first, int64_t count) {
+void cg_run(const CgState &s, const NodeOperator *nodes, RowsProduct *rows, int64_t first, int64_t count) {
     const c10::cuda::CUDAGuard guard(s.p.device());
     void *stream = c10::cuda::getCurrentCUDAStream(s.p.device().index()).stream();
     const int64_t k = s.k, n = s.n;
@@ -88,10 +89,12 @@ void cg_run(const CgState &s, NodeOperator *nodes, RowsProduct *rows, int64_t fi
         raise_on(km_cg_segment_sums_f32(k, bp, s.blocks, s.seg_blocks, static_cast<double *>(to.data_ptr()), stream));
     };
     TORCH_CHECK((nodes != nullptr) != (rows != nullptr), "one kind of product");
+    const Tensor scratch = nodes != nullptr ? nodes->nodes(k) : Tensor();
+    float *at_nodes = nodes != nullptr ? scratch.data_ptr<float>() : nullptr;
     for (int64_t it = first; it < first + count; it++) {
         if (nodes != nullptr) {
-            if (it == first) nodes->compress(s.p, k);
-            nodes->product(k, q, p, s.sigma2, bp);
+            if (it == first) nodes->compress(s.p, k, at_nodes);
+            nodes->product(k, at_nodes, q, p, s.sigma2, bp);
         } else {
             rows->run();
             raise_on(km_cg_q_dots_f32(k, q, p, (float)s.sigma2, 0, n, bp, nullptr, 0, nullptr, 0, stream));
@@ -101,7 +104,7 @@ void cg_run(const CgState &s, NodeOperator *nodes, RowsProduct *rows, int64_t fi
                                      s.rs_row(it), bp, s.row(s.alphas, it), stream));
         totals(s.send2);
         if (nodes != nullptr && it + 1 < first + count)
-            nodes->update_p(s, it);
+            nodes->update_p(s, it, at_nodes);
         else
             raise_on(km_cg_update_p_f32(k, p, r, 0, n, s.send2.data_ptr(), s.send2.numel(), 1, (int32_t)s.slots, s.rs_row(it), s.rs_row(it + 1),
                                         s.ynorm.const_data_ptr<float>(), s.row(s.history, it + 1), s.row(s.betas, it), stream));

@@ -22,23 +22,23 @@ class NodeOperator {
     Tensor plan() const { return plan_.slice(0, 0, 5); }
     void build(int64_t lo, int64_t hi, int64_t nodes, int64_t max_blocks);
     // out = the window's rows of K v
-    void matvec(const Tensor &v, const Tensor &out);
+    void matvec(const Tensor &v, const Tensor &out) const;
 
-    void compress(const Tensor &v, int64_t k);
-    void update_p(const CgState &s, int64_t it);
-    void product(int64_t k, float *out, const float *p, double sigma2, float *block_partials);
+    Tensor nodes(int64_t k) const;
+    void compress(const Tensor &v, int64_t k, float *nodes) const;
+    void update_p(const CgState &s, int64_t it, float *nodes) const;
+    void product(int64_t k, const float *nodes, float *out, const float *p, double sigma2, float *block_partials) const;
 
   private:
-    float *nodes(int64_t k);
     void *stream() const { return c10::cuda::getCurrentCUDAStream(x_.device().index()).stream(); }
     int kid_;
     int64_t n_, R_, begin_, count_, P_ = 0, max_blocks_ = 0, blk0_ = 0, blk1_ = 0;
-    Tensor x_, params_, start_, end_, centre_, plan_, lambda_, matrix_, nodes_;
+    Tensor x_, params_, start_, end_, centre_, plan_, lambda_, matrix_;
     km_batch kb_{};
     km_view vparams_{};
 };
 
-void cg_run(const CgState &s, NodeOperator *nodes, RowsProduct *rows, int64_t first, int64_t count);
+void cg_run(const CgState &s, const NodeOperator *nodes, RowsProduct *rows, int64_t first, int64_t count);
 
 // z_c^T log(A) z_c for every column of a CG run, fp64 on the device
 Tensor log_forms(const Tensor &alphas, const Tensor &betas, const Tensor &residual_norms, const Tensor &z_norm2, double converged);
