@@ -84,6 +84,9 @@ Problem::Problem(int64_t kernel_type, const Tensor &tx1, const Tensor &tx2, cons
         for (size_t d = 0; d < batch.size(); d++) kb.size[d] = batch[d];
     }
     x1 = view(tx1, 1), x2 = view(tx2, 1), params = view(tparams, 1), start = view(tstart, 1), end = view(tend, 1);
+    all_columns_ = row_blocks > 1 && tstart.storage_offset() > 0 && tend.storage_offset() == 0 && tstart.strides() == tend.strides() &&
+                   tstart.is_alias_of(tend) &&
+                   tstart.storage().nbytes() == 2 * sizeof(int32_t) * (size_t)tstart.storage_offset();
 }
 
 int64_t Problem::items() const {

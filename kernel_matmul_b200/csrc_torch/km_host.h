@@ -73,9 +73,10 @@ struct Problem {
     km_view view(const Tensor &t, int nonbatch);
     Tensor empty(std::initializer_list<int64_t> tail, const Tensor &like) const;
     int64_t items() const;
-    // Every row block has the same range (ranges.make_ranges without a cutoff says so by the stride of
-    // start and end): all columns, presumably.
-    bool one_range() const { return row_blocks > 1 && start.stride[0] == 0 && end.stride[0] == 0; }
+    // Presumably every row block sees all columns: the ranges come from ranges.make_ranges without a
+    // cutoff, which lays them out as the two halves of one storage, end first.  (A hint: the values are
+    // looked at on the device.)
+    bool one_range() const { return all_columns_; }
     bool try_nodes(int64_t path) const {
         if (path == PATH_NODES) return true;
         if (path != PATH_AUTO) return false;
@@ -84,7 +85,7 @@ struct Problem {
     void *stream() const { return c10::cuda::getCurrentCUDAStream(device).stream(); }
 
   private:
-    bool flat_ = false;
+    bool flat_ = false, all_columns_ = false;
 };
 
 Tensor workspace(const Tensor &like, size_t bytes);

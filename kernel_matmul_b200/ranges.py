@@ -57,9 +57,10 @@ def make_ranges(
     rows = int(math.ceil(m / block_size))
     if cutoff is None:
         n = x2.shape[-1] if x2 is not None else m
-        # one value for all row blocks: its stride tells the products that there is only one range
-        start = torch.zeros(1, dtype=torch.int32, device=out_device).expand(*batch_shape, rows)
-        end = torch.full((1,), n, dtype=torch.int32, device=out_device).expand(*batch_shape, rows)
+        # both in one storage, end first: tells the products that it is presumably all columns (the
+        # values are looked at on the device all the same)
+        both = torch.empty(2, *batch_shape, rows, dtype=torch.int32, device=out_device)
+        end, start = both[0].fill_(n), both[1].zero_()
         return start, end
 
     dev = _device_for(x1)
