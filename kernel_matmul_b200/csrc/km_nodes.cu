@@ -424,7 +424,7 @@ struct CompressShape {
 template <int COLS>
 __global__ void __launch_bounds__(128) nodes_compress_kernel(const CompressArgs p) {
     const NodesArgs &a = p.a;
-    if (!a.hdr->use) return;
+    if (!__shfl_sync(0xffffffffu, a.hdr->use, 0)) return;  // (warp-uniform: another CTA may clear it meanwhile)
     constexpr int STAGE = CompressShape<COLS>::STAGE;
     extern __shared__ __align__(16) float smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -441,6 +441,7 @@ __global__ void __launch_bounds__(128) nodes_compress_kernel(const CompressArgs 
     const bool shared = p.slots == 1;
     const int c0 = shared ? a.hdr->first[level] : a.classes[slot * NODES_LEVELS + level], c1 = shared ? a.hdr->first[level + 1] : c0 + 1;
     const int row_count = (int)min((int64_t)a.block, p.rows - row0), steps = (row_count + CP_ROWS - 1) / CP_ROWS;
+    bool finite = true;
 
     for (int cls = c0; cls < c1; cls++) {
         const int P = a.hdr->P[cls];
@@ -505,12 +506,20 @@ __global__ void __launch_bounds__(128) nodes_compress_kernel(const CompressArgs 
                 }
                 if (mine) {
 #pragma unroll
-                    for (int j = 0; j < 4; j++)
+                    for (int j = 0; j < 4; j++) {
                         if (j <= last) *reinterpret_cast<ulonglong2 *>(out + (q + j) * p.kq + c) = make_ulonglong2(acc[j][0], acc[j][1]);
+#pragma unroll
+                        for (int h = 0; h < 2; h++) {
+                            float v0, v1;
+                            unpack2(acc[j][h], v0, v1);
+                            finite = finite && fabsf(v0) <= NODES_MAX_OPERAND && fabsf(v1) <= NODES_MAX_OPERAND;
+                        }
+                    }
                 }
             }
         }
     }
+    if (!finite) a.hdr->use = 0;  // (the kernels after this one see it)
 }
 
 // What the product and the gradient at the nodes share.  A CTA of four warps works on one batch and KC

@@ -37,7 +37,12 @@ constexpr float NODES_EPS = 3e-8f;      // bound on the interpolation error, rel
 // by powers of NODES_RATIO.  The longest of some hundred blocks of uniform points is 1.3 times the mean.
 constexpr int NODES_LEVELS = 4;
 constexpr float NODES_RATIO = 1.15f;
-constexpr float NODES_MIN_H = 1e-18f;   // half-length given to an interval of coincident points
+// Half-length given to an interval of coincident points: short enough for the square of a distance between
+// its nodes to vanish, as that of the points does.
+constexpr float NODES_MIN_H = 1e-25f;
+// Operands that are not finite, or near overflow, at the nodes are left to the direct kernels: sums of
+// Lagrange polynomials of either sign would turn an infinity into NaN.
+constexpr float NODES_MAX_OPERAND = 1e30f;
 
 // Smallest P whose error bound is below NODES_EPS on an interval of half-length h; > NODES_MAX if
 // none (or for non-finite arguments).  `lane` of 32 lanes tries one rho; the result is in every lane.

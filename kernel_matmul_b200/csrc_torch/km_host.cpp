@@ -125,6 +125,15 @@ Tensor workspace(const Tensor &like, size_t bytes) {
     return at::empty({(int64_t)std::max<size_t>(bytes, 256)}, like.options().dtype(at::kByte).requires_grad(false));
 }
 
+// The same, or an undefined tensor where the device has not that much memory left.
+static Tensor workspace_if_free(const Tensor &like, size_t bytes) {
+    try {
+        return workspace(like, bytes);
+    } catch (const c10::OutOfMemoryError &) {
+        return Tensor();
+    }
+}
+
 static std::string shape_of(const Tensor &t) {
     std::ostringstream s;
     s << t.sizes();
@@ -141,8 +150,8 @@ Tensor matmul(int64_t kernel_type, const Tensor &x1, const Tensor &x2, const Ten
     const km_view vr = p.view(rhs, 2), vo = p.view(out, 2);
     if (p.try_nodes(path)) {
         const size_t bytes = km_matmul_nodes_workspace_bytes(&p.kb, p.m, p.n, k, &p.x1, &p.x2, &vr, p.one_range());
-        if (bytes > 0) {
-            Tensor ws = workspace(x1, bytes);
+        const Tensor ws = bytes > 0 ? workspace_if_free(x1, bytes) : Tensor();
+        if (ws.defined()) {
             raise_on(km_matmul_nodes_f32(p.kid, &p.kb, p.m, p.n, k, &p.x1, &p.x2, &vr, &p.params, &p.start, &p.end, &vo, p.one_range(),
                                          ws.data_ptr(), ws.numel(), p.stream()));
             return out;
@@ -172,8 +181,8 @@ Tensor bilinear(int64_t kernel_type, const Tensor &x1, const Tensor &x2, const T
     const km_view vl = p.view(left, 2), vr = p.view(right, 2), vg = p.view(grad, 1);
     if (p.try_nodes(path)) {
         const size_t bytes = km_grad_nodes_workspace_bytes(p.kid, &p.kb, p.m, p.n, k, &p.x1, &p.x2, &vl, &vr, p.one_range());
-        if (bytes > 0) {
-            Tensor ws = workspace(x1, bytes);
+        const Tensor ws = bytes > 0 ? workspace_if_free(x1, bytes) : Tensor();
+        if (ws.defined()) {
             raise_on(km_bilinear_derivative_nodes_f32(p.kid, &p.kb, p.m, p.n, k, &p.x1, &p.x2, &vl, &vr, &p.params, &p.start, &p.end, &vg,
                                                       p.one_range(), ws.data_ptr(), ws.numel(), p.stream()));
             return grad;
