@@ -357,6 +357,14 @@ KM_API int km_index_f32(int kernel_type, const km_batch *batch, int64_t m, int64
                  const int32_t *const *batch_indices, const int32_t *row, const int32_t *col,
                  float *out, void *stream);
 
+/* The same, and distances[l] = x1[row[l]] - x2[col[l]] (a marker where the lookup has no entry), for the
+ * gradient below: float[L]. */
+KM_API int km_index_distances_f32(int kernel_type, const km_batch *batch, int64_t m, int64_t n, int64_t L,
+                 const km_view *x1, const km_view *x2, const km_view *params,
+                 const km_view *start, const km_view *end,
+                 const int32_t *const *batch_indices, const int32_t *row, const int32_t *col,
+                 float *out, float *distances, void *stream);
+
 /* grad[b, q] = d/d theta_q sum_l [batch(l) == b] out_grad[l] * K[b, row[l], col[l]].  Replaces
  * index_bwd.call(..., out_grad) (native/index_bwd/index_bwd.cpp:6-27, index_bwd.cu:65-112).
  * grad (B.., P) every element written.  workspace: km_index_bwd_workspace_bytes(...) bytes. */
@@ -368,6 +376,11 @@ KM_API int km_index_bwd_f32(int kernel_type, const km_batch *batch, int64_t m, i
                      const int32_t *const *batch_indices, const int32_t *row,
                      const int32_t *col, const float *out_grad, const km_view *grad,
                      void *workspace, size_t workspace_bytes, void *stream);
+
+/* The same gradient from the distances that km_index_distances_f32 wrote for these lookups. */
+KM_API int km_index_bwd_distances_f32(int kernel_type, const km_batch *batch, int64_t L, const km_view *params,
+                     const int32_t *const *batch_indices, const float *distances, const float *out_grad,
+                     const km_view *grad, void *workspace, size_t workspace_bytes, void *stream);
 
 /* ---------------------------------------------------------------------------------------
  * Band construction on the device (the reference runs these on one CPU thread after a

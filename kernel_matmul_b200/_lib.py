@@ -92,6 +92,10 @@ def _load() -> ctypes.CDLL:
     lib.km_index_bwd_workspace_bytes.argtypes = [ctypes.c_int, bp]
     lib.km_index_bwd_f32.restype = ctypes.c_int
     lib.km_index_bwd_f32.argtypes = [ctypes.c_int, bp, i64, i64, i64, wp, wp, wp, wp, wp, pp, vp, vp, vp, wp, vp, sz, vp]
+    lib.km_index_distances_f32.restype = ctypes.c_int
+    lib.km_index_distances_f32.argtypes = [ctypes.c_int, bp, i64, i64, i64, wp, wp, wp, wp, wp, pp, vp, vp, vp, vp, vp]
+    lib.km_index_bwd_distances_f32.restype = ctypes.c_int
+    lib.km_index_bwd_distances_f32.argtypes = [ctypes.c_int, bp, i64, wp, pp, vp, vp, wp, vp, sz, vp]
     lib.km_make_ranges_f32.restype = ctypes.c_int
     lib.km_make_ranges_f32.argtypes = [i64, i64, i64, vp, vp, ctypes.c_float, i32, i32, vp, vp, vp, vp]
     lib.km_make_ranges_symmetric_f32.restype = ctypes.c_int
@@ -162,7 +166,7 @@ EXPORTED = [
     "km_bilinear_derivative_nodes_f32", "km_positive_params_f32", "km_positive_params_bwd_f32", "km_grad_workspace_bytes", "km_grad_tc_workspace_bytes", "km_bilinear_derivative_tc_f32",
     "km_matmul_bwd_tc_f32",
     "km_bilinear_derivative_f32", "km_bilinear_derivative_static_f32", "km_matmul_bwd_f32", "km_dense_f32", "km_dense_bwd_f32",
-    "km_index_f32", "km_index_bwd_workspace_bytes", "km_index_bwd_f32", "km_make_ranges_f32",
+    "km_index_f32", "km_index_bwd_workspace_bytes", "km_index_bwd_f32", "km_index_distances_f32", "km_index_bwd_distances_f32", "km_make_ranges_f32",
     "km_make_ranges_symmetric_f32", "km_make_ranges_symmetric_cutoffs_f32", "km_transpose_ranges_i32", "km_count_entries",
     "km_probe_fp32_peak", "km_probe_sfu_peak", "km_selftest_bounded_wait", "km_selftest_set_wait_polls",
     "km_cg_block_dots_f32", "km_cg_q_dots_f32", "km_cg_segment_sums_f32", "km_cg_init_scalars_f32", "km_cg_update_xr_f32",

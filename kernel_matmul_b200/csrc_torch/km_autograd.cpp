@@ -50,18 +50,20 @@ struct IndexFunction : torch::autograd::Function<IndexFunction> {
     static Tensor forward(AutogradContext *ctx, const Tensor &x1, const Tensor &x2, const Tensor &params, const Tensor &start,
                           const Tensor &end, const std::vector<Tensor> &batch_indices, const Tensor &row, const Tensor &col,
                           int64_t kernel_type) {
-        variable_list saved{x1, x2, params, start, end, row, col};
+        Tensor distances;
+        Tensor out = index(kernel_type, x1, x2, params, start, end, batch_indices, row, col, params.requires_grad() ? &distances : nullptr);
+        variable_list saved{x1, x2, params, start, end, row, col, distances};
         saved.insert(saved.end(), batch_indices.begin(), batch_indices.end());
         ctx->save_for_backward(std::move(saved));
         ctx->saved_data["kernel_type"] = kernel_type;
-        return index(kernel_type, x1, x2, params, start, end, batch_indices, row, col);
+        return out;
     }
     static variable_list backward(AutogradContext *ctx, variable_list grads) {
         const auto s = ctx->get_saved_variables();
         Tensor g;
         if (ctx->needs_input_grad(2))
-            g = at::sum_to(index_bwd(ctx->saved_data["kernel_type"].toInt(), s[0], s[1], s[2], s[3], s[4], {s.begin() + 7, s.end()},
-                                     s[5], s[6], grads[0]),
+            g = at::sum_to(index_bwd(ctx->saved_data["kernel_type"].toInt(), s[0], s[1], s[2], s[3], s[4], {s.begin() + 8, s.end()},
+                                     s[5], s[6], grads[0], s[7].defined() ? &s[7] : nullptr),
                            s[2].sizes());
         variable_list r(9);
         r[2] = g;

@@ -303,19 +303,25 @@ struct Lookups {
 };
 
 Tensor index(int64_t kernel_type, const Tensor &x1, const Tensor &x2, const Tensor &params, const Tensor &start, const Tensor &end,
-             const std::vector<Tensor> &batch_indices, const Tensor &row, const Tensor &col) {
+             const std::vector<Tensor> &batch_indices, const Tensor &row, const Tensor &col, Tensor *distances) {
     Problem p(kernel_type, x1, x2, params, start, end, {});
     Lookups l(p, "index", batch_indices, row, col);
     const c10::cuda::CUDAGuard guard(x1.device());
     Tensor out = at::empty(l.shape, x1.options().requires_grad(false));
-    raise_on(km_index_f32(p.kid, &p.kb, p.m, p.n, l.count, &p.x1, &p.x2, &p.params, &p.start, &p.end, l.batch, l.row, l.col,
-                          out.data_ptr<float>(), p.stream()));
+    if (distances != nullptr) {
+        *distances = at::empty(l.shape, x1.options().requires_grad(false));
+        raise_on(km_index_distances_f32(p.kid, &p.kb, p.m, p.n, l.count, &p.x1, &p.x2, &p.params, &p.start, &p.end, l.batch, l.row, l.col,
+                                        out.data_ptr<float>(), distances->data_ptr<float>(), p.stream()));
+    } else {
+        raise_on(km_index_f32(p.kid, &p.kb, p.m, p.n, l.count, &p.x1, &p.x2, &p.params, &p.start, &p.end, l.batch, l.row, l.col,
+                              out.data_ptr<float>(), p.stream()));
+    }
     return out;
 }
 
 Tensor index_bwd(int64_t kernel_type, const Tensor &x1, const Tensor &x2, const Tensor &params, const Tensor &start,
                  const Tensor &end, const std::vector<Tensor> &batch_indices, const Tensor &row, const Tensor &col,
-                 const Tensor &out_grad) {
+                 const Tensor &out_grad, const Tensor *distances) {
     Problem p(kernel_type, x1, x2, params, start, end, {});
     Lookups l(p, "index_bwd", batch_indices, row, col);
     check_f32(out_grad);
@@ -324,8 +330,14 @@ Tensor index_bwd(int64_t kernel_type, const Tensor &x1, const Tensor &x2, const 
     Tensor grad = p.empty({num_params(kernel_type)}, x1);
     const km_view vg = p.view(grad, 1);
     Tensor ws = workspace(x1, km_index_bwd_workspace_bytes(p.kid, &p.kb));
-    raise_on(km_index_bwd_f32(p.kid, &p.kb, p.m, p.n, l.count, &p.x1, &p.x2, &p.params, &p.start, &p.end, l.batch, l.row, l.col,
-                              og.const_data_ptr<float>(), &vg, ws.data_ptr(), ws.numel(), p.stream()));
+    if (distances != nullptr) {
+        const Tensor d = distances->contiguous();
+        raise_on(km_index_bwd_distances_f32(p.kid, &p.kb, l.count, &p.params, l.batch, d.const_data_ptr<float>(), og.const_data_ptr<float>(),
+                                            &vg, ws.data_ptr(), ws.numel(), p.stream()));
+    } else {
+        raise_on(km_index_bwd_f32(p.kid, &p.kb, p.m, p.n, l.count, &p.x1, &p.x2, &p.params, &p.start, &p.end, l.batch, l.row, l.col,
+                                  og.const_data_ptr<float>(), &vg, ws.data_ptr(), ws.numel(), p.stream()));
+    }
     return grad;
 }
 

@@ -99,11 +99,12 @@ Tensor bilinear(int64_t kernel_type, const Tensor &x1, const Tensor &x2, const T
 Tensor dense(int64_t kernel_type, const Tensor &x1, const Tensor &x2, const Tensor &params, const Tensor &start, const Tensor &end);
 Tensor dense_bwd(int64_t kernel_type, const Tensor &x1, const Tensor &x2, const Tensor &params, const Tensor &start,
                  const Tensor &end, const Tensor &out_grad);
+// `distances`: where to put the distances of the lookups, from which their gradient needs no points
 Tensor index(int64_t kernel_type, const Tensor &x1, const Tensor &x2, const Tensor &params, const Tensor &start, const Tensor &end,
-             const std::vector<Tensor> &batch_indices, const Tensor &row, const Tensor &col);
+             const std::vector<Tensor> &batch_indices, const Tensor &row, const Tensor &col, Tensor *distances = nullptr);
 Tensor index_bwd(int64_t kernel_type, const Tensor &x1, const Tensor &x2, const Tensor &params, const Tensor &start,
                  const Tensor &end, const std::vector<Tensor> &batch_indices, const Tensor &row, const Tensor &col,
-                 const Tensor &out_grad);
+                 const Tensor &out_grad, const Tensor *distances = nullptr);
 
 // matmul for a window of row blocks, optionally summed over the batch, with everything but the launch
 // done once: for loops that call the same product on the same buffers (whose contents change) many

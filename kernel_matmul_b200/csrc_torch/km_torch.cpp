@@ -185,8 +185,16 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
           nogil());
     m.def("dense", &kmh::dense, nogil());
     m.def("dense_bwd", &kmh::dense_bwd, nogil());
-    m.def("index", &kmh::index, nogil());
-    m.def("index_bwd", &kmh::index_bwd, nogil());
+    using torch::Tensor;
+    using Indices = std::vector<Tensor>;
+    m.def("index", [](int64_t kt, const Tensor &x1, const Tensor &x2, const Tensor &params, const Tensor &start, const Tensor &end,
+                      const Indices &batch, const Tensor &row, const Tensor &col) {
+        return kmh::index(kt, x1, x2, params, start, end, batch, row, col);
+    }, nogil());
+    m.def("index_bwd", [](int64_t kt, const Tensor &x1, const Tensor &x2, const Tensor &params, const Tensor &start, const Tensor &end,
+                          const Indices &batch, const Tensor &row, const Tensor &col, const Tensor &out_grad) {
+        return kmh::index_bwd(kt, x1, x2, params, start, end, batch, row, col, out_grad);
+    }, nogil());
     m.def("make_ranges", &make_ranges);
     m.def("make_ranges_symmetric", &make_ranges_symmetric);
     m.def("transpose_ranges", &transpose_ranges);
