@@ -229,6 +229,7 @@ __global__ void __launch_bounds__(32 * (128 / (32 * RPT)) * WN, 384 / (32 * (128
 template <int KT, int KB, int RPT, int WN>
 __global__ void __launch_bounds__(32 * (128 / (32 * RPT)) * WN)
     matmul_fma_cluster_kernel(const MatmulArgs<float> a) {
+    if (a.gate.closed()) return;
     constexpr int WM = 128 / (32 * RPT);
     constexpr int THREADS = 32 * WM * WN;
     extern __shared__ __align__(16) float smem[];

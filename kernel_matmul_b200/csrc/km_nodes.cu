@@ -79,9 +79,12 @@ __device__ __forceinline__ int nodes_needed_for(int kt, const float *theta, int6
 
 // Extents of every block (a warp each), alignment of every band, and -- the CTA that finishes last --
 // the number of nodes of every kernel of the batch at every half-length.
-__global__ void __launch_bounds__(256) nodes_plan_kernel(const NodesArgs a, int kernel_type) {
+// (Time is latency, most of it the last CTA's: 16 kernels on 512 blocks took 21 us with 256 threads and the
+// classes listed in shared memory.)
+constexpr int PLAN_THREADS = 512, PLAN_WARPS = PLAN_THREADS / 32;
+__global__ void __launch_bounds__(PLAN_THREADS) nodes_plan_kernel(const NodesArgs a, int kernel_type) {
     const int lane = threadIdx.x & 31;
-    const int64_t warps = (int64_t)gridDim.x * 8, first = blockIdx.x * 8LL + (threadIdx.x >> 5);
+    const int64_t warps = (int64_t)gridDim.x * PLAN_WARPS, first = blockIdx.x * (int64_t)PLAN_WARPS + (threadIdx.x >> 5);
     const int64_t boxes1 = a.slots1 * a.R, boxes = boxes1 + (a.same ? 0 : a.slots2 * a.C);
     float longest = 0.0f;
     int bad = 0;
@@ -94,8 +97,7 @@ __global__ void __launch_bounds__(256) nodes_plan_kernel(const NodesArgs a, int 
         float lo = INFINITY, hi = -INFINITY;
         bool nan = false;
         const int *order = one ? a.order1 : a.order2;
-#pragma unroll 4
-        for (int i = lane; i < a.block; i += 32) {
+        const auto see = [&](int i) {
             const int64_t row = block * a.block + i;
             if (row < rows) {
                 const float e = base[point_row(order, row) * x.s0];
@@ -103,6 +105,12 @@ __global__ void __launch_bounds__(256) nodes_plan_kernel(const NodesArgs a, int 
                 hi = fmaxf(hi, e);
                 nan = nan || !(fabsf(e) < INFINITY);
             }
+        };
+        if (order != nullptr) {  // in order: the first and the last point (all are finite, or `bad` is set)
+            if (lane < 2) see(lane == 0 ? 0 : (int)min((int64_t)a.block, rows - block * a.block) - 1);
+        } else {
+#pragma unroll
+            for (int i = 0; i < KM_BLOCK_SIZE; i += 32) see(i + lane);
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
@@ -140,7 +148,7 @@ __global__ void __launch_bounds__(256) nodes_plan_kernel(const NodesArgs a, int 
         s_last = atomicAdd(&a.hdr->done, 1) == (int)gridDim.x - 1;
         s_fits = 1;
     }
-    for (int i = threadIdx.x; i < NODES_LEVELS * (NODES_MAX / 2 + 1); i += 256) (&s_class[0][0])[i] = 0;
+    for (int i = threadIdx.x; i < NODES_LEVELS * (NODES_MAX / 2 + 1); i += PLAN_THREADS) (&s_class[0][0])[i] = 0;
     __syncthreads();
     if (!s_last) return;
     __threadfence();
@@ -149,7 +157,7 @@ __global__ void __launch_bounds__(256) nodes_plan_kernel(const NodesArgs a, int 
 #pragma unroll
     for (int l = 1; l < NODES_LEVELS; l++) h[l] = h[l - 1] * (1.0f / NODES_RATIO);
     const bool any_bad = *reinterpret_cast<volatile int *>(&a.hdr->bad) != 0;
-    for (int64_t w = threadIdx.x >> 5; w < a.batch.count * NODES_LEVELS; w += 8) {
+    for (int64_t w = threadIdx.x >> 5; w < a.batch.count * NODES_LEVELS; w += PLAN_WARPS) {
         const int l = (int)(w % NODES_LEVELS);
         const float *theta = batch_ptr(a.params, decompose(a.batch, w / NODES_LEVELS));
         // (fewer classes where batches share the points: every class has its own Lagrange matrices)
@@ -166,18 +174,22 @@ __global__ void __launch_bounds__(256) nodes_plan_kernel(const NodesArgs a, int 
     }
     __syncthreads();
     const bool use = !any_bad && s_fits;
-    // warp l lists the classes of level l (NODES_LEVELS <= 8 warps): counted from the largest node count
-    // down while they fit; smaller ones are served by the smallest that does (the largest always fits)
-    __shared__ int s_count[NODES_LEVELS], s_smallest[NODES_LEVELS];
+    // warp l lists the classes of level l: counted from the largest node count down while they fit; smaller
+    // ones are served by the smallest that does (the largest always fits)
+    static_assert(NODES_LEVELS <= PLAN_WARPS && NODES_MAX / 2 < 64, "a warp per level, a bit per node count");
+    __shared__ int s_count[NODES_LEVELS];
     const int l = threadIdx.x >> 5;
-    if (l < NODES_LEVELS && lane == 0 && use) {
-        int count = 0, total = 0, smallest = 0;
-        for (int i = NODES_MAX / 2; i >= 2; i--) {
-            if (!s_class[l][i]) continue;
-            if (count == NODES_CLASSES_PER_LEVEL || total + 2 * i > a.cap) break;
-            count++, total += 2 * i, smallest = i;
+    unsigned long long needed = 0, kept = 0;  // bits: P / 2
+    if (l < NODES_LEVELS && use) {
+        needed = __ballot_sync(0xffffffffu, s_class[l][lane] != 0);
+        needed |= (unsigned long long)__ballot_sync(0xffffffffu, lane + 32 <= NODES_MAX / 2 && s_class[l][min(lane + 32, NODES_MAX / 2)] != 0) << 32;
+        int total = 0;
+        for (unsigned long long left = needed; left != 0;) {
+            const int i = 63 - __clzll((long long)left);
+            if (__popcll(kept) == NODES_CLASSES_PER_LEVEL || total + 2 * i > a.cap) break;
+            kept |= 1ull << i, left &= ~(1ull << i), total += 2 * i;
         }
-        s_count[l] = count, s_smallest[l] = smallest;
+        if (lane == 0) s_count[l] = __popcll(kept);
     }
     __syncthreads();
     if (l < NODES_LEVELS && lane == 0 && use) {
@@ -186,13 +198,13 @@ __global__ void __launch_bounds__(256) nodes_plan_kernel(const NodesArgs a, int 
         a.hdr->h[l] = h[l];
         a.hdr->first[l] = at;
         if (l == NODES_LEVELS - 1) a.hdr->first[NODES_LEVELS] = at + s_count[l];
-        for (int i = 2; i < s_smallest[l]; i++) s_class[l][i] = at;
-        for (int i = s_smallest[l]; i <= NODES_MAX / 2; i++) {
-            if (!s_class[l][i]) continue;
+        for (unsigned long long left = needed; left != 0; left &= left - 1) {
+            const int i = __ffsll((long long)left) - 1;
+            s_class[l][i] = at;
+            if (!((kept >> i) & 1)) continue;
             a.hdr->P[at] = s_P[at] = 2 * i;
             a.hdr->off[at] = off;
-            s_h[at] = h[l];
-            s_class[l][i] = at++;
+            s_h[at++] = h[l];
             off += 2 * i;
         }
     }
@@ -206,17 +218,17 @@ __global__ void __launch_bounds__(256) nodes_plan_kernel(const NodesArgs a, int 
     }
     __syncthreads();
     if (!use) return;
-    for (int c = threadIdx.x >> 5; c < s_count[0] + s_count[1] + s_count[2] + s_count[3]; c += 8)
+    for (int c = threadIdx.x >> 5; c < s_count[0] + s_count[1] + s_count[2] + s_count[3]; c += PLAN_WARPS)
         for (int q = lane; q < s_P[c]; q += 32) s_node_class[s_node_first[c] + q] = (unsigned char)c;
     __syncthreads();
-    for (int64_t w = threadIdx.x; w < a.batch.count * NODES_LEVELS; w += 256) a.classes[w] = s_class[w % NODES_LEVELS][a.classes[w] / 2];
+    for (int64_t w = threadIdx.x; w < a.batch.count * NODES_LEVELS; w += PLAN_THREADS) a.classes[w] = s_class[w % NODES_LEVELS][a.classes[w] / 2];
     // offsets, then weights, of all classes: one node per thread and round
-    for (int i = threadIdx.x; i < s_nodes; i += 256) {
+    for (int i = threadIdx.x; i < s_nodes; i += PLAN_THREADS) {
         const int c = s_node_class[i], q = i - s_node_first[c];
         s_delta[i] = a.hdr->delta[c][q] = node_offset(s_h[c], q, s_P[c]);
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < s_nodes; i += 256) {
+    for (int i = threadIdx.x; i < s_nodes; i += PLAN_THREADS) {
         const int c = s_node_class[i], q = i - s_node_first[c];
         a.hdr->weight[c][q] = node_weight(s_delta + s_node_first[c], s_h[c], q, s_P[c]);
     }
@@ -336,7 +348,9 @@ __global__ void __launch_bounds__(1024) sort_scan_kernel(SortTables *t, int *bad
         before += c[i];
     }
     if (threadIdx.x == 1023) t->first[SORT_BUCKETS] = before;
-    if (over) *bad = 1;
+    // (the bits of NaNs lie beyond those of the infinities)
+    const bool finite = ordered_value(~t->lo) > -INFINITY && ordered_value(t->hi) < INFINITY;
+    if (over || !finite) *bad = 1;
 }
 
 __global__ void __launch_bounds__(256) sort_place_kernel(View<const float> x, int64_t n, SortTables *t, int *order) {
@@ -408,115 +422,124 @@ struct CompressArgs {
     float *out;
 };
 
-constexpr int CP_ROWS = 32;              // rows per stage
-constexpr int CP_NODES = 40;             // nodes per pass
-constexpr int CP_LS = CP_ROWS + 1;
+constexpr int CP_ROWS = 128;             // rows at a time
+constexpr int CP_NODES = 40;             // nodes at a time
+constexpr int CP_LS = CP_ROWS + 4;       // (lanes of neighbouring nodes read neighbouring 16 bytes)
 template <int COLS>
 struct CompressShape {
-    static constexpr int STAGE = CP_ROWS * COLS + CP_NODES * CP_LS + 3 & ~3;  // floats: operand rows, then Lagrange matrix
-    static constexpr size_t SMEM = 4 * 2 * STAGE * sizeof(float);
+    static constexpr int LAMBDA = CP_ROWS * COLS, PARTS = LAMBDA + CP_NODES * CP_LS;  // floats before them
+    static constexpr size_t SMEM = (PARTS + 4 * 32 * 16) * sizeof(float);
 };
 
-// A warp per (slot, block, COLS columns), no synchronisation beyond the warp: the block's rows pass
-// through two stages of 32 rows (operand and Lagrange matrix, cp.async), a lane owning 4 nodes x 4 columns
-// (8 shared-memory words read for 8 packed FMAs).  More than 40 nodes, or more units than lanes, take
-// further passes over the rows.
+// A CTA per (slot, block, COLS columns), and per class where an operand is shared by all batches.  What it
+// needs of 128 rows -- operand and Lagrange matrix -- is fetched at once; a warp takes 32 of the rows, a
+// lane 4 nodes (a quarter of them apart) x 4 columns of them, four rows at a time: 8 shared-memory reads of 16 bytes for
+// 32 packed FMAs.  The warps' sums are added in order.  More than 40 nodes, or more units than lanes, go over
+// the rows again, which for blocks of 128 are still there.
+// (One warp per block and 32 columns, through stages of 32 rows, had 512 - 2000 warps on the GPU and waited: 42 us instead of
+// 22 for 65 536 shared rows x 16 columns, 125 instead of 54 for 131 072 x 128 in blocks of 1024, 145 instead of
+// 112 for 4 x 262 144 x 32.)
 template <int COLS>
 __global__ void __launch_bounds__(128) nodes_compress_kernel(const CompressArgs p) {
     const NodesArgs &a = p.a;
-    if (!__shfl_sync(0xffffffffu, a.hdr->use, 0)) return;  // (warp-uniform: another CTA may clear it meanwhile)
-    constexpr int STAGE = CompressShape<COLS>::STAGE;
+    __shared__ int s_use;
+    if (threadIdx.x == 0) s_use = a.hdr->use;  // (once: another CTA may clear it meanwhile)
+    __syncthreads();
+    if (!s_use) return;
+    using Shape = CompressShape<COLS>;
     extern __shared__ __align__(16) float smem[];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    float *stages = smem + warp * 2 * STAGE;
+    float *vs = smem, *ls = smem + Shape::LAMBDA, *parts = smem + Shape::PARTS;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const int64_t chunks = (p.kq + COLS - 1) / COLS;
-    const int64_t item = blockIdx.x * 4LL + warp;
-    if (item >= chunks * p.slots * p.blocks) return;
-    const int64_t chunk = item % chunks, box = item / chunks, slot = box / p.blocks, block = box % p.blocks;
+    const int64_t chunk = blockIdx.x % chunks, box = blockIdx.x / chunks, slot = box / p.blocks, block = box % p.blocks;
+    const int64_t x_slot = p.x_slots == 1 ? 0 : slot;
+    const int level = level_of(a.hdr, p.half[x_slot * p.blocks + block]);
+    const int cls = p.slots == 1 ? a.hdr->first[level] + (int)blockIdx.y : a.classes[slot * NODES_LEVELS + level];
+    if (p.slots == 1 && cls >= a.hdr->first[level + 1]) return;
     const int k0 = (int)chunk * COLS, kc = (int)min((int64_t)COLS, p.kq - k0);  // a multiple of 4
     const float *v = batch_ptr(p.v, decompose(a.batch, slot));
-    const int64_t row0 = block * a.block, x_slot = p.x_slots == 1 ? 0 : slot;
-    const int groups = kc / 4;
-    const int level = level_of(a.hdr, p.half[x_slot * p.blocks + block]);
-    const bool shared = p.slots == 1;
-    const int c0 = shared ? a.hdr->first[level] : a.classes[slot * NODES_LEVELS + level], c1 = shared ? a.hdr->first[level + 1] : c0 + 1;
+    const int64_t row0 = block * a.block;
+    const int groups = kc / 4, P = a.hdr->P[cls];
     const int row_count = (int)min((int64_t)a.block, p.rows - row0), steps = (row_count + CP_ROWS - 1) / CP_ROWS;
+    const float *lambda_cls = p.lambda + ((x_slot * p.blocks + block) * node_rows(a, p.x_slots) + node_first(a, p.x_slots, cls)) * a.block;
+    float *out_cls = p.out + (box * node_rows(a, p.slots) + node_first(a, p.slots, cls)) * p.kq + k0;
     bool finite = true;
 
-    for (int cls = c0; cls < c1; cls++) {
-        const int P = a.hdr->P[cls];
-        const float *lambda_cls =
-            p.lambda + ((x_slot * p.blocks + block) * node_rows(a, p.x_slots) + node_first(a, p.x_slots, cls)) * a.block;
-        float *out_cls = p.out + (box * node_rows(a, p.slots) + node_first(a, p.slots, cls)) * p.kq + k0;
-        for (int p0 = 0; p0 < P; p0 += CP_NODES) {
-            const int Pn = min(CP_NODES, P - p0);
-            const float *lambda = lambda_cls + p0 * a.block;
-            float *out = out_cls + p0 * p.kq;
-            const auto load = [&](int step, int which) {
-                float *vs = stages + which * STAGE, *ls = vs + CP_ROWS * COLS;
+    for (int p0 = 0; p0 < P; p0 += CP_NODES) {
+        const int Pn = min(CP_NODES, P - p0), quads = (Pn + 3) / 4, units = quads * groups;
+        for (int u0 = 0; u0 < units; u0 += 32) {
+            const int unit = u0 + lane;
+            const bool mine = unit < units;
+            const int q = mine ? unit % quads : 0, c = mine ? (unit / quads) * 4 : 0;  // nodes q, q + quads, ..
+            int at[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) at[j] = min(q + j * quads, Pn - 1) * CP_LS;
+            f32x2 acc[4][2] = {};
+            for (int step = 0; step < steps; step++) {
                 const int r = step * CP_ROWS, count = min(CP_ROWS, row_count - r);
-                if (p.vec) {
-                    for (int e = lane; e < CP_ROWS * groups; e += 32) {
-                        const int i = e / groups, c = (e - i * groups) * 4;
-                        if (i < count)
-                            cp_async16(vs + i * COLS + c, v + point_row(p.order, row0 + r + i) * p.v.s0 + k0 + c);
-                        else
-                            *reinterpret_cast<float4 *>(vs + i * COLS + c) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                if (steps > 1 || u0 == 0) {
+                    __syncthreads();  // (what was there is done with)
+                    if (steps > 1 || p0 == 0) {
+                        if (p.vec) {
+                            for (int e = t; e < CP_ROWS * groups; e += 128) {
+                                const int i = e / groups, ce = (e - i * groups) * 4;
+                                if (i < count)
+                                    cp_async16(vs + i * COLS + ce, v + point_row(p.order, row0 + r + i) * p.v.s0 + k0 + ce);
+                                else
+                                    *reinterpret_cast<float4 *>(vs + i * COLS + ce) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                            }
+                        } else {
+                            for (int e = t; e < CP_ROWS * kc; e += 128) {
+                                const int i = e / kc, ce = e - i * kc;
+                                if (i < count && k0 + ce < a.k)
+                                    cp_async4(vs + i * COLS + ce, v + point_row(p.order, row0 + r + i) * p.v.s0 + (k0 + ce) * p.v.s1);
+                                else
+                                    vs[i * COLS + ce] = 0.0f;
+                            }
+                        }
                     }
-                } else {
-                    for (int e = lane; e < CP_ROWS * kc; e += 32) {
-                        const int i = e / kc, c = e - i * kc;
-                        if (i < count && k0 + c < a.k)
-                            cp_async4(vs + i * COLS + c, v + point_row(p.order, row0 + r + i) * p.v.s0 + (k0 + c) * p.v.s1);
-                        else
-                            vs[i * COLS + c] = 0.0f;
-                    }
+                    const float *lambda = lambda_cls + p0 * a.block + r;
+                    for (int n = warp; n < Pn; n += 4) cp_async16(ls + n * CP_LS + lane * 4, lambda + n * a.block + lane * 4);
+                    cp_async_commit();
+                    cp_async_wait<0>();
+                    __syncthreads();
                 }
-                for (int q = 0; q < Pn; q++) cp_async4(ls + q * CP_LS + lane, lambda + q * a.block + r + lane);
-                cp_async_commit();
-            };
-            const int quads = (Pn + 3) / 4, units = quads * groups;
-            for (int u0 = 0; u0 < units; u0 += 32) {
-                const int unit = u0 + lane;
-                const bool mine = unit < units;
-                const int q = mine ? (unit % quads) * 4 : 0, c = mine ? (unit / quads) * 4 : 0;
-                const int last = Pn - 1 - q;  // (P is even, not always a multiple of 4)
-                const int at0 = q * CP_LS, at1 = at0 + CP_LS, at2 = at0 + (last >= 2 ? 2 : 0) * CP_LS, at3 = at0 + (last >= 3 ? 3 : 0) * CP_LS;
-                f32x2 acc[4][2] = {};
-                load(0, 0);
-                for (int step = 0; step < steps; step++) {
-                    if (step + 1 < steps) {
-                        load(step + 1, (step + 1) & 1);
-                        cp_async_wait<1>();
-                    } else {
-                        cp_async_wait<0>();
-                    }
-                    __syncwarp();
-                    const float *w0 = stages + (step & 1) * STAGE + c, *ls = stages + (step & 1) * STAGE + CP_ROWS * COLS;
-#pragma unroll 8
-                    for (int i = 0; i < CP_ROWS; i++) {
-                        const ulonglong2 w = *reinterpret_cast<const ulonglong2 *>(w0 + i * COLS);
-                        const f32x2 a0 = splat2(ls[at0 + i]), a1 = splat2(ls[at1 + i]), a2 = splat2(ls[at2 + i]), a3 = splat2(ls[at3 + i]);
-                        acc[0][0] = fma2(a0, w.x, acc[0][0]), acc[0][1] = fma2(a0, w.y, acc[0][1]);
-                        acc[1][0] = fma2(a1, w.x, acc[1][0]), acc[1][1] = fma2(a1, w.y, acc[1][1]);
-                        acc[2][0] = fma2(a2, w.x, acc[2][0]), acc[2][1] = fma2(a2, w.y, acc[2][1]);
-                        acc[3][0] = fma2(a3, w.x, acc[3][0]), acc[3][1] = fma2(a3, w.y, acc[3][1]);
-                    }
-                    __syncwarp();
-                }
-                if (mine) {
+#pragma unroll 2
+                for (int i = warp * 32; i < warp * 32 + 32; i += 4) {
+                    float l[4][4];
 #pragma unroll
                     for (int j = 0; j < 4; j++) {
-                        if (j <= last) *reinterpret_cast<ulonglong2 *>(out + (q + j) * p.kq + c) = make_ulonglong2(acc[j][0], acc[j][1]);
+                        const float4 f = *reinterpret_cast<const float4 *>(ls + at[j] + i);
+                        l[j][0] = f.x, l[j][1] = f.y, l[j][2] = f.z, l[j][3] = f.w;
+                    }
 #pragma unroll
-                        for (int h = 0; h < 2; h++) {
-                            float v0, v1;
-                            unpack2(acc[j][h], v0, v1);
-                            finite = finite && fabsf(v0) <= NODES_MAX_OPERAND && fabsf(v1) <= NODES_MAX_OPERAND;
+                    for (int d = 0; d < 4; d++) {
+                        const ulonglong2 w = *reinterpret_cast<const ulonglong2 *>(vs + (i + d) * COLS + c);
+#pragma unroll
+                        for (int j = 0; j < 4; j++) {
+                            const f32x2 f = splat2(l[j][d]);
+                            acc[j][0] = fma2(f, w.x, acc[j][0]), acc[j][1] = fma2(f, w.y, acc[j][1]);
                         }
                     }
                 }
             }
+            // [warp][j][lane][4]: a warp adds up the sums of one j
+#pragma unroll
+            for (int j = 0; j < 4; j++) *reinterpret_cast<ulonglong2 *>(parts + ((warp * 4 + j) * 32 + lane) * 4) = make_ulonglong2(acc[j][0], acc[j][1]);
+            __syncthreads();
+            float4 o = *reinterpret_cast<const float4 *>(parts + (warp * 32 + lane) * 4);
+#pragma unroll
+            for (int w = 1; w < 4; w++) {
+                const float4 x = *reinterpret_cast<const float4 *>(parts + ((w * 4 + warp) * 32 + lane) * 4);
+                o.x += x.x, o.y += x.y, o.z += x.z, o.w += x.w;
+            }
+            const int node = q + warp * quads;
+            if (mine && node < Pn) {
+                *reinterpret_cast<float4 *>(out_cls + (p0 + node) * p.kq + c) = o;
+                finite = finite && fmaxf(fmaxf(fabsf(o.x), fabsf(o.y)), fmaxf(fabsf(o.z), fabsf(o.w))) <= NODES_MAX_OPERAND &&
+                         !isnan(o.x) && !isnan(o.y) && !isnan(o.z) && !isnan(o.w);
+            }
+            if (steps == 1 && u0 + 32 < units) __syncthreads();  // (parts are written again; elsewhere the next fetch waits)
         }
     }
     if (!finite) a.hdr->use = 0;  // (the kernels after this one see it)
@@ -1112,8 +1135,9 @@ static int nodes_compress(const NodesArgs &a, const NodesLayout &l, const View<c
         const cudaError_t err = cudaFuncSetAttribute(nodes_compress_kernel<COLS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                      (int)CompressShape<COLS>::SMEM);
         if (err != cudaSuccess) return cuda_fail(err, "cudaFuncSetAttribute(interpolation)");
-        const int64_t ctas = ceil_div(c.slots * c.blocks * ceil_div(l.kq, COLS), 4);
-        nodes_compress_kernel<COLS><<<(unsigned)ctas, 128, CompressShape<COLS>::SMEM, s>>>(c);
+        // (a shared operand: a CTA per class that the plan may have made, most of which return at once)
+        const dim3 grid((unsigned)(c.slots * c.blocks * ceil_div(l.kq, COLS)), c.slots == 1 && a.batch.count > 1 ? NODES_CLASSES_PER_LEVEL : 1);
+        nodes_compress_kernel<COLS><<<grid, 128, CompressShape<COLS>::SMEM, s>>>(c);
         return (int)KM_OK;
     };
     const int rc = l.kq <= 16 ? launch(Int<16>()) : launch(Int<32>());
@@ -1140,8 +1164,8 @@ static int nodes_begin(NodesArgs &a, const NodesLayout &l, int kernel_type, unsi
         if (rc != KM_OK) return rc;
         a.order1 = reinterpret_cast<const int *>(ws + l.order1), a.order2 = reinterpret_cast<const int *>(ws + l.order2);
     }
-    const int64_t boxes = l.slots1 * l.R + (l.same ? 0 : l.slots2 * l.C), work = std::max(ceil_div(boxes, 8), ceil_div(a.batch.count * ceil_div(a.m, KM_BLOCK_SIZE), 256));
-    nodes_plan_kernel<<<(unsigned)std::min<int64_t>(work, 148 * 4), 256, 0, s>>>(a, kernel_type);
+    const int64_t boxes = l.slots1 * l.R + (l.same ? 0 : l.slots2 * l.C), work = std::max(ceil_div(boxes, PLAN_WARPS), ceil_div(a.batch.count * ceil_div(a.m, KM_BLOCK_SIZE), PLAN_THREADS));
+    nodes_plan_kernel<<<(unsigned)std::min<int64_t>(work, 148 * 2), PLAN_THREADS, 0, s>>>(a, kernel_type);
     KM_CHECK_LAUNCH("interpolation: plan launch");
     nodes_lambda_kernel<<<(unsigned)(boxes * (l.block / 128)), 128, 0, s>>>(a);
     KM_CHECK_LAUNCH("interpolation: Lagrange matrices launch");

@@ -69,11 +69,13 @@ __device__ __forceinline__ float node_offset(float h, int q, int P) { return h *
 // Barycentric weight of node q, scaled by (2 / h)^P: 1 / prod_r (delta_q - delta_r) of the ROUNDED
 // offsets, in fp64, so that the Lagrange polynomials are those of the very points kappa is taken at.
 __device__ __forceinline__ float node_weight(const float *delta, float h, int q, int P) {
-    const double s = 2.0 / (double)h;
-    double w = 1.0;
-    for (int r = 0; r < P; r++)
-        if (r != q) w *= ((double)delta[q] - (double)delta[r]) * s;
-    return (float)(1.0 / w);
+    const double s = 2.0 / (double)h, d = (double)delta[q];
+    double w[2] = {1.0, 1.0};  // (P is even)
+    for (int r = 0; r < P; r += 2) {
+        if (r != q) w[0] *= (d - (double)delta[r]) * s;
+        if (r + 1 != q) w[1] *= (d - (double)delta[r + 1]) * s;
+    }
+    return (float)(1.0 / (w[0] * w[1]));
 }
 
 }  // namespace km
