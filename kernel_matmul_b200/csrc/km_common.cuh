@@ -68,11 +68,22 @@ inline View<T> make_view(const km_view *v, const Batch &b) {
 __host__ __device__ inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
 // Runs a kernel only if *flag == want (always for a null flag): the choice between interpolation and
-// direct evaluation (km_nodes.cu) is made on the device.
+// direct evaluation (km_nodes.cu) is made on the device.  Kernels behind a gate are launched so that they may start while
+// their predecessor drains (launch_gated), and closed() is the first thing they ask: behind a closed gate
+// they are over by then but for the first CTA, which stays until the predecessor is complete, so that the
+// chain is complete when its last kernel is; behind an open one all of them wait for it.  The flag itself
+// has been final since before the chain's first kernel.  (8192 CTAs of a gated kernel that only return take
+// 36 us.)
 struct Gate {
     const int *flag = nullptr;
     int want = 0;
-    __device__ __forceinline__ bool closed() const { return flag != nullptr && *flag != want; }
+    __device__ __forceinline__ bool closed() const {
+        if (flag == nullptr) return false;
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+        const bool run = *flag == want;
+        if (run || (blockIdx.x == 0 && blockIdx.y == 0)) asm volatile("griddepcontrol.wait;" ::: "memory");
+        return !run;
+    }
 };
 
 // Second stage of every gradient op (km_grad.cu): per batch, add `units` partial records of
@@ -90,6 +101,8 @@ int matmul_direct(int kernel_type, const km_batch *batch, int64_t m, int64_t n, 
 int matmul_tc_direct(int kernel_type, const km_batch *batch, int64_t m, int64_t n, int64_t k, const km_view *x1, const km_view *x2,
                      const km_view *rhs, const km_view *params, const km_view *start, const km_view *end, const km_view *out,
                      void *workspace, size_t workspace_bytes, Gate gate, void *stream);
+// Zeroes what matmul_tc_direct behind a gate needs zeroed of its workspace.
+int matmul_tc_prepare(const Batch &batch, int64_t k, const View<const float> &rhs, void *workspace, cudaStream_t s);
 int grad_direct(int kernel_type, const km_batch *batch, int64_t m, int64_t n, int64_t k, const km_view *x1, const km_view *x2,
                 const km_view *left, const km_view *right, const km_view *params, const km_view *start, const km_view *end,
                 const km_view *grad, void *workspace, size_t workspace_bytes, Gate gate, void *stream);
@@ -101,10 +114,10 @@ int grad_tc_direct(int kernel_type, const km_batch *batch, int64_t m, int64_t n,
 // launch): the kernel calls grid_wait() before it touches what the predecessor writes.  In chains of
 // kernels of a few microseconds the launch latency between two of them is otherwise a third of the time.
 template <typename... P, typename... A>
-inline int launch_chained(const char *what, void (*kernel)(P...), unsigned ctas, unsigned threads, size_t smem, cudaStream_t stream,
+inline int launch_chained(const char *what, void (*kernel)(P...), dim3 ctas, unsigned threads, size_t smem, cudaStream_t stream,
                           A &&...args) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(ctas);
+    cfg.gridDim = ctas;
     cfg.blockDim = dim3(threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
@@ -117,6 +130,16 @@ inline int launch_chained(const char *what, void (*kernel)(P...), unsigned ctas,
     return err == cudaSuccess ? (int)KM_OK : cuda_fail(err, what);
 }
 
+// The same for a kernel behind a gate; an ordinary launch without one.
+template <typename... P, typename... A>
+inline int launch_gated(const char *what, const Gate &gate, void (*kernel)(P...), unsigned ctas, unsigned threads, size_t smem,
+                        cudaStream_t stream, A &&...args) {
+    if (gate.flag != nullptr) return launch_chained(what, kernel, ctas, threads, smem, stream, std::forward<A>(args)...);
+    kernel<<<ctas, threads, smem, stream>>>(std::forward<A>(args)...);
+    const cudaError_t err = cudaGetLastError();
+    return err == cudaSuccess ? (int)KM_OK : cuda_fail(err, what);
+}
+
 // ---------------------------------------------------------------------------- device side
 
 // The predecessor's results are complete and visible; the successor may start once every CTA is here.
@@ -124,6 +147,9 @@ __device__ __forceinline__ void grid_wait() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
+
+// The successor may start once every CTA has called this.
+__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // Flattened batch index -> per-dimension indices (row-major over the batch dims).
 struct BatchIndex {

@@ -215,19 +215,19 @@ __global__ void __launch_bounds__(256) grad_finish_kernel(Batch batch, int64_t u
 }
 
 template <typename PT>
-static void launch_finish_typed(int kernel_type, const Batch &batch, int64_t units, const PT *partials,
+static int launch_finish_typed(int kernel_type, const Batch &batch, int64_t units, const PT *partials,
                                 const View<const float> &params, const View<float> &grad, cudaStream_t stream, Gate gate) {
     const unsigned blocks = (unsigned)batch.count;
+    const auto launch = [&](auto kernel) {
+        return launch_gated("gradient finish launch", gate, kernel, blocks, 256, 0, stream, batch, units, partials, params, grad, gate);
+    };
     switch (kernel_type) {
     case KM_KERNEL_RBF:
-        grad_finish_kernel<KM_KERNEL_RBF, PT><<<blocks, 256, 0, stream>>>(batch, units, partials, params, grad, gate);
-        break;
+        return launch(grad_finish_kernel<KM_KERNEL_RBF, PT>);
     case KM_KERNEL_SPECTRAL:
-        grad_finish_kernel<KM_KERNEL_SPECTRAL, PT><<<blocks, 256, 0, stream>>>(batch, units, partials, params, grad, gate);
-        break;
+        return launch(grad_finish_kernel<KM_KERNEL_SPECTRAL, PT>);
     default:
-        grad_finish_kernel<KM_KERNEL_LOCALLY_PERIODIC, PT><<<blocks, 256, 0, stream>>>(batch, units, partials, params, grad, gate);
-        break;
+        return launch(grad_finish_kernel<KM_KERNEL_LOCALLY_PERIODIC, PT>);
     }
 }
 
@@ -240,11 +240,8 @@ int launch_grad_finish(int kernel_type, const Batch &batch, int64_t units, const
         return KM_ERR_UNSUPPORTED;
     }
     if (partials_fp64)
-        launch_finish_typed(kernel_type, batch, units, static_cast<const double *>(partials), params, grad, stream, gate);
-    else
-        launch_finish_typed(kernel_type, batch, units, static_cast<const float *>(partials), params, grad, stream, gate);
-    KM_CHECK_LAUNCH("gradient finish launch");
-    return KM_OK;
+        return launch_finish_typed(kernel_type, batch, units, static_cast<const double *>(partials), params, grad, stream, gate);
+    return launch_finish_typed(kernel_type, batch, units, static_cast<const float *>(partials), params, grad, stream, gate);
 }
 
 template <int KT, int KB, int RPT, int WN>
@@ -257,9 +254,7 @@ static int launch_grad(const GradArgs &a, cudaStream_t stream) {
         set_error("gradient: too many work items (%lld)", (long long)items);
         return KM_ERR_UNSUPPORTED;
     }
-    grad_band_kernel<KT, KB, RPT, WN><<<(unsigned)items, THREADS, smem, stream>>>(a);
-    KM_CHECK_LAUNCH("gradient band launch");
-    return KM_OK;
+    return launch_gated("gradient band launch", a.gate, grad_band_kernel<KT, KB, RPT, WN>, (unsigned)items, THREADS, smem, stream, a);
 }
 
 template <int KT>

@@ -457,9 +457,7 @@ static int launch_grad_tc(const GradTcArgs &a, cudaStream_t s) {
     auto kernel = grad_tc_kernel<KT, G>;
     cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err != cudaSuccess) return cuda_fail(err, "cudaFuncSetAttribute(grad_tc)");
-    kernel<<<(unsigned)items, 128 * G + 32, smem, s>>>(a);
-    KM_CHECK_LAUNCH("gradient (tensor cores) launch");
-    return KM_OK;
+    return launch_gated("gradient (tensor cores) launch", a.gate, kernel, (unsigned)items, 128 * G + 32, smem, s, a);
 }
 
 // consumer groups for up to 16 columns (one group: more registers per thread; measured equal for
@@ -526,8 +524,9 @@ static int grad_tc_entry(const char *name, int kernel_type, const km_batch *batc
         KM_REQUIRE(n == 0 || (x2->data && right->data), KM_ERR_INVALID_ARGUMENT, "%s: null data pointer", name);
         const int64_t total = slots * a.kblocks * tiles * (int64_t)GT_COLS * a.kp;
         const unsigned blocks = (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(total, 256), 148 * 32));
-        grad_tc_images_kernel<<<blocks, 256, 0, s>>>(a.batch, slots, n, k, a.kp, a.kblocks, tiles, rv, images, a.status, gate);
-        KM_CHECK_LAUNCH("gradient (tensor cores) pre-pass launch");
+        rc = launch_gated("gradient (tensor cores) pre-pass launch", gate, grad_tc_images_kernel, blocks, 256, 0, s, a.batch, slots, n, k, a.kp,
+                          a.kblocks, tiles, rv, images, a.status, gate);
+        if (rc != KM_OK) return rc;
         switch (kernel_type) {
         case KM_KERNEL_RBF: rc = dispatch_grad_tc<KM_KERNEL_RBF>(a, s); break;
         case KM_KERNEL_SPECTRAL: rc = dispatch_grad_tc<KM_KERNEL_SPECTRAL>(a, s); break;

@@ -548,9 +548,7 @@ static int launch_matmul(const MatmulArgs<float> &a, cudaStream_t stream) {
             return KM_OK;
         }
     }
-    kernel<<<(unsigned)items, THREADS, smem, stream>>>(a);
-    KM_CHECK_LAUNCH("km_matmul_f32 launch");
-    return KM_OK;
+    return launch_gated("km_matmul_f32 launch", a.gate, kernel, (unsigned)items, THREADS, smem, stream, a);
 }
 
 template <int KT, bool SUM>

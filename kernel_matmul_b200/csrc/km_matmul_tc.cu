@@ -625,9 +625,7 @@ static int launch_tc_n(const TcArgs &a, cudaStream_t s) {
     constexpr size_t smem = TcCfg<N>::SMEM_BYTES;
     cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err != cudaSuccess) return cuda_fail(err, "cudaFuncSetAttribute(matmul_tc)");
-    kernel<<<(unsigned)items, TcCfg<N>::THREADS, smem, s>>>(a);
-    KM_CHECK_LAUNCH("km_matmul_tc_f32 launch");
-    return KM_OK;
+    return launch_gated("km_matmul_tc_f32 launch", a.gate, kernel, (unsigned)items, TcCfg<N>::THREADS, smem, s, a);
 }
 
 template <int KT>
@@ -636,6 +634,16 @@ static int launch_tc(const TcArgs &a, int n_pad, cudaStream_t s) {
     if (n_pad == 32) return launch_tc_n<KT, 32>(a, s);
     if (n_pad == 64) return launch_tc_n<KT, 64>(a, s);
     return launch_tc_n<KT, 128>(a, s);
+}
+
+static int tc_zero_scales(int64_t slots, int64_t k, void *workspace, cudaStream_t s) {
+    unsigned char *scales = static_cast<unsigned char *>(workspace) + TC_STATUS_BYTES;
+    const cudaError_t err = cudaMemsetAsync(scales, 0, tc_scale_bytes(slots, tc_k_blocks(k)), s);
+    return err == cudaSuccess ? (int)KM_OK : cuda_fail(err, "km_matmul_tc_f32 cudaMemsetAsync");
+}
+
+int matmul_tc_prepare(const Batch &batch, int64_t k, const View<const float> &rhs, void *workspace, cudaStream_t s) {
+    return tc_zero_scales(tc_slots(batch, rhs), k, workspace, s);
 }
 
 static int tc_matmul(int kernel_type, TcArgs a, const View<const float> &rhs, void *workspace, cudaStream_t s) {
@@ -655,15 +663,18 @@ static int tc_matmul(int kernel_type, TcArgs a, const View<const float> &rhs, vo
     a.col_inv_scale = reinterpret_cast<const float *>(scales) + TC_MAX_N;
     a.gave_up = gave_up_word();
     a.wait_polls = current_wait_polls();
-    cudaError_t err = cudaMemsetAsync(scales, 0, tc_scale_bytes(slots, kblocks), s);
-    if (err != cudaSuccess) return cuda_fail(err, "km_matmul_tc_f32 cudaMemsetAsync");
+    int rc = KM_OK;
+    if (a.gate.flag == nullptr) rc = tc_zero_scales(slots, a.k, workspace, s);  // (behind a gate: matmul_tc_prepare, a memset would break the chain)
+    if (rc != KM_OK) return rc;
     const unsigned max_blocks = (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(a.n, 16), 148 * 8));
-    tc_colmax_kernel<<<max_blocks, 256, 0, s>>>(a.batch, slots, a.n, a.k, n_pad, (int)kblocks, rhs, scales, a.status, a.gate);
-    KM_CHECK_LAUNCH("km_matmul_tc_f32 column-maximum launch");
+    rc = launch_gated("km_matmul_tc_f32 column-maximum launch", a.gate, tc_colmax_kernel, max_blocks, 256, 0, s, a.batch, slots, a.n, a.k,
+                          n_pad, (int)kblocks, rhs, scales, a.status, a.gate);
+    if (rc != KM_OK) return rc;
     const int64_t total = slots * kblocks * supers * (int64_t)(TC_SCOLS * n_pad);
     const unsigned blocks = (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(total, 256), 148 * 32));
-    tc_rhs_images_kernel<<<blocks, 256, 0, s>>>(a.batch, slots, a.n, a.k, n_pad, (int)kblocks, supers, rhs, images, scales, a.gate);
-    KM_CHECK_LAUNCH("km_matmul_tc_f32 pre-pass launch");
+    rc = launch_gated("km_matmul_tc_f32 pre-pass launch", a.gate, tc_rhs_images_kernel, blocks, 256, 0, s, a.batch, slots, a.n, a.k, n_pad,
+                      (int)kblocks, supers, rhs, images, scales, a.gate);
+    if (rc != KM_OK) return rc;
     switch (kernel_type) {
     case KM_KERNEL_RBF: return launch_tc<KM_KERNEL_RBF>(a, n_pad, s);
     case KM_KERNEL_SPECTRAL: return launch_tc<KM_KERNEL_SPECTRAL>(a, n_pad, s);

@@ -1,5 +1,8 @@
 // Products and gradients by blockwise interpolation (km_nodes.cuh has the method and its error bound).
 //
+// The kernels of a call are chained by programmatic dependent launches, each waiting for its predecessor before
+// anything but operands is read; those behind the gate wait in Gate::closed.
+//
 // A call is: extents of the blocks and choice of P (nodes_plan_kernel), Lagrange matrices
 // (nodes_lambda_kernel), rhs / left / right at the nodes (nodes_compress_kernel), then the product
 // (nodes_product_kernel, which also takes its result back to the 128 rows) or the gradient
@@ -83,6 +86,7 @@ __device__ __forceinline__ int nodes_needed_for(int kt, const float *theta, int6
 // classes listed in shared memory.)
 constexpr int PLAN_THREADS = 512, PLAN_WARPS = PLAN_THREADS / 32;
 __global__ void __launch_bounds__(PLAN_THREADS) nodes_plan_kernel(const NodesArgs a, int kernel_type) {
+    grid_release();
     const int lane = threadIdx.x & 31;
     const int64_t warps = (int64_t)gridDim.x * PLAN_WARPS, first = blockIdx.x * (int64_t)PLAN_WARPS + (threadIdx.x >> 5);
     const int64_t boxes1 = a.slots1 * a.R, boxes = boxes1 + (a.same ? 0 : a.slots2 * a.C);
@@ -238,6 +242,7 @@ __global__ void __launch_bounds__(PLAN_THREADS) nodes_plan_kernel(const NodesArg
 // lambda[q][row] = (w_q / (x - xi_q)) / sum of the same.
 __global__ void __launch_bounds__(128) nodes_lambda_kernel(const NodesArgs a) {
     const NodesHeader *hdr = a.hdr;
+    grid_wait();
     if (!hdr->use) return;
     __shared__ float delta[NODES_MAX], weight[NODES_MAX];
     const int64_t boxes1 = a.slots1 * a.R;
@@ -442,25 +447,54 @@ struct CompressShape {
 template <int COLS>
 __global__ void __launch_bounds__(128) nodes_compress_kernel(const CompressArgs p) {
     const NodesArgs &a = p.a;
-    __shared__ int s_use;
-    if (threadIdx.x == 0) s_use = a.hdr->use;  // (once: another CTA may clear it meanwhile)
-    __syncthreads();
-    if (!s_use) return;
     using Shape = CompressShape<COLS>;
     extern __shared__ __align__(16) float smem[];
     float *vs = smem, *ls = smem + Shape::LAMBDA, *parts = smem + Shape::PARTS;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    __shared__ int s_use;
     const int64_t chunks = (p.kq + COLS - 1) / COLS;
     const int64_t chunk = blockIdx.x % chunks, box = blockIdx.x / chunks, slot = box / p.blocks, block = box % p.blocks;
     const int64_t x_slot = p.x_slots == 1 ? 0 : slot;
-    const int level = level_of(a.hdr, p.half[x_slot * p.blocks + block]);
-    const int cls = p.slots == 1 ? a.hdr->first[level] + (int)blockIdx.y : a.classes[slot * NODES_LEVELS + level];
-    if (p.slots == 1 && cls >= a.hdr->first[level + 1]) return;
     const int k0 = (int)chunk * COLS, kc = (int)min((int64_t)COLS, p.kq - k0);  // a multiple of 4
     const float *v = batch_ptr(p.v, decompose(a.batch, slot));
     const int64_t row0 = block * a.block;
-    const int groups = kc / 4, P = a.hdr->P[cls];
+    const int groups = kc / 4;
     const int row_count = (int)min((int64_t)a.block, p.rows - row0), steps = (row_count + CP_ROWS - 1) / CP_ROWS;
+    const auto fetch_rows = [&](int r) {
+        const int count = min(CP_ROWS, row_count - r);
+        if (p.vec) {
+            for (int e = t; e < CP_ROWS * groups; e += 128) {
+                const int i = e / groups, ce = (e - i * groups) * 4;
+                if (i < count)
+                    cp_async16(vs + i * COLS + ce, v + point_row(p.order, row0 + r + i) * p.v.s0 + k0 + ce);
+                else
+                    *reinterpret_cast<float4 *>(vs + i * COLS + ce) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            }
+        } else {
+            for (int e = t; e < CP_ROWS * kc; e += 128) {
+                const int i = e / kc, ce = e - i * kc;
+                if (i < count && k0 + ce < a.k)
+                    cp_async4(vs + i * COLS + ce, v + point_row(p.order, row0 + r + i) * p.v.s0 + (k0 + ce) * p.v.s1);
+                else
+                    vs[i * COLS + ce] = 0.0f;
+            }
+        }
+    };
+    // the operand was there before the plan, whose results come through a chain of loads: it is on the way
+    // meanwhile (but not where there is a CTA per class, most of which have nothing to do)
+    const bool early = gridDim.y == 1;
+    if (early) fetch_rows(0);
+    grid_wait();
+    if (t == 0) s_use = a.hdr->use;  // (once: another CTA may clear it meanwhile)
+    __syncthreads();
+    const int level = level_of(a.hdr, p.half[x_slot * p.blocks + block]);
+    const int cls = p.slots == 1 ? a.hdr->first[level] + (int)blockIdx.y : a.classes[slot * NODES_LEVELS + level];
+    if (!s_use || (p.slots == 1 && cls >= a.hdr->first[level + 1])) {
+        cp_async_commit();
+        cp_async_wait<0>();
+        return;
+    }
+    const int P = a.hdr->P[cls];
     const float *lambda_cls = p.lambda + ((x_slot * p.blocks + block) * node_rows(a, p.x_slots) + node_first(a, p.x_slots, cls)) * a.block;
     float *out_cls = p.out + (box * node_rows(a, p.slots) + node_first(a, p.slots, cls)) * p.kq + k0;
     bool finite = true;
@@ -476,28 +510,11 @@ __global__ void __launch_bounds__(128) nodes_compress_kernel(const CompressArgs 
             for (int j = 0; j < 4; j++) at[j] = min(q + j * quads, Pn - 1) * CP_LS;
             f32x2 acc[4][2] = {};
             for (int step = 0; step < steps; step++) {
-                const int r = step * CP_ROWS, count = min(CP_ROWS, row_count - r);
+                const int r = step * CP_ROWS;
                 if (steps > 1 || u0 == 0) {
                     __syncthreads();  // (what was there is done with)
-                    if (steps > 1 || p0 == 0) {
-                        if (p.vec) {
-                            for (int e = t; e < CP_ROWS * groups; e += 128) {
-                                const int i = e / groups, ce = (e - i * groups) * 4;
-                                if (i < count)
-                                    cp_async16(vs + i * COLS + ce, v + point_row(p.order, row0 + r + i) * p.v.s0 + k0 + ce);
-                                else
-                                    *reinterpret_cast<float4 *>(vs + i * COLS + ce) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                            }
-                        } else {
-                            for (int e = t; e < CP_ROWS * kc; e += 128) {
-                                const int i = e / kc, ce = e - i * kc;
-                                if (i < count && k0 + ce < a.k)
-                                    cp_async4(vs + i * COLS + ce, v + point_row(p.order, row0 + r + i) * p.v.s0 + (k0 + ce) * p.v.s1);
-                                else
-                                    vs[i * COLS + ce] = 0.0f;
-                            }
-                        }
-                    }
+                    const bool there = early && p0 == 0 && u0 == 0 && step == 0;
+                    if ((steps > 1 || p0 == 0) && !there) fetch_rows(r);
                     const float *lambda = lambda_cls + p0 * a.block + r;
                     for (int n = warp; n < Pn; n += 4) cp_async16(ls + n * CP_LS + lane * 4, lambda + n * a.block + lane * 4);
                     cp_async_commit();
@@ -777,6 +794,7 @@ struct NodesProductArgs {
 template <int KT, int KC>
 __global__ void __launch_bounds__(128, NodeShape<KC>::CTAS) nodes_product_kernel(const NodesProductArgs p) {
     const NodesArgs &a = p.a;
+    grid_wait();
     if (!a.hdr->use) return;
     using Fn = KernelFn<KT>;
     constexpr int KC2 = KC / 2, QS = NodeShape<KC>::QS;
@@ -942,6 +960,7 @@ struct NodesGradArgs {
 template <int KT, int KC>
 __global__ void __launch_bounds__(128, NodeShape<KC>::CTAS) nodes_grad_kernel(const NodesGradArgs p) {
     const NodesArgs &a = p.a;
+    grid_wait();
     if (!a.hdr->use) return;
     using Fn = KernelFn<KT>;
     constexpr int KC2 = KC / 2, NS = Fn::NSUMS;
@@ -1137,13 +1156,9 @@ static int nodes_compress(const NodesArgs &a, const NodesLayout &l, const View<c
         if (err != cudaSuccess) return cuda_fail(err, "cudaFuncSetAttribute(interpolation)");
         // (a shared operand: a CTA per class that the plan may have made, most of which return at once)
         const dim3 grid((unsigned)(c.slots * c.blocks * ceil_div(l.kq, COLS)), c.slots == 1 && a.batch.count > 1 ? NODES_CLASSES_PER_LEVEL : 1);
-        nodes_compress_kernel<COLS><<<grid, 128, CompressShape<COLS>::SMEM, s>>>(c);
-        return (int)KM_OK;
+        return launch_chained("interpolation: operand launch", nodes_compress_kernel<COLS>, grid, 128, CompressShape<COLS>::SMEM, s, c);
     };
-    const int rc = l.kq <= 16 ? launch(Int<16>()) : launch(Int<32>());
-    if (rc != KM_OK) return rc;
-    KM_CHECK_LAUNCH("interpolation: operand launch");
-    return KM_OK;
+    return l.kq <= 16 ? launch(Int<16>()) : launch(Int<32>());
 }
 
 static int nodes_begin(NodesArgs &a, const NodesLayout &l, int kernel_type, unsigned char *ws, cudaStream_t s) {
@@ -1167,9 +1182,7 @@ static int nodes_begin(NodesArgs &a, const NodesLayout &l, int kernel_type, unsi
     const int64_t boxes = l.slots1 * l.R + (l.same ? 0 : l.slots2 * l.C), work = std::max(ceil_div(boxes, PLAN_WARPS), ceil_div(a.batch.count * ceil_div(a.m, KM_BLOCK_SIZE), PLAN_THREADS));
     nodes_plan_kernel<<<(unsigned)std::min<int64_t>(work, 148 * 2), PLAN_THREADS, 0, s>>>(a, kernel_type);
     KM_CHECK_LAUNCH("interpolation: plan launch");
-    nodes_lambda_kernel<<<(unsigned)(boxes * (l.block / 128)), 128, 0, s>>>(a);
-    KM_CHECK_LAUNCH("interpolation: Lagrange matrices launch");
-    return KM_OK;
+    return launch_chained("interpolation: Lagrange matrices launch", nodes_lambda_kernel, (unsigned)(boxes * (l.block / 128)), 128, 0, s, a);
 }
 
 template <int KT, int KC>
@@ -1177,18 +1190,16 @@ static int launch_nodes_product(const NodesProductArgs &p, cudaStream_t s) {
     auto kernel = nodes_product_kernel<KT, KC>;
     const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)NodeShape<KC>::SMEM);
     if (err != cudaSuccess) return cuda_fail(err, "cudaFuncSetAttribute(interpolation)");
-    kernel<<<(unsigned)(p.a.batch.count * (p.wpr == 1 ? ceil_div(p.a.R, 4) : p.a.R) * p.k_chunks), 128, NodeShape<KC>::SMEM, s>>>(p);
-    KM_CHECK_LAUNCH("interpolation: product launch");
-    return KM_OK;
+    return launch_chained("interpolation: product launch", kernel, (unsigned)(p.a.batch.count * (p.wpr == 1 ? ceil_div(p.a.R, 4) : p.a.R) * p.k_chunks),
+                          128, NodeShape<KC>::SMEM, s, p);
 }
 template <int KT, int KC>
 static int launch_nodes_grad(const NodesGradArgs &p, cudaStream_t s) {
     auto kernel = nodes_grad_kernel<KT, KC>;
     const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)NodeShape<KC>::SMEM);
     if (err != cudaSuccess) return cuda_fail(err, "cudaFuncSetAttribute(interpolation)");
-    kernel<<<(unsigned)(p.a.batch.count * (p.wpr == 1 ? ceil_div(p.a.R, 4) : p.a.R) * p.k_chunks), 128, NodeShape<KC>::SMEM, s>>>(p);
-    KM_CHECK_LAUNCH("interpolation: gradient launch");
-    return KM_OK;
+    return launch_chained("interpolation: gradient launch", kernel, (unsigned)(p.a.batch.count * (p.wpr == 1 ? ceil_div(p.a.R, 4) : p.a.R) * p.k_chunks),
+                          128, NodeShape<KC>::SMEM, s, p);
 }
 #define KM_NODES_DISPATCH(launch, args)                                                                \
     [&](int kt, int kc) {                                                                              \
@@ -1284,6 +1295,10 @@ extern "C" int km_matmul_nodes_f32(int kernel_type, const km_batch *batch, int64
                "km_matmul_nodes_f32: workspace of %zu bytes needed (256-byte aligned), %zu given", l.total, workspace_bytes);
     unsigned char *ws = static_cast<unsigned char *>(workspace);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (k >= 9) {
+        rc = matmul_tc_prepare(b, k, make_view<const float>(rhs, b), ws + l.direct, s);
+        if (rc != KM_OK) return rc;
+    }
     NodesProductArgs p;
     p.a = nodes_args(c, b);
     rc = nodes_begin(p.a, l, kernel_type, ws, s);
