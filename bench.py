@@ -21,11 +21,11 @@ Printed keys (one JSON line, rank 0):
              ``kernel_matmul_b200.host.cg_solve_from_host`` with HOST (pinned) buffers: every rank
              copies x, params and its rows of Y to the device, builds the band, iterates, and copies
              its rows of the solution back;
-  roofline   the dominant kernel (``matmul_sum_ph_kernel``: the batch sum with the operator's phase
-             vectors written once per solve by a pre-pass; ``KM_SUM_PHASES=0`` selects
-             ``matmul_sum_tc_kernel``, which evaluates them in every product) against the measured dense bf16 rate
-             (its three fp16 MMAs per 16 phase values are what bounds it), its time taken with CUDA
-             events around the product inside the timed iterations;
+  roofline   the product, by CUDA events around it inside the timed iterations: the operator laid out
+             once between interpolation nodes (``node_product_kernel``) against the measured HBM rate;
+             or, with ``KM_SUM_PHASES=1`` / ``0``, the kernels that evaluate every entry (``matmul_sum_ph_kernel`` with
+             precomputed phase vectors, ``matmul_sum_tc_kernel`` without) against the measured dense bf16
+             rate (their three fp16 MMAs per 16 phase values are what bounds them);
   cpu_baseline  the dense PyTorch formulation (materialise every K_b, mask by ranges, matmul, sum)
              in fp32 on all host cores, on a seeded sample of row blocks of the same product,
              extrapolated linearly in entries;
@@ -472,8 +472,9 @@ def measure_mixture(w, dev, steps: int, path: str, fp32_peak: float, sfu_peak: f
         step_ms.append(e0.elapsed_time(e2))
     ops.check(dev)
     fwd, bwd = statistics.mean(fwd_ms), statistics.mean(bwd_ms)
-    fwd_name = "matmul_tc_kernel" if tc_fwd else "matmul_fma_kernel"
-    bwd_name = "grad_tc_kernel" if tc_bwd else "grad_band_kernel"
+    by_nodes = path == "auto" and not tc_fwd  # (what the automatic path does at this size)
+    fwd_name = "nodes_product_kernel" if by_nodes else ("matmul_tc_kernel" if tc_fwd else "matmul_fma_kernel")
+    bwd_name = "nodes_grad_kernel" if by_nodes else ("grad_tc_kernel" if tc_bwd else "grad_band_kernel")
     kernels = {
         fwd_name: {"ms": fwd, "sfu_per_entry": TC_FWD[kt][1] if tc_fwd else GEN_FWD[kt][1],
                    "contraction": "tcgen05.mma kind::f16 (fp16 hi/lo split)" if tc_fwd else "fma.rn.f32x2",
@@ -488,6 +489,10 @@ def measure_mixture(w, dev, steps: int, path: str, fp32_peak: float, sfu_peak: f
         kd["achieved_sfu_tops"] = E * kd["sfu_per_entry"] / (kd["ms"] * 1e-3) / 1e12
         kd["frac_sfu"] = kd["achieved_sfu_tops"] / sfu_peak
         kd["traffic"] = dram_traffic("spectral_mixture", kname) if w.n == 65536 else None
+        if by_nodes:
+            kd["contraction"] = "between interpolation nodes (fma.rn.f32x2)"
+            kd["note"] = ("all kernels of the call; rates and fractions count the work of evaluating every entry, which "
+                          "interpolation does not do: they may exceed 1")
     ms_per_step = statistics.mean(step_ms)
     res = {
         "config": config_of(w, E), "path": path, "ms_per_step": ms_per_step, "value": 2.0 * E * k / (ms_per_step * 1e-3),
@@ -812,6 +817,24 @@ def run_cg(args, rank: int, world: int, local: int) -> None:
                            "the library's live calibration kernels.  The metric counts component entries (B per unique "
                            "entry), as the reference would evaluate them",
         }
+        nodes = op.current_nodes()
+        if nodes is not None:
+            # a product reads the node matrix (P^2 values per pair of 128-point blocks in the band), the Lagrange
+            # matrices of its columns and of its rows, the vector, and writes and reads the vector at the nodes
+            P = int(nodes.plan().tolist()[3])
+            col_blocks, row_blocks = (op.hi - op.lo) / 128, (op.row1 - op.row0) / 128
+            product_bytes = 4.0 * (e_unique / 128**2 * P * P + (col_blocks + row_blocks) * P * 128 + (op.hi - op.lo) * k
+                                   + 2 * col_blocks * P * k + op.rows * k)
+            hbm = peaks.get("hbm_gbs", 6650.0)
+            roofline = {
+                "bound": "hbm", "kernel": "node_product_kernel (with node_compress_kernel)", "achieved": product_bytes / t_prod / 1e9,
+                "peak": hbm, "unit": "GB/s", "frac": product_bytes / t_prod / 1e9 / hbm, "product_ms": product_ms,
+                "algorithmic_bytes_per_product": product_bytes, "nodes_per_block": P,
+                "peak_source": "MEASURED_PEAKS.json hbm_gbs" if peaks else "fallback 6650 GB/s (MEASURED_PEAKS.json absent)",
+                "what": "the operator is a matrix between P Chebyshev points per 128-point block, summed over the components and "
+                        "laid out once per operator (inside the end-to-end figure, outside the timed iterations); the metric "
+                        "counts component entries, as the reference would evaluate them",
+            }
         line = {
             "metric": METRIC, "value": units / (ms_per_step * 1e-3), "unit": UNIT, "n_gpus": world,
             "steps": args.steps, "warmup": warm, "ms_per_step": ms_per_step,
@@ -820,7 +843,8 @@ def run_cg(args, rank: int, world: int, local: int) -> None:
             "exchange": op.mode,
             "phase_vectors": ("written once per operator by a pre-pass (%.2f GB workspace per rank; inside the end-to-end "
                               "figure, outside the timed iterations)" % (phase_ws.numel() / 1e9)) if phase_ws is not None
-                             else "evaluated inside every product (KM_SUM_PHASES=0)",
+                             else ("none: operator laid out between nodes" if nodes is not None
+                                   else "evaluated inside every product (KM_SUM_PHASES=0)"),
             "collective": {"single": "none (one rank)",
                            "halo": f"2 NCCL all_gather_into_tensor per iteration: [{op.halo_above} + {op.halo_below} halo rows "
                                    f"of q + segment sums of p.q] and [segment sums of r.r]",
@@ -836,7 +860,8 @@ def run_cg(args, rank: int, world: int, local: int) -> None:
                     "relative_residual": e2e_residual,
                     "what": "host.cg_solve_from_host: pinned host x, params, Y rows in; band, operator set-up, "
                             f"{iters} iterations; solution rows out"},
-            # per iteration: product (tensor-core kernel + FMA-pipe companion), q/dots, 2 x segment sums, 2 x update
+            # per iteration: product (compression + node product, or tensor-core kernel + FMA-pipe companion),
+            # q/dots, 2 x segment sums, 2 x update
             "gpu_launches": 7 * args.steps,
             "iteration_breakdown_ms": breakdown,
             "relative_residual_after_timed_region": residual,
