@@ -45,6 +45,10 @@ constexpr int64_t TENSOR_CORE_MIN_K = 9, GRAD_TENSOR_CORE_MIN_K = 8, TENSOR_CORE
 // (batch, row block) items from which the automatic path tries blockwise interpolation
 // (km_matmul_nodes_f32): its four small passes take about 10 us more than they save below.
 constexpr int64_t NODES_MIN_ITEMS = 512;
+// With a band, both sides share an interval: where one has this many times the other's points, the blocks
+// of the sparser are too long for it (5003 test points against 50 021: 100 nodes and more) and the call would pay
+// 25 us for finding out.
+constexpr int64_t NODES_MAX_RATIO = 8;
 // Without a cutoff: kernel entries from which it does (the points have to be put in order first).
 constexpr int64_t NODES_MIN_ENTRIES = 1LL << 27;
 
@@ -80,7 +84,8 @@ struct Problem {
     bool try_nodes(int64_t path) const {
         if (path == PATH_NODES) return true;
         if (path != PATH_AUTO) return false;
-        return one_range() ? m * n * (items() / row_blocks) >= NODES_MIN_ENTRIES : items() >= NODES_MIN_ITEMS;
+        if (one_range()) return m * n * (items() / row_blocks) >= NODES_MIN_ENTRIES;
+        return items() >= NODES_MIN_ITEMS && std::max(m, n) < NODES_MAX_RATIO * std::min(m, n);
     }
     void *stream() const { return c10::cuda::getCurrentCUDAStream(device).stream(); }
 
