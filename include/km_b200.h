@@ -518,12 +518,15 @@ KM_API int km_cg_log_forms_f32(int64_t iterations, int64_t k, const float *alpha
 
 /* ---------------------------------------------------------------------------------------
  * The operator of a CG solve by blockwise interpolation (see km_matmul_nodes_f32), laid out once and
- * applied many times.  K = sum over the batch of params of kernels that share the points x (n values,
- * x_stride elements apart) and the band start / end (contiguous, one per row block).
+ * applied many times.  K = sum over the batch of params of spectral kernels that share the points x (n
+ * values, x_stride elements apart), the band start / end (contiguous, one per row block) and the
+ * lengthscale, applied to up to KM_NODE_MAX_COLUMNS columns: the case of the tensor-core batch sum of
+ * km_matmul_rows_f32, whose entries have errors of the same size, a part of the kernel's maximum.
  *  - plan: looks at points, band and parameters; `plan` (KM_NODE_PLAN_BYTES, 8-byte aligned) begins with
  *    five int64: first and last column the row blocks of the window read, a checksum of the whole
- *    band, the nodes per block (0: this operator cannot be laid out so) and the widest band of the
- *    window in blocks; `centre` receives one value per row block.
+ *    band, the nodes per block (0: this operator cannot be laid out so) and the widest band of any
+ *    row block in blocks; `centre` receives one value per row block.  With x and params NULL only the
+ *    first three are found out.
  *  - build, with these as `nodes` and `max_blocks`: lambda (row blocks x nodes x 128 floats) and
  *    matrix (row blocks of the window x max_blocks x nodes x nodes floats).
  *  - compress: nodes (row blocks x nodes x ceil4(k)) = lambda^T v for blocks [block_begin, block_end).
@@ -533,10 +536,11 @@ KM_API int km_cg_log_forms_f32(int64_t iterations, int64_t k, const float *alpha
  * No reference counterpart (its solves call matmul once per iteration).
  * ------------------------------------------------------------------------------------- */
 #define KM_NODE_PLAN_BYTES 128
-KM_API int km_node_operator_plan_f32(int kernel_type, const km_batch *batch, int64_t n, const float *x, int64_t x_stride,
+#define KM_NODE_MAX_COLUMNS 16
+KM_API int km_node_operator_plan_f32(const km_batch *batch, int64_t n, const float *x, int64_t x_stride,
                                      const km_view *params, const int32_t *start, const int32_t *end, int64_t row_block_begin,
                                      int64_t row_block_count, float *centre, void *plan, void *stream);
-KM_API int km_node_operator_build_f32(int kernel_type, const km_batch *batch, int64_t n, const float *x, int64_t x_stride,
+KM_API int km_node_operator_build_f32(const km_batch *batch, int64_t n, const float *x, int64_t x_stride,
                                       const km_view *params, const int32_t *start, const int32_t *end, int64_t row_block_begin,
                                       int64_t row_block_count, const float *centre, const void *plan, int64_t nodes,
                                       int64_t max_blocks, float *lambda, float *matrix, void *stream);

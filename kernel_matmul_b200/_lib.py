@@ -142,9 +142,9 @@ def _load() -> ctypes.CDLL:
     lib.km_cg_log_forms_f32.argtypes = [i64, i64, vp, vp, vp, vp, f32, vp, vp]
     ip = vp
     lib.km_node_operator_plan_f32.restype = ctypes.c_int
-    lib.km_node_operator_plan_f32.argtypes = [ctypes.c_int, bp, i64, vp, i64, wp, ip, ip, i64, i64, vp, vp, vp]
+    lib.km_node_operator_plan_f32.argtypes = [bp, i64, vp, i64, wp, ip, ip, i64, i64, vp, vp, vp]
     lib.km_node_operator_build_f32.restype = ctypes.c_int
-    lib.km_node_operator_build_f32.argtypes = [ctypes.c_int, bp, i64, vp, i64, wp, ip, ip, i64, i64, vp, vp, i64, i64, vp, vp, vp]
+    lib.km_node_operator_build_f32.argtypes = [bp, i64, vp, i64, wp, ip, ip, i64, i64, vp, vp, i64, i64, vp, vp, vp]
     lib.km_node_compress_f32.restype = ctypes.c_int
     lib.km_node_compress_f32.argtypes = [i64, i64, i64, vp, vp, vp, i64, i64, vp]
     lib.km_node_update_p_f32.restype = ctypes.c_int

@@ -53,8 +53,8 @@ BLOCK_SIZE = 128
 MAX_SEGMENTS = 64
 
 
-#: points from which a solve lays its operator out as a node matrix; below, the kernels are evaluated in
-#: every product
+#: points from which a solve over a sum of spectral components lays its operator out as a node matrix;
+#: below, the kernels are evaluated in every product
 NODE_OPERATOR_MIN_ROWS = 4096
 #: most memory for the node matrix of a rank
 NODE_OPERATOR_MAX_BYTES = 16 << 30
@@ -221,10 +221,14 @@ class ShardedOperator:
         """Operator backed by ``ops.matmul_rows`` (sum over the batch of ``params`` if batched);
         ``start`` / ``end`` are one band ``(R,)`` shared by all components.
 
-        From ``NODE_OPERATOR_MIN_ROWS`` points, where the points' blocks are short enough against what
-        the kernel varies over (sorted points; bands aligned to blocks), the operator is laid out as a
-        matrix between the nodes of blockwise interpolation (``km_node_operator_build_f32``), summed over
-        all components, once; a product then reads it instead of evaluating kernels.
+        A sum of 2 to 1024 spectral components with one lengthscale on ``NODE_OPERATOR_MIN_ROWS`` points and
+        more, where the points' blocks are short enough against what the kernel varies over (sorted points;
+        bands aligned to blocks), is laid out as a matrix between the nodes of blockwise interpolation
+        (``km_node_operator_build_f32``) once; a product of up to 16 columns then reads it instead of
+        evaluating kernels.  These are the sums whose products otherwise run on the tensor cores, with an error per
+        entry that is as large a part of the kernel's maximum.  Every other operator is evaluated: those
+        kernels hold each entry to about 1e-6 of itself, and tens of CG steps on a system of condition
+        number 1000 turn a change of their last bits into 1e-4 of a gradient of the marginal likelihood.
 
         ``phases``: for a sum of spectral components, write the per-point phase vectors once now
         (``ops.prepare_sum_phases``: about ``16 B n`` bytes for ``B`` components) so that every product
@@ -235,7 +239,7 @@ class ShardedOperator:
         import os
 
         from . import _C, ops
-        from ._lib import KERNEL_TYPES
+        from ._lib import KM_MAX_BATCH_DIMS
 
         n = x.shape[-1]
         batched = params.dim() > 1
@@ -267,7 +271,8 @@ class ShardedOperator:
             return call
 
         def matvec_rows(v: Tensor, rb_begin: int, rb_count: int, out: Tensor) -> None:
-            by_nodes = current_nodes() if (rb_begin, rb_count) == (begin, count) and v.is_contiguous() and out.is_contiguous() else None
+            whole = (rb_begin, rb_count) == (begin, count) and v.is_contiguous() and out.is_contiguous()
+            by_nodes = current_nodes(v.shape[-1]) if whole else None
             if by_nodes is not None:
                 by_nodes.matvec(v, out)
             else:
@@ -279,19 +284,22 @@ class ShardedOperator:
         rank = dist.get_rank(group) if world > 1 else 0
         R = -(-n // BLOCK_SIZE)
         begin, count = row_block_window(R, rank, world)
+        may_lay_out = (not direct and n >= NODE_OPERATOR_MIN_ROWS and kernel_type == "spectral" and x.dim() == 1
+                       and 1 <= len(B) <= KM_MAX_BATCH_DIMS and 2 <= B.numel() <= 1024)
+
         # the columns this rank's row blocks read, a checksum of the whole band, and how many nodes
         # per block and blocks per band a node operator would have (one host synchronisation, at
         # set-up only)
         def plan_nodes():
-            plan = _C.NodeOperator(KERNEL_TYPES.get(kernel_type, -1), x, params, start.reshape(-1)[:R], end.reshape(-1)[:R], begin, count)
+            looked_at = (x, params) if may_lay_out else (None, None)
+            plan = _C.NodeOperator(n, *looked_at, start.reshape(-1)[:R], end.reshape(-1)[:R], begin, count)
             return (plan, *(int(v) for v in plan.plan().tolist()))
 
         def versions():
             return tuple(None if t.is_inference() else t._version for t in (x, params, start, end))
 
         def usable(node_count: int, widest: int) -> bool:
-            return (not direct and n >= NODE_OPERATOR_MIN_ROWS and node_count > 0
-                    and 4 * count * widest * node_count**2 <= NODE_OPERATOR_MAX_BYTES)
+            return node_count > 0 and 4 * count * widest * node_count**2 <= NODE_OPERATOR_MAX_BYTES
 
         laid_out = versions()
         plan, lo, hi, checksum, node_count, widest = plan_nodes()
@@ -302,10 +310,12 @@ class ShardedOperator:
             phase_ws = ops.prepare_sum_phases(kernel_type, x, x, params, rows=(begin * BLOCK_SIZE, min(n, (begin + count) * BLOCK_SIZE)),
                                               cols=(max(0, min(lo, n)), max(0, min(hi, n))))
 
-        def current_nodes():
-            """The node operator, laid out again if points, parameters or band were written to since;
-            ``None``: the products evaluate the kernels."""
+        def current_nodes(k: int = 1):
+            """The node operator for products of ``k`` columns, laid out again if points, parameters or band
+            were written to since; ``None``: the products evaluate the kernels."""
             nonlocal nodes, laid_out
+            if k > _C.NODE_MAX_COLUMNS:
+                return None
             if nodes is not None and versions() != laid_out:
                 laid_out = versions()
                 again, now_lo, now_hi, _, node_count, widest = plan_nodes()
@@ -441,7 +451,7 @@ class CGSolver:
                 getattr(op, "rows_product", None) is not None:
             from . import _C
 
-            nodes = op.current_nodes()
+            nodes = op.current_nodes(self.k)
             rows = None if nodes is not None else op.rows_product(self.p[: op.n], op.begin, op.count, self.kp[op.row0: op.row1])
             state = _C.CgState(self.x, self.r, self.p, self.kp, self.bp, self.rs, self.ynorm, self.history, self.alphas, self.betas,
                                self.send1, self.send2, op.n, self.k, op.count, op.seg_blocks, op.segs_per_rank, op.sigma2)

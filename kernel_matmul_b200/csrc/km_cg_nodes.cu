@@ -3,9 +3,13 @@
 // A solve applies ONE operator many times, so what the products of km_nodes.cu form on every call is
 // laid out once here: P nodes per block of 128 points (one interval length for all blocks), the
 // Lagrange matrices, and the kernel matrix between the nodes,
-//     G[r][c - c_lo(r)][q][p] = sum_b scale_b kappa_b(xi_{r,p} - xi_{c,q}),
+//     G[r][c - c_lo(r)][q][p] = exp(-tau^2 / 2 l^2) sum_b s_b cos(2 pi f_b tau),   tau = xi_{r,p} - xi_{c,q},
 // summed over all components of the operator: whatever their number, a product then reads
-// P^2 values per pair of blocks instead of evaluating 128^2 x components.  With P = 14 that is 0.56 GB for
+// P^2 values per pair of blocks instead of evaluating 128^2 x components.  An entry's error is a part of the
+// kernel's MAXIMUM (km_nodes.cuh), as that of the tensor-core batch sum is, so only operators that run on that
+// one otherwise are laid out: sums of 2 and more spectral components with one lengthscale, for up to
+// KM_NODE_MAX_COLUMNS columns.  The FMA kernels that evaluate all others hold every entry to 1e-6 of ITSELF, and
+// tens of CG steps bring a difference in the entries' last bits back a thousand times larger.  With P = 14 that is 0.56 GB for
 // 4 million points and a band of 22 blocks; a product is 85 us of HBM time for it, 135 us for the vectors
 // and Lagrange matrices, where the sum of 64 components took 11 ms on the tensor cores.
 //
@@ -23,8 +27,8 @@ constexpr int NODE_OP_MAX = 32;  // most nodes per block of an operator
 struct NodePlan {
     long long lo, hi;        // columns read by the row blocks of the window
     long long checksum;      // of the whole band
-    long long P;             // nodes per block; 0: not this way (band not aligned, or too many nodes)
-    long long max_blocks;    // widest band of the window, in blocks
+    long long P;             // nodes per block; 0: not this way (band not aligned, several lengthscales, too many nodes)
+    long long max_blocks;    // widest band of any row block, in blocks
     int max_h_bits, done, bad, width;
     int lo_bits, hi_bits;
 };
@@ -40,12 +44,12 @@ struct NodePlanArgs {
     NodePlan *plan;
 };
 
-template <int KT>
+// (x null: lo, hi and checksum only, P 0)
 __global__ void __launch_bounds__(256) node_plan_kernel(const NodePlanArgs a) {
     const int lane = threadIdx.x & 31;
     float longest = 0.0f;
     int bad = 0;
-    for (int64_t v = blockIdx.x * 8LL + (threadIdx.x >> 5); v < a.R; v += gridDim.x * 8LL) {
+    for (int64_t v = blockIdx.x * 8LL + (threadIdx.x >> 5); a.x != nullptr && v < a.R; v += gridDim.x * 8LL) {
         float lo = INFINITY, hi = -INFINITY;
         bool nan = false;
 #pragma unroll
@@ -75,14 +79,14 @@ __global__ void __launch_bounds__(256) node_plan_kernel(const NodePlanArgs a) {
         if (r >= a.rb0 && r < a.rb1) first = min(first, s), last = max(last, e);
         if (s >= e) continue;
         bad |= s < 0 || s % KM_BLOCK_SIZE != 0 || (e < a.n && e % KM_BLOCK_SIZE != 0);
-        if (r >= a.rb0 && r < a.rb1) width = max(width, (int)((min((int64_t)e, a.n) - s + KM_BLOCK_SIZE - 1) / KM_BLOCK_SIZE));
+        width = max(width, (int)((min((int64_t)e, a.n) - s + KM_BLOCK_SIZE - 1) / KM_BLOCK_SIZE));
     }
     first = __reduce_min_sync(0xffffffffu, first);
     last = __reduce_max_sync(0xffffffffu, last);
     width = __reduce_max_sync(0xffffffffu, width);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    __shared__ int s_last, s_p;
+    __shared__ int s_last, s_p, s_lengthscales;
     bad = __syncthreads_or(bad);
     if (lane == 0) {
         atomicMax(&a.plan->max_h_bits, __float_as_int(longest));
@@ -97,16 +101,19 @@ __global__ void __launch_bounds__(256) node_plan_kernel(const NodePlanArgs a) {
         if (bad) a.plan->bad = 1;
         __threadfence();
         s_last = atomicAdd(&a.plan->done, 1) == (int)gridDim.x - 1;
-        s_p = 0;
+        s_p = a.x != nullptr ? 0 : 4096;
+        s_lengthscales = 1;
     }
     __syncthreads();
     if (!s_last) return;
     __threadfence();
     volatile NodePlan *plan = a.plan;
     const float h = __int_as_float(plan->max_h_bits);
-    for (int64_t b = threadIdx.x >> 5; b < a.batch.count; b += 8) {
-        const int p = nodes_needed<KT>(batch_ptr(a.params, decompose(a.batch, b)), a.params.s0, h, lane);
+    for (int64_t b = threadIdx.x >> 5; a.x != nullptr && b < a.batch.count; b += 8) {
+        const float *theta = batch_ptr(a.params, decompose(a.batch, b));
+        const int p = nodes_needed<KM_KERNEL_SPECTRAL>(theta, a.params.s0, h, lane);
         if (lane == 0) atomicMax(&s_p, p);
+        if (lane == 0 && !(theta[0] == a.params.data[0])) s_lengthscales = 2;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -114,7 +121,7 @@ __global__ void __launch_bounds__(256) node_plan_kernel(const NodePlanArgs a) {
         plan->lo = a.rb1 > a.rb0 ? INT_MAX - plan->lo_bits : 0;
         plan->hi = a.rb1 > a.rb0 ? plan->hi_bits : 0;
         plan->checksum = plan->checksum & ((1ll << 61) - 1);
-        plan->P = (plan->bad == 0 && P <= NODE_OP_MAX) ? P : 0;
+        plan->P = (plan->bad == 0 && s_lengthscales == 1 && P <= NODE_OP_MAX) ? P : 0;
         plan->max_blocks = plan->width;
     }
 }
@@ -172,14 +179,12 @@ __global__ void __launch_bounds__(128) node_lambda_kernel(const NodeOpArgs a) {
 // hold all rows.  Components are the outer loop: the phase factors of the nodes are the same for
 // all pairs and lie in shared memory, all that changes from pair to pair is the phase of the centres'
 // distance (reduced in fp64), so a component costs 4 FMAs per pair to rotate the row's factors and 2 per
-// entry; where all spectral components share a lengthscale the envelope multiplies the finished sum.
+// entry; the envelope, one for all components, multiplies the finished sum.
 constexpr int GB_PAIRS = 6;
 constexpr int GB_COMPS = 32;  // components per chunk
 
-template <int KT>
 __global__ void __launch_bounds__(128) node_matrix_kernel(const NodeOpArgs a) {
-    using Fn = KernelFn<KT>;
-    constexpr bool SPECTRAL = KT == KM_KERNEL_SPECTRAL;
+    using Fn = KernelFn<KM_KERNEL_SPECTRAL>;
     __shared__ float delta[NODE_OP_MAX + 8];
     __shared__ __align__(16) float2 node_phase[GB_COMPS][NODE_OP_MAX + 8];  // cos, sin of W delta
     __shared__ float2 pair_phase[4][GB_PAIRS][GB_COMPS];
@@ -201,10 +206,6 @@ __global__ void __launch_bounds__(128) node_matrix_kernel(const NodeOpArgs a) {
     float D[GB_PAIRS];
 #pragma unroll
     for (int i = 0; i < GB_PAIRS; i++) D[i] = i < pairs ? centre - a.centre[c_lo + first + i] : 0.0f;
-    bool one_ell = SPECTRAL;
-    if constexpr (SPECTRAL)
-        for (int64_t b = lane; b < a.batch.count; b += 32) one_ell = one_ell && batch_ptr(a.params, decompose(a.batch, b))[0] == a.params.data[0];
-    one_ell = __all_sync(0xffffffffu, one_ell);
 
     const int q_step = 8 * (32 / width);
     for (int round = 0; round * q_step < P; round++) {
@@ -222,22 +223,20 @@ __global__ void __launch_bounds__(128) node_matrix_kernel(const NodeOpArgs a) {
                 const int b = i / P, q = i % P;
                 Fn fn;
                 fn.init(batch_ptr(a.params, decompose(a.batch, b0 + b)), a.params.s0);
-                float c = 1.0f, sn = 0.0f;
-                if constexpr (Fn::PHASE) sincospif(fn.phase_half_turns() * delta[q], &sn, &c);
+                float c, sn;
+                sincospif(fn.phase_half_turns() * delta[q], &sn, &c);
                 node_phase[b][q] = make_float2(c, sn);
                 if (q == 0) scales[b] = fn.scale;
             }
-            if constexpr (Fn::PHASE) {
-                if (lane < comps) {
-                    Fn fn;
-                    fn.init(batch_ptr(a.params, decompose(a.batch, b0 + lane)), a.params.s0);
+            if (lane < comps) {
+                Fn fn;
+                fn.init(batch_ptr(a.params, decompose(a.batch, b0 + lane)), a.params.s0);
 #pragma unroll
-                    for (int i = 0; i < GB_PAIRS; i++) {
-                        const double turns = (double)fn.phase_half_turns() * (double)D[i];
-                        float c, sn;
-                        sincospif((float)(turns - 2.0 * rint(0.5 * turns)), &sn, &c);
-                        pair_phase[warp][i][lane] = make_float2(c, sn);
-                    }
+                for (int i = 0; i < GB_PAIRS; i++) {
+                    const double turns = (double)fn.phase_half_turns() * (double)D[i];
+                    float c, sn;
+                    sincospif((float)(turns - 2.0 * rint(0.5 * turns)), &sn, &c);
+                    pair_phase[warp][i][lane] = make_float2(c, sn);
                 }
             }
             __syncthreads();
@@ -247,37 +246,13 @@ __global__ void __launch_bounds__(128) node_matrix_kernel(const NodeOpArgs a) {
                 float2 col[8];
 #pragma unroll
                 for (int j = 0; j < 8; j++) col[j] = node_phase[b][qs + j];
-                if (SPECTRAL && one_ell) {
 #pragma unroll
-                    for (int i = 0; i < GB_PAIRS; i++) {
-                        if (i >= pairs) break;
-                        const float2 ph = pair_phase[warp][i][b];
-                        const float rc = scale * (ph.x * row_phase.x - ph.y * row_phase.y), rs = scale * (ph.y * row_phase.x + ph.x * row_phase.y);
+                for (int i = 0; i < GB_PAIRS; i++) {
+                    if (i >= pairs) break;
+                    const float2 ph = pair_phase[warp][i][b];
+                    const float rc = scale * (ph.x * row_phase.x - ph.y * row_phase.y), rs = scale * (ph.y * row_phase.x + ph.x * row_phase.y);
 #pragma unroll
-                        for (int j = 0; j < 8; j++) acc[i][j] = fmaf(rc, col[j].x, fmaf(rs, col[j].y, acc[i][j]));
-                    }
-                } else {
-                    Fn fn;
-                    fn.init(batch_ptr(a.params, decompose(a.batch, b0 + b)), a.params.s0);
-#pragma unroll
-                    for (int i = 0; i < GB_PAIRS; i++) {
-                        if (i >= pairs) break;
-                        float rc = 1.0f, rs = 0.0f;
-                        if constexpr (Fn::PHASE) {
-                            const float2 ph = pair_phase[warp][i][b];
-                            rc = ph.x * row_phase.x - ph.y * row_phase.y, rs = ph.y * row_phase.x + ph.x * row_phase.y;
-                        }
-                        const float y = D[i] + dp;
-#pragma unroll
-                        for (int j = 0; j < 8; j += 2) {
-                            f32x2 cs = 0ull;
-                            if constexpr (Fn::PHASE) cs = pack2(rc * col[j].x + rs * col[j].y, rc * col[j + 1].x + rs * col[j + 1].y);
-                            float k0, k1;
-                            unpack2(fn.unscaled2_ph(pack2(y - delta[qs + j], y - delta[qs + j + 1]), cs, 0ull), k0, k1);
-                            acc[i][j] = fmaf(scale, k0, acc[i][j]);
-                            acc[i][j + 1] = fmaf(scale, k1, acc[i][j + 1]);
-                        }
-                    }
+                    for (int j = 0; j < 8; j++) acc[i][j] = fmaf(rc, col[j].x, fmaf(rs, col[j].y, acc[i][j]));
                 }
             }
         }
@@ -290,12 +265,8 @@ __global__ void __launch_bounds__(128) node_matrix_kernel(const NodeOpArgs a) {
 #pragma unroll
                 for (int j = 0; j < 8; j++) {
                     if (q0 + j >= P) break;
-                    float v = acc[i][j];
-                    if (SPECTRAL && one_ell) {
-                        const float tau = (D[i] + dp) - delta[q0 + j];
-                        v *= exp2f(c0 * tau * tau);
-                    }
-                    out[(q0 + j) * P] = v;
+                    const float tau = (D[i] + dp) - delta[q0 + j];
+                    out[(q0 + j) * P] = acc[i][j] * exp2f(c0 * tau * tau);
                 }
             }
         }
@@ -580,22 +551,12 @@ __global__ void __launch_bounds__(128) node_product_kernel(const NodeProductArgs
 }
 
 template <typename F>
-static int node_dispatch_kt(int kernel_type, F f) {
-    switch (kernel_type) {
-    case KM_KERNEL_RBF: return f(std::integral_constant<int, KM_KERNEL_RBF>());
-    case KM_KERNEL_SPECTRAL: return f(std::integral_constant<int, KM_KERNEL_SPECTRAL>());
-    default: return f(std::integral_constant<int, KM_KERNEL_LOCALLY_PERIODIC>());
-    }
-}
-
-template <int MAX_KC, typename F>
 static int node_dispatch_kc(int64_t k, F f) {
     if (k <= 1) return f(std::integral_constant<int, 1>());
     if (k <= 2) return f(std::integral_constant<int, 2>());
     if (k <= 4) return f(std::integral_constant<int, 4>());
     if (k <= 8) return f(std::integral_constant<int, 8>());
-    if (k <= 16 || MAX_KC == 16) return f(std::integral_constant<int, 16>());
-    return f(std::integral_constant<int, MAX_KC>());
+    return f(std::integral_constant<int, 16>());
 }
 
 static int node_compress(NodeVectorArgs g, cudaStream_t s) {
@@ -605,48 +566,50 @@ static int node_compress(NodeVectorArgs g, cudaStream_t s) {
     if (g.blk1 <= g.blk0 && g.r == nullptr) return KM_OK;
     // (an update always runs one CTA: it keeps the residual history)
     const unsigned ctas = (unsigned)std::max<int64_t>(1, g.blk1 - g.blk0);
-    return node_dispatch_kc<16>(g.k, [&](auto kc) {
+    return node_dispatch_kc(g.k, [&](auto kc) {
         return launch_chained("node compression launch", node_compress_kernel<decltype(kc)::value>, ctas, 128, 0, s, g);
     });
 }
 
 }  // namespace km
 
-extern "C" int km_node_operator_plan_f32(int kernel_type, const km_batch *batch, int64_t n, const float *x, int64_t x_stride,
+extern "C" int km_node_operator_plan_f32(const km_batch *batch, int64_t n, const float *x, int64_t x_stride,
                                          const km_view *params, const int32_t *start, const int32_t *end, int64_t row_block_begin,
                                          int64_t row_block_count, float *centre, void *plan, void *stream) {
     using namespace km;
-    KM_REQUIRE(valid_kernel_type(kernel_type) && batch && params, KM_ERR_INVALID_ARGUMENT, "km_node_operator_plan_f32: bad arguments");
-    NodePlanArgs a;
-    const int rc = make_batch(batch, &a.batch);
-    if (rc != KM_OK) return rc;
+    KM_REQUIRE((x == nullptr) == (params == nullptr) && (x == nullptr || batch), KM_ERR_INVALID_ARGUMENT,
+               "km_node_operator_plan_f32: bad arguments");
+    NodePlanArgs a = {};
+    if (x != nullptr) {
+        const int rc = make_batch(batch, &a.batch);
+        if (rc != KM_OK) return rc;
+        KM_REQUIRE(a.batch.count >= 1 && params->data && centre, KM_ERR_INVALID_ARGUMENT, "km_node_operator_plan_f32: bad arguments");
+        a.params = make_view<const float>(params, a.batch);
+    }
     const int64_t R = ceil_div(n, KM_BLOCK_SIZE);
-    KM_REQUIRE(n >= 1 && n <= 0x7fffffffLL - 256 && a.batch.count >= 1 && row_block_begin >= 0 && row_block_count >= 0 &&
+    KM_REQUIRE(n >= 1 && n <= 0x7fffffffLL - 256 && row_block_begin >= 0 && row_block_count >= 0 &&
                    row_block_begin + row_block_count <= R,
                KM_ERR_INVALID_ARGUMENT, "km_node_operator_plan_f32: bad sizes");
-    KM_REQUIRE(x && params->data && start && end && centre && plan && (uintptr_t)plan % 8 == 0, KM_ERR_INVALID_ARGUMENT,
-               "km_node_operator_plan_f32: null pointer");
+    KM_REQUIRE(start && end && plan && (uintptr_t)plan % 8 == 0, KM_ERR_INVALID_ARGUMENT, "km_node_operator_plan_f32: null pointer");
     a.n = n, a.R = R, a.rb0 = row_block_begin, a.rb1 = row_block_begin + row_block_count;
-    a.x = x, a.xs = x_stride, a.params = make_view<const float>(params, a.batch), a.start = start, a.end = end;
+    a.x = x, a.xs = x_stride, a.start = start, a.end = end;
     a.centre = centre, a.plan = static_cast<NodePlan *>(plan);
     static_assert(sizeof(NodePlan) <= KM_NODE_PLAN_BYTES, "plan size");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const cudaError_t err = cudaMemsetAsync(plan, 0, sizeof(NodePlan), s);
     if (err != cudaSuccess) return cuda_fail(err, "km_node_operator_plan_f32");
     const unsigned ctas = (unsigned)std::min<int64_t>(ceil_div(R, 8), 148 * 4);
-    return node_dispatch_kt(kernel_type, [&](auto kt) {
-        node_plan_kernel<decltype(kt)::value><<<ctas, 256, 0, s>>>(a);
-        KM_CHECK_LAUNCH("km_node_operator_plan_f32 launch");
-        return (int)KM_OK;
-    });
+    node_plan_kernel<<<ctas, 256, 0, s>>>(a);
+    KM_CHECK_LAUNCH("km_node_operator_plan_f32 launch");
+    return KM_OK;
 }
 
-extern "C" int km_node_operator_build_f32(int kernel_type, const km_batch *batch, int64_t n, const float *x, int64_t x_stride,
+extern "C" int km_node_operator_build_f32(const km_batch *batch, int64_t n, const float *x, int64_t x_stride,
                                           const km_view *params, const int32_t *start, const int32_t *end, int64_t row_block_begin,
                                           int64_t row_block_count, const float *centre, const void *plan, int64_t nodes,
                                           int64_t max_blocks, float *lambda, float *matrix, void *stream) {
     using namespace km;
-    KM_REQUIRE(valid_kernel_type(kernel_type) && batch && params, KM_ERR_INVALID_ARGUMENT, "km_node_operator_build_f32: bad arguments");
+    KM_REQUIRE(batch && params, KM_ERR_INVALID_ARGUMENT, "km_node_operator_build_f32: bad arguments");
     NodeOpArgs a;
     const int rc = make_batch(batch, &a.batch);
     if (rc != KM_OK) return rc;
@@ -667,17 +630,15 @@ extern "C" int km_node_operator_build_f32(int kernel_type, const km_batch *batch
     const int64_t items = row_block_count * ceil_div(max_blocks, GB_PAIRS);
     if (items == 0) return KM_OK;
     KM_REQUIRE(items <= 0x7fffffffLL, KM_ERR_UNSUPPORTED, "km_node_operator_build_f32: too many blocks");
-    return node_dispatch_kt(kernel_type, [&](auto kt) {
-        node_matrix_kernel<decltype(kt)::value><<<(unsigned)ceil_div(items, 4), 128, 0, s>>>(a);
-        KM_CHECK_LAUNCH("km_node_operator_build_f32 launch");
-        return (int)KM_OK;
-    });
+    node_matrix_kernel<<<(unsigned)ceil_div(items, 4), 128, 0, s>>>(a);
+    KM_CHECK_LAUNCH("km_node_operator_build_f32 launch");
+    return KM_OK;
 }
 
 extern "C" int km_node_compress_f32(int64_t k, int64_t n, int64_t nodes_per_block, const float *lambda, const float *v, float *nodes,
                                     int64_t block_begin, int64_t block_end, void *stream) {
     using namespace km;
-    KM_REQUIRE(k >= 1 && n >= 1 && nodes_per_block >= 4 && nodes_per_block <= NODE_OP_MAX && block_begin >= 0 && block_end >= block_begin &&
+    KM_REQUIRE(k >= 1 && k <= KM_NODE_MAX_COLUMNS && n >= 1 && nodes_per_block >= 4 && nodes_per_block <= NODE_OP_MAX && block_begin >= 0 && block_end >= block_begin &&
                    block_end <= ceil_div(n, KM_BLOCK_SIZE) && lambda && v && nodes,
                KM_ERR_INVALID_ARGUMENT, "km_node_compress_f32: bad arguments");
     NodeVectorArgs g{};
@@ -691,7 +652,7 @@ extern "C" int km_node_update_p_f32(int64_t k, int64_t n, int64_t nodes_per_bloc
                                     int64_t seg_rank_stride_bytes, int32_t seg_ranks, int32_t seg_slots, const float *rs_old,
                                     float *rs_new, const float *ynorm, float *history_row, float *beta_row, void *stream) {
     using namespace km;
-    KM_REQUIRE(k >= 1 && n >= 1 && nodes_per_block >= 4 && nodes_per_block <= NODE_OP_MAX && block_begin >= 0 && block_end >= block_begin &&
+    KM_REQUIRE(k >= 1 && k <= KM_NODE_MAX_COLUMNS && n >= 1 && nodes_per_block >= 4 && nodes_per_block <= NODE_OP_MAX && block_begin >= 0 && block_end >= block_begin &&
                    block_end <= ceil_div(n, KM_BLOCK_SIZE) && lambda && p && r && nodes && rr_seg_sums && rs_old && rs_new &&
                    rs_old != rs_new && (history_row == nullptr || ynorm) && seg_ranks >= 1 && seg_slots >= 0 && seg_rank_stride_bytes % 8 == 0,
                KM_ERR_INVALID_ARGUMENT, "km_node_update_p_f32: bad arguments");
@@ -708,7 +669,7 @@ extern "C" int km_node_product_f32(int64_t k, int64_t n, int64_t nodes_per_block
                                    int64_t row_block_begin, int64_t row_block_count, float *out, const float *p, float sigma2,
                                    float *block_partials, void *stream) {
     using namespace km;
-    KM_REQUIRE(k >= 1 && n >= 1 && nodes_per_block >= 4 && nodes_per_block <= NODE_OP_MAX && row_block_begin >= 0 && row_block_count >= 0 &&
+    KM_REQUIRE(k >= 1 && k <= KM_NODE_MAX_COLUMNS && n >= 1 && nodes_per_block >= 4 && nodes_per_block <= NODE_OP_MAX && row_block_begin >= 0 && row_block_count >= 0 &&
                    row_block_begin + row_block_count <= ceil_div(n, KM_BLOCK_SIZE) && row_block_count <= 0x7fffffffLL && start && end &&
                    lambda && nodes && out && (matrix || max_blocks == 0) && (p == nullptr || block_partials),
                KM_ERR_INVALID_ARGUMENT, "km_node_product_f32: bad arguments");
@@ -732,6 +693,5 @@ extern "C" int km_node_product_f32(int64_t k, int64_t n, int64_t nodes_per_block
     };
     if (k <= 4) return launch(std::integral_constant<int, 4>());
     if (k <= 8) return launch(std::integral_constant<int, 8>());
-    if (k <= 16) return launch(std::integral_constant<int, 16>());
-    return launch(std::integral_constant<int, 32>());
+    return launch(std::integral_constant<int, 16>());
 }

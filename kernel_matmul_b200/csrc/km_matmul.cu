@@ -564,6 +564,9 @@ static int dispatch_matmul(MatmulArgs<float> &a, cudaStream_t stream) {
     return launch_matmul<KT, 32, 2, 2, SUM>(a, stream);
 }
 
+// (the operator laid out between nodes stands in for the tensor-core batch sum and for nothing else)
+static_assert(KM_NODE_MAX_COLUMNS == SUM_TC_MAX_K, "columns of the node operator");
+
 static int matmul_entry(const char *name, int kernel_type, const km_batch *batch, int64_t m, int64_t n, int64_t k,
                         const km_view *x1, const km_view *x2, const km_view *rhs, const km_view *params,
                         const km_view *start, const km_view *end, const km_view *out, int64_t rb_begin,

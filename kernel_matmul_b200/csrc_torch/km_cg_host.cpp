@@ -5,27 +5,32 @@
 
 namespace kmh {
 
-NodeOperator::NodeOperator(int64_t kernel_type, const Tensor &x, const Tensor &params, const Tensor &start, const Tensor &end,
-                           int64_t row_block_begin, int64_t row_block_count)
-    : kid_((int)kernel_type), begin_(row_block_begin), count_(row_block_count), x_(x), params_(params) {
-    check_f32(x), check_f32(params), check_i32(start), check_i32(end);
-    TORCH_CHECK(x.dim() == 1 && params.dim() >= 1 && params.size(-1) == num_params(kernel_type), "x must be (n,) and params (.., P)");
-    n_ = x.size(0);
+NodeOperator::NodeOperator(int64_t n, const std::optional<Tensor> &x, const std::optional<Tensor> &params, const Tensor &start,
+                           const Tensor &end, int64_t row_block_begin, int64_t row_block_count)
+    : n_(n), begin_(row_block_begin), count_(row_block_count) {
+    check_i32(start), check_i32(end);
     R_ = (n_ + KM_BLOCK_SIZE - 1) / KM_BLOCK_SIZE;
     TORCH_CHECK(start.numel() >= R_ && end.numel() >= R_, "start / end must have ", R_, " entries");
     start_ = start.reshape({-1}).contiguous(), end_ = end.reshape({-1}).contiguous();
-    if (params_.dim() - 1 > KM_MAX_BATCH_DIMS) params_ = params_.reshape({-1, params_.size(-1)});
-    const int nb = (int)params_.dim() - 1;
-    kb_.ndim = nb;
-    for (int d = 0; d < nb; d++) kb_.size[d] = params_.size(d), vparams_.batch_stride[d] = params_.stride(d);
-    vparams_.data = params_.data_ptr();
-    vparams_.stride[0] = params_.stride(nb);
-    const c10::cuda::CUDAGuard guard(x.device());
-    const auto opt = x.options().requires_grad(false);
-    centre_ = at::empty({std::max<int64_t>(R_, 1)}, opt);
+    const c10::cuda::CUDAGuard guard(start_.device());
+    const auto opt = start_.options().requires_grad(false);
     plan_ = at::empty({KM_NODE_PLAN_BYTES / 8}, opt.dtype(at::kLong));
-    raise_on(km_node_operator_plan_f32(kid_, &kb_, n_, x_.const_data_ptr<float>(), x_.stride(0), &vparams_, start_.const_data_ptr<int32_t>(),
-                                       end_.const_data_ptr<int32_t>(), begin_, count_, centre_.data_ptr<float>(), plan_.data_ptr(), stream()));
+    if (x.has_value()) {
+        check_f32(*x), check_f32(*params);
+        x_ = *x, params_ = *params;
+        TORCH_CHECK(x_.dim() == 1 && x_.size(0) == n_ && params_.dim() >= 1 && params_.size(-1) == num_params(KM_KERNEL_SPECTRAL),
+                    "x must be (n,) and params (.., 3)");
+        if (params_.dim() - 1 > KM_MAX_BATCH_DIMS) params_ = params_.reshape({-1, params_.size(-1)});
+        const int nb = (int)params_.dim() - 1;
+        kb_.ndim = nb;
+        for (int d = 0; d < nb; d++) kb_.size[d] = params_.size(d), vparams_.batch_stride[d] = params_.stride(d);
+        vparams_.data = params_.data_ptr();
+        vparams_.stride[0] = params_.stride(nb);
+        centre_ = at::empty({std::max<int64_t>(R_, 1)}, opt.dtype(at::kFloat));
+    }
+    raise_on(km_node_operator_plan_f32(&kb_, n_, x ? x_.const_data_ptr<float>() : nullptr, x ? x_.stride(0) : 0, x ? &vparams_ : nullptr,
+                                       start_.const_data_ptr<int32_t>(), end_.const_data_ptr<int32_t>(), begin_, count_,
+                                       x ? centre_.data_ptr<float>() : nullptr, plan_.data_ptr(), stream()));
 }
 
 void NodeOperator::build(int64_t lo, int64_t hi, int64_t nodes, int64_t max_blocks) {
@@ -36,7 +41,7 @@ void NodeOperator::build(int64_t lo, int64_t hi, int64_t nodes, int64_t max_bloc
     blk0_ = std::min(blk0_, blk1_);
     lambda_ = at::empty({R_ * P_ * KM_BLOCK_SIZE}, opt);
     matrix_ = at::empty({std::max<int64_t>(1, count_ * max_blocks * P_ * P_)}, opt);
-    raise_on(km_node_operator_build_f32(kid_, &kb_, n_, x_.const_data_ptr<float>(), x_.stride(0), &vparams_, start_.const_data_ptr<int32_t>(),
+    raise_on(km_node_operator_build_f32(&kb_, n_, x_.const_data_ptr<float>(), x_.stride(0), &vparams_, start_.const_data_ptr<int32_t>(),
                                         end_.const_data_ptr<int32_t>(), begin_, count_, centre_.const_data_ptr<float>(), plan_.data_ptr(),
                                         P_, max_blocks_, lambda_.data_ptr<float>(), matrix_.data_ptr<float>(), stream()));
 }
@@ -69,7 +74,8 @@ void NodeOperator::matvec(const Tensor &v, const Tensor &out) const {
     TORCH_CHECK(v.dim() == 2 && v.size(0) == n_ && v.is_contiguous() && out.dim() == 2 && out.is_contiguous() && out.size(1) == v.size(1),
                 "v must be a contiguous (n, k) tensor and out (rows, k)");
     const int64_t rows = std::max<int64_t>(0, std::min(n_, (begin_ + count_) * KM_BLOCK_SIZE) - begin_ * KM_BLOCK_SIZE);
-    TORCH_CHECK(out.size(0) == rows, "out must have ", rows, " rows");
+    TORCH_CHECK(out.size(0) == rows && v.size(1) <= KM_NODE_MAX_COLUMNS, "out must have ", rows, " rows and at most ",
+                KM_NODE_MAX_COLUMNS, " columns");
     const c10::cuda::CUDAGuard guard(x_.device());
     const Tensor scratch = nodes(v.size(1));
     compress(v, v.size(1), scratch.data_ptr<float>());

@@ -15,8 +15,9 @@ struct CgState {
 
 class NodeOperator {
   public:
-    // Looks at points, band and parameters of a window of row blocks; `plan()` tells what came of it.
-    NodeOperator(int64_t kernel_type, const Tensor &x, const Tensor &params, const Tensor &start, const Tensor &end,
+    // Looks at the band -- and, of a sum of spectral components, at points and parameters -- for a window of row
+    // blocks of n points; `plan()` tells what came of it.
+    NodeOperator(int64_t n, const std::optional<Tensor> &x, const std::optional<Tensor> &params, const Tensor &start, const Tensor &end,
                  int64_t row_block_begin, int64_t row_block_count);
     // int64 on the device: lo, hi, checksum, nodes per block (0: not this way), widest band in blocks
     Tensor plan() const { return plan_.slice(0, 0, 5); }
@@ -30,8 +31,7 @@ class NodeOperator {
     void product(int64_t k, const float *nodes, float *out, const float *p, double sigma2, float *block_partials) const;
 
   private:
-    void *stream() const { return c10::cuda::getCurrentCUDAStream(x_.device().index()).stream(); }
-    int kid_;
+    void *stream() const { return c10::cuda::getCurrentCUDAStream(start_.device().index()).stream(); }
     int64_t n_, R_, begin_, count_, P_ = 0, max_blocks_ = 0, blk0_ = 0, blk1_ = 0;
     Tensor x_, params_, start_, end_, centre_, plan_, lambda_, matrix_;
     km_batch kb_{};

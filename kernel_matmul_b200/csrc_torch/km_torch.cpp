@@ -141,6 +141,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.attr("KERNEL_LOCALLY_PERIODIC") = (int)KM_KERNEL_LOCALLY_PERIODIC;
     m.attr("TENSOR_CORE_MIN_K") = kmh::TENSOR_CORE_MIN_K;
     m.attr("GRAD_TENSOR_CORE_MIN_K") = kmh::GRAD_TENSOR_CORE_MIN_K;
+    m.attr("NODE_MAX_COLUMNS") = KM_NODE_MAX_COLUMNS;
     m.attr("TENSOR_CORE_MIN_ITEMS") = kmh::TENSOR_CORE_MIN_ITEMS;
     // the package's own error types; without the package (the extension loaded by itself) RuntimeError
     py::register_exception_translator([](std::exception_ptr p) {
@@ -223,7 +224,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         .def_property_readonly("out", &kmh::RowsProduct::out)
         .def_property_readonly("tensor_cores", &kmh::RowsProduct::tensor_cores);
     py::class_<kmh::NodeOperator>(m, "NodeOperator")
-        .def(py::init<int64_t, const Tensor &, const Tensor &, const Tensor &, const Tensor &, int64_t, int64_t>())
+        .def(py::init<int64_t, const std::optional<Tensor> &, const std::optional<Tensor> &, const Tensor &, const Tensor &, int64_t,
+                      int64_t>())
         .def("plan", &kmh::NodeOperator::plan)
         .def("build", &kmh::NodeOperator::build, nogil())
         .def("matvec", &kmh::NodeOperator::matvec, nogil());

@@ -190,7 +190,8 @@ def test_ranges_without_cutoff_are_ordinary_tensors():
 @pytest.mark.parametrize("n", [4096, 4097, 5000])
 @pytest.mark.parametrize("kt,components,width", [("rbf", 0, 100.0), ("spectral", 3, 100.0), ("spectral", 40, 60.0), ("locally_periodic", 2, 200.0)])
 def test_cg_operator_laid_out_once(n, kt, components, width):
-    """K v from the node matrix, P <= 16 and beyond, one and several chunks of components and columns."""
+    """K v from the node matrix, P <= 16 and beyond, one and several chunks of components and columns;
+    operators other than sums of spectral components with one lengthscale are evaluated."""
     from kernel_matmul_b200 import ranges
     from kernel_matmul_b200.cg import ShardedOperator
 
@@ -198,9 +199,11 @@ def test_cg_operator_laid_out_once(n, kt, components, width):
 
     x = torch.sort(torch.rand(n) * (n / width))[0]
     params = make_params(kt, (components,) if components else ())
+    if kt == "spectral":
+        params[..., 0] = 0.9
     start, end = ranges.make_ranges(3.0, x.cuda())
     op = ShardedOperator.from_kernel(kt, x.cuda(), params.cuda(), start, end, 0.1)
-    assert op.current_nodes() is not None
+    assert (op.current_nodes() is not None) == (kt == "spectral") and op.current_nodes(17) is None
     B = (components,) if components else ()
     rows = torch.arange(n - 384 - n % 128, n)  # the last row blocks (the oracle takes its time)
     first = int(rows[0]) // 128
@@ -220,17 +223,17 @@ def test_cg_operator_follows_its_parameters():
 
     n, k = 6000, 8
     x = torch.sort(torch.rand(n) * 60)[0].cuda()
-    params = torch.tensor([1.0, 1.2], device="cuda")
+    params = torch.tensor([[1.0, 0.0, 1.2], [1.0, 0.4, 0.7]], device="cuda")
     start, end = ranges.make_ranges(3.0, x)
-    op = ShardedOperator.from_kernel("rbf", x, params, start, end, 0.1)
+    op = ShardedOperator.from_kernel("spectral", x, params, start, end, 0.1)
     v = torch.randn(n, k, device="cuda")
     before = op.apply(v)
-    params.copy_(torch.tensor([0.7, 0.9]))
-    fresh = ShardedOperator.from_kernel("rbf", x, params.clone(), start, end, 0.1)
+    params.copy_(torch.tensor([[0.7, 0.1, 0.9], [0.7, 0.5, 0.8]]))
+    fresh = ShardedOperator.from_kernel("spectral", x, params.clone(), start, end, 0.1)
     after = op.apply(v)
-    assert torch.equal(after, fresh.apply(v)) and not torch.equal(after, before)
-    params[0] = 0.004  # a block spans many lengthscales: evaluated directly
-    assert rel_err(op.apply(v), ShardedOperator.from_kernel("rbf", x, params, start, end, 0.1, phases=False).apply(v)) <= TOL
+    assert fresh.current_nodes() is not None and torch.equal(after, fresh.apply(v)) and not torch.equal(after, before)
+    params[:, 0] = 0.004  # a block spans many lengthscales: evaluated directly
+    assert rel_err(op.apply(v), ShardedOperator.from_kernel("spectral", x, params, start, end, 0.1, phases=False).apply(v)) <= TOL
 
     vs = [torch.randn(n, k, device="cuda") for _ in range(4)]
     ref = [fresh.apply(w) for w in vs]
@@ -243,6 +246,27 @@ def test_cg_operator_follows_its_parameters():
                 got.append(fresh.apply(w))
         torch.cuda.synchronize()
         assert all(torch.equal(g, r) for g, r in zip(got, ref))
+
+
+@pytest.mark.parametrize("form", ["rbf", "spectral", "locally_periodic", "several lengthscales", "one component", "points of their own"])
+@pytest.mark.parametrize("k", [8, 16])
+def test_solves_of_operators_that_are_not_laid_out(form, k):
+    """Iterates to the bit those of the kernels evaluated in every product, which is what CG steps leave of a
+    relative accuracy of 1e-6 per entry (the node matrix has an error relative to its largest entry)."""
+    from kernel_matmul_b200 import ranges
+    from kernel_matmul_b200.cg import ShardedOperator, conjugate_gradient
+
+    n, kt = 5000, form if form in KERNEL_TYPES else "spectral"
+    x = (torch.sort(torch.rand(n))[0] * 50).cuda()
+    batch = {"several lengthscales": (3,), "one component": (1,), "points of their own": (2,)}.get(form, ())
+    if form == "points of their own":
+        kt, x = "rbf", torch.stack([x, x + 0.01])
+    params = make_params(kt, batch, 0.3).cuda()  # lengthscales up to 0.6: the band cuts off at 5 of them
+    start, end = ranges.make_ranges(3.0, x[0] if x.dim() == 2 else x)
+    y = torch.randn(n, k, device="cuda")
+    solves = [conjugate_gradient(ShardedOperator.from_kernel(kt, x, params, start, end, 0.2, phases=p), y, 30) for p in (None, False)]
+    assert torch.equal(solves[0].solution, solves[1].solution) and torch.equal(solves[0].residual_norms, solves[1].residual_norms)
+    assert bool(solves[0].solution.isfinite().all())
 
 
 def test_log_forms_on_the_device_match_the_eigenvalues():
