@@ -709,7 +709,10 @@ struct NodeItem {
             }
             if (l == row_level) P = col_P[l], row_class = col_class[l];
         }
-        stage_floats = max(col_P[0], P) * NodeShape<KC>::QS;  // (the longest half-length has the most nodes)
+        // The most nodes this kernel has at any half-length: NOT always those of the longest, as every level of
+        // the plan merges its smaller classes into larger ones by itself.
+        stage_floats = max(max(col_P[0], col_P[1]), max(col_P[2], col_P[3])) * NodeShape<KC>::QS;
+        static_assert(NODES_LEVELS == 4, "stage_floats");
         stages = 8 * stage_floats <= NodeShape<KC>::TILE_FLOATS ? 2 : 1;
         tiles = smem + (threadIdx.x >> 5) * stages * stage_floats;
         __syncthreads();

@@ -98,6 +98,79 @@ def test_batch_forms(form):
         _both(kt, x, x, rhs, torch.randn(*batch, n, k), params[kt], start, end)
 
 
+def _half_lengths(x):
+    """Half-lengths of the 128-point blocks of (.., n) sorted points."""
+    blocks = [x[..., i:i + 128] for i in range(0, x.shape[-1], 128)]
+    return torch.stack([0.5 * (b[..., -1] - b[..., 0]) for b in blocks], dim=-1)
+
+
+def _nodes_by_level(kt, params, longest, unit, cap, classes=8, eps=3e-8):
+    """The plan of csrc/km_nodes.cu restated: nodes of every kernel at the four half-lengths, after each level
+    has kept its largest classes and merged the others into them."""
+    rho = 1.1 * 2.0 ** (0.17 * torch.arange(32, dtype=torch.float64))
+    out = []
+    for level in range(4):
+        b = 0.5 * longest / 1.15**level * (rho - 1 / rho)
+        need = []
+        for theta in params.double():
+            be = (b / theta[0]) ** 2
+            log_m = 0.5 * be + torch.log1p(be)
+            if kt == "spectral":
+                log_m = log_m + 2 * torch.pi * theta[1].abs() * b
+            if kt == "locally_periodic":
+                log_m = log_m + (torch.cosh((2 * torch.pi * b / theta[2]).clamp(max=300)) - 1) / theta[1]
+            p = ((log_m + torch.log(4 / (rho - 1)) - torch.log(torch.tensor(eps))) / torch.log(rho)).min().item()
+            need.append(max(4, -(-int(-(-p // 1)) // unit) * unit))
+        kept = []
+        for p in sorted(set(need), reverse=True):
+            if len(kept) == classes or sum(kept) + p > cap:
+                break
+            kept.append(p)
+        out.append([min(q for q in kept if q >= p) for p in need])
+    return torch.tensor(out).T
+
+
+@pytest.mark.parametrize("kt,why", [("spectral", "more than eight classes"), ("locally_periodic", "more than eight classes"),
+                                    ("spectral", "more nodes than there is room for")])
+@pytest.mark.parametrize("shared", [True, False])
+@pytest.mark.parametrize("k", [5, 20])
+def test_levels_that_merge_different_classes(kt, why, shared, k):
+    """Kernels that have MORE nodes on shorter intervals, because their class was merged there and not on the
+    longest: what a warp stages of an operand is larger than the longest interval's nodes."""
+    from oracle import oracle as O
+
+    g = torch.Generator().manual_seed(3)
+    n = 1500
+    room = why == "more nodes than there is room for"
+    batch = 3 if room else 16
+    k = min(k, 16) if room and not shared else k
+    x = torch.sort(torch.rand(*(() if shared else (batch,)), n, generator=g) * (26 if room and kt == "spectral" else 11))[0]
+    halves = _half_lengths(x).reshape(-1, 12)
+    longest = halves.max().item()
+    levels = sum((halves <= longest / 1.15**i).long() for i in range(1, 4))
+    unit, cap = (4, 160) if shared else (2, 160)
+    for _ in range(4000):
+        u = torch.rand(batch, 4, generator=g)
+        if kt == "spectral":
+            params = torch.stack([0.7 + 0.8 * u[:, 0], 2.0 + 3.0 * u[:, 1] if room else 6.0 * u[:, 1], 0.8 + u[:, 3]], dim=-1)
+        else:
+            params = torch.stack([0.7 + 0.8 * u[:, 0], 0.3 + u[:, 1], 0.35 + 2.0 * u[:, 2], 0.8 + u[:, 3]], dim=-1)
+        nodes = _nodes_by_level(kt, params, longest, unit, cap)
+        if nodes.max() > (80 if k <= 16 else 64):
+            continue
+        at = [levels[0] if shared else levels[i] for i in range(batch)]
+        hit = [i for i in range(batch) if any(nodes[i, at[i][c]] > max(nodes[i, 0], nodes[i, at[i][r]]) for r in range(12)
+                                               for c in range(max(0, r - 1), min(12, r + 2)))]
+        if hit:
+            break
+    else:
+        raise AssertionError("no such parameters found")
+    xe = x.expand(batch, n)
+    start, end = O.make_ranges(1.2, x)
+    _both(kt, xe, xe, torch.randn(n, k).expand(batch, n, k) if shared else torch.randn(batch, n, k), torch.randn(batch, n, k), params,
+          start.expand(batch, -1), end.expand(batch, -1))
+
+
 @pytest.mark.parametrize("case", ["band not aligned", "nan point", "points in no order", "many periods", "empty bands", "equal points"])
 def test_steps_aside(case):
     """Inputs that interpolation must leave to the direct kernels, or take with an empty interval."""
