@@ -72,15 +72,18 @@ __host__ __device__ inline int64_t ceil_div(int64_t a, int64_t b) { return (a + 
 // their predecessor drains (launch_gated), and closed() is the first thing they ask: behind a closed gate
 // they are over by then but for the first CTA, which stays until the predecessor is complete, so that the
 // chain is complete when its last kernel is; behind an open one all of them wait for it.  The flag itself
-// has been final since before the chain's first kernel.  (8192 CTAs of a gated kernel that only return take
-// 36 us.)
+// has been final since before the chain's first kernel started, but it is read before any wait: by an acquire
+// load, as kernels before that one have read and changed it and left it in the SM's L1.  (8192 CTAs of a gated kernel
+// that only return take 36 us.)
 struct Gate {
     const int *flag = nullptr;
     int want = 0;
     __device__ __forceinline__ bool closed() const {
         if (flag == nullptr) return false;
         asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-        const bool run = *flag == want;
+        int now;
+        asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(now) : "l"(flag) : "memory");
+        const bool run = now == want;
         if (run || (blockIdx.x == 0 && blockIdx.y == 0)) asm volatile("griddepcontrol.wait;" ::: "memory");
         return !run;
     }
