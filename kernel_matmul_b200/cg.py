@@ -225,8 +225,10 @@ class ShardedOperator:
         more, where the points' blocks are short enough against what the kernel varies over (sorted points;
         bands aligned to blocks), is laid out as a matrix between the nodes of blockwise interpolation
         (``km_node_operator_build_f32``) once; a product of up to 16 columns then reads it instead of
-        evaluating kernels.  These are the sums whose products otherwise run on the tensor cores, with an error per
-        entry that is as large a part of the kernel's maximum.  Every other operator is evaluated: those
+        evaluating kernels.  These are the sums whose products otherwise run on the tensor cores.  Against 64 bits
+        (4 to 64 components, 1 to 16 columns) products of random vectors are off by 2.1e-7 - 2.6e-7 from the
+        node matrix and by 3.0e-7 - 7.9e-7 from the tensor cores, and entries, taken by one-hot columns, by
+        up to 5.8e-7 and 9.6e-7 of the kernel's maximum.  Every other operator is evaluated: those
         kernels hold each entry to about 1e-6 of itself, and tens of CG steps on a system of condition
         number 1000 turn a change of their last bits into 1e-4 of a gradient of the marginal likelihood.
 

@@ -148,7 +148,7 @@ Tensor matmul(int64_t kernel_type, const Tensor &x1, const Tensor &x2, const Ten
     const c10::cuda::CUDAGuard guard(x1.device());
     Tensor out = p.empty({p.m, k}, x1);
     const km_view vr = p.view(rhs, 2), vo = p.view(out, 2);
-    if (p.try_nodes(path)) {
+    if (p.try_nodes(path, k, TENSOR_CORE_MIN_K)) {
         const size_t bytes = km_matmul_nodes_workspace_bytes(&p.kb, p.m, p.n, k, &p.x1, &p.x2, &vr, p.one_range());
         const Tensor ws = bytes > 0 ? workspace_if_free(x1, bytes) : Tensor();
         if (ws.defined()) {
@@ -179,7 +179,7 @@ Tensor bilinear(int64_t kernel_type, const Tensor &x1, const Tensor &x2, const T
     const c10::cuda::CUDAGuard guard(x1.device());
     Tensor grad = p.empty({num_params(kernel_type)}, x1);
     const km_view vl = p.view(left, 2), vr = p.view(right, 2), vg = p.view(grad, 1);
-    if (p.try_nodes(path)) {
+    if (p.try_nodes(path, k, GRAD_TENSOR_CORE_MIN_K)) {
         const size_t bytes = km_grad_nodes_workspace_bytes(p.kid, &p.kb, p.m, p.n, k, &p.x1, &p.x2, &vl, &vr, p.one_range());
         const Tensor ws = bytes > 0 ? workspace_if_free(x1, bytes) : Tensor();
         if (ws.defined()) {

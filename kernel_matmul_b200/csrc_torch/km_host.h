@@ -42,8 +42,12 @@ enum Path : int64_t { PATH_AUTO = 0, PATH_FMA = 1, PATH_TC = 2, PATH_NODES = 3 }
 // kernels hardly depends on the width, and their pre-passes are two or three small launches.
 constexpr int64_t TENSOR_CORE_MIN_K = 9, GRAD_TENSOR_CORE_MIN_K = 8, TENSOR_CORE_MIN_ITEMS = 256;
 
-// (batch, row block) items from which the automatic path tries blockwise interpolation
-// (km_matmul_nodes_f32): its four small passes take about 10 us more than they save below.
+// The automatic path tries blockwise interpolation (km_matmul_nodes_f32) only where the tensor-core kernels
+// run otherwise, and from this many (batch, row block) items: its four small passes take about 10 us more
+// than they save below.  Against 64 bits products of random operands have relative errors (2-norm) of 2.1e-7 - 3.2e-7
+// by interpolation, 8.9e-7 - 1.4e-6 on the tensor cores and 2.4e-7 - 1.0e-6 on the FMA pipe, which holds small
+// entries to 1e-6 of themselves (one-hot columns, entries of 1e-4 - 1e-3 of the largest, worst relative error: RBF 3e-6,
+// 3e-4 and 1e-6, locally periodic with a lengthscale of 0.6 3e-5, 2e-4 and 2e-6): what ran on the FMA pipe stays there.
 constexpr int64_t NODES_MIN_ITEMS = 512;
 // With a band, both sides share an interval: where one has this many times the other's points, the blocks
 // of the sparser are too long for it (5003 test points against 50 021: 100 nodes and more) and the call would pay
@@ -81,9 +85,10 @@ struct Problem {
     // cutoff, which lays them out as the two halves of one storage, end first.  (A hint: the values are
     // looked at on the device.)
     bool one_range() const { return all_columns_; }
-    bool try_nodes(int64_t path) const {
+    // `k` columns, of an op that takes the tensor cores from `min_k` columns on
+    bool try_nodes(int64_t path, int64_t k, int64_t min_k) const {
         if (path == PATH_NODES) return true;
-        if (path != PATH_AUTO) return false;
+        if (path != PATH_AUTO || k < min_k || items() < TENSOR_CORE_MIN_ITEMS) return false;
         if (one_range()) return m * n * (items() / row_blocks) >= NODES_MIN_ENTRIES;
         return items() >= NODES_MIN_ITEMS && std::max(m, n) < NODES_MAX_RATIO * std::min(m, n);
     }

@@ -206,6 +206,31 @@ def test_steps_aside(case):
     _both(kt, x, x, torch.randn(n, k), torch.randn(n, k), params, start, end)
 
 
+@pytest.mark.parametrize("kt", KERNEL_TYPES)
+@pytest.mark.parametrize("form", ["band", "all columns"])
+def test_what_ran_on_the_fma_pipe_stays_there(kt, form):
+    """Up to 8 columns, gradients of up to 7, and fewer than 256 items without a cutoff: to the bit the FMA
+    kernels, which hold every entry to about 1e-6 of itself."""
+    from kernel_matmul_b200 import ops, ranges
+
+    def check(n, k, grad_k, batch):
+        x = torch.sort(torch.rand(n) * (n / 100))[0].cuda()
+        start, end = ranges.make_ranges(2.0 if form == "band" else None, x)
+        xs, params = x.expand(*batch, n), make_params(kt, batch).cuda()
+        args = (params, start.expand(*batch, -1), end.expand(*batch, -1))
+        rhs, left = torch.randn(n, max(k, grad_k), device="cuda"), torch.randn(n, max(k, grad_k), device="cuda")
+        auto, fma = (ops.matmul(kt, xs, xs, rhs[:, :k], *args, path=p) for p in ("auto", "fma"))
+        assert torch.equal(auto, fma)
+        auto, fma = (ops.bilinear_derivative(kt, xs, xs, left[:, :grad_k], rhs[:, :grad_k], *args, path=p) for p in ("auto", "fma"))
+        assert torch.equal(auto, fma)
+
+    if form == "band":
+        check(33000, 8, 7, (2,))  # 516 items
+    else:
+        check(11600, 16, 16, ())  # 91 items, 2^27 entries
+        check(33000, 8, 7, ())
+
+
 @pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan"), 3e38])
 @pytest.mark.parametrize("k", [3, 12])
 def test_operands_that_are_not_finite_or_near_overflow(value, k):
