@@ -25,6 +25,7 @@ from torch import Tensor
 
 from . import _C, ranges
 from ._lib import KERNEL_TYPES
+from .configurations import get_kernel_type_defines
 
 try:  # optional third-party base class
     from linear_operator import LinearOperator as _LinearOperator
@@ -89,9 +90,6 @@ class _OperatorCore:
             raise ValueError("x1 and x2 must have shapes (..., M, 1) and (..., N, 1), respectively")
         if symmetric is None:
             symmetric = x1.shape == x2.shape and torch.equal(x1, x2)
-        if kernel_type == "compact":
-            raise NotImplementedError("the 'compact' kernel is not part of this build")
-        self._kid = KERNEL_TYPES.get(kernel_type, -1)  # (-1: refused by the ops)
         self._x1, self._x2, self._params, self._start, self._end, self._x1v, self._x2v = _C.expand_operator(
             x1, x2, params, start, end)
         self._kernel_type = kernel_type
@@ -99,6 +97,14 @@ class _OperatorCore:
         self._symmetric = bool(symmetric)
 
     # -- helpers ---------------------------------------------------------------------------
+    @property
+    def _kid(self) -> int:
+        """Runtime kernel type of the ops.  An operator of another kernel can be made and asked for its shape;
+        its products are refused, by name."""
+        if self._kernel_type not in KERNEL_TYPES:
+            get_kernel_type_defines(self._kernel_type)  # raises
+        return KERNEL_TYPES[self._kernel_type]
+
     def _core_size(self) -> torch.Size:
         return torch.Size((*self._batch_shape, self._x1.size(-2), self._x2.size(-2)))
 

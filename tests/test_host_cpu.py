@@ -140,3 +140,19 @@ def test_torch_extension_exports_the_ten_reference_functions():
         _C.matmul(0, x, x, torch.rand(10, 1), torch.ones(2), s, s)
     with pytest.raises(RuntimeError, match="x must be a CUDA tensor"):
         _C.make_ranges_symmetric(x[None], 1.0, 128)
+
+
+@pytest.mark.parametrize("kernel_type,error", [("compact", NotImplementedError), ("no such kernel", KeyError)])
+def test_operators_of_kernels_that_are_not_there_are_refused_by_name(kernel_type, error):
+    """At the product, as before it is launched; the operator itself can be made."""
+    from kernel_matmul_b200.linear_operator import KernelMatmulOperator
+
+    x = torch.arange(5.0).unsqueeze(-1)
+    start, end = torch.zeros(1, dtype=torch.int32), torch.full((1,), 5, dtype=torch.int32)
+    op = KernelMatmulOperator(x, x, torch.ones(2), start, end, kernel_type=kernel_type, symmetric=True)
+    assert op.shape == (5, 5)
+    index = torch.zeros(1, dtype=torch.int32)
+    for call in (lambda: op.matmul(torch.ones(5, 1)), op.to_dense, lambda: op.bilinear_derivative(torch.ones(5, 1), torch.ones(5, 1)),
+                 lambda: op.get_indices(index, index)):
+        with pytest.raises(error, match=kernel_type):
+            call()
