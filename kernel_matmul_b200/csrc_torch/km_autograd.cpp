@@ -75,14 +75,15 @@ struct IndexFunction : torch::autograd::Function<IndexFunction> {
 struct PositiveParams : torch::autograd::Function<PositiveParams> {
     static variable_list forward(AutogradContext *ctx, at::TensorList raw_in, double lower_bound, int64_t lengthscales,
                                  std::optional<double> cutoff_factor) {
-        std::vector<Tensor> raw;
+        std::vector<Tensor> raw, dense;
         const float *ptr[KM_MAX_PARAMS];
         TORCH_CHECK(raw_in.size() >= 1 && raw_in.size() <= KM_MAX_PARAMS, "1 to ", KM_MAX_PARAMS, " raw parameters");
         for (const Tensor &t : raw_in) {
             check_f32(t);
             TORCH_CHECK(t.sizes() == raw_in[0].sizes() && t.device() == raw_in[0].device(), "raw parameters must share shape and device");
-            raw.push_back(t.contiguous());
-            ptr[raw.size() - 1] = raw.back().const_data_ptr<float>();
+            raw.push_back(t);  // (saved as given: the gradient's own derivative goes through it)
+            dense.push_back(t.contiguous());
+            ptr[raw.size() - 1] = dense.back().const_data_ptr<float>();
         }
         const c10::cuda::CUDAGuard guard(raw[0].device());
         Shape shape(raw[0].sizes().begin(), raw[0].sizes().end());
@@ -109,9 +110,11 @@ struct PositiveParams : torch::autograd::Function<PositiveParams> {
         }
         const float *ptr[KM_MAX_PARAMS];
         float *to[KM_MAX_PARAMS];
+        std::vector<Tensor> dense;
         Tensor flat = g.reshape({-1, (int64_t)raw.size()});
         for (size_t q = 0; q < raw.size(); q++) {
-            ptr[q] = raw[q].const_data_ptr<float>();
+            dense.push_back(raw[q].contiguous());
+            ptr[q] = dense.back().const_data_ptr<float>();
             out[q] = at::empty(raw[q].sizes(), raw[q].options().requires_grad(false));
             to[q] = out[q].data_ptr<float>();
         }

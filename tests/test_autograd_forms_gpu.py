@@ -45,6 +45,23 @@ def test_parameters_have_second_derivatives():
         torch.testing.assert_close(a, b, rtol=1e-6, atol=1e-6)
 
 
+def test_second_derivatives_of_parameters_that_are_not_contiguous():
+    from kernel_matmul_b200 import kernels
+
+    m = kernels.SpectralKernelMatmulModule(cutoff=1.0, batch_shape=torch.Size((2, 3))).cuda()
+    for name, raw in list(m.named_parameters()):
+        setattr(m, name, torch.nn.Parameter(torch.randn(3, 2, device="cuda").t()))
+    leaves = list(m.parameters())
+    assert not any(p.is_contiguous() for p in leaves)
+    grads = {}
+    for name, params in (("kernel", m.params()), ("expressions", _expressions(m))):
+        first = torch.autograd.grad((params**3).sum(), leaves, create_graph=True)
+        second = torch.autograd.grad(sum((g**2).sum() for g in first), leaves)
+        grads[name] = [*first, *second]
+    for a, b in zip(grads["kernel"], grads["expressions"]):
+        torch.testing.assert_close(a, b, rtol=1e-6, atol=1e-6)
+
+
 def test_parameters_under_forward_mode_vmap_and_tracing():
     import torch.autograd.forward_ad as fwAD
 
