@@ -309,7 +309,12 @@ Tensor index(int64_t kernel_type, const Tensor &x1, const Tensor &x2, const Tens
     const c10::cuda::CUDAGuard guard(x1.device());
     Tensor out = at::empty(l.shape, x1.options().requires_grad(false));
     if (distances != nullptr) {
-        *distances = at::empty(l.shape, x1.options().requires_grad(false));
+        try {
+            *distances = at::empty(l.shape, x1.options().requires_grad(false));
+        } catch (const c10::OutOfMemoryError &) {  // the gradient goes back to the points
+        }
+    }
+    if (distances != nullptr && distances->defined()) {
         raise_on(km_index_distances_f32(p.kid, &p.kb, p.m, p.n, l.count, &p.x1, &p.x2, &p.params, &p.start, &p.end, l.batch, l.row, l.col,
                                         out.data_ptr<float>(), distances->data_ptr<float>(), p.stream()));
     } else {

@@ -109,7 +109,8 @@ Tensor bilinear(int64_t kernel_type, const Tensor &x1, const Tensor &x2, const T
 Tensor dense(int64_t kernel_type, const Tensor &x1, const Tensor &x2, const Tensor &params, const Tensor &start, const Tensor &end);
 Tensor dense_bwd(int64_t kernel_type, const Tensor &x1, const Tensor &x2, const Tensor &params, const Tensor &start,
                  const Tensor &end, const Tensor &out_grad);
-// `distances`: where to put the distances of the lookups, from which their gradient needs no points
+// `distances`: where to put the distances of the lookups, from which their gradient needs no points (left
+// undefined where the device has no memory for them)
 Tensor index(int64_t kernel_type, const Tensor &x1, const Tensor &x2, const Tensor &params, const Tensor &start, const Tensor &end,
              const std::vector<Tensor> &batch_indices, const Tensor &row, const Tensor &col, Tensor *distances = nullptr);
 Tensor index_bwd(int64_t kernel_type, const Tensor &x1, const Tensor &x2, const Tensor &params, const Tensor &start,

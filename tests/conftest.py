@@ -5,6 +5,7 @@
 """
 from __future__ import annotations
 
+import contextlib
 import os
 import random
 import sys
@@ -42,6 +43,19 @@ def seed(request) -> int:
     random.seed(s)
     torch.manual_seed(s)
     return s
+
+
+@contextlib.contextmanager
+def memory_left(nbytes: int):
+    """At most ``nbytes`` more than now for PyTorch's allocator, which refuses the rest as out of memory."""
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(0).total_memory
+    torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + nbytes) / total)
+    try:
+        yield
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
 
 
 KERNEL_TYPES = ["rbf", "spectral", "locally_periodic"]

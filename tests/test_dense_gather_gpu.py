@@ -3,7 +3,7 @@ against the fp64 oracle; tolerances as in ``test_ops_gpu.py``."""
 import pytest
 import torch
 
-from conftest import KERNEL_TYPES, assert_grad_close, make_params, rel_err
+from conftest import KERNEL_TYPES, assert_grad_close, make_params, memory_left, rel_err
 
 pytestmark = pytest.mark.gpu
 
@@ -82,3 +82,30 @@ def test_gather_of_points_that_are_not_finite():
     out = op.get_indices(row, torch.zeros_like(row))
     assert out.isnan().tolist() == [False, True, False, False, False]
     assert torch.autograd.grad(out.sum(), p)[0].isnan().all()
+
+
+def test_gather_without_memory_for_the_distances():
+    """The values fit, the distances beside them do not: the gradient goes back to the points."""
+    from kernel_matmul_b200 import ranges
+    from kernel_matmul_b200.linear_operator import KernelMatmulOperator
+
+    n, count = 3000, 1 << 24  # 64 MB of values
+    x = torch.sort(torch.rand(n, device="cuda") * 30)[0]
+    start, end = ranges.make_ranges(4.0, x)
+    row = torch.randint(0, n, (count,), dtype=torch.int32, device="cuda")
+    col = (row + torch.randint(-200, 200, (count,), dtype=torch.int32, device="cuda")).clamp_(0, n - 1)
+    w = torch.randn(count, device="cuda")
+    p = torch.tensor([1.0, 1.2], device="cuda", requires_grad=True)
+    op = KernelMatmulOperator(x[:, None], x[:, None], p, start, end, kernel_type="rbf", symmetric=True)
+    out = op.get_indices(row, col)
+    want = torch.autograd.grad(out, p, w)[0]
+    expected = out.detach().cpu()
+    del out
+    with memory_left((64 + 24) << 20):
+        out = op.get_indices(row, col)
+        with pytest.raises(torch.OutOfMemoryError):
+            torch.empty(count, device="cuda")
+        got = torch.autograd.grad(out, p, w)[0]
+    assert torch.equal(out.detach().cpu(), expected)
+    # (sums of 2^24 terms of either sign: fp32 within a thread's share, fp64 beyond)
+    assert_grad_close(got, want, torch.full_like(want, float(w.abs().sum()) * 0.1))
