@@ -529,6 +529,10 @@ KM_API int km_cg_log_forms_f32(int64_t iterations, int64_t k, const float *alpha
  *    first three are found out.
  *  - build, with these as `nodes` and `max_blocks`: lambda (row blocks x nodes x 128 floats) and
  *    matrix (row blocks of the window x max_blocks x nodes x nodes floats).
+ *    All that is laid out follows from the values points, parameters and band have then: hand the kernels copies of
+ *    them that nothing writes to (a band that has become wider would read past the matrix).
+ *  - changed: *changed = whether points, parameters (batch.., 3) or band (views with one stride) differ in any bit
+ *    from such copies (contiguous).
  *  - compress: nodes (row blocks x nodes x ceil4(k)) = lambda^T v for blocks [block_begin, block_end).
  *  - update_p: the same behind p = r + beta p on these blocks (arguments as km_cg_update_p_f32).
  *  - product: the window's rows of K v from its nodes; with p not null of K v + sigma2 p, and the
@@ -544,6 +548,9 @@ KM_API int km_node_operator_build_f32(const km_batch *batch, int64_t n, const fl
                                       const km_view *params, const int32_t *start, const int32_t *end, int64_t row_block_begin,
                                       int64_t row_block_count, const float *centre, const void *plan, int64_t nodes,
                                       int64_t max_blocks, float *lambda, float *matrix, void *stream);
+KM_API int km_node_operator_changed(const km_batch *batch, int64_t n, const float *x, int64_t x_stride, const km_view *params,
+                                    const km_view *start, const km_view *end, const float *own_x, const float *own_params,
+                                    const int32_t *own_start, const int32_t *own_end, int32_t *changed, void *stream);
 KM_API int km_node_compress_f32(int64_t k, int64_t n, int64_t nodes_per_block, const float *lambda, const float *v, float *nodes,
                                 int64_t block_begin, int64_t block_end, void *stream);
 KM_API int km_node_update_p_f32(int64_t k, int64_t n, int64_t nodes_per_block, const float *lambda, float *p, const float *r,

@@ -145,6 +145,8 @@ def _load() -> ctypes.CDLL:
     lib.km_node_operator_plan_f32.argtypes = [bp, i64, vp, i64, wp, ip, ip, i64, i64, vp, vp, vp]
     lib.km_node_operator_build_f32.restype = ctypes.c_int
     lib.km_node_operator_build_f32.argtypes = [bp, i64, vp, i64, wp, ip, ip, i64, i64, vp, vp, i64, i64, vp, vp, vp]
+    lib.km_node_operator_changed.restype = ctypes.c_int
+    lib.km_node_operator_changed.argtypes = [bp, i64, vp, i64, wp, wp, wp, vp, vp, vp, vp, vp, vp]
     lib.km_node_compress_f32.restype = ctypes.c_int
     lib.km_node_compress_f32.argtypes = [i64, i64, i64, vp, vp, vp, i64, i64, vp]
     lib.km_node_update_p_f32.restype = ctypes.c_int
@@ -170,7 +172,7 @@ EXPORTED = [
     "km_make_ranges_symmetric_f32", "km_make_ranges_symmetric_cutoffs_f32", "km_transpose_ranges_i32", "km_count_entries",
     "km_probe_fp32_peak", "km_probe_sfu_peak", "km_selftest_bounded_wait", "km_selftest_set_wait_polls",
     "km_cg_block_dots_f32", "km_cg_q_dots_f32", "km_cg_segment_sums_f32", "km_cg_init_scalars_f32", "km_cg_update_xr_f32",
-    "km_cg_update_p_f32", "km_cg_log_forms_f32", "km_node_operator_plan_f32", "km_node_operator_build_f32", "km_node_compress_f32", "km_node_update_p_f32",
+    "km_cg_update_p_f32", "km_cg_log_forms_f32", "km_node_operator_plan_f32", "km_node_operator_build_f32", "km_node_operator_changed", "km_node_compress_f32", "km_node_update_p_f32",
     "km_node_product_f32", "km_sum_phases_workspace_bytes", "km_sum_phases_prepare_f32", "km_matmul_rows_phases_f32",
 ]
 

@@ -156,6 +156,8 @@ class ShardedOperator:
         if mode not in ("auto", "halo", "allgather"):
             raise ValueError(f"unknown mode {mode!r}")
         self.n = n
+        #: the laid-out operator for products of ``k`` columns, or ``None`` (operators of ``from_kernel``)
+        self.current_nodes: Callable | None = None
         self.sigma2 = float(sigma2)
         self.matvec_rows = matvec_rows
         self.group = group
@@ -274,7 +276,7 @@ class ShardedOperator:
 
         def matvec_rows(v: Tensor, rb_begin: int, rb_count: int, out: Tensor) -> None:
             whole = (rb_begin, rb_count) == (begin, count) and v.is_contiguous() and out.is_contiguous()
-            by_nodes = current_nodes(v.shape[-1]) if whole else None
+            by_nodes = current_nodes(v.shape[-1], look=False) if whole else None
             if by_nodes is not None:
                 by_nodes.matvec(v, out)
             else:
@@ -294,7 +296,8 @@ class ShardedOperator:
         # set-up only)
         def plan_nodes():
             looked_at = (x, params) if may_lay_out else (None, None)
-            plan = _C.NodeOperator(n, *looked_at, start.reshape(-1)[:R], end.reshape(-1)[:R], begin, count)
+            band = (t[(0,) * (t.dim() - 1)][:R] for t in (start, end))
+            plan = _C.NodeOperator(n, *looked_at, *band, begin, count)
             return (plan, *(int(v) for v in plan.plan().tolist()))
 
         def versions():
@@ -312,18 +315,27 @@ class ShardedOperator:
             phase_ws = ops.prepare_sum_phases(kernel_type, x, x, params, rows=(begin * BLOCK_SIZE, min(n, (begin + count) * BLOCK_SIZE)),
                                               cols=(max(0, min(lo, n)), max(0, min(hi, n))))
 
-        def current_nodes(k: int = 1):
+        def current_nodes(k: int = 1, look: bool = True):
             """The node operator for products of ``k`` columns, laid out again if points, parameters or band
-            were written to since; ``None``: the products evaluate the kernels."""
+            have other values by now; ``None``: the products evaluate the kernels.  PyTorch's version counters
+            tell of most writes.  With ``look``, and for inference tensors, which have no counter, the
+            values themselves are compared (one host synchronisation), so that writes through ``.data`` or by
+            other libraries are followed too.  Under stream capture there is nothing but the counters, and a
+            product after a write evaluates the kernels."""
             nonlocal nodes, laid_out
-            if k > _C.NODE_MAX_COLUMNS:
+            if nodes is None or k > _C.NODE_MAX_COLUMNS:
                 return None
-            if nodes is not None and versions() != laid_out:
-                laid_out = versions()
+            now = versions()
+            if now == laid_out and not look and None not in now:
+                return nodes
+            if torch.cuda.is_current_stream_capturing():
+                return nodes if now == laid_out else None
+            if nodes.changed():
                 again, now_lo, now_hi, _, node_count, widest = plan_nodes()
                 if usable(node_count, widest):
                     again.build(now_lo, now_hi, node_count, widest)
                 nodes = again if usable(node_count, widest) else None
+            laid_out = now
             return nodes
 
         op = cls(n, sigma2, matvec_rows, group=group, device=x.device, col_range=(lo, hi) if count > 0 else (0, 0),
@@ -332,6 +344,13 @@ class ShardedOperator:
         op.current_nodes = current_nodes
         op.rows_product = rows_product
         return op
+
+    def look(self, k: int) -> None:
+        """Lay the operator out again if what it was laid out from has other values by now, however that
+        came about.  ``apply``, ``apply_rows`` and, at its start, a solve do this; ``matvec_rows`` by itself
+        follows the writes that PyTorch's version counters tell of."""
+        if self.current_nodes is not None:
+            self.current_nodes(k)
 
     # ---- the operator applied to a full vector (tests, diagnostics)
 
@@ -343,6 +362,7 @@ class ShardedOperator:
         """This rank's rows of ``(K + sigma^2 I) v`` for a full ``v`` -> ``(rows, k)``."""
         out = torch.empty(self.rows, v.shape[-1], device=v.device, dtype=v.dtype)
         if self.rows > 0:
+            self.look(v.shape[-1])
             self.matvec_rows(v, self.begin, self.count, out)
             out.add_(self.local(v), alpha=self.sigma2)
         return out
@@ -407,6 +427,7 @@ class CGSolver:
         self.alphas = torch.zeros(max_iterations, k, device=dev, dtype=dt)
         self.betas = torch.zeros(max_iterations, k, device=dev, dtype=dt)
         self.it = 0
+        self._looked = False  # whether this solve has looked at what its operator was laid out from (``look``)
         #: set to a callable ``mark(name)`` to be told where the phases of ``step()`` begin
         #: (bench.py records CUDA events there for its per-phase breakdown)
         self.mark = None
@@ -473,6 +494,9 @@ class CGSolver:
         mark = self.mark or (lambda name: None)
         mark("product")
         if op.rows > 0:
+            if not self._looked:
+                op.look(k)
+                self._looked = True
             op.matvec_rows(self.p[: op.n], op.begin, op.count, self.kp[op.row0: op.row1])
         mark("q_dots")
         V.q_dots(self.kp, self.p, op.sigma2, op.row0, op.row1, self.bp, self.send1, self.top_off, self.top_rows,

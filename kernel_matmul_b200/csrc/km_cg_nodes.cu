@@ -140,6 +140,32 @@ struct NodeOpArgs {
     int P, max_blocks;
 };
 
+// Whether points, parameters or band differ in any bit from the copies an operator was laid out from.  (4 million
+// points and 64 components: 5 us.)
+struct NodeChangedArgs {
+    Batch batch;
+    int64_t n, R;
+    const float *x;
+    int64_t xs;
+    View<const float> params;
+    const int *start, *end;
+    int64_t ss, es;
+    const float *own_x, *own_params;
+    const int *own_start, *own_end;
+    int *changed;
+};
+__global__ void __launch_bounds__(256) node_changed_kernel(const NodeChangedArgs a) {
+    const int64_t first = blockIdx.x * 256LL + threadIdx.x, step = gridDim.x * 256LL;
+    const auto bits = [](float v) { return __float_as_uint(v); };
+    bool differs = false;
+    for (int64_t i = first; i < a.n; i += step) differs |= bits(a.x[i * a.xs]) != bits(a.own_x[i]);
+    for (int64_t r = first; r < a.R; r += step) differs |= a.start[r * a.ss] != a.own_start[r] || a.end[r * a.es] != a.own_end[r];
+    constexpr int P = 3;  // parameters of a spectral component
+    for (int64_t i = first; i < a.batch.count * P; i += step)
+        differs |= bits(batch_ptr(a.params, decompose(a.batch, i / P))[(i % P) * a.params.s0]) != bits(a.own_params[i]);
+    if (differs) *a.changed = 1;
+}
+
 // Lagrange matrix of every block: thread = row.
 __global__ void __launch_bounds__(128) node_lambda_kernel(const NodeOpArgs a) {
     __shared__ float delta[NODE_OP_MAX], weight[NODE_OP_MAX];
@@ -423,7 +449,7 @@ __global__ void __launch_bounds__(128) node_product_kernel(const NodeProductArgs
     float *qs = gs + max(g.chunk * P, 4 * P * KC4);  // [chunk][KC4]
     const int s = g.start[r], e = g.end[r];
     const int64_t c_lo = s < e ? s / KM_BLOCK_SIZE : 0;
-    const int count = s < e ? (int)((min((int64_t)e, g.n) + KM_BLOCK_SIZE - 1) / KM_BLOCK_SIZE - c_lo) * P : 0;
+    const int count = s < e ? max(0, (int)((min((int64_t)e, g.n) + KM_BLOCK_SIZE - 1) / KM_BLOCK_SIZE - c_lo)) * P : 0;
     const float *G = g.G + (int64_t)blockIdx.x * g.max_blocks * P * P;
     const float *lambda = g.lambda + r * P * KM_BLOCK_SIZE;
     for (int i = t; i < P * (KM_BLOCK_SIZE / 4); i += 128) cp_async16(ls + i * 4, lambda + i * 4);
@@ -632,6 +658,29 @@ extern "C" int km_node_operator_build_f32(const km_batch *batch, int64_t n, cons
     KM_REQUIRE(items <= 0x7fffffffLL, KM_ERR_UNSUPPORTED, "km_node_operator_build_f32: too many blocks");
     node_matrix_kernel<<<(unsigned)ceil_div(items, 4), 128, 0, s>>>(a);
     KM_CHECK_LAUNCH("km_node_operator_build_f32 launch");
+    return KM_OK;
+}
+
+extern "C" int km_node_operator_changed(const km_batch *batch, int64_t n, const float *x, int64_t x_stride, const km_view *params,
+                                        const km_view *start, const km_view *end, const float *own_x, const float *own_params,
+                                        const int32_t *own_start, const int32_t *own_end, int32_t *changed, void *stream) {
+    using namespace km;
+    KM_REQUIRE(batch && params && start && end, KM_ERR_INVALID_ARGUMENT, "km_node_operator_changed: bad arguments");
+    NodeChangedArgs a = {};
+    const int rc = make_batch(batch, &a.batch);
+    if (rc != KM_OK) return rc;
+    KM_REQUIRE(n >= 1 && n <= 0x7fffffffLL - 256 && x && params->data && start->data && end->data && own_x && own_params && own_start &&
+                   own_end && changed,
+               KM_ERR_INVALID_ARGUMENT, "km_node_operator_changed: bad arguments");
+    a.n = n, a.R = ceil_div(n, KM_BLOCK_SIZE), a.x = x, a.xs = x_stride, a.params = make_view<const float>(params, a.batch);
+    a.start = static_cast<const int *>(start->data), a.ss = start->stride[0];
+    a.end = static_cast<const int *>(end->data), a.es = end->stride[0];
+    a.own_x = own_x, a.own_params = own_params, a.own_start = own_start, a.own_end = own_end, a.changed = changed;
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    const cudaError_t err = cudaMemsetAsync(changed, 0, sizeof(int32_t), s);
+    if (err != cudaSuccess) return cuda_fail(err, "km_node_operator_changed");
+    node_changed_kernel<<<(unsigned)std::min<int64_t>(ceil_div(n, 256), 148 * 8), 256, 0, s>>>(a);
+    KM_CHECK_LAUNCH("km_node_operator_changed launch");
     return KM_OK;
 }
 

@@ -11,39 +11,68 @@ NodeOperator::NodeOperator(int64_t n, const std::optional<Tensor> &x, const std:
     check_i32(start), check_i32(end);
     R_ = (n_ + KM_BLOCK_SIZE - 1) / KM_BLOCK_SIZE;
     TORCH_CHECK(start.numel() >= R_ && end.numel() >= R_, "start / end must have ", R_, " entries");
-    start_ = start.reshape({-1}).contiguous(), end_ = end.reshape({-1}).contiguous();
+    TORCH_CHECK(start.dim() == 1 && end.dim() == 1, "start and end must have one dimension");
+    start_ = start, end_ = end;
     const c10::cuda::CUDAGuard guard(start_.device());
     const auto opt = start_.options().requires_grad(false);
     plan_ = at::empty({KM_NODE_PLAN_BYTES / 8}, opt.dtype(at::kLong));
+    km_view params_now{};
     if (x.has_value()) {
         check_f32(*x), check_f32(*params);
         x_ = *x, params_ = *params;
-        TORCH_CHECK(x_.dim() == 1 && x_.size(0) == n_ && params_.dim() >= 1 && params_.size(-1) == num_params(KM_KERNEL_SPECTRAL),
+        TORCH_CHECK(x_.dim() == 1 && x_.size(0) == n_ && params_.dim() >= 1 && params_.size(-1) == num_params(KM_KERNEL_SPECTRAL) &&
+                        params_.dim() - 1 <= KM_MAX_BATCH_DIMS,
                     "x must be (n,) and params (.., 3)");
-        if (params_.dim() - 1 > KM_MAX_BATCH_DIMS) params_ = params_.reshape({-1, params_.size(-1)});
-        const int nb = (int)params_.dim() - 1;
-        kb_.ndim = nb;
-        for (int d = 0; d < nb; d++) kb_.size[d] = params_.size(d), vparams_.batch_stride[d] = params_.stride(d);
-        vparams_.data = params_.data_ptr();
-        vparams_.stride[0] = params_.stride(nb);
+        kb_.ndim = (int)params_.dim() - 1;
+        for (int d = 0; d < kb_.ndim; d++) kb_.size[d] = params_.size(d);
+        params_now = params_view(params_);
         centre_ = at::empty({std::max<int64_t>(R_, 1)}, opt.dtype(at::kFloat));
     }
-    raise_on(km_node_operator_plan_f32(&kb_, n_, x ? x_.const_data_ptr<float>() : nullptr, x ? x_.stride(0) : 0, x ? &vparams_ : nullptr,
-                                       start_.const_data_ptr<int32_t>(), end_.const_data_ptr<int32_t>(), begin_, count_,
+    const Tensor s = start_.contiguous(), e = end_.contiguous();
+    raise_on(km_node_operator_plan_f32(&kb_, n_, x ? x_.const_data_ptr<float>() : nullptr, x ? x_.stride(0) : 0, x ? &params_now : nullptr,
+                                       s.const_data_ptr<int32_t>(), e.const_data_ptr<int32_t>(), begin_, count_,
                                        x ? centre_.data_ptr<float>() : nullptr, plan_.data_ptr(), stream()));
+}
+
+km_view NodeOperator::params_view(const Tensor &params) const {
+    km_view v{};
+    v.data = params.data_ptr();
+    for (int d = 0; d < kb_.ndim; d++) v.batch_stride[d] = params.stride(d);
+    v.stride[0] = params.stride(kb_.ndim);
+    return v;
 }
 
 void NodeOperator::build(int64_t lo, int64_t hi, int64_t nodes, int64_t max_blocks) {
     const c10::cuda::CUDAGuard guard(x_.device());
     const auto opt = x_.options().requires_grad(false);
+    const auto copy = [](const Tensor &t) { return t.detach().clone(at::MemoryFormat::Contiguous); };
     P_ = nodes, max_blocks_ = max_blocks;
     blk0_ = std::max<int64_t>(0, lo) / KM_BLOCK_SIZE, blk1_ = (std::min(hi, n_) + KM_BLOCK_SIZE - 1) / KM_BLOCK_SIZE;
     blk0_ = std::min(blk0_, blk1_);
+    own_x_ = copy(x_), own_params_ = copy(params_), own_start_ = copy(start_), own_end_ = copy(end_);
     lambda_ = at::empty({R_ * P_ * KM_BLOCK_SIZE}, opt);
     matrix_ = at::empty({std::max<int64_t>(1, count_ * max_blocks * P_ * P_)}, opt);
-    raise_on(km_node_operator_build_f32(&kb_, n_, x_.const_data_ptr<float>(), x_.stride(0), &vparams_, start_.const_data_ptr<int32_t>(),
-                                        end_.const_data_ptr<int32_t>(), begin_, count_, centre_.const_data_ptr<float>(), plan_.data_ptr(),
-                                        P_, max_blocks_, lambda_.data_ptr<float>(), matrix_.data_ptr<float>(), stream()));
+    const km_view own_params = params_view(own_params_);
+    raise_on(km_node_operator_build_f32(&kb_, n_, own_x_.const_data_ptr<float>(), 1, &own_params, own_start_.const_data_ptr<int32_t>(),
+                                        own_end_.const_data_ptr<int32_t>(), begin_, count_, centre_.const_data_ptr<float>(),
+                                        plan_.data_ptr(), P_, max_blocks_, lambda_.data_ptr<float>(), matrix_.data_ptr<float>(), stream()));
+}
+
+bool NodeOperator::changed() const {
+    // (a tensor may have been given other memory)
+    if (x_.sizes() != own_x_.sizes() || params_.sizes() != own_params_.sizes() || start_.sizes() != own_start_.sizes() ||
+        end_.sizes() != own_end_.sizes())
+        return true;
+    const c10::cuda::CUDAGuard guard(own_x_.device());
+    const Tensor flag = at::empty({1}, own_start_.options());
+    const km_view params_now = params_view(params_);
+    km_view s{}, e{};
+    s.data = start_.data_ptr(), s.stride[0] = start_.stride(0), e.data = end_.data_ptr(), e.stride[0] = end_.stride(0);
+    raise_on(km_node_operator_changed(&kb_, n_, x_.const_data_ptr<float>(), x_.stride(0), &params_now, &s, &e,
+                                      own_x_.const_data_ptr<float>(), own_params_.const_data_ptr<float>(),
+                                      own_start_.const_data_ptr<int32_t>(), own_end_.const_data_ptr<int32_t>(), flag.data_ptr<int32_t>(),
+                                      stream()));
+    return flag.item<int32_t>() != 0;
 }
 
 // Scratch of a product: one per call or run, on its stream, so that an operator may be applied on several
@@ -64,7 +93,7 @@ void NodeOperator::update_p(const CgState &s, int64_t it, float *nodes) const {
 }
 
 void NodeOperator::product(int64_t k, const float *nodes, float *out, const float *p, double sigma2, float *block_partials) const {
-    raise_on(km_node_product_f32(k, n_, P_, max_blocks_, start_.const_data_ptr<int32_t>(), end_.const_data_ptr<int32_t>(),
+    raise_on(km_node_product_f32(k, n_, P_, max_blocks_, own_start_.const_data_ptr<int32_t>(), own_end_.const_data_ptr<int32_t>(),
                                  lambda_.const_data_ptr<float>(), matrix_.const_data_ptr<float>(), nodes, begin_, count_, out, p, (float)sigma2,
                                  block_partials, stream()));
 }

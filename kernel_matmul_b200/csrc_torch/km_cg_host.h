@@ -21,7 +21,11 @@ class NodeOperator {
                  int64_t row_block_begin, int64_t row_block_count);
     // int64 on the device: lo, hi, checksum, nodes per block (0: not this way), widest band in blocks
     Tensor plan() const { return plan_.slice(0, 0, 5); }
+    // Copies points, parameters and band and lays the operator out from the copies, which is what all products use.
     void build(int64_t lo, int64_t hi, int64_t nodes, int64_t max_blocks);
+    // Whether any of them has another value than its copy by now, however it was written to (waits for the
+    // device; not under stream capture).
+    bool changed() const;
     // out = the window's rows of K v
     void matvec(const Tensor &v, const Tensor &out) const;
 
@@ -33,9 +37,11 @@ class NodeOperator {
   private:
     void *stream() const { return c10::cuda::getCurrentCUDAStream(start_.device().index()).stream(); }
     int64_t n_, R_, begin_, count_, P_ = 0, max_blocks_ = 0, blk0_ = 0, blk1_ = 0;
-    Tensor x_, params_, start_, end_, centre_, plan_, lambda_, matrix_;
+    km_view params_view(const Tensor &params) const;
+    Tensor x_, params_, start_, end_;                      // the caller's
+    Tensor own_x_, own_params_, own_start_, own_end_;      // contiguous copies
+    Tensor centre_, plan_, lambda_, matrix_;
     km_batch kb_{};
-    km_view vparams_{};
 };
 
 void cg_run(const CgState &s, const NodeOperator *nodes, RowsProduct *rows, int64_t first, int64_t count);

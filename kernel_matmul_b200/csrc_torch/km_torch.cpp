@@ -228,6 +228,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
                       int64_t>())
         .def("plan", &kmh::NodeOperator::plan)
         .def("build", &kmh::NodeOperator::build, nogil())
+        .def("changed", &kmh::NodeOperator::changed, nogil())
         .def("matvec", &kmh::NodeOperator::matvec, nogil());
     py::class_<kmh::CgState>(m, "CgState")
         .def(py::init([](const Tensor &x, const Tensor &r, const Tensor &p, const Tensor &kp, const Tensor &bp, const Tensor &rs,

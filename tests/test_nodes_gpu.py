@@ -346,6 +346,78 @@ def test_cg_operator_follows_its_parameters():
         assert all(torch.equal(g, r) for g, r in zip(got, ref))
 
 
+@pytest.mark.parametrize("write", ["data", "inference tensors"])
+@pytest.mark.parametrize("what", ["lengthscale", "scale", "points", "wider band", "narrower band"])
+@pytest.mark.parametrize("use", ["apply", "steps", "run"])
+def test_cg_operator_follows_writes_that_are_not_counted(write, what, use):
+    """Version counters do not tell of writes through ``.data`` nor of any to inference tensors."""
+    from kernel_matmul_b200 import ranges
+    from kernel_matmul_b200.cg import CGSolver, ShardedOperator
+
+    n, k = 4500, 3
+
+    def inputs():
+        x = (torch.sort(torch.rand(n, generator=torch.Generator().manual_seed(1)))[0] * 45).cuda()
+        return [x, torch.tensor([[0.6, 0.0, 1.2], [0.6, 0.4, 0.7]], device="cuda"), *ranges.make_ranges(2.4, x)]
+
+    def change(t):
+        x, params, start, end = (a.data for a in t)
+        if what == "lengthscale":
+            params[:, 0] = 0.5
+        elif what == "scale":
+            params[1, 2] = 0.9
+        elif what == "points":
+            x.mul_(1.01)
+        else:
+            s, e = ranges.make_ranges(4.0 if what == "wider band" else 1.9, x)
+            start.copy_(s), end.copy_(e)
+
+    def result(op):
+        y = torch.randn(n, k, generator=torch.Generator().manual_seed(2)).cuda()
+        if use == "apply":
+            return op.apply(y)
+        solver = CGSolver(op, y, 8)
+        if use == "run":
+            solver.run(8)
+        else:
+            for _ in range(8):
+                solver.step()
+        return solver.solution()
+
+    with torch.inference_mode(write == "inference tensors"):
+        t = inputs()
+        op = ShardedOperator.from_kernel("spectral", *t, 0.2)
+        assert op.current_nodes() is not None
+        before = result(op)
+        change(t)
+        after = result(op)
+        fresh = ShardedOperator.from_kernel("spectral", *(a.clone() for a in t), 0.2)
+        assert fresh.current_nodes() is not None
+        assert torch.equal(after, result(fresh)) and not torch.equal(after, before)
+
+
+def test_band_that_becomes_wider_during_a_solve_is_not_read():
+    """Products read the band that the matrix was laid out for, not the caller's tensors."""
+    from kernel_matmul_b200 import ranges
+    from kernel_matmul_b200.cg import CGSolver, ShardedOperator
+
+    n, k = 4500, 3
+    x = torch.sort(torch.rand(n, device="cuda") * 45)[0]
+    params = torch.tensor([[0.6, 0.0, 1.2], [0.6, 0.4, 0.7]], device="cuda")
+    start, end = ranges.make_ranges(2.4, x)
+    y = torch.randn(n, k, device="cuda")
+    ops = [ShardedOperator.from_kernel("spectral", x, params, s, e, 0.2) for s, e in ((start.clone(), end.clone()), (start, end))]
+    wide = ranges.make_ranges(4.0, x)
+    solvers = [CGSolver(op, y, 8) for op in ops]
+    for solver in solvers:
+        solver.step()
+    start.data.copy_(wide[0]), end.data.copy_(wide[1])
+    for solver in solvers:
+        for _ in range(7):
+            solver.step()
+    assert torch.equal(solvers[0].solution(), solvers[1].solution())
+
+
 @pytest.mark.parametrize("form", ["rbf", "spectral", "locally_periodic", "several lengthscales", "one component", "points of their own"])
 @pytest.mark.parametrize("k", [8, 16])
 def test_solves_of_operators_that_are_not_laid_out(form, k):
