@@ -56,8 +56,15 @@ MAX_SEGMENTS = 64
 #: points from which a solve over a sum of spectral components lays its operator out as a node matrix;
 #: below, the kernels are evaluated in every product
 NODE_OPERATOR_MIN_ROWS = 4096
-#: most memory for the node matrix of a rank
+#: most memory for the node matrix and the Lagrange matrices of a whole system
 NODE_OPERATOR_MAX_BYTES = 16 << 30
+
+
+def fits_as_nodes(row_blocks: int, widest: int, nodes: int) -> bool:
+    """Whether a system of ``row_blocks`` with a band of up to ``widest`` blocks and ``nodes`` nodes per block (0:
+    cannot be) is laid out.  Of the whole system, not of a rank's part of it: all rank counts must evaluate it
+    in the same way, as they give the same iterates."""
+    return nodes > 0 and 4 * row_blocks * nodes * (widest * nodes + BLOCK_SIZE) <= NODE_OPERATOR_MAX_BYTES
 
 
 def segment_layout(num_row_blocks: int, world_size: int) -> tuple[int, int, int]:
@@ -150,7 +157,7 @@ class ShardedOperator:
 
     def __init__(self, n: int, sigma2: float, matvec_rows: Callable[[Tensor, int, int, Tensor], None],
                  group=None, device: torch.device | None = None, col_range: tuple[int, int] | None = None,
-                 band_checksum: int = 0, vector_ops=None, mode: str = "auto"):
+                 band_checksum: int = 0, vector_ops=None, mode: str = "auto", laid_out: bool = False):
         import torch.distributed as dist
 
         if mode not in ("auto", "halo", "allgather"):
@@ -180,12 +187,12 @@ class ShardedOperator:
         hi = max(min(n, -(-hi // BLOCK_SIZE) * BLOCK_SIZE), self.row1)
         if self.rows == 0:
             lo = hi = self.row0 = self.row1 = min(self.row0, n)
-        self._agree(lo, hi, band_checksum, col_range is not None, mode)
+        self._agree(lo, hi, band_checksum, col_range is not None, mode, laid_out)
 
     # ---- set-up: the ranks compare what they were given and settle the exchange layout
 
-    def _agree(self, lo: int, hi: int, band_checksum: int, banded: bool, mode: str) -> None:
-        mine = [self.n, self.R, int(band_checksum), lo, hi, self.row0, self.row1, int(banded)]
+    def _agree(self, lo: int, hi: int, band_checksum: int, banded: bool, mode: str, laid_out: bool) -> None:
+        mine = [self.n, self.R, int(band_checksum), lo, hi, self.row0, self.row1, int(banded), int(laid_out)]
         if self.world > 1:
             t = torch.tensor(mine, dtype=torch.int64, device=self.device if self.device is not None else "cpu")
             every = torch.empty(self.world * len(mine), dtype=torch.int64, device=t.device)
@@ -198,6 +205,8 @@ class ShardedOperator:
                 raise ShardMismatchError(
                     f"rank {rk} describes a different system than rank 0: (n, row blocks, band checksum) = "
                     f"{tuple(row[:3])} against {tuple(table[0][:3])}")
+        #: whether every rank has laid its rows out: either all of them use that, or none does
+        self.laid_out = all(row[8] for row in table)
         below = max(row[5] - row[3] for row in table)  # most rows any rank needs from the rank before it
         above = max(row[4] - row[6] for row in table)  # ... from the rank after it
         owned = [row[6] - row[5] for row in table]
@@ -303,17 +312,10 @@ class ShardedOperator:
         def versions():
             return tuple(None if t.is_inference() else t._version for t in (x, params, start, end))
 
-        def usable(node_count: int, widest: int) -> bool:
-            return node_count > 0 and 4 * count * widest * node_count**2 <= NODE_OPERATOR_MAX_BYTES
-
         laid_out = versions()
         plan, lo, hi, checksum, node_count, widest = plan_nodes()
-        if usable(node_count, widest):
-            plan.build(lo, hi, node_count, widest)
+        if fits_as_nodes(R, widest, node_count) and plan.build(lo, hi, node_count, widest):
             nodes = plan
-        elif phases and batched and count > 0:
-            phase_ws = ops.prepare_sum_phases(kernel_type, x, x, params, rows=(begin * BLOCK_SIZE, min(n, (begin + count) * BLOCK_SIZE)),
-                                              cols=(max(0, min(lo, n)), max(0, min(hi, n))))
 
         def current_nodes(k: int = 1, look: bool = True):
             """The node operator for products of ``k`` columns, laid out again if points, parameters or band
@@ -331,15 +333,20 @@ class ShardedOperator:
             if torch.cuda.is_current_stream_capturing():
                 return nodes if now == laid_out else None
             if nodes.changed():
+                nodes = None  # (its memory is what the new one takes)
                 again, now_lo, now_hi, _, node_count, widest = plan_nodes()
-                if usable(node_count, widest):
-                    again.build(now_lo, now_hi, node_count, widest)
-                nodes = again if usable(node_count, widest) else None
+                if fits_as_nodes(R, widest, node_count) and again.build(now_lo, now_hi, node_count, widest):
+                    nodes = again
             laid_out = now
             return nodes
 
         op = cls(n, sigma2, matvec_rows, group=group, device=x.device, col_range=(lo, hi) if count > 0 else (0, 0),
-                 band_checksum=checksum, mode=mode)
+                 band_checksum=checksum, mode=mode, laid_out=nodes is not None)
+        if not op.laid_out:  # here or on another rank
+            nodes = None
+            if phases and batched and count > 0:
+                phase_ws = ops.prepare_sum_phases(kernel_type, x, x, params, rows=(begin * BLOCK_SIZE, min(n, (begin + count) * BLOCK_SIZE)),
+                                                  cols=(max(0, min(lo, n)), max(0, min(hi, n))))
         op.phase_workspace = phase_ws  # (None: the products evaluate the phase vectors themselves)
         op.current_nodes = current_nodes
         op.rows_product = rows_product

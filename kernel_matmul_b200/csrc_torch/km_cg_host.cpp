@@ -42,20 +42,26 @@ km_view NodeOperator::params_view(const Tensor &params) const {
     return v;
 }
 
-void NodeOperator::build(int64_t lo, int64_t hi, int64_t nodes, int64_t max_blocks) {
+bool NodeOperator::build(int64_t lo, int64_t hi, int64_t nodes, int64_t max_blocks) {
     const c10::cuda::CUDAGuard guard(x_.device());
     const auto opt = x_.options().requires_grad(false);
     const auto copy = [](const Tensor &t) { return t.detach().clone(at::MemoryFormat::Contiguous); };
     P_ = nodes, max_blocks_ = max_blocks;
     blk0_ = std::max<int64_t>(0, lo) / KM_BLOCK_SIZE, blk1_ = (std::min(hi, n_) + KM_BLOCK_SIZE - 1) / KM_BLOCK_SIZE;
     blk0_ = std::min(blk0_, blk1_);
-    own_x_ = copy(x_), own_params_ = copy(params_), own_start_ = copy(start_), own_end_ = copy(end_);
-    lambda_ = at::empty({R_ * P_ * KM_BLOCK_SIZE}, opt);
-    matrix_ = at::empty({std::max<int64_t>(1, count_ * max_blocks * P_ * P_)}, opt);
+    try {
+        lambda_ = at::empty({R_ * P_ * KM_BLOCK_SIZE}, opt);
+        matrix_ = at::empty({std::max<int64_t>(1, count_ * max_blocks * P_ * P_)}, opt);
+        own_x_ = copy(x_), own_params_ = copy(params_), own_start_ = copy(start_), own_end_ = copy(end_);
+    } catch (const c10::OutOfMemoryError &) {
+        lambda_ = matrix_ = own_x_ = own_params_ = own_start_ = own_end_ = Tensor();
+        return false;
+    }
     const km_view own_params = params_view(own_params_);
     raise_on(km_node_operator_build_f32(&kb_, n_, own_x_.const_data_ptr<float>(), 1, &own_params, own_start_.const_data_ptr<int32_t>(),
                                         own_end_.const_data_ptr<int32_t>(), begin_, count_, centre_.const_data_ptr<float>(),
                                         plan_.data_ptr(), P_, max_blocks_, lambda_.data_ptr<float>(), matrix_.data_ptr<float>(), stream()));
+    return true;
 }
 
 bool NodeOperator::changed() const {

@@ -22,7 +22,8 @@ class NodeOperator {
     // int64 on the device: lo, hi, checksum, nodes per block (0: not this way), widest band in blocks
     Tensor plan() const { return plan_.slice(0, 0, 5); }
     // Copies points, parameters and band and lays the operator out from the copies, which is what all products use.
-    void build(int64_t lo, int64_t hi, int64_t nodes, int64_t max_blocks);
+    // False, and nothing is kept, where the device has not that much memory left.
+    bool build(int64_t lo, int64_t hi, int64_t nodes, int64_t max_blocks);
     // Whether any of them has another value than its copy by now, however it was written to (waits for the
     // device; not under stream capture).
     bool changed() const;

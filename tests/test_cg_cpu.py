@@ -173,3 +173,35 @@ def test_a_non_finite_residual_is_reported():
     good = CGSolver(ShardedOperator(K.shape[0], 0.05, _dense_matvec(K), vector_ops=TorchVectorOps()), y)
     good.step()
     good.check_finite()
+
+
+def _laid_out_worker(rank, world, port, out_dir):
+    os.environ["MASTER_ADDR"] = "127.0.0.1"
+    os.environ["MASTER_PORT"] = str(port)
+    dist.init_process_group("gloo", rank=rank, world_size=world)
+    try:
+        x, K, _ = _system(n=1500)
+        make = lambda laid_out: ShardedOperator(1500, 0.05, _dense_matvec(K, x), vector_ops=TorchVectorOps(), laid_out=laid_out)  # noqa: E731
+        got = [make(True).laid_out, make(rank == 0).laid_out, make(rank == 1).laid_out, make(False).laid_out]
+        torch.save(got, os.path.join(out_dir, f"rank{rank}.pt"))
+    finally:
+        dist.destroy_process_group()
+
+
+def test_ranks_use_a_laid_out_operator_all_or_none(tmp_path):
+    port = 29500 + (os.getpid() % 2000) + 60
+    mp.spawn(_laid_out_worker, args=(2, port, str(tmp_path)), nprocs=2, join=True)
+    for rank in range(2):
+        assert torch.load(os.path.join(tmp_path, f"rank{rank}.pt")) == [True, False, False, False]
+
+
+def test_size_of_a_laid_out_operator():
+    """4 n nodes (band + 1) bytes per block, all of it counted; nothing of it depends on the rank."""
+    from kernel_matmul_b200.cg import NODE_OPERATOR_MAX_BYTES, fits_as_nodes
+
+    R, nodes, widest = 32768, 14, 22
+    assert fits_as_nodes(R, widest, nodes) and not fits_as_nodes(R, widest, 0)
+    most = NODE_OPERATOR_MAX_BYTES // (4 * nodes * (widest * nodes + 128))
+    assert fits_as_nodes(most, widest, nodes) and not fits_as_nodes(most + 1, widest, nodes)
+    # the Lagrange matrices alone
+    assert not fits_as_nodes(NODE_OPERATOR_MAX_BYTES // (4 * nodes * 128) + 1, 0, nodes)

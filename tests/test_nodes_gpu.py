@@ -7,7 +7,7 @@ both."""
 import pytest
 import torch
 
-from conftest import KERNEL_TYPES, assert_grad_close, make_params, rel_err
+from conftest import KERNEL_TYPES, assert_grad_close, make_params, memory_left, rel_err
 
 pytestmark = pytest.mark.gpu
 
@@ -394,6 +394,56 @@ def test_cg_operator_follows_writes_that_are_not_counted(write, what, use):
         fresh = ShardedOperator.from_kernel("spectral", *(a.clone() for a in t), 0.2)
         assert fresh.current_nodes() is not None
         assert torch.equal(after, result(fresh)) and not torch.equal(after, before)
+
+
+def _wide_system():
+    """800 000 points, 16 nodes per block and bands of 20 blocks: 130 MB of node matrix, 50 MB of Lagrange matrices."""
+    from kernel_matmul_b200 import ranges
+
+    n = 800000
+    x = torch.sort(torch.rand(n, device="cuda") * (n / 200))[0]
+    params = torch.tensor([[1.5, 0.0, 0.6], [1.5, 2.0, 0.5]], device="cuda")
+    return x, params, *ranges.make_ranges(6.0, x), torch.randn(n, 2, device="cuda")
+
+
+def test_cg_operator_without_memory_for_its_matrix():
+    """Evaluated, as where it is asked to be."""
+    from kernel_matmul_b200.cg import ShardedOperator
+
+    x, params, start, end, y = _wide_system()
+    want = ShardedOperator.from_kernel("spectral", x, params, start, end, 0.1, phases=True).apply(y).cpu()
+    with memory_left(135 << 20):  # (90 MB for the phase vectors)
+        op = ShardedOperator.from_kernel("spectral", x, params, start, end, 0.1)
+        assert op.current_nodes() is None and op.phase_workspace is not None
+        assert torch.equal(op.apply(y).cpu(), want)
+    assert ShardedOperator.from_kernel("spectral", x, params, start, end, 0.1).current_nodes() is not None
+
+
+def test_cg_operator_is_laid_out_again_in_its_own_memory():
+    from kernel_matmul_b200.cg import ShardedOperator
+
+    x, params, start, end, y = _wide_system()
+    op = ShardedOperator.from_kernel("spectral", x, params, start, end, 0.1)
+    op.apply(y)
+    with memory_left(80 << 20):
+        params[1, 2] = 0.7
+        again = op.apply(y)
+        assert op.current_nodes() is not None
+    assert torch.equal(again, ShardedOperator.from_kernel("spectral", x, params, start, end, 0.1).apply(y))
+
+
+def test_plan_of_the_cg_operator_is_the_same_for_every_window():
+    """Nodes and blocks by which all ranks decide whether a system is laid out."""
+    from kernel_matmul_b200 import _C, ranges
+
+    n = 6000
+    x = torch.sort(torch.rand(n, device="cuda") ** 2 * 60)[0]  # denser, with wider bands, at one end
+    params = torch.tensor([[0.6, 0.0, 1.2], [0.6, 0.4, 0.7]], device="cuda")
+    start, end = ranges.make_ranges(2.4, x)
+    R = start.shape[0]
+    plans = [_C.NodeOperator(n, x, params, start, end, b, c).plan().tolist() for b, c in ((0, R), (0, R // 2), (R // 2, R - R // 2), (R, 0))]
+    assert all(p[2:] == plans[0][2:] for p in plans) and plans[0][4] == int((end - start).max() + 127) // 128
+    assert _C.NodeOperator(n, None, None, start, end, 0, R).plan().tolist()[:4] == plans[0][:3] + [0]
 
 
 def test_band_that_becomes_wider_during_a_solve_is_not_read():
