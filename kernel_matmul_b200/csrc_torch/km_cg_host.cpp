@@ -3,6 +3,8 @@
 // Python took 350 us.
 #include "km_cg_host.h"
 
+#include <c10/cuda/CUDAGraphsC10Utils.h>
+
 namespace kmh {
 
 NodeOperator::NodeOperator(int64_t n, const std::optional<Tensor> &x, const std::optional<Tensor> &params, const Tensor &start,
@@ -61,7 +63,17 @@ bool NodeOperator::build(int64_t lo, int64_t hi, int64_t nodes, int64_t max_bloc
     raise_on(km_node_operator_build_f32(&kb_, n_, own_x_.const_data_ptr<float>(), 1, &own_params, own_start_.const_data_ptr<int32_t>(),
                                         own_end_.const_data_ptr<int32_t>(), begin_, count_, centre_.const_data_ptr<float>(),
                                         plan_.data_ptr(), P_, max_blocks_, lambda_.data_ptr<float>(), matrix_.data_ptr<float>(), stream()));
+    laid_out_on_ = c10::cuda::getCurrentCUDAStream(x_.device().index());
+    laid_out_.record(*laid_out_on_);
     return true;
+}
+
+void NodeOperator::use() const {
+    const auto now = c10::cuda::getCurrentCUDAStream(own_x_.device().index());
+    // (a capture waits for nothing outside it, and begins behind a synchronisation)
+    if (now == *laid_out_on_ || c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) return;
+    laid_out_.block(now);
+    for (const Tensor *t : {&lambda_, &matrix_, &own_start_, &own_end_, &own_x_, &own_params_}) t->record_stream(now);
 }
 
 bool NodeOperator::changed() const {
@@ -70,6 +82,7 @@ bool NodeOperator::changed() const {
         end_.sizes() != own_end_.sizes())
         return true;
     const c10::cuda::CUDAGuard guard(own_x_.device());
+    use();
     const Tensor flag = at::empty({1}, own_start_.options());
     const km_view params_now = params_view(params_);
     km_view s{}, e{};
@@ -112,6 +125,7 @@ void NodeOperator::matvec(const Tensor &v, const Tensor &out) const {
     TORCH_CHECK(out.size(0) == rows && v.size(1) <= KM_NODE_MAX_COLUMNS, "out must have ", rows, " rows and at most ",
                 KM_NODE_MAX_COLUMNS, " columns");
     const c10::cuda::CUDAGuard guard(x_.device());
+    use();
     const Tensor scratch = nodes(v.size(1));
     compress(v, v.size(1), scratch.data_ptr<float>());
     product(v.size(1), scratch.const_data_ptr<float>(), out.data_ptr<float>(), nullptr, 0.0, nullptr);
@@ -130,6 +144,7 @@ void cg_run(const CgState &s, const NodeOperator *nodes, RowsProduct *rows, int6
         raise_on(km_cg_segment_sums_f32(k, bp, s.blocks, s.seg_blocks, static_cast<double *>(to.data_ptr()), stream));
     };
     TORCH_CHECK((nodes != nullptr) != (rows != nullptr), "one kind of product");
+    if (nodes != nullptr) nodes->use();
     const Tensor scratch = nodes != nullptr ? nodes->nodes(k) : Tensor();
     float *at_nodes = nodes != nullptr ? scratch.data_ptr<float>() : nullptr;
     for (int64_t it = first; it < first + count; it++) {

@@ -1,5 +1,7 @@
 #pragma once
 
+#include <ATen/cuda/CUDAEvent.h>
+
 #include "km_host.h"
 
 namespace kmh {
@@ -30,6 +32,9 @@ class NodeOperator {
     // out = the window's rows of K v
     void matvec(const Tensor &v, const Tensor &out) const;
 
+    // Called before products on the current stream: they come after the layout, which may have been made on
+    // another, and its memory is not given away before they are done.
+    void use() const;
     Tensor nodes(int64_t k) const;
     void compress(const Tensor &v, int64_t k, float *nodes) const;
     void update_p(const CgState &s, int64_t it, float *nodes) const;
@@ -42,6 +47,8 @@ class NodeOperator {
     Tensor x_, params_, start_, end_;                      // the caller's
     Tensor own_x_, own_params_, own_start_, own_end_;      // contiguous copies
     Tensor centre_, plan_, lambda_, matrix_;
+    mutable at::cuda::CUDAEvent laid_out_;
+    std::optional<c10::cuda::CUDAStream> laid_out_on_;
     km_batch kb_{};
 };
 

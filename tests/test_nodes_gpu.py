@@ -432,6 +432,27 @@ def test_cg_operator_is_laid_out_again_in_its_own_memory():
     assert torch.equal(again, ShardedOperator.from_kernel("spectral", x, params, start, end, 0.1).apply(y))
 
 
+def test_cg_operator_laid_out_on_another_stream():
+    """Products on a stream come after a layout that a product on another one has just made, and its memory
+    outlives them."""
+    from kernel_matmul_b200.cg import ShardedOperator
+
+    x, params, start, end, y = _wide_system()
+    op = ShardedOperator.from_kernel("spectral", x, params, start, end, 0.1)
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    for scale in (0.7, 0.8, 0.9):
+        params[1, 2] = scale
+        for stream in streams:
+            stream.wait_stream(torch.cuda.current_stream())
+        got = []
+        for stream in streams:  # the first lays out again
+            with torch.cuda.stream(stream):
+                got.append(op.apply(y))
+        torch.cuda.synchronize()
+        want = ShardedOperator.from_kernel("spectral", x, params, start, end, 0.1).apply(y)
+        assert torch.equal(got[0], want) and torch.equal(got[1], want)
+
+
 def test_plan_of_the_cg_operator_is_the_same_for_every_window():
     """Nodes and blocks by which all ranks decide whether a system is laid out."""
     from kernel_matmul_b200 import _C, ranges
