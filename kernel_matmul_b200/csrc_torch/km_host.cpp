@@ -224,7 +224,12 @@ RowsProduct::RowsProduct(int64_t kernel_type, const Tensor &x1, const Tensor &x2
     int64_t items = count_;
     for (int64_t b : p_.batch) items *= b;
     tc_ = !sum_ && rows > 0 && (path == PATH_TC || (path == PATH_AUTO && k_ >= TENSOR_CORE_MIN_K && items >= TENSOR_CORE_MIN_ITEMS));
-    rhs_ = p_.view(rhs, 2);
+    set_views();
+    if (sum_ && phases.has_value()) phases_ = *phases;
+}
+
+void RowsProduct::set_views() {
+    rhs_ = p_.view(keep_[2], 2);
     if (sum_) {
         vout_ = km_view{};
         vout_.data = out_.data_ptr();
@@ -232,18 +237,21 @@ RowsProduct::RowsProduct(int64_t kernel_type, const Tensor &x1, const Tensor &x2
     } else {
         vout_ = p_.view(out_, 2);
     }
-    if (sum_ && phases.has_value()) phases_ = *phases;
-    if (tc_) workspace_ = workspace(x1, km_matmul_tc_workspace_bytes(&p_.kb, p_.n, k_, &rhs_));
 }
 
 void RowsProduct::run() {
     poll_gave_up(p_.device);
     const c10::cuda::CUDAGuard guard((c10::DeviceIndex)p_.device);
+    if (!p_.keep.empty()) {  // (more batch dims than the ABI carries: what was flattened may be a copy, of other contents by now)
+        p_ = Problem(p_.kid, keep_[0], keep_[1], keep_[3], keep_[4], keep_[5], {{&keep_[2], 2}});
+        set_views();
+    }
     void *stream = p_.stream();
-    if (tc_)
+    if (tc_) {
+        const Tensor ws = workspace(keep_[0], km_matmul_tc_workspace_bytes(&p_.kb, p_.n, k_, &rhs_));
         raise_on(km_matmul_tc_rows_f32(p_.kid, &p_.kb, p_.m, p_.n, k_, &p_.x1, &p_.x2, &rhs_, &p_.params, &p_.start, &p_.end, &vout_,
-                                       begin_, count_, workspace_.data_ptr(), workspace_.numel(), stream));
-    else if (phases_.defined())
+                                       begin_, count_, ws.data_ptr(), ws.numel(), stream));
+    } else if (phases_.defined())
         raise_on(km_matmul_rows_phases_f32(p_.kid, &p_.kb, p_.m, p_.n, k_, &p_.x1, &p_.x2, &rhs_, &p_.params, &p_.start, &p_.end,
                                            &vout_, begin_, count_, phases_.data_ptr(), phases_.numel(), stream));
     else

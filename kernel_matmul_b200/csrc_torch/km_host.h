@@ -125,13 +125,14 @@ class RowsProduct {
     RowsProduct(int64_t kernel_type, const Tensor &x1, const Tensor &x2, const Tensor &rhs, const Tensor &params, const Tensor &start,
                 const Tensor &end, int64_t row_block_begin, int64_t row_block_count, bool sum_batches,
                 const std::optional<Tensor> &out, int64_t path, const std::optional<Tensor> &phases);
-    void run();  // on the current stream
+    void run();  // on the current stream, with scratch of its own
     const Tensor &out() const { return out_; }
     bool tensor_cores() const { return tc_; }
 
   private:
+    void set_views();
     Problem p_;
-    Tensor out_, phases_, workspace_;
+    Tensor out_, phases_;
     std::vector<Tensor> keep_;
     km_view rhs_, vout_;
     int64_t k_, begin_, count_;

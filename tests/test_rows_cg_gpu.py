@@ -307,3 +307,22 @@ def test_batch_sum_on_tensor_cores(B, k, sum_kernel_variant):
                     end.expand(B, -1)).sum(0)
     out2 = ops.matmul_rows(args[0], args[1], args[2], args[3], d(params2), args[5], args[6], sum_batches=True)
     assert rel_err(out2, ref2) <= 1e-5
+
+
+@pytest.mark.parametrize("path_k", [3, 12])
+def test_prepared_product_of_many_batch_dims_sees_new_contents(path_k):
+    """More batch dims than the C ABI carries, which do not collapse without a copy: contents that change
+    between calls are those of the call."""
+    from kernel_matmul_b200 import ops, ranges
+
+    n, batch = 700, (2, 3, 2, 1, 2)
+    x = torch.sort(torch.rand(2, 1, 2, 1, 1, n, device="cuda") * 6)[0]
+    params = make_params("rbf", batch).cuda()
+    start, end = ranges.make_ranges(2.0, x[0, 0, 0, 0, 0])
+    rhs = torch.randn(2, 1, 2, 1, 2, n, path_k, device="cuda")
+    out = torch.empty(*batch, n, path_k, device="cuda")
+    call = ops.prepare_matmul_rows("rbf", x, x, rhs, params, start, end, row_block_begin=0, row_block_count=-(-n // 128), sum_batches=False, out=out)
+    for _ in range(2):
+        call()
+        assert torch.equal(out, ops.matmul_rows("rbf", x, x, rhs, params, start, end))
+        x.mul_(1.1), rhs.neg_(), params.mul_(0.9)
