@@ -72,18 +72,21 @@ __host__ __device__ inline int64_t ceil_div(int64_t a, int64_t b) { return (a + 
 // their predecessor drains (launch_gated), and closed() is the first thing they ask: behind a closed gate
 // they are over by then but for the first CTA, which stays until the predecessor is complete, so that the
 // chain is complete when its last kernel is; behind an open one all of them wait for it.  The flag itself
-// has been final since before the chain's first kernel started, but it is read before any wait: by an acquire
-// load, as kernels before that one have read and changed it and left it in the SM's L1.  (8192 CTAs of a gated kernel
-// that only return take 36 us.)
+// is final when the chain's first kernel starts, but it is read before any wait: past the SM's L1,
+// in which kernels before that one may have left it as it was.  (8192 CTAs of a gated kernel that only return take
+// 36 us.)
+__device__ __forceinline__ int load_flag(const int *flag) {  // (an acquire would throw the L1 of the running kernels away)
+    int v;
+    asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(flag) : "memory");
+    return v;
+}
 struct Gate {
     const int *flag = nullptr;
     int want = 0;
     __device__ __forceinline__ bool closed() const {
         if (flag == nullptr) return false;
         asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-        int now;
-        asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(now) : "l"(flag) : "memory");
-        const bool run = now == want;
+        const bool run = load_flag(flag) == want;
         if (run || (blockIdx.x == 0 && blockIdx.y == 0)) asm volatile("griddepcontrol.wait;" ::: "memory");
         return !run;
     }
