@@ -1157,8 +1157,10 @@ static int nodes_compress(const NodesArgs &a, const NodesLayout &l, const View<c
         const cudaError_t err = cudaFuncSetAttribute(nodes_compress_kernel<COLS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                      (int)CompressShape<COLS>::SMEM);
         if (err != cudaSuccess) return cuda_fail(err, "cudaFuncSetAttribute(interpolation)");
-        // (a shared operand: a CTA per class that the plan may have made, most of which return at once)
-        const dim3 grid((unsigned)(c.slots * c.blocks * ceil_div(l.kq, COLS)), c.slots == 1 && a.batch.count > 1 ? NODES_CLASSES_PER_LEVEL : 1);
+        // (a shared operand: a CTA per class that the plan may have made -- one per kernel at most --, of which many
+        // return at once; 12 000 that do take 30 us)
+        const dim3 grid((unsigned)(c.slots * c.blocks * ceil_div(l.kq, COLS)),
+                        c.slots == 1 ? (unsigned)std::min<int64_t>(a.batch.count, NODES_CLASSES_PER_LEVEL) : 1);
         return launch_chained("interpolation: operand launch", nodes_compress_kernel<COLS>, grid, 128, CompressShape<COLS>::SMEM, s, c);
     };
     return l.kq <= 16 ? launch(Int<16>()) : launch(Int<32>());

@@ -48,10 +48,21 @@ constexpr int64_t TENSOR_CORE_MIN_K = 9, GRAD_TENSOR_CORE_MIN_K = 8, TENSOR_CORE
 // by interpolation, 8.9e-7 - 1.4e-6 on the tensor cores and 2.4e-7 - 1.0e-6 on the FMA pipe, which holds small
 // entries to 1e-6 of themselves (one-hot columns, entries of 1e-4 - 1e-3 of the largest, worst relative error: RBF 3e-6,
 // 3e-4 and 1e-6, locally periodic with a lengthscale of 0.6 3e-5, 2e-4 and 2e-6): what ran on the FMA pipe stays there.
+//
+// Bands of 6 blocks and more gain from 512 items on; gradients of up to 16 columns gain nothing on 6 blocks there (factor
+// 0.9 - 1.05 of the direct kernels' time; products 0.7 - 0.8), bands of 3 blocks lose up to 1.1 on products of up to
+// four kernels and up to 1.6 on such gradients, and gain from 2048 items on.  A call that the device declines (bands not
+// aligned to blocks, intervals too long) takes 1.03 - 1.25 times its time, a gradient of 9 columns on 512 items 1.4.
 constexpr int64_t NODES_MIN_ITEMS = 512;
+// Row blocks of a kernel from which it does: the plan takes 0.25 us per kernel, in one CTA, and the last column blocks of a
+// band are as dear as the first.  512 and 2048 kernels on one block each took 150 and 490 us, directly 27 and 51;
+// 256 on three blocks 111 and 47, 64 on eight blocks 70 and 44; 32 on 32 blocks 0.8 - 0.9 of the direct time at a
+// band of 6 blocks.
+constexpr int64_t NODES_MIN_ROW_BLOCKS = 32;
 // With a band, both sides share an interval: where one has this many times the other's points, the blocks
-// of the sparser are too long for it (5003 test points against 50 021: 100 nodes and more) and the call would pay
-// 25 us for finding out.
+// of the sparser may be too long for it (5003 test points against 50 021 at 100 per unit: 100 nodes and more) and the
+// call would pay 25 us for finding out.  Not measured over densities and lengthscales: smooth kernels on dense points,
+// which a longer interval would do for, are evaluated directly too.
 constexpr int64_t NODES_MAX_RATIO = 8;
 // Without a cutoff: kernel entries from which it does (the points have to be put in order first).
 constexpr int64_t NODES_MIN_ENTRIES = 1LL << 27;
@@ -88,7 +99,7 @@ struct Problem {
     // `k` columns, of an op that takes the tensor cores from `min_k` columns on
     bool try_nodes(int64_t path, int64_t k, int64_t min_k) const {
         if (path == PATH_NODES) return true;
-        if (path != PATH_AUTO || k < min_k || items() < TENSOR_CORE_MIN_ITEMS) return false;
+        if (path != PATH_AUTO || k < min_k || items() < TENSOR_CORE_MIN_ITEMS || row_blocks < NODES_MIN_ROW_BLOCKS) return false;
         if (one_range()) return m * n * (items() / row_blocks) >= NODES_MIN_ENTRIES;
         return items() >= NODES_MIN_ITEMS && std::max(m, n) < NODES_MAX_RATIO * std::min(m, n);
     }

@@ -231,6 +231,19 @@ def test_what_ran_on_the_fma_pipe_stays_there(kt, form):
         check(33000, 8, 7, ())
 
 
+@pytest.mark.parametrize("batch,n,cutoff", [(600, 100, 2.0), (40, 31 * 128, 2.0), (40, 31 * 128, None)])
+def test_batches_of_small_problems_are_evaluated_directly(batch, n, cutoff):
+    """Whatever their number, kernels of fewer than 32 row blocks run on the tensor cores."""
+    from kernel_matmul_b200 import ops, ranges
+
+    x = torch.sort(torch.rand(n) * (n / 100))[0].cuda()
+    start, end = ranges.make_ranges(cutoff, x)
+    rhs, left = torch.randn(n, 16, device="cuda"), torch.randn(n, 16, device="cuda")
+    args = (make_params("rbf", (batch,)).cuda(), start.expand(batch, -1), end.expand(batch, -1))
+    assert torch.equal(*(ops.matmul("rbf", x, x, rhs, *args, path=p) for p in ("auto", "tc")))
+    assert torch.equal(*(ops.bilinear_derivative("rbf", x, x, left, rhs, *args, path=p) for p in ("auto", "tc")))
+
+
 @pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan"), 3e38])
 @pytest.mark.parametrize("k", [3, 12])
 def test_operands_that_are_not_finite_or_near_overflow(value, k):
