@@ -48,6 +48,9 @@ constexpr int64_t TENSOR_CORE_MIN_K = 9, GRAD_TENSOR_CORE_MIN_K = 8, TENSOR_CORE
 // by interpolation, 8.9e-7 - 1.4e-6 on the tensor cores and 2.4e-7 - 1.0e-6 on the FMA pipe, which holds small
 // entries to 1e-6 of themselves (one-hot columns, entries of 1e-4 - 1e-3 of the largest, worst relative error: RBF 3e-6,
 // 3e-4 and 1e-6, locally periodic with a lengthscale of 0.6 3e-5, 2e-4 and 2e-6): what ran on the FMA pipe stays there.
+// Gradients of random operands are off by 1e-11 - 2.6e-10 of the sum of their terms' magnitudes, 1.6e-10 - 1e-9 on the tensor
+// cores; of single entries, constant and smooth operands by up to 4e-7, 6e-7 there (an RBF lengthscale's by up to 1.2e-7
+// against 1.0e-7).
 //
 // Bands of 6 blocks and more gain from 512 items on; gradients of up to 16 columns gain nothing on 6 blocks there (factor
 // 0.9 - 1.05 of the direct kernels' time; products 0.7 - 0.8), bands of 3 blocks lose up to 1.1 on products of up to

@@ -2,12 +2,13 @@
 sizes and in the forms where its kernels branch, and the direct kernels where it must step aside.
 
 Tolerances: products 1e-5 of the largest value and gradients as in ``conftest.assert_grad_close``, the
-criteria of the direct kernels; the interpolation's own bound, 3e-8 of kappa's maximum per entry, is below
-both."""
+criteria of the direct kernels; the interpolation's own error, up to 3e-8 of kappa's maximum per entry and 2.1e-7
+of that of a gradient's factor (``test_nodes_cpu.py``), is below both."""
 import pytest
 import torch
 
 from conftest import KERNEL_TYPES, assert_grad_close, make_params, memory_left, rel_err
+from test_nodes_cpu import nodes_by_level
 
 pytestmark = pytest.mark.gpu
 
@@ -104,32 +105,6 @@ def _half_lengths(x):
     return torch.stack([0.5 * (b[..., -1] - b[..., 0]) for b in blocks], dim=-1)
 
 
-def _nodes_by_level(kt, params, longest, unit, cap, classes=8, eps=3e-8):
-    """The plan of csrc/km_nodes.cu restated: nodes of every kernel at the four half-lengths, after each level
-    has kept its largest classes and merged the others into them."""
-    rho = 1.1 * 2.0 ** (0.17 * torch.arange(32, dtype=torch.float64))
-    out = []
-    for level in range(4):
-        b = 0.5 * longest / 1.15**level * (rho - 1 / rho)
-        need = []
-        for theta in params.double():
-            be = (b / theta[0]) ** 2
-            log_m = 0.5 * be + torch.log1p(be)
-            if kt == "spectral":
-                log_m = log_m + 2 * torch.pi * theta[1].abs() * b
-            if kt == "locally_periodic":
-                log_m = log_m + (torch.cosh((2 * torch.pi * b / theta[2]).clamp(max=300)) - 1) / theta[1]
-            p = ((log_m + torch.log(4 / (rho - 1)) - torch.log(torch.tensor(eps))) / torch.log(rho)).min().item()
-            need.append(max(4, -(-int(-(-p // 1)) // unit) * unit))
-        kept = []
-        for p in sorted(set(need), reverse=True):
-            if len(kept) == classes or sum(kept) + p > cap:
-                break
-            kept.append(p)
-        out.append([min(q for q in kept if q >= p) for p in need])
-    return torch.tensor(out).T
-
-
 @pytest.mark.parametrize("kt,why", [("spectral", "more than eight classes"), ("locally_periodic", "more than eight classes"),
                                     ("spectral", "more nodes than there is room for")])
 @pytest.mark.parametrize("shared", [True, False])
@@ -155,7 +130,7 @@ def test_levels_that_merge_different_classes(kt, why, shared, k):
             params = torch.stack([0.7 + 0.8 * u[:, 0], 2.0 + 3.0 * u[:, 1] if room else 6.0 * u[:, 1], 0.8 + u[:, 3]], dim=-1)
         else:
             params = torch.stack([0.7 + 0.8 * u[:, 0], 0.3 + u[:, 1], 0.35 + 2.0 * u[:, 2], 0.8 + u[:, 3]], dim=-1)
-        nodes = _nodes_by_level(kt, params, longest, unit, cap)
+        nodes = nodes_by_level(kt, params, longest, unit, cap)
         if nodes.max() > (80 if k <= 16 else 64):
             continue
         at = [levels[0] if shared else levels[i] for i in range(batch)]
