@@ -435,6 +435,27 @@ def reference_cuda_timing(kind: str, kernel_type: str, k: int, call_args: tuple,
 # ------------------------------------------------------------------------ spectral mixture (config 2)
 
 
+def direct_kernel_rates(kt, k, E, fwd, bwd, tc_fwd, tc_bwd, fp32_peak, sfu_peak, traffic_known) -> dict:
+    """Rates of the kernels that evaluate every entry of the band (``E`` entries; ``fwd`` / ``bwd`` ms)."""
+    kernels = {
+        "matmul_tc_kernel" if tc_fwd else "matmul_fma_kernel": {
+            "ms": fwd, "sfu_per_entry": TC_FWD[kt][1] if tc_fwd else GEN_FWD[kt][1],
+            "contraction": "tcgen05.mma kind::f16 (fp16 hi/lo split)" if tc_fwd else "fma.rn.f32x2",
+            "fp32_instr_per_entry": TC_FWD[kt][0] if tc_fwd else fp32_instr_fwd(kt, k)},
+        "grad_tc_kernel" if tc_bwd else "grad_band_kernel": {
+            "ms": bwd, "sfu_per_entry": TC_BWD[kt][1] if tc_bwd else GEN_BWD[kt][1],
+            "contraction": "tcgen05.mma kind::tf32 (3xTF32)" if tc_bwd else "fma.rn.f32x2",
+            "fp32_instr_per_entry": TC_BWD[kt][0] if tc_bwd else fp32_instr_bwd(kt, k)},
+    }
+    for kname, kd in kernels.items():
+        kd["achieved_tflops"] = 2.0 * E * kd["fp32_instr_per_entry"] / (kd["ms"] * 1e-3) / 1e12
+        kd["frac_fp32"] = kd["achieved_tflops"] / fp32_peak
+        kd["achieved_sfu_tops"] = E * kd["sfu_per_entry"] / (kd["ms"] * 1e-3) / 1e12
+        kd["frac_sfu"] = kd["achieved_sfu_tops"] / sfu_peak
+        kd["traffic"] = dram_traffic("spectral_mixture", kname) if traffic_known else None
+    return kernels
+
+
 def measure_mixture(w, dev, steps: int, path: str, fp32_peak: float, sfu_peak: float, with_e2e: bool, with_ref: bool) -> dict:
     """Forward product + matmul_bwd of the spectral mixture: resident inputs, CUDA events, L2 flushed
     between steps.  Returns times, roofline fractions per kernel and (optionally) the end-to-end
@@ -472,35 +493,29 @@ def measure_mixture(w, dev, steps: int, path: str, fp32_peak: float, sfu_peak: f
         step_ms.append(e0.elapsed_time(e2))
     ops.check(dev)
     fwd, bwd = statistics.mean(fwd_ms), statistics.mean(bwd_ms)
-    by_nodes = path == "auto" and not tc_fwd  # (what the automatic path does at this size)
-    fwd_name = "nodes_product_kernel" if by_nodes else ("matmul_tc_kernel" if tc_fwd else "matmul_fma_kernel")
-    bwd_name = "nodes_grad_kernel" if by_nodes else ("grad_tc_kernel" if tc_bwd else "grad_band_kernel")
-    kernels = {
-        fwd_name: {"ms": fwd, "sfu_per_entry": TC_FWD[kt][1] if tc_fwd else GEN_FWD[kt][1],
-                   "contraction": "tcgen05.mma kind::f16 (fp16 hi/lo split)" if tc_fwd else "fma.rn.f32x2",
-                   "fp32_instr_per_entry": TC_FWD[kt][0] if tc_fwd else fp32_instr_fwd(kt, k)},
-        bwd_name: {"ms": bwd, "sfu_per_entry": TC_BWD[kt][1] if tc_bwd else GEN_BWD[kt][1],
-                   "contraction": "tcgen05.mma kind::tf32 (3xTF32)" if tc_bwd else "fma.rn.f32x2",
-                   "fp32_instr_per_entry": TC_BWD[kt][0] if tc_bwd else fp32_instr_bwd(kt, k)},
-    }
-    for kname, kd in kernels.items():
-        kd["achieved_tflops"] = 2.0 * E * kd["fp32_instr_per_entry"] / (kd["ms"] * 1e-3) / 1e12
-        kd["frac_fp32"] = kd["achieved_tflops"] / fp32_peak
-        kd["achieved_sfu_tops"] = E * kd["sfu_per_entry"] / (kd["ms"] * 1e-3) / 1e12
-        kd["frac_sfu"] = kd["achieved_sfu_tops"] / sfu_peak
-        kd["traffic"] = dram_traffic("spectral_mixture", kname) if w.n == 65536 else None
-        if by_nodes:
-            kd["contraction"] = "between interpolation nodes (fma.rn.f32x2)"
-            kd["note"] = ("all kernels of the call; rates and fractions count the work of evaluating every entry, which "
-                          "interpolation does not do: they may exceed 1")
+    by_nodes = path == "auto" and not tc_fwd and k >= ops.TENSOR_CORE_MIN_K  # (what the automatic path does at this size)
+    if by_nodes:
+        # bytes that the calls cannot do without: points and rhs read and the product written; points, rhs and its
+        # gradient read (what interpolation evaluates follows from the points: no count of entries or FLOPs here)
+        hbm = measured_peaks().get("hbm_gbs", 6650.0)
+        kernels = {name: {"ms": ms, "bound": "hbm", "bytes": 4.0 * (n + n * k + B * n * k), "contraction": "between interpolation nodes "
+                          "(fma.rn.f32x2)", "what": "all kernels of the call"}
+                   for name, ms in (("nodes_product_kernel", fwd), ("nodes_grad_kernel", bwd))}
+        for kd in kernels.values():
+            kd["achieved_gbs"] = kd["bytes"] / (kd["ms"] * 1e-3) / 1e9
+            kd["frac_hbm"] = kd["achieved_gbs"] / hbm
+    else:
+        kernels = direct_kernel_rates(kt, k, E, fwd, bwd, tc_fwd, tc_bwd, fp32_peak, sfu_peak, w.n == 65536)
     ms_per_step = statistics.mean(step_ms)
     res = {
         "config": config_of(w, E), "path": path, "ms_per_step": ms_per_step, "value": 2.0 * E * k / (ms_per_step * 1e-3),
         "unit": UNIT, "steps": steps, "l2": "flushed between steps (256 MB write)", "kernels": kernels,
         "fp32_peak_tflops": fp32_peak, "sfu_peak_tops": sfu_peak,
-        "bound": "fp32 (FFMA issue rate measured live; the contraction runs on the tensor cores at a few % of their peak, "
+        "bound": "hbm (bytes of the operands; the time is FP32 issue between the nodes, launches and operands to the nodes)" if by_nodes else
+                 "fp32 (FFMA issue rate measured live; the contraction runs on the tensor cores at a few % of their peak, "
                  "what bounds the kernels is generating the kernel entries)",
-        "gpu_launches_per_step": (3 if tc_fwd else 1) + (3 if tc_bwd else 2),
+        # interpolation: plan, Lagrange matrices, operand(s), product / gradient and finish, and the gated direct kernels
+        "gpu_launches_per_step": (4 + 3) + (6 + 3) if by_nodes else (3 if tc_fwd else 1) + (3 if tc_bwd else 2),
     }
     if with_e2e:
         hx, hrhs = w.x.pin_memory(), w.rhs.contiguous().pin_memory()
@@ -537,7 +552,7 @@ def measure_single_op(name: str, dev, steps: int, fp32_peak: float, sfu_peak: fl
     events, L2 flushed between steps).  Workloads:
       rbf_small                  RBF forward, n = 4096, k = 1 (launch-latency bound)
       locally_periodic_bilinear  bilinear_derivative, batch 4, n = 262144, k = 32
-      rbf_unbanded               unbanded RBF forward, n = 131072, k = 128 (tensor cores)
+      rbf_unbanded               unbanded RBF forward, n = 131072, k = 128 (between interpolation nodes)
       rbf_unbanded_index         2^24 random (row, col) gathers
     """
     from kernel_matmul_b200 import ops, ranges, workloads
@@ -565,8 +580,8 @@ def measure_single_op(name: str, dev, steps: int, fp32_peak: float, sfu_peak: fl
         kt, k = "locally_periodic", w.rhs.shape[-1]
         E = int(ops.count_entries(w.n, w.n, start, end))
         fn = lambda: ops.bilinear_derivative(kt, xb, xb, lhs, rhs, params, start, end)  # noqa: E731
-        model = {"bound": "fp32", "fp32_instr": TC_BWD[kt][0], "sfu": TC_BWD[kt][1]}
-        units, kernel = E * k, "grad_tc_kernel"
+        model = {"bound": "hbm", "bytes": 4.0 * (w.n + 2 * B * w.n * k), "what": "points, left and right"}
+        units, kernel = E * k, "nodes_grad_kernel (with all kernels of the call)"
         if with_ref:
             ref = reference_cuda_timing("bilinear_derivative", kt, k, (xb, xb, lhs, rhs, params.contiguous(), start, end), reps=1)
     elif name == "rbf_unbanded":
@@ -576,8 +591,8 @@ def measure_single_op(name: str, dev, steps: int, fp32_peak: float, sfu_peak: fl
         rhs, params = w.rhs.to(dev), w.params.to(dev)
         kt, k, E = "rbf", w.rhs.shape[-1], w.n * w.n
         fn = lambda: ops.matmul(kt, x, x, rhs, params, start, end)  # noqa: E731
-        model = {"bound": "tensor", "tensor_flops": 3 * 2.0 * E * k, "fp32_instr": TC_FWD[kt][0], "sfu": TC_FWD[kt][1]}
-        units, kernel = E * k, "matmul_tc_kernel"
+        model = {"bound": "hbm", "bytes": 4.0 * (w.n + 2 * w.n * k), "what": "points, rhs and product"}
+        units, kernel = E * k, "nodes_product_kernel (with all kernels of the call)"
         if with_ref:
             ref = reference_cuda_timing("matmul", kt, k, tuple(t.unsqueeze(0) for t in (x, x, rhs, params, start, end)), reps=1)
     elif name == "rbf_unbanded_index":
@@ -588,7 +603,7 @@ def measure_single_op(name: str, dev, steps: int, fp32_peak: float, sfu_peak: fl
         row, col = w.extra["row"].to(dev), w.extra["col"].to(dev)
         L = row.numel()
         fn = lambda: ops.index("rbf", x, x, params, start, end, (), row, col)  # noqa: E731
-        model = {"bound": "hbm", "bytes": 12 * L}
+        model = {"bound": "hbm", "bytes": 12 * L, "what": "row, col and value of every lookup"}
         units, kernel, E, k, kt = L, "index_kernel", L, 1, "rbf"
     else:
         raise SystemExit(f"unknown workload {name}")
@@ -605,14 +620,9 @@ def measure_single_op(name: str, dev, steps: int, fp32_peak: float, sfu_peak: fl
     ops.check(dev)
     t = statistics.mean(ms) * 1e-3
     roof = {"bound": model["bound"], "kernel": kernel, "traffic": dram_traffic(name, kernel)}
-    if model["bound"] == "tensor":
-        f16_peak = peaks.get("bf16_tflops", 1590.0)
-        roof.update(achieved=model["tensor_flops"] / t / 1e12, peak=f16_peak, unit="TFLOP/s",
-                    peak_source="MEASURED_PEAKS.json bf16_tflops (burst); achieved counts the 3 fp16 MMAs per product",
-                    frac_sfu=E * model["sfu"] / t / 1e12 / sfu_peak)
-    elif model["bound"] == "hbm":
+    if model["bound"] == "hbm":
         roof.update(achieved=model["bytes"] / t / 1e9, peak=peaks.get("hbm_gbs", 6650.0), unit="GB/s",
-                    peak_source="MEASURED_PEAKS.json hbm_gbs; algorithmic bytes = row + col + out per lookup")
+                    peak_source="MEASURED_PEAKS.json hbm_gbs; algorithmic bytes: " + model["what"])
     else:
         roof.update(achieved=2.0 * E * model["fp32_instr"] / t / 1e12, peak=fp32_peak, unit="TFLOP/s",
                     peak_source="live FFMA probe", frac_sfu=E * model["sfu"] / t / 1e12 / sfu_peak)
@@ -932,7 +942,10 @@ def run_mixture(args, rank: int, world: int, local: int) -> None:
             "warmup": 3, "ms_per_step": ms, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
             "dtype": "f32", "data": "synthetic", "config": res["config"], "path": args.path, "l2": res["l2"],
             "per_rank": "own batch of components (same seeded parameters on every rank), no collective",
-            "roofline": {"bound": "fp32", "kernel": dom, "achieved": d["achieved_tflops"], "peak": fp32_peak, "unit": "TFLOP/s",
+            "roofline": {"bound": "hbm", "kernel": dom, "achieved": d["achieved_gbs"], "peak": measured_peaks().get("hbm_gbs", 6650.0),
+                         "unit": "GB/s", "frac": d["frac_hbm"], "traffic": None, "peak_source": "MEASURED_PEAKS.json hbm_gbs; algorithmic "
+                         "bytes = points, operands and results", "kernels": kernels} if "frac_hbm" in d else
+                        {"bound": "fp32", "kernel": dom, "achieved": d["achieved_tflops"], "peak": fp32_peak, "unit": "TFLOP/s",
                          "frac": d["frac_fp32"], "traffic": d["traffic"], "traffic_source": "profiles/dram_traffic.json",
                          "peak_source": "measured live: km_probe_fp32_peak (FFMA issue rate of all SMs)",
                          "fp32_peak_tflops": fp32_peak, "sfu_peak_tops": sfu_peak, "kernels": kernels},
