@@ -86,6 +86,7 @@ std::tuple<Tensor, Tensor> band(double cutoff, const Tensor &x1, const std::opti
         kmh::check_f32(*x2);
         TORCH_CHECK(x2->dim() == x1.dim() && x2->sizes().slice(0, x1.dim() - 1) == x1.sizes().slice(0, x1.dim() - 1),
                     "x1 and x2 must share their batch dimensions");
+        TORCH_CHECK(x2->device() == x1.device(), "all tensors must be on the same CUDA device");
         const Tensor c = x2->contiguous();
         kmh::raise_on(km_make_ranges_f32(B, m, x2->size(-1), a.const_data_ptr<float>(), c.const_data_ptr<float>(), (float)cutoff,
                                          (int32_t)block, align ? 1 : 0, start.data_ptr<int32_t>(), end.data_ptr<int32_t>(),
@@ -101,6 +102,7 @@ std::tuple<Tensor, Tensor> band(double cutoff, const Tensor &x1, const std::opti
 // Symmetric bands of B kernels with cutoffs (B,) over x (n,) or (B, n): (B, R) each, or (R,) with `single`.
 std::tuple<Tensor, Tensor> band_cutoffs(const Tensor &cutoffs, const Tensor &x, int64_t block, bool single) {
     kmh::check_f32(cutoffs), kmh::check_f32(x);
+    TORCH_CHECK(cutoffs.device() == x.device(), "all tensors must be on the same CUDA device");
     const c10::cuda::CUDAGuard guard(x.device());
     const int64_t n = x.size(-1), R = (n + block - 1) / block, B = cutoffs.size(0);
     const Tensor a = x.contiguous(), c = cutoffs.contiguous();

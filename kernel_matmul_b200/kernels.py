@@ -62,7 +62,7 @@ def _band(x1: Tensor, x2: Tensor, symmetric: bool, cutoff: float | Tensor | None
     xs = x1.squeeze(-1)
     if isinstance(cutoff, Tensor):
         if symmetric and xs.dim() == 1 and xs.is_cuda and xs.dtype == torch.float32:
-            return _C.band_cutoffs(cutoff.detach(), xs, _BLOCK_SIZE, True)
+            return _C.band_cutoffs(cutoff.detach().to(xs.device), xs, _BLOCK_SIZE, True)
         cutoff = float(cutoff)
     if symmetric:
         return make_ranges(cutoff, xs, align=True)

@@ -65,7 +65,7 @@ def make_ranges(
 
     dev = _device_for(x1)
     x1d = x1 if x1.is_cuda and x1.dtype == torch.float32 else x1.detach().to(device=dev, dtype=torch.float32)
-    if x2 is not None and not (x2.is_cuda and x2.dtype == torch.float32):
+    if x2 is not None and not (x2.device == dev and x2.dtype == torch.float32):
         x2 = x2.detach().to(device=dev, dtype=torch.float32)
     start, end = _C.band(float(cutoff), x1d, x2, block_size, align)
     return (start, end) if x1.is_cuda else (start.to(out_device), end.to(out_device))

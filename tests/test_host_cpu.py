@@ -156,3 +156,34 @@ def test_operators_of_kernels_that_are_not_there_are_refused_by_name(kernel_type
                  lambda: op.get_indices(index, index)):
         with pytest.raises(error, match=kernel_type):
             call()
+
+
+def test_band_of_points_on_another_gpu_is_made_of_a_copy(monkeypatch):
+    """make_ranges moves x2 to x1's device, whatever GPU it is on (tensors that only have the attributes)."""
+    from kernel_matmul_b200 import ranges
+
+    class Points:
+        dtype, is_cuda = torch.float32, True
+
+        def __init__(self, index):
+            self.device, self.shape = torch.device("cuda", index), (256,)
+
+        def detach(self):
+            return self
+
+        def to(self, *, device, dtype):
+            moved = Points(0)
+            moved.device, moved.dtype = device, dtype
+            return moved
+
+    seen = []
+
+    class Extension:
+        @staticmethod
+        def band(cutoff, x1, x2, block, align):
+            seen.append((x1.device, x2.device))
+            return "start", "end"
+
+    monkeypatch.setattr(ranges, "_C", Extension)
+    assert ranges.make_ranges(1.0, Points(0), Points(1), align=True) == ("start", "end")
+    assert seen == [(torch.device("cuda", 0), torch.device("cuda", 0))]
