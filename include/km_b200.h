@@ -134,10 +134,10 @@ KM_API int km_workspace_status(const void *workspace, int32_t *status_out, void 
 KM_API int km_take_gave_up(int32_t device, int32_t *what);
 
 /* ---------------------------------------------------------------------------------------
- * The same product by blockwise interpolation where its error bound allows: between blocks of 128
- * sorted points kappa is a polynomial to fp32 rounding (error below 1e-8 of kappa's maximum, bounded
- * from the block extents and the parameters on the device), so the product is taken between P = 4 .. 64
- * Chebyshev points per block, with Lagrange matrices on both sides.  Calls whose bands are not
+ * The same product by blockwise interpolation where the points allow: between blocks of 128
+ * sorted points kappa is a polynomial to fp32 rounding (to about 3e-8 of kappa's maximum), so the product is taken
+ * between P = 4 .. 80 Chebyshev points per block, with Lagrange matrices on both sides; P is chosen on the device
+ * from the blocks' extents and the parameters.  Calls whose bands are not
  * aligned to blocks, or that would need more points, are evaluated directly (km_matmul_tc_f32 from 9
  * columns, km_matmul_f32 below): the kernels of both ways are launched and the device decides.
  * all_columns != 0: the caller expects every row block to see all columns (no cutoff); the points, shared by

@@ -20,6 +20,11 @@ The value of ``log det Khat`` comes from the same solve (stochastic Lanczos quad
 ``beta_j`` of the CG run on ``z_i`` are the entries of the Lanczos tridiagonal ``T_i`` of ``Khat``
 started at ``z_i`` (``T[j,j] = 1/alpha_j + beta_{j-1}/alpha_{j-1}``, ``T[j,j+1] = sqrt(beta_j)/alpha_j``),
 and ``z^T log(Khat) z ~ |z|^2 e_1^T log(T) e_1``; the mean over the probes estimates the trace.
+
+How exact they are in fp32: tens of CG steps at a condition number of 1000 bring a relative rounding of
+1e-7 in the products back as 4e-6 - 1e-5 in the solves, 1e-7 - 3e-6 in value and log-determinant.  The gradients are
+differences of two terms that nearly cancel: any change in the products' last bits moves ``grad_params`` by up
+to 4e-4 and ``grad_sigma2`` by up to 6e-4 of themselves (14 systems of 2000 to 54 000 points).
 """
 from __future__ import annotations
 
