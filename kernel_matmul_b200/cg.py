@@ -313,7 +313,7 @@ class ShardedOperator:
             return tuple(None if t.is_inference() else t._version for t in (x, params, start, end))
 
         laid_out = versions()
-        plan, lo, hi, checksum, node_count, widest = plan_nodes()
+        plan, lo, hi, checksum, node_count, widest = plan_nodes() if n > 0 else (None, 0, 0, 0, 0, 0)
         if fits_as_nodes(R, widest, node_count) and plan.build(lo, hi, node_count, widest):
             nodes = plan
 

@@ -69,6 +69,7 @@ bool NodeOperator::build(int64_t lo, int64_t hi, int64_t nodes, int64_t max_bloc
 }
 
 void NodeOperator::use() const {
+    TORCH_CHECK(laid_out_on_.has_value(), "the operator has not been laid out");
     const auto now = c10::cuda::getCurrentCUDAStream(own_x_.device().index());
     // (a capture waits for nothing outside it, and begins behind a synchronisation)
     if (now == *laid_out_on_ || c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) return;

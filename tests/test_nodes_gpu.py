@@ -420,6 +420,22 @@ def test_cg_operator_is_laid_out_again_in_its_own_memory():
     assert torch.equal(again, ShardedOperator.from_kernel("spectral", x, params, start, end, 0.1).apply(y))
 
 
+def test_cg_operators_without_points_and_before_their_layout():
+    from kernel_matmul_b200 import _C, ranges
+    from kernel_matmul_b200.cg import ShardedOperator
+
+    x, params = torch.empty(0, device="cuda"), torch.tensor([[0.6, 0.0, 1.2], [0.6, 0.4, 0.7]], device="cuda")
+    none = torch.empty(0, dtype=torch.int32, device="cuda")
+    for p in (params, params[0]):
+        op = ShardedOperator.from_kernel("spectral", x, p, none, none, 0.1)
+        assert op.apply(torch.empty(0, 3, device="cuda")).shape == (0, 3)
+    x = torch.sort(torch.rand(5000, device="cuda") * 50)[0]
+    start, end = ranges.make_ranges(2.4, x)
+    plan = _C.NodeOperator(5000, x, params, start, end, 0, start.shape[0])
+    with pytest.raises(RuntimeError, match="not been laid out"):
+        plan.matvec(torch.ones(5000, 1, device="cuda"), torch.empty(5000, 1, device="cuda"))
+
+
 def test_cg_operator_laid_out_on_another_stream():
     """Products on a stream come after a layout that a product on another one has just made, and its memory
     outlives them."""
